@@ -13,6 +13,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB_PATH = os.path.join(_HERE, "libfkda.so")
 _lib = None
+_fwd_fast = None
 
 FLAG_SCAN_SIMT = 0x1
 FLAG_SCAN_PLAIN = 0x2
@@ -85,6 +86,19 @@ def lib():
             getattr(L, name).restype = ci
         _lib = L
     return _lib
+
+
+def _load_host():
+    """The native host path (csrc/fkda_host.cpp), loaded with the library on the first call."""
+    global _fwd_fast
+    lib()
+    try:
+        from . import _fkda_host
+    except ImportError as e:
+        raise RuntimeError(f"the native host path of flash_kda cannot be loaded ({e}): build it with "
+                           "`python -m flashkda_b200.build`") from e
+    _fwd_fast = _fkda_host.fwd_fast
+    return _fwd_fast
 
 
 def last_error() -> str:
@@ -223,6 +237,14 @@ def fwd(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state
     tensor of at least `get_workspace_size(B*T, H, N)` bytes; by default one is allocated per
     call from torch's caching allocator, as the reference does (flash_kda/__init__.py:38).
     """
+    if workspace is None and not flags:
+        # the ordinary call: checked, given scratch memory and launched natively; False = something is not in order
+        done = (_fwd_fast or _load_host())(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state,
+                                           final_state, cu_seqlens)
+        if done is True:
+            return None
+        if done is not False:
+            raise RuntimeError(done)
     p, ws = _params(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state, final_state,
                     cu_seqlens, workspace, flags)
     with torch.cuda.device(q.device):

@@ -8,12 +8,15 @@ travels with the source tree; it is never installed into site-packages.
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libfkda.so")
+HOST_SRC = os.path.join(CSRC, "fkda_host.cpp")
+HOST_EXT = os.path.join(HERE, "_fkda_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["fkda_api.cu", "fkda_prepare.cu", "fkda_prepare_tc.cu", "fkda_scan.cu", "fkda_scan2.cu", "fkda_scan_short.cu", "fkda_segscan.cu", "fkda_short16.cu", "fkda_refmode.cu", "fkda_aux.cu", "fkda_static_ws.cu"]
 HEADERS = [os.path.join(CSRC, "fkda_common.cuh"), os.path.join(os.path.dirname(HERE), "include", "fkda.h"),
            os.path.join(os.path.dirname(HERE), "include", "fkda_testing.h")]
@@ -37,6 +40,24 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _build_host(force):
+    """The host path of `fwd` (checks, scratch memory, launch), a CPython extension on top of libfkda.so and torch."""
+    if not force and not _stale(HOST_EXT, [HOST_SRC, LIB] + HEADERS[1:2]):
+        return ""
+    import torch
+    tdir = os.path.dirname(os.path.abspath(torch.__file__))
+    inc, libdir = os.path.join(tdir, "include"), os.path.join(tdir, "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"),
+           "-isystem", sysconfig.get_paths()["include"], HOST_SRC, "-o", HOST_EXT, LIB, "-Wl,-rpath,$ORIGIN", f"-L{libdir}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    return r.stderr
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ_DIR, exist_ok=True)
     nvcc = _nvcc()
@@ -56,9 +77,10 @@ def build(force=False, verbose=False):
     with ThreadPoolExecutor(max_workers=len(sources)) as ex:
         objs = list(ex.map(compile_one, sources))
     if force or _stale(LIB, objs):
-        r = subprocess.run([nvcc, "-shared", "-o", LIB] + objs + ["-lcudart"], capture_output=True, text=True)
+        r = subprocess.run([nvcc, "-shared", "-Xlinker", "-soname=libfkda.so", "-o", LIB] + objs + ["-lcudart"], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    logs["fkda_host.cpp"] = _build_host(force)
     if verbose:
         for src, log in logs.items():
             print(f"==== {src}\n{log}")

@@ -84,7 +84,18 @@ int segments_for(int64_t chains, int64_t chunks_per_seq, int64_t flags, int* seg
     return static_cast<int>(forced);
   }
   if (flags & FKDA_FLAG_SCAN_LOOKAHEAD) return 1;
-  return fkda::plan_segments(chains, chunks_per_seq, seg_chunks, fkda::device_sm_count());
+  // The planner tries up to 158 run counts with a dozen 64-bit divisions each (several microseconds), and a call asks
+  // twice; it is a pure function of these three numbers, so each thread keeps its last answer.
+  thread_local struct { int64_t chains = -1, chunks = -1; int sms = -1, n = 1, len = 0; } last;
+  const int sms = fkda::device_sm_count();
+  if (last.chains != chains || last.chunks != chunks_per_seq || last.sms != sms) {
+    last.n = fkda::plan_segments(chains, chunks_per_seq, &last.len, sms);
+    last.chains = chains;
+    last.chunks = chunks_per_seq;
+    last.sms = sms;
+  }
+  *seg_chunks = last.len;
+  return last.n;
 }
 
 // `varlen` < 0: size for whichever mode needs more (the upper bound T_total/32 + N covers both).
@@ -119,7 +130,14 @@ bool make_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_pe
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-int validate(const fkda_fwd_params* p, Layout* L) {
+// whether the call takes the fused short-sequence kernel, which needs the workspace for its status word only
+bool fused_short(const fkda_fwd_params* p) {
+  const bool any_t = (p->flags & 0xff57u) == FKDA_FLAG_FUSED_ANY_T;
+  return p->cu_seqlens == nullptr && p->T > 0 && (any_t || (p->T <= fkda::kFusedMaxT && (p->flags & 0xff57u) == 0));
+}
+
+// `whole_call`: the operator (fkda_fwd) rather than one of its stages
+int validate(const fkda_fwd_params* p, Layout* L, bool whole_call = false) {
   if (!p) return fail(FKDA_ERR_INVALID_ARGUMENT, "params is NULL");
   if (!p->q || !p->k || !p->v || !p->g || !p->beta || !p->out) return fail(FKDA_ERR_INVALID_ARGUMENT, "q, k, v, g, beta and out must be non-NULL");
   if (!p->A_log || !p->dt_bias) return fail(FKDA_ERR_INVALID_ARGUMENT, "A_log and dt_bias must be non-NULL");
@@ -145,16 +163,24 @@ int validate(const fkda_fwd_params* p, Layout* L) {
   if (L->chunks_per_head * p->H > 0x7fffffffLL) return fail(FKDA_ERR_INVALID_ARGUMENT, "too many (chunk, head) pairs for one call");
   if (!p->workspace) return fail(FKDA_ERR_INVALID_ARGUMENT, "workspace is NULL");
   if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return fail(FKDA_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
-  if (p->workspace_bytes < L->total_bytes)
-    return fail(FKDA_ERR_WORKSPACE_TOO_SMALL, "workspace has %lld bytes, %lld needed", (long long)p->workspace_bytes, (long long)L->total_bytes);
+  // (a caller who can read the status word sized the workspace by fkda_get_workspace_size, which is held to)
+  const int64_t needed = whole_call && (p->flags & FKDA_FLAG_STATUS_UNREAD) && fused_short(p) ? fkda::kWsHeaderBytes : L->total_bytes;
+  if (p->workspace_bytes < needed)
+    return fail(FKDA_ERR_WORKSPACE_TOO_SMALL, "workspace has %lld bytes, %lld needed", (long long)p->workspace_bytes, (long long)needed);
   return FKDA_OK;
+}
+
+// The status word starts at zero.  (Varlen calls: the chunk-prefix kernel, which runs first and alone, clears it.)
+cudaError_t clear_status(const fkda_fwd_params* p, cudaStream_t stream) {
+  if (p->flags & FKDA_FLAG_STATUS_UNREAD) return cudaSuccess;
+  return cudaMemsetAsync(p->workspace, 0, fkda::kWsHeaderBytes, stream);
 }
 
 int do_prepare(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, int wait_limit_us = 0, int first_load_only = 0) {
   uint8_t* ws = static_cast<uint8_t*>(p->workspace);
   int* status = reinterpret_cast<int*>(ws);
   int* prefix = reinterpret_cast<int*>(ws + L.prefix_off);
-  cudaError_t e = cudaMemsetAsync(ws, 0, fkda::kWsHeaderBytes, stream);
+  cudaError_t e = p->cu_seqlens ? cudaSuccess : clear_status(p, stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(status)");
   if (p->cu_seqlens) {
     e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), p->B * p->T, static_cast<int>(p->H), L.n_segs, prefix, status, stream);
@@ -295,6 +321,14 @@ int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen
   return FKDA_OK;
 }
 
+int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes) {
+  Layout L;
+  if (!p || !bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "NULL pointer");
+  if (!make_layout(p->B * p->T, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
+  *bytes = (p->flags & FKDA_FLAG_STATUS_UNREAD) && fused_short(p) ? fkda::kWsHeaderBytes : L.total_bytes;
+  return FKDA_OK;
+}
+
 int fkda_prepare(const fkda_fwd_params* p, void* cuda_stream) {
   Layout L;
   int rc = validate(p, &L);
@@ -311,7 +345,7 @@ int fkda_scan(const fkda_fwd_params* p, void* cuda_stream) {
 
 int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
   Layout L;
-  int rc = validate(p, &L);
+  int rc = validate(p, &L, true);
   if (rc != FKDA_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   if (p->flags & FKDA_FLAG_REFERENCE_ROUNDING) {
@@ -327,10 +361,9 @@ int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
     if (e != cudaSuccess) return cuda_fail(e, "reference-rounding kernel launch");
     return FKDA_OK;
   }
-  const bool fused_any_t = (p->flags & 0xff57u) == FKDA_FLAG_FUSED_ANY_T;
-  if (p->cu_seqlens == nullptr && p->T > 0 && (fused_any_t || (p->T <= fkda::kFusedMaxT && (p->flags & 0xff57u) == 0))) {
+  if (fused_short(p)) {
     // short fixed-length sequences (a continuation step): one fused kernel, no operand records
-    cudaError_t e = cudaMemsetAsync(p->workspace, 0, fkda::kWsHeaderBytes, stream);
+    cudaError_t e = clear_status(p, stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(status)");
     e = fkda::launch_short16(static_cast<const __nv_bfloat16*>(p->q), static_cast<const __nv_bfloat16*>(p->k),
                              static_cast<const __nv_bfloat16*>(p->v), static_cast<const __nv_bfloat16*>(p->g),

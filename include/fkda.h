@@ -55,6 +55,9 @@ typedef enum fkda_state_dtype { FKDA_STATE_NONE = 0, FKDA_STATE_BF16 = 1, FKDA_S
 #define FKDA_FLAG_PREPARE_TCGEN05 0x80u
 /* The same stage on the earlier kernel (vectorised global loads, mma.sync products).  Same operand records. */
 #define FKDA_FLAG_PREPARE_MMA_SYNC 0x20000u
+/* Nobody will read the status word of this call's workspace (scratch memory that the caller of the caller never sees): it
+ * is left uninitialised where no kernel needs it, which saves a memset node in front of a call of a few microseconds. */
+#define FKDA_FLAG_STATUS_UNREAD 0x40000u
 /* Cut every sequence of the batch into n (2..255) runs walked in parallel, whatever the planner would
  * choose; the workspace must then be sized with fkda_get_workspace_size_flags.  Together with FKDA_FLAG_SCAN_PLAIN or
  * FKDA_FLAG_SCAN_LOOKAHEAD both passes over the runs use that recurrence kernel (otherwise each pass picks the faster
@@ -99,6 +102,10 @@ int fkda_get_workspace_size_flags(int64_t T_total, int64_t H, int64_t N, int64_t
  * T_total/32 + N chunks), where fkda_get_workspace_size covers both forms.  No counterpart in the reference. */
 int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t flags,
                                int64_t* bytes);
+
+/* The same for one call: the bytes of workspace that fkda_fwd will need for exactly these sizes and flags (`workspace`,
+ * `workspace_bytes` and the data pointers other than cu_seqlens are not looked at). */
+int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes);
 
 /* The planner of the segment-parallel recurrence: into how many runs (1 = none) a batch with `chains`
  * = N*H chains of `chunks_per_sequence` 32-token chunks is cut, and the run length in chunks.  (For a varlen batch the call plans with the average sequence length and
