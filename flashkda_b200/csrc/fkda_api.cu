@@ -19,6 +19,9 @@ cudaError_t launch_prepare_pipe(const PrepParams& p, cudaStream_t stream);
 cudaError_t launch_scan(const ScanParams& p, cudaStream_t stream);
 cudaError_t launch_scan_simt(const ScanParams& p, cudaStream_t stream);
 cudaError_t launch_scan2(const ScanParams& p, cudaStream_t stream);
+cudaError_t launch_recur_split(const ScanParams& p, const __nv_bfloat16* v, int rows, cudaStream_t stream);
+cudaError_t launch_operands(const PrepParams& p, bool one_per_cta, cudaStream_t stream);
+cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream_t stream);
 cudaError_t launch_scan_short(const ScanParams& p, int sm_count, cudaStream_t stream);
 cudaError_t launch_short16(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* g,
                            const __nv_bfloat16* beta, const float* A_log, const float* dt_bias, const void* initial_state,
@@ -28,7 +31,7 @@ cudaError_t launch_refmode(const __nv_bfloat16* q, const __nv_bfloat16* k, const
                            const __nv_bfloat16* beta, const float* A_log, const float* dt_bias, const void* initial_state,
                            void* final_state, __nv_bfloat16* out, const int64_t* cu_seqlens, int64_t N, int64_t T, int64_t T_total,
                            int H, int state_fp32, float scale, float gate_scale, cudaStream_t stream);
-cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_chunks, float* seg_buf, int kernel_choice,
+cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_chunks, float* seg_buf, int kernel_choice, const __nv_bfloat16* v,
                                   cudaStream_t stream);
 #ifdef FKDA_TUNING
 void set_prepare_trace(long long* buf);
@@ -176,6 +179,30 @@ cudaError_t clear_status(const fkda_fwd_params* p, cudaStream_t stream) {
   return cudaMemsetAsync(p->workspace, 0, fkda::kWsHeaderBytes, stream);
 }
 
+fkda::PrepParams prep_params(const fkda_fwd_params* p, const Layout& L) {
+  uint8_t* ws = static_cast<uint8_t*>(p->workspace);
+  fkda::PrepParams q{};
+  q.q = static_cast<const __nv_bfloat16*>(p->q);
+  q.k = static_cast<const __nv_bfloat16*>(p->k);
+  q.v = static_cast<const __nv_bfloat16*>(p->v);
+  q.g = static_cast<const __nv_bfloat16*>(p->g);
+  q.beta = static_cast<const __nv_bfloat16*>(p->beta);
+  q.A_log = p->A_log;
+  q.dt_bias = p->dt_bias;
+  q.cu_seqlens = p->cu_seqlens;
+  q.chunk_prefix = reinterpret_cast<const int*>(ws + L.prefix_off);
+  q.records = ws + L.records_off;
+  q.status = reinterpret_cast<int*>(ws);
+  q.T = p->T;
+  q.T_total = p->B * p->T;
+  q.H = static_cast<int>(p->H);
+  q.N = static_cast<int>(p->N);
+  q.total_chunks = static_cast<int>(L.chunks_per_head);
+  q.scale = p->scale;
+  q.gate_scale = static_cast<float>(static_cast<double>(p->lower_bound) * 1.4426950408889634);
+  return q;
+}
+
 int do_prepare(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, int wait_limit_us = 0, int first_load_only = 0) {
   uint8_t* ws = static_cast<uint8_t*>(p->workspace);
   int* status = reinterpret_cast<int*>(ws);
@@ -186,25 +213,7 @@ int do_prepare(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, i
     e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), p->B * p->T, static_cast<int>(p->H), L.n_segs, prefix, status, stream);
     if (e != cudaSuccess) return cuda_fail(e, "chunk_prefix launch");
   }
-  fkda::PrepParams q{};
-  q.q = static_cast<const __nv_bfloat16*>(p->q);
-  q.k = static_cast<const __nv_bfloat16*>(p->k);
-  q.v = static_cast<const __nv_bfloat16*>(p->v);
-  q.g = static_cast<const __nv_bfloat16*>(p->g);
-  q.beta = static_cast<const __nv_bfloat16*>(p->beta);
-  q.A_log = p->A_log;
-  q.dt_bias = p->dt_bias;
-  q.cu_seqlens = p->cu_seqlens;
-  q.chunk_prefix = prefix;
-  q.records = ws + L.records_off;
-  q.status = status;
-  q.T = p->T;
-  q.T_total = p->B * p->T;
-  q.H = static_cast<int>(p->H);
-  q.N = static_cast<int>(p->N);
-  q.total_chunks = static_cast<int>(L.chunks_per_head);
-  q.scale = p->scale;
-  q.gate_scale = static_cast<float>(static_cast<double>(p->lower_bound) * 1.4426950408889634);
+  fkda::PrepParams q = prep_params(p, L);
   q.wait_limit_us = wait_limit_us;
   q.first_load_only = first_load_only;
 #ifdef FKDA_TUNING
@@ -250,7 +259,7 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   else if ((p->flags & (FKDA_FLAG_SCAN_PLAIN | FKDA_FLAG_SCAN_LOOKAHEAD)) && L.n_segs > 1) {
     // a forced run count together with a forced kernel: both passes on that kernel
     e = fkda::launch_scan_segmented(s, L.n_segs, L.seg_chunks, reinterpret_cast<float*>(ws + L.seg_off),
-                                    (p->flags & FKDA_FLAG_SCAN_PLAIN) ? 1 : 2, stream);
+                                    (p->flags & FKDA_FLAG_SCAN_PLAIN) ? 1 : 2, nullptr, stream);
   } else if (p->flags & FKDA_FLAG_SCAN_PLAIN) e = fkda::launch_scan(s, stream);
   else if (!(p->flags & FKDA_FLAG_SCAN_LOOKAHEAD) && p->cu_seqlens == nullptr && p->T > 0 &&
              (p->T <= 2 * fkda::kChunk || (p->T <= 5 * fkda::kChunk && p->N * p->H > sms))) {
@@ -275,9 +284,86 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
     }
   } else if (L.n_segs > 1) {
     // few long chains: cut them into runs that are walked in parallel
-    e = fkda::launch_scan_segmented(s, L.n_segs, L.seg_chunks, reinterpret_cast<float*>(ws + L.seg_off), 0, stream);
+    e = fkda::launch_scan_segmented(s, L.n_segs, L.seg_chunks, reinterpret_cast<float*>(ws + L.seg_off), 0, nullptr, stream);
   } else e = fkda::launch_scan2(s, stream);
   if (e != cudaSuccess) return cuda_fail(e, "scan launch");
+  return FKDA_OK;
+}
+
+// Runs per sequence for the walk over compact records (1: whole sequences), at most `most` of them, and their length.
+// Hundredths of a microsecond per chunk step, measured: a chain split over four or two CTAs (fkda_recur_split.cu) or in one
+// CTA (fkda_recur.cu), the latter with and without outputs; a pass costs about 8 us beside its steps, the chaining of
+// the maps 3 us per run and wave of its CTAs.
+int plan_runs(int64_t chains, int64_t chunks, int most, int sms, int* len) {
+  constexpr int64_t kQuad = 60, kHalf = 80, kOne = 132, kQuiet = 95;
+  const int64_t whole = (chains * 4 <= sms ? kQuad : chains * 2 <= sms ? kHalf : kOne * ((chains + sms - 1) / sms)) * chunks;
+  int64_t best = whole;
+  int best_n = 1;
+  for (int64_t n = 3; n <= most; ++n) {
+    const int64_t l = (chunks + n - 1) / n;
+    if (l < 8) break;
+    if ((n - 1) * l >= chunks) continue;       // the last run would be empty
+    const int64_t pass1 = (chains * (2 * n - 3) + sms - 1) / sms * kQuiet * l, run0 = kOne * l;
+    const int64_t pass2 = (chains * (n - 1) + sms - 1) / sms * kOne * l;
+    const int64_t cost = (pass1 > run0 ? pass1 : run0) + pass2 + 1600 + 300 * (n - 2) * ((chains * 8 + sms - 1) / sms);
+    if (cost < best) {
+      best = cost;
+      best_n = static_cast<int>(n);
+    }
+  }
+  if (best * 10 > whole * 9) best_n = 1;
+  *len = static_cast<int>((chunks + best_n - 1) / best_n);
+  return best_n;
+}
+
+// The forward pass over compact records (fkda_record.cuh): token-parallel stage, then the recurrence in the form that suits
+// the number of chains.
+int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
+  uint8_t* ws = static_cast<uint8_t*>(p->workspace);
+  int* status = reinterpret_cast<int*>(ws);
+  const int64_t chains = p->N * p->H, T_total = p->B * p->T;
+  const int sms = fkda::device_sm_count();
+  int runs = 1, run_len = 0;
+  if (L.n_segs > 1) {
+    thread_local struct { int64_t chains = -1, chunks = -1; int most = 0, sms = 0, n = 1, len = 0; } last;
+    // (packed batches: the longest sequence sets the time either way; its length is on the device, a third above the average is assumed)
+    const int64_t tokens = p->cu_seqlens ? (p->N > 1 ? T_total * 4 / (p->N * 3) : T_total) : p->T;
+    const int64_t chunks = (tokens + fkda::kChunk - 1) / fkda::kChunk;
+    if (last.chains != chains || last.chunks != chunks || last.most != L.n_segs || last.sms != sms) {
+      last.n = plan_runs(chains, chunks, L.n_segs, sms, &last.len);
+      last.chains = chains;
+      last.chunks = chunks;
+      last.most = L.n_segs;
+      last.sms = sms;
+    }
+    runs = last.n;
+    run_len = last.len;
+  }
+  cudaError_t e = cudaSuccess;
+  if (p->cu_seqlens)
+    e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), T_total, static_cast<int>(p->H), runs,
+                                  reinterpret_cast<int*>(ws + L.prefix_off), status, stream);
+  else e = clear_status(p, stream);
+  if (e != cudaSuccess) return cuda_fail(e, "scheduling launch");
+  e = fkda::launch_operands(prep_params(p, L), (p->flags & FKDA_FLAG_PREPARE_TCGEN05) != 0, stream);
+  if (e != cudaSuccess) return cuda_fail(e, "token-parallel launch");
+  fkda::ScanParams s = scan_params(p, L);
+  const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
+  if (runs > 1) {
+    e = fkda::launch_scan_segmented(s, runs, run_len, reinterpret_cast<float*>(ws + L.seg_off), 0, v, stream);
+  } else {
+    s.seg_chunks_dev = nullptr;
+    // Fewer chains than a quarter or half of the SMs: a chain's time is what counts, it is split over four or two CTAs.
+    // (FKDA_FLAG_SCAN_NO_SEGMENTS: one CTA walks the whole chain.)
+    const bool split = (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS) == 0;
+    if (split && chains * 4 <= sms) e = fkda::launch_recur_split(s, v, 32, stream);
+    else if (split && chains * 2 <= sms) e = fkda::launch_recur_split(s, v, 64, stream);
+    else {
+      s.next_walk = p->cu_seqlens ? status + 3 : nullptr;
+      e = fkda::launch_recur(s, v, stream);
+    }
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "recurrence launch");
   return FKDA_OK;
 }
 
@@ -375,6 +461,12 @@ int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
     if (e != cudaSuccess) return cuda_fail(e, "short-sequence kernel launch");
     return FKDA_OK;
   }
+  // No kernel of the two-stage form is asked for: compact records.  (Packed batches with FKDA_FLAG_SCAN_NO_SEGMENTS take the
+  // two-stage form: the whole walk on kernels that share nothing with the runs it is compared against.)
+  const bool cross_check = p->cu_seqlens != nullptr && (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS);
+  if (p->B * p->T > 0 && !cross_check && (p->flags & ~static_cast<uint32_t>(FKDA_FLAG_STATUS_UNREAD | FKDA_FLAG_SCAN_NO_SEGMENTS | FKDA_FLAG_NO_FUSED_SHORT |
+                                                            FKDA_FLAG_PREPARE_TCGEN05)) == 0)
+    return do_compact(p, L, stream);
   rc = do_prepare(p, L, stream);
   if (rc != FKDA_OK) return rc;
   return do_scan(p, L, stream);

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <type_traits>
 
 namespace fkda {
 
@@ -170,6 +171,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // generic-proxy writes to shared memory -> visible to the async proxy (bulk copies, tcgen05.mma)
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// Programmatic dependent launch: a kernel launched by launch_after (below) may start while the kernel before it in the stream
+// is still running; everything up to this wait (barrier set-up, tensor-memory allocation) then overlaps with that
+// kernel's end.  Nothing that an earlier kernel writes or reads may be touched before it.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- bulk async copies (the TMA engine, untiled form; 16-byte aligned addresses and sizes) ------
 __device__ __forceinline__ void bulk_g2s(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
@@ -431,6 +437,7 @@ struct ScanParams {
   const int* select;           // device word, or nullptr: the kernel runs only if *select == select_want
   int select_want;
   const int* seg_chunks_dev;   // varlen batches: run length decided on the device from the longest sequence (else nullptr)
+  int* next_walk;              // persistent recurrence kernel: device counter (zeroed) that hands out the walks, or nullptr (in turn)
   // Test aids of the look-ahead kernel's give-up path (both 0 in production): a wait limit in microseconds instead of
   // the default, and a number of records after which the copy producer stops issuing copies, so that the consumers'
   // next wait runs out with nothing in flight.
@@ -477,6 +484,22 @@ struct SmemOptIn {
     return e;
   }
 };
+
+// Launch that lets the kernel's set-up overlap with the end of the stream's previous kernel (grid_dependency_wait).
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
 
 // Fixed-length sequences of at most this many tokens take the fused short-sequence kernel (fkda_short16.cu).
 constexpr int64_t kFusedMaxT = 32;

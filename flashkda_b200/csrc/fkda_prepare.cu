@@ -35,7 +35,8 @@ __global__ void chunk_prefix_kernel(const int64_t* __restrict__ cu, int N, int64
     carry = 0;
     longest = 0;
     prefix[0] = 0;
-    *status = kStatusOk;
+    status[0] = kStatusOk;
+    status[3] = 0;                 // chains handed out by the fused kernel
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

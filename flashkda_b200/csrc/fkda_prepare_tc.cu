@@ -21,9 +21,8 @@
 // products use k+ = khat 2^(G - P) and k- = khat 2^(P - G): both stay inside 2^(+-115.4) for lower_bound >= -5
 // (16 tokens x 5 x log2 e), every needed product k+_i k-_j (j <= i) is <= 1 in magnitude, and one 32 x 32 product
 // covers both sub-blocks and their cross block.  w' is formed from k+ and multiplied by 2^P per channel on the way out.
-#include <cuda.h>
-
 #include "fkda_common.cuh"
+#include "fkda_tma.cuh"
 
 namespace fkda {
 namespace prep_tc {
@@ -32,38 +31,7 @@ namespace prep_tc {
 static long long* g_trace = nullptr;      // timeline buffer of a tuning build (see the trace macros of the kernels)
 #endif
 
-// ---- PTX wrappers used only here ------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
-// the same box into the L2 only (no shared-memory destination, nothing to wait for)
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0),
-               "r"(c1), "r"(c2)
-               : "memory");
-}
-__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-// 16 lanes x 32 columns in the accumulator-fragment shape: registers 4j, 4j+1 = (lane t/4, columns 8j + 2(t%4), +1),
-// 4j+2, 4j+3 = (lane t/4 + 8, same columns), j = 0..3
-__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-// stores the transposes of four 8x8 tiles of 16-bit elements held as mma fragments (thread t: row t/4, columns 2(t%4), +1);
-// lane 8m + r supplies the address of row r of tile m
-__device__ __forceinline__ void stsm_x4_trans(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-               : "memory");
-}
+// ---- PTX wrapper used only here ------------------------------------------------------------------------------------
 __device__ __forceinline__ void st_global_16(void* p, const uint4& v) {
   asm volatile("st.global.v4.b32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -352,40 +320,6 @@ __device__ __forceinline__ void up_row(const uint32_t (&u)[32], uint8_t* up, int
     *reinterpret_cast<uint4*>(row + cb * 128) =
         make_uint4(pack_bf16(__uint_as_float(u[8 * cb]), __uint_as_float(u[8 * cb + 1])), pack_bf16(__uint_as_float(u[8 * cb + 2]), __uint_as_float(u[8 * cb + 3])),
                    pack_bf16(__uint_as_float(u[8 * cb + 4]), __uint_as_float(u[8 * cb + 5])), pack_bf16(__uint_as_float(u[8 * cb + 6]), __uint_as_float(u[8 * cb + 7])));
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// The driver's tensor-map encoder, looked up once through the runtime (no link-time dependency on the driver library).
-EncodeTiledFn encode_tiled_fn() {
-  static std::atomic<EncodeTiledFn> cached{nullptr};
-  EncodeTiledFn fn = cached.load(std::memory_order_acquire);
-  if (fn != nullptr) return fn;
-  void* ptr = nullptr;
-  cudaDriverEntryPointQueryResult qres;
-  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess ||
-      ptr == nullptr) {
-    (void)cudaGetLastError();
-    return nullptr;
-  }
-  fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  cached.store(fn, std::memory_order_release);
-  return fn;
-}
-
-// [T_total][H][128] bf16 tensor as a 3-d map (channel, head, token) read in [32 tok][1 head][64 ch] boxes with the
-// 128-byte swizzle; tokens past T_total read as zero.
-bool make_map(CUtensorMap* map, const void* base, int64_t T_total, int H) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (fn == nullptr) return false;
-  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kD), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T_total)};
-  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(kD) * 2, static_cast<cuuint64_t>(kD) * 2 * static_cast<cuuint64_t>(H)};
-  const cuuint32_t box[3] = {64, 1, static_cast<cuuint32_t>(kChunk)};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace prep_tc
@@ -992,8 +926,8 @@ prepare_tc4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 cudaError_t launch_prepare_pipe(const PrepParams& p, cudaStream_t stream) {
   if (p.total_chunks == 0 || p.H == 0 || p.T_total == 0) return cudaSuccess;
   CUtensorMap tq, tk, tg, tv;
-  if (!prep_tc::make_map(&tq, p.q, p.T_total, p.H) || !prep_tc::make_map(&tk, p.k, p.T_total, p.H) ||
-      !prep_tc::make_map(&tg, p.g, p.T_total, p.H) || !prep_tc::make_map(&tv, p.v, p.T_total, p.H))
+  if (!make_map(&tq, p.q, p.T_total, p.H) || !make_map(&tk, p.k, p.T_total, p.H) ||
+      !make_map(&tg, p.g, p.T_total, p.H) || !make_map(&tv, p.v, p.T_total, p.H))
     return cudaErrorInvalidValue;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in.ensure(prep_pipe::prepare_pipe_kernel, prep_pipe::kSmemBytes);
@@ -1016,8 +950,8 @@ bool prepare_tc4_applicable(const PrepParams& p) {
 cudaError_t launch_prepare_tc4(const PrepParams& p, cudaStream_t stream) {
   if (p.total_chunks == 0 || p.H == 0 || p.T_total == 0) return cudaSuccess;
   CUtensorMap tq, tk, tg, tv;
-  if (!prep_tc::make_map(&tq, p.q, p.T_total, p.H) || !prep_tc::make_map(&tk, p.k, p.T_total, p.H) ||
-      !prep_tc::make_map(&tg, p.g, p.T_total, p.H) || !prep_tc::make_map(&tv, p.v, p.T_total, p.H))
+  if (!make_map(&tq, p.q, p.T_total, p.H) || !make_map(&tk, p.k, p.T_total, p.H) ||
+      !make_map(&tg, p.g, p.T_total, p.H) || !make_map(&tv, p.v, p.T_total, p.H))
     return cudaErrorInvalidValue;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in.ensure(prep_tc4::prepare_tc4_kernel, prep_tc4::kSmemBytes);

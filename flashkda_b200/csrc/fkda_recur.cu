@@ -1,0 +1,569 @@
+// Inter-chunk recurrence of the KDA prefill over compact records: the state of a (sequence, head) chain in registers, the
+// output products on tcgen05.
+//
+// Replaces the reference's K2 (csrc/smxx/fwd_kernel2.cuh:115-839).  The rows v of S^T never meet each other in the
+// recurrence, so four warps hold 32 rows each as fp32 mma.sync accumulator fragments, and everything on the serial chain
+// stays in the fragment layout:
+//     R^T = v^T - S^T k+^T     A = the state registers rounded to bf16, B = -k+ rows by ldmatrix; the accumulators start
+//                              from v^T, which a transposing ldmatrix brings from its TMA tile     [32 v x 32 tok]
+//     U^T = R^T (T diag(beta))^T
+//     S^T = S^T diag(e) + U^T kr      A = U^T, the packed accumulators of the line above; accumulators = the state
+// No trip through tensor memory or shared memory lies on that chain and no rendezvous between warps; a chunk waits for its
+// record only.  (With the state in tensor memory, fkda_scan2.cu, a chunk costs a commit, a read, a decay and a write of the
+// whole state per step.)
+//     O^T = S^T q+^T + U^T mqk^T
+// is off the chain: the bf16 copies of S^T and U^T are left in tensor memory, one thread issues the ten products, four
+// other warps write the result.
+//
+// What bounds it: a warp's 140 mma.sync of 8 cycles on its sub-partition (1120 cycles per chunk), the ten tcgen05.mma, each of
+// which keeps the tensor cores from them for about 50 cycles, and the latencies in between: 2470 cycles per chunk (1720
+// with the output products left out).  Two warps of 16 rows per sub-partition read every operand twice as often and end at
+// the shared-memory pipe (2650); the output products on mma.sync in the output warps: 2700.  4 x 8192 tokens x 32 heads, fp32
+// state: 0.340 ms over records of 0.96 GB (4.4 TB/s).
+//
+// Warps 0-3: recurrence; 4-7: output, and one of them each the output products and the copies.  The code of a
+// recurrence warp and of the output warp on the same SM sub-partition together stay near 8 KB: beyond that a sub-partition's
+// instruction cache misses and straight-line code runs at three cycles per instruction and warp at best.
+#include "fkda_common.cuh"
+#include "fkda_record.cuh"
+#include "fkda_tma.cuh"
+
+namespace fkda {
+namespace recur {
+
+constexpr int kThreads = 256;                      // two warps per SM sub-partition: 255 registers each
+constexpr int kStages = 5;
+constexpr int kStageBytes = 37 * 1024;             // v tile (two swizzled [32 tok][64 ch] halves) | record
+static_assert(8192 + kCrBytes <= kStageBytes, "stage");
+constexpr int kSmStg = kStages * kStageBytes;      // output staging: [32 tok][32 v] per output warp
+constexpr int kStgStride = 80;                     // bytes per token: conflict-free stmatrix
+constexpr int kInfos = 16;
+constexpr int kSmInfo = kSmStg + 4 * 32 * kStgStride;
+constexpr int kSmBars = kSmInfo + kInfos * 32;
+constexpr int kSmMisc = kSmBars + 256;
+constexpr int kSmem = kSmMisc + 16;
+static_assert(kSmem <= 227 * 1024, "shared memory plan");
+// tensor memory columns.  The copies of S and U follow the stages: a stage is refilled only once the output products of
+// its chunk, which read both, are complete, so a full stage means that its copies may be written over.
+constexpr uint32_t kTmemCols = 512;
+constexpr int kOBufs = 3;
+constexpr uint32_t kColSb = 0;                     // kStages x 64: bf16 copy of S^T [v][k], two k per column
+constexpr uint32_t kColUt = kColSb + 64 * kStages; // kStages x 16: bf16 U^T [v][tok]
+constexpr uint32_t kColO = kColUt + 16 * kStages;  // kOBufs x 32: O^T [v][tok]
+static_assert(kColO + 32 * kOBufs <= kTmemCols, "tensor memory plan");
+enum { B_FULL = 0, B_EMPTY = kStages, B_U = 2 * kStages, B_O = 3 * kStages, B_O_FREE = B_O + kOBufs, B_COUNT = B_O_FREE + kOBufs };
+static_assert(B_COUNT * 8 <= 256, "barrier area");
+
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t (&a)[4], const uint32_t (&b)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]),
+               "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3])
+               : "memory");
+}
+
+// What the copying thread says about a chunk (written before its stage's barrier is armed).
+struct Info {
+  long long out_off;   // element offset of the first token's row in `out`
+  int len;             // valid tokens
+  int flags;
+  int walk;            // index of the walk (chain, or run of a chain) for chain_view
+  int pad[3];
+};
+static_assert(sizeof(Info) == 32, "info");
+enum { kFirst = 1, kLast = 2, kEmpty = 4 /* no tokens: the state is handed through */, kQuiet = 8 /* no outputs wanted */, kEnd = 16 };
+
+// The chunks of one walk on the recurrence warps, from stage s (phase par) on; ready: that stage is known to be full.  S: rows v = row0 + 16 vt + g (+ 8), columns 8 jt + 2 t, + 1.
+template <bool kOut>
+__device__ __forceinline__ bool walk(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int nchunks, int64_t tokens, bool zero_v,
+                                     int row0, int lane, volatile int* abort_flag, int& s, uint32_t& par, bool& ready) {
+  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+  const int mi = lane >> 3, r = lane & 7, t = lane & 3;
+  const uint32_t kn_lane = 8192 + kCrKN + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
+  const uint32_t kr_lane = 8192 + kCrKR + mi * 2048 + r * 16;
+  const uint32_t v_lane = (row0 >> 6) * 4096 + lane * 128;
+  const uint32_t tb_lane = 8192 + kCrTB + r * 16;
+  for (int c = 0; c < nchunks; ++c) {
+    if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) return false;
+    const uint32_t stage = sbase + s * kStageBytes;
+
+    // R^T = v^T - S^T k+^T: the accumulators start from v^T; operands of a k-step are loaded during the one before
+    float R[2][4][4];
+    {
+      uint32_t x[4][4];              // v^T: channel blocks of 8 rows; register = token block
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ldsm_x4_trans(stage + v_lane + ((((row0 >> 3) + i) & 7) ^ r) * 16, x[i][0], x[i][1], x[i][2], x[i][3]);
+      const int64_t left = tokens - static_cast<int64_t>(c) * kChunk;
+      if (left < kChunk || zero_v) {   // rows past the sequence end belong to somebody else
+        const int len = zero_v ? 0 : static_cast<int>(left);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const uint32_t keep = (8 * nt + 2 * t < len ? 0xffffu : 0u) | (8 * nt + 2 * t + 1 < len ? 0xffff0000u : 0u);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i][nt] &= keep;
+        }
+      }
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          R[vt][nt][0] = bf_lo(x[2 * vt][nt]);
+          R[vt][nt][1] = bf_hi(x[2 * vt][nt]);
+          R[vt][nt][2] = bf_lo(x[2 * vt + 1][nt]);
+          R[vt][nt][3] = bf_hi(x[2 * vt + 1][nt]);
+        }
+    }
+    uint32_t bb[2][8];
+    ldsm_x4(stage + kn_lane, bb[0][0], bb[0][1], bb[0][2], bb[0][3]);
+    ldsm_x4(stage + kn_lane + 4096, bb[0][4], bb[0][5], bb[0][6], bb[0][7]);
+    if (kOut) tc_fence_after();
+    const uint32_t sb = tq + kColSb + 64 * s;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t a[2][16];               // bf16 copy of the state: A fragments of four k-steps, and 32 columns of tensor memory
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          a[vt][2 * j] = pack_bf16(S[vt][8 * half + j][0], S[vt][8 * half + j][1]);
+          a[vt][2 * j + 1] = pack_bf16(S[vt][8 * half + j][2], S[vt][8 * half + j][3]);
+        }
+        if (kOut) tmem_st_16x128b_x8(sb + (static_cast<uint32_t>(16 * vt) << 16) + 32 * half, a[vt]);
+      }
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4) {
+        const int ks = 4 * half + k4;
+        const uint32_t(&B)[8] = bb[ks & 1];
+        if (ks < 7) {
+          uint32_t(&N)[8] = bb[(ks + 1) & 1];
+          ldsm_x4(stage + kn_lane + (ks + 1) * 256, N[0], N[1], N[2], N[3]);
+          ldsm_x4(stage + kn_lane + 4096 + (ks + 1) * 256, N[4], N[5], N[6], N[7]);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int vt = 0; vt < 2; ++vt)
+            mma_bf16_16816(R[vt][nt], a[vt][4 * k4], a[vt][4 * k4 + 1], a[vt][4 * k4 + 2], a[vt][4 * k4 + 3], B[2 * nt], B[2 * nt + 1]);
+      }
+    }
+    // U^T = R^T (T diag(beta))^T
+    uint32_t l[4], m[4], n[4];       // T diag(beta): token tiles 0 and 1 (tokens 0-15 only: lower triangle), 2, 3
+    ldsm_x4(stage + tb_lane + (mi >> 1) * 512 + (mi & 1) * 128, l[0], l[1], l[2], l[3]);
+    ldsm_x4(stage + tb_lane + 1024 + mi * 128, m[0], m[1], m[2], m[3]);
+    ldsm_x4(stage + tb_lane + 1536 + mi * 128, n[0], n[1], n[2], n[3]);
+    uint32_t kr[2][4];
+    ldsm_x4_trans(stage + kr_lane, kr[0][0], kr[0][1], kr[0][2], kr[0][3]);
+    uint32_t u[2][2][4];             // A fragments, k-step = 16 tokens: first of R^T, then of U^T
+    auto as_operand = [&](uint32_t(&d)[2][4], const float(&x)[4][4]) {
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)  // e & 1: rows + 8, e >> 1: tokens + 8
+          d[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
+    };
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt) as_operand(u[vt], R[vt]);
+    {
+      float U[2][4][4];
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) U[vt][nt][0] = U[vt][nt][1] = U[vt][nt][2] = U[vt][nt][3] = 0.f;
+        mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
+        mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[2], l[3]);
+        mma_bf16_16816(U[vt][2], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
+        mma_bf16_16816(U[vt][3], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], n[0], n[1]);
+        mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
+        mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
+      }
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) {
+        as_operand(u[vt], U[vt]);
+        if (kOut) {
+          const uint32_t ut = tq + (static_cast<uint32_t>(16 * vt) << 16) + kColUt + 16 * s;
+          tmem_st_16x128b_x4(ut, u[vt][0], u[vt][1]);
+        }
+      }
+    }
+    // S^T = S^T diag(e) + U^T kr; the next stage's barrier is looked at meanwhile
+    const float2* e2 = reinterpret_cast<const float2*>(smem + s * kStageBytes + 8192 + kCrE) + t;
+    const int s1 = s + 1 == kStages ? 0 : s + 1;
+    const uint32_t par1 = s1 == 0 ? par ^ 1u : par;
+    ready = mbar_test(bar(B_FULL + s1), par1);
+#pragma unroll
+    for (int jt = 0; jt < 16; ++jt) {
+      const uint32_t(&B)[4] = kr[jt & 1];
+      if (jt < 15) {
+        uint32_t(&N)[4] = kr[(jt + 1) & 1];
+        ldsm_x4_trans(stage + kr_lane + (jt + 1) * 128, N[0], N[1], N[2], N[3]);
+      }
+      const float2 e = e2[4 * jt];
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) {
+        uint32_t y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[vt][jt][k]);
+        mul2(y[0], y[1], e);
+        mul2(y[2], y[3], e);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) S[vt][jt][k] = __uint_as_float(y[k]);
+      }
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+          mma_bf16_16816(S[vt][jt], u[vt][ks][0], u[vt][ks][1], u[vt][ks][2], u[vt][ks][3], B[2 * ks], B[2 * ks + 1]);
+    }
+    if (kOut) {
+      tmem_wait_st();
+      tc_fence_before();
+    }
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(bar(B_U + s));
+      mbar_arrive(bar(B_EMPTY + s));
+    }
+    s = s1;
+    par = par1;
+  }
+  return true;
+}
+
+__device__ __forceinline__ void load_state(float (&S)[2][16][4], const ChainView& cv, int row0, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int vt = 0; vt < 2; ++vt) {
+    const int v = row0 + 16 * vt + g;
+    if (cv.init_mode == 1) {
+      const float* src = static_cast<const float*>(cv.init_base) + v * kD + 2 * t;
+#pragma unroll
+      for (int jt = 0; jt < 16; ++jt) {
+        const float2 lo = __ldg(reinterpret_cast<const float2*>(src + 8 * jt)), hi = __ldg(reinterpret_cast<const float2*>(src + 8 * kD + 8 * jt));
+        S[vt][jt][0] = lo.x; S[vt][jt][1] = lo.y; S[vt][jt][2] = hi.x; S[vt][jt][3] = hi.y;
+      }
+    } else if (cv.init_mode == 2) {
+      const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(cv.init_base) + v * kD + 2 * t;
+#pragma unroll
+      for (int jt = 0; jt < 16; ++jt) {
+        const uint32_t lo = __ldg(reinterpret_cast<const uint32_t*>(src + 8 * jt)), hi = __ldg(reinterpret_cast<const uint32_t*>(src + 8 * kD + 8 * jt));
+        S[vt][jt][0] = bf_lo(lo); S[vt][jt][1] = bf_hi(lo); S[vt][jt][2] = bf_lo(hi); S[vt][jt][3] = bf_hi(hi);
+      }
+    } else {
+#pragma unroll
+      for (int jt = 0; jt < 16; ++jt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[vt][jt][i] = (cv.init_mode == 3 && 8 * jt + 2 * t + (i & 1) == v + 8 * (i >> 1)) ? 1.f : 0.f;
+    }
+  }
+}
+__device__ __forceinline__ void store_state(const float (&S)[2][16][4], const ChainView& cv, int row0, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int vt = 0; vt < 2; ++vt) {
+    const int v = row0 + 16 * vt + g;
+    if (cv.fin_fp32) {
+      float* dst = static_cast<float*>(cv.fin_base) + static_cast<size_t>(v) * cv.fin_stride + 2 * t;
+#pragma unroll
+      for (int jt = 0; jt < 16; ++jt) {
+        *reinterpret_cast<float2*>(dst + 8 * jt) = make_float2(S[vt][jt][0], S[vt][jt][1]);
+        *reinterpret_cast<float2*>(dst + 8 * cv.fin_stride + 8 * jt) = make_float2(S[vt][jt][2], S[vt][jt][3]);
+      }
+    } else {
+      __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(cv.fin_base) + v * kD + 2 * t;
+#pragma unroll
+      for (int jt = 0; jt < 16; ++jt) {
+        *reinterpret_cast<uint32_t*>(dst + 8 * jt) = pack_bf16(S[vt][jt][0], S[vt][jt][1]);
+        *reinterpret_cast<uint32_t*>(dst + 8 * kD + 8 * jt) = pack_bf16(S[vt][jt][2], S[vt][jt][3]);
+      }
+    }
+  }
+}
+
+// kStream: the CTA is persistent and goes through its walks (whole chains; with kSeg runs of a chain, see fkda_segscan.cu) as
+// one stream of chunks, so that records, v and state of the next walk are on their way while the last chunks of this one
+// are computed.  Equal lengths: walks in turn, every other round backwards; packed batches take the next longest
+// sequence from a device counter.  Otherwise one walk per CTA: a chunk costs 8 % less (2470 against 2680 cycles: the loop
+// has no registers to spare and every value kept for the stream is felt), a walk 3 us more.
+template <bool kSeg, bool kStream>
+__global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constant__ CUtensorMap tm_v, const ScanParams p, const int walks) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sbase = smem_u32(smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kSmMisc + 4);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kSmMisc);
+  Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
+  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+  if (tid == 0) {
+    *abort_flag = (sbase & 1023u) != 0u ? 1 : 0;       // the swizzled tiles need this alignment: report instead of computing garbage
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(bar(B_FULL + s), 1);
+      mbar_init(bar(B_EMPTY + s), 4 + 1);              // recurrence warps + commit of the output products
+      mbar_init(bar(B_U + s), 4);
+    }
+    for (int i = 0; i < kOBufs; ++i) {
+      mbar_init(bar(B_O + i), 1);
+      mbar_init(bar(B_O_FREE + i), 4);
+    }
+    fence_mbar_init();
+  }
+  if (warp == 4) {
+    tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  bool ok = *abort_flag == 0;
+  grid_dependency_wait();
+
+  if (warp < 4) {
+    // ===== recurrence ================================================================================================
+    const int row0 = 32 * warp;
+    const uint32_t tq = tmem + (static_cast<uint32_t>(row0) << 16);
+    float S[2][16][4];
+    int s = 0;
+    uint32_t par = 0;
+    bool ready = false;
+    for (int i = 0; ok;) {
+      int walk_index = static_cast<int>(blockIdx.x);
+      if (kStream) {
+        if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
+        const volatile Info* f = infos + (i & (kInfos - 1));
+        walk_index = f->walk;
+        ready = true;
+        if (f->flags & kEnd) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(B_U + s));
+          break;
+        }
+      }
+      const ChainView cv = chain_view<kSeg>(p, walk_index);
+      load_state(S, cv, row0, lane);
+      if (cv.nchunks == 0) {             // an empty sequence: its one item has nothing to compute
+        if (!ready && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar(B_U + s));
+          mbar_arrive(bar(B_EMPTY + s));
+        }
+        if (++s == kStages) { s = 0; par ^= 1u; }
+        ready = false;
+        ++i;
+      } else if (!kSeg || cv.write_out) {
+        ok = walk<true>(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, false, row0, lane, abort_flag, s, par, ready);
+      } else {
+        ok = walk<false>(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, cv.zero_up, row0, lane, abort_flag, s, par, ready);
+      }
+      if (ok && cv.fin_base != nullptr) store_state(S, cv, row0, lane);
+      if (!kStream) break;
+      i += cv.nchunks;
+    }
+  } else {
+    const int w = warp - 4, mi = lane >> 3, r = lane & 7;
+    const uint32_t tq = tmem + (static_cast<uint32_t>(32 * w) << 16) + kColO;
+    const uint32_t stg = sbase + kSmStg + w * 32 * kStgStride;
+    const uint8_t* src = smem + kSmStg + w * 32 * kStgStride + (lane >> 2) * kStgStride + (lane & 3) * 16;
+    __nv_bfloat16* const out0 = p.out + static_cast<size_t>(lane >> 2) * p.H * kD + 32 * w + (lane & 3) * 8;
+    const size_t step = static_cast<size_t>(8) * p.H * kD;      // eight tokens on
+
+    // ===== one lane of the second warp: the stream of chunks into the ring ==========================================
+    struct { long long bos, eos; const uint8_t* rec; int walk, h, c, n, flags, turn; bool ended; } cur{};
+    int copied = 0;
+    int cs = 0;                        // stage of the next item
+    auto copy = [&]() {
+      const int s = cs;
+      Info* f = infos + (copied & (kInfos - 1));
+      if (cur.c == cur.n) {            // the next walk
+        if (!kStream && cur.turn > 0) {
+          cur.ended = true;
+          return;
+        }
+        const int base = cur.turn * static_cast<int>(gridDim.x);
+        const int walk = !kStream ? static_cast<int>(blockIdx.x) : p.next_walk != nullptr ? atomicAdd(p.next_walk, 1)
+                                                : base + ((cur.turn & 1) ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x));
+        ++cur.turn;
+        if (walk >= walks || walk < 0) {
+          // (the last round may be shorter than the grid: a CTA without a walk in it is done, there is no round after it)
+          cur.ended = true;
+          f->flags = kEnd;
+          mbar_arrive(bar(B_FULL + s));
+          if (++cs == kStages) cs = 0;
+          ++copied;
+          return;
+        }
+        const ChainView cv = chain_view<kSeg>(p, walk);
+        cur.walk = walk;
+        cur.h = cv.h;
+        cur.bos = cv.bos;
+        cur.eos = cv.eos;
+        cur.c = 0;
+        cur.n = cv.nchunks > 0 ? cv.nchunks : 1;
+        cur.flags = (cv.nchunks > 0 ? 0 : kEmpty) | (cv.write_out ? 0 : kQuiet);
+        cur.rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
+        if (copied > 0 && (cv.init_mode == 1 || cv.init_mode == 2)) bulk_prefetch_l2(cv.init_base, kD * kD * (cv.init_mode == 1 ? 4 : 2));
+      }
+      const long long t0 = cur.bos + static_cast<long long>(cur.c) * kChunk;
+      f->out_off = (t0 * p.H + cur.h) * kD;
+      f->len = cur.eos - t0 < kChunk ? static_cast<int>(cur.eos - t0) : kChunk;
+      f->walk = cur.walk;
+      f->flags = (cur.flags & (kEmpty | kQuiet)) | (cur.c == 0 ? kFirst : 0) | (cur.c + 1 == cur.n ? kLast : 0);
+      if (cur.flags & kEmpty) {
+        mbar_arrive(bar(B_FULL + s));
+      } else {
+        const uint32_t dst = sbase + s * kStageBytes;
+        mbar_arrive_expect_tx(bar(B_FULL + s), kCrBytes + 8192);
+        bulk_g2s(dst + 8192, cur.rec + static_cast<size_t>(cur.c) * kCrBytes, kCrBytes, bar(B_FULL + s));
+        tma_load_3d(dst, &tm_v, 0, cur.h, static_cast<int>(t0), bar(B_FULL + s));
+        tma_load_3d(dst + 4096, &tm_v, 64, cur.h, static_cast<int>(t0), bar(B_FULL + s));
+      }
+      ++cur.c;
+      ++copied;
+      if (++cs == kStages) cs = 0;
+    };
+    // ===== one lane of the first warp: O^T = S^T q+^T + U^T mqk^T of item i ==========================================
+    int issued = 0;                    // items whose commits are under way
+    int ps = 0, po = 0;                // stage and output buffer of the next item, with their phases
+    uint32_t ps_par = 0, po_par = 1;
+    auto products = [&](int i) -> bool {
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 32, 0, 0);
+      const int s = ps, o = po;
+      if (!mbar_wait_parked(bar(B_U + s), ps_par, abort_flag)) return false;
+      if (i >= kOBufs && !mbar_wait_parked(bar(B_O_FREE + o), po_par, abort_flag)) return false;
+      if (++ps == kStages) { ps = 0; ps_par ^= 1u; }
+      if (++po == kOBufs) { po = 0; po_par ^= 1u; }
+      const int flags = static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags;
+      if (flags & (kEmpty | kQuiet | kEnd)) {
+        mbar_arrive(bar(B_O + o));
+        if (!(flags & kEnd)) mbar_arrive(bar(B_EMPTY + s));
+        return true;
+      }
+      tc_fence_after();
+      const uint32_t base = sbase + s * kStageBytes + 8192;
+      const uint32_t d = tmem + kColO + 32 * o;
+      const uint64_t bq = umma_desc(base + kCrQP, 128, 2048), bm = umma_desc(base + kCrMQK, 128, 512);
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) umma_ts(d, tmem + kColSb + 64 * s + 8 * ks, bq + ks * 16, idesc, ks > 0);
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) umma_ts(d, tmem + kColUt + 16 * s + 8 * ks, bm + ks * 16, idesc, 1);
+      umma_commit(bar(B_O + o));
+      umma_commit(bar(B_EMPTY + s));
+      issued = i + 1;
+      return true;
+    };
+
+    int n_one = 0;                     // (one walk per CTA) its items
+    if (!kStream) {
+      n_one = chain_view<kSeg>(p, static_cast<int>(blockIdx.x)).nchunks;
+      if (n_one == 0) n_one = 1;
+    }
+    if (w == 1 && lane == 0 && ok)
+      for (int k = 0; k < kStages && !cur.ended; ++k) copy();
+    if (w == 0 && lane == 0 && ok) ok = products(0);
+    bool end_ahead = false;            // (first warp) the end of the stream has been passed on
+    int i = 0, o = 0, es = 0;          // item; its output buffer and its stage with their phases
+    uint32_t o_par = 0, es_par = 0;
+    for (; kStream || i < n_one; ++i) {
+      if (w == 0) {
+        // the products of the next item before the output of this one
+        if (lane == 0 && ok && !end_ahead) {
+          end_ahead = kStream ? (static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags & kEnd) != 0 : i + 1 == n_one;
+          if (!end_ahead) ok = products(i + 1);
+        }
+        __syncwarp();
+      }
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait_parked(bar(B_O + o), o_par, abort_flag))) { ok = false; break; }
+      const volatile Info* f = infos + (i & (kInfos - 1));
+      const int flags = f->flags;
+      if (flags & kEnd) break;
+      if (!(flags & (kEmpty | kQuiet))) {
+        const long long off = f->out_off;
+        const int len = f->len;
+        tc_fence_after();
+        uint32_t y[2][16];
+        tmem_ld_16x256b_x4(tq + 32 * o, y[0]);
+        tmem_ld_16x256b_x4(tq + (16u << 16) + 32 * o, y[1]);
+        tmem_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(B_O_FREE + o));
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const uint32_t* x = y[vt] + 8 * k;
+            auto pk2 = [&](int e) { return pack_bf16(__uint_as_float(x[e]), __uint_as_float(x[e + 1])); };
+            stsm_x4_trans(stg + (8 * (2 * k + (mi >> 1)) + r) * kStgStride + vt * 32 + (mi & 1) * 16, pk2(0), pk2(2), pk2(4), pk2(6));
+          }
+        __syncwarp();
+        __nv_bfloat16* dst = out0 + off;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (8 * k + (lane >> 2) < len) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src + 8 * k * kStgStride);
+          dst += step;
+        }
+        __syncwarp();
+      } else {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(B_O_FREE + o));
+      }
+      if (w == 1 && lane == 0 && !cur.ended) {
+        if (!mbar_wait_parked(bar(B_EMPTY + es), es_par, abort_flag)) ok = false;
+        else copy();
+      }
+      if (++o == kOBufs) { o = 0; o_par ^= 1u; }
+      if (++es == kStages) { es = 0; es_par ^= 1u; }
+    }
+    if (w == 0 && lane == 0 && issued > 0) {
+      // the commits issued last must land before the CTA may exit (a stage that was refilled since has had its commit)
+      const int k = issued - 1;
+      const uint64_t t0 = globaltimer_ns();
+      if (!ok) {
+        while (!mbar_try_wait(bar(B_O + k % kOBufs), (k / kOBufs) & 1))
+          if (globaltimer_ns() - t0 > 20000000ull) break;
+      } else if (i - k < kStages) {
+        while (ok && !mbar_try_wait(bar(B_EMPTY + k % kStages), (k / kStages) & 1))
+          if (globaltimer_ns() - t0 > kWaitLimitNs) ok = false;
+      }
+    }
+    if (w == 1 && lane == 0 && (!ok || *abort_flag > 0)) {
+      // (giving up) copies in flight must land before the CTA's shared memory goes away
+      for (int c = copied > kStages ? copied - kStages : 0; c < copied; ++c) {
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(bar(B_FULL + c % kStages), (c / kStages) & 1))
+          if (globaltimer_ns() - t0 > 20000000ull) break;
+      }
+    }
+  }
+  if (!ok || *abort_flag > 0) atomicCAS(p.status, kStatusOk, kStatusWaitTimeout);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 4) {
+    tc_fence_after();
+    tmem_dealloc(tmem, kTmemCols);
+  }
+}
+
+}  // namespace recur
+
+// v: the value tensor [T_total][H][128]
+cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream_t stream) {
+  int64_t walks = static_cast<int64_t>(p.N) * p.H;
+  if (p.seg_chunks > 0) walks *= p.seg_pass == 1 ? 2 * p.n_segs - 3 : p.n_segs - 1;
+  if (walks <= 0) return cudaSuccess;
+  CUtensorMap tv;
+  if (!make_map(&tv, v, p.T_total, p.H)) return cudaErrorInvalidValue;
+  // More walks than SMs and short ones on average: one persistent CTA per SM.  (At 24 chunks the 3 us a walk costs more
+  // in a CTA of its own are what the tighter chunk loop saves.)
+  const int64_t sms = device_sm_count();
+  const bool stream_form = p.seg_chunks == 0 && walks > sms && (p.T_total + static_cast<int64_t>(p.N) * (kChunk / 2)) / kChunk <= 24 * static_cast<int64_t>(p.N);
+  auto kernel = p.seg_chunks > 0 ? recur::recur_kernel<true, false> : stream_form ? recur::recur_kernel<false, true> : recur::recur_kernel<false, false>;
+  static SmemOptIn opt_in[3];
+  cudaError_t e = opt_in[p.seg_chunks > 0 ? 1 : stream_form ? 2 : 0].ensure(kernel, recur::kSmem);
+  if (e != cudaSuccess) return e;
+  return launch_after(kernel, static_cast<unsigned>(stream_form ? sms : walks), recur::kThreads, recur::kSmem, stream, tv, p, static_cast<int>(walks));
+}
+
+}  // namespace fkda

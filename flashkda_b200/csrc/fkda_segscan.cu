@@ -13,6 +13,7 @@
 namespace fkda {
 
 cudaError_t launch_scan2(const ScanParams& p, cudaStream_t stream);
+cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream_t stream);
 cudaError_t launch_scan(const ScanParams& p, cudaStream_t stream);
 
 namespace {
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(256) seg_combine_kernel(float* seg_buf, int n_
 
 }  // namespace
 
-cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_chunks, float* seg_buf, int kernel_choice,
+// v: the value tensor where the records are the compact ones (both passes then run on the register-resident kernel), else nullptr
+cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_chunks, float* seg_buf, int kernel_choice, const __nv_bfloat16* v,
                                   cudaStream_t stream) {
   ScanParams p = base;
   p.seg_chunks = seg_chunks;
@@ -172,7 +174,7 @@ cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_ch
   pass_cost_x100(chains * (n_segs - 1), &compact2, sms);
   if (kernel_choice) compact1 = compact2 = kernel_choice == 1;   // forced: 1 compact, 2 look-ahead
   p.seg_pass = 1;
-  cudaError_t e = compact1 ? launch_scan(p, stream) : launch_scan2(p, stream);
+  cudaError_t e = v != nullptr ? launch_recur(p, v, stream) : compact1 ? launch_scan(p, stream) : launch_scan2(p, stream);
   if (e != cudaSuccess) return e;
   if (n_segs > 2) {
     static SmemOptIn opt_in;
@@ -184,7 +186,7 @@ cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_ch
     if (e != cudaSuccess) return e;
   }
   p.seg_pass = 2;
-  return compact2 ? launch_scan(p, stream) : launch_scan2(p, stream);
+  return v != nullptr ? launch_recur(p, v, stream) : compact2 ? launch_scan(p, stream) : launch_scan2(p, stream);
 }
 
 }  // namespace fkda

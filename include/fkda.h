@@ -113,13 +113,14 @@ int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes);
  * counterpart: its recurrence kernel always walks a whole sequence per CTA (csrc/smxx/fwd_kernel2.cuh:434-742). */
 int fkda_plan_segments(int64_t chains, int64_t chunks_per_sequence, int* segments, int* chunks_per_segment);
 
-/* The whole operator (replaces fwd(), csrc/flash_kda.cpp:28-217), enqueued on `stream`: prepare + scan, or, for
- * fixed-length sequences of at most 32 tokens, one fused kernel that uses the workspace for its status word only. */
+/* The whole operator (replaces fwd(), csrc/flash_kda.cpp:28-217), enqueued on `stream`: a token-parallel stage and a
+ * recurrence over compact operand records, or, for fixed-length sequences of at most 32 tokens, one fused kernel that
+ * uses the workspace for its status word only.  With kernel-selection flags: fkda_prepare followed by fkda_scan. */
 int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream);
 
-/* The two stages on their own, for tests and profiling.  fkda_prepare fills the workspace
- * (reference K1, csrc/smxx/fwd_kernel1.cuh:107); fkda_scan consumes it (reference K2,
- * csrc/smxx/fwd_kernel2.cuh:115).  fkda_fwd == fkda_prepare followed by fkda_scan. */
+/* The two-stage form over the larger record (w', u' instead of k+, T diag(beta)), stage by stage, for tests and profiling.
+ * fkda_prepare fills the workspace (reference K1, csrc/smxx/fwd_kernel1.cuh:107); fkda_scan consumes it (reference K2,
+ * csrc/smxx/fwd_kernel2.cuh:115). */
 int fkda_prepare(const fkda_fwd_params* p, void* cuda_stream);
 int fkda_scan(const fkda_fwd_params* p, void* cuda_stream);
 

@@ -1,0 +1,47 @@
+"""GPU: the forward pass over compact records at the sizes where its kernels can go wrong - around the 32-token chunk, its
+16-token halves and the rings of the copies; batches on either side of the lines between the forms of the recurrence (a chain
+split over four or two CTAs, one CTA per chain, the persistent form, runs); empty sequences; every state form."""
+import pytest
+import torch
+
+import flashkda_b200 as F
+import oracle
+from flashkda_b200.workloads import Workload, make_inputs
+from helpers import OUT_MAX_ABS, STATE_REL, max_abs, rel_fro, to_cuda
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "chunk_edges_split4": Workload("c", H=3, seq_lens=[1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 97], state_in="fp32", state_out="fp32"),
+    "ring_lengths_split4": Workload("c", H=2, B=3, T=32 * 9 + 5, state_in="bf16", state_out="bf16"),
+    "split2": Workload("c", H=25, B=2, T=33 + 64, state_out="fp32"),
+    "one_cta": Workload("c", H=40, B=3, T=32 * 6 + 1, state_in="fp32", state_out="fp32"),
+    "one_cta_no_state": Workload("c", H=100, B=1, T=48),
+    "persistent_two_rounds": Workload("c", H=50, B=6, T=70, state_in="bf16", state_out="bf16"),
+    "persistent_packed_with_empty": Workload("c", H=16, seq_lens=[0, 5, 33, 0, 64, 1, 31, 32, 100, 0, 2, 47], state_in="fp32", state_out="fp32"),
+    "runs": Workload("c", H=2, B=1, T=32 * 700 + 9, state_in="fp32", state_out="fp32", lower_bound=-1.0),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_compact_path_matches_the_recurrence(name):
+    w = CASES[name]
+    x = make_inputs(w)
+    xc = to_cuda(x)
+    out = torch.full_like(xc["v"], float("nan"))
+    fin = None if xc["final_state"] is None else torch.full_like(xc["final_state"], float("nan"))
+    B, T = x["q"].shape[:2]
+    ws = torch.empty(F.get_workspace_size(B * T, w.H, w.N), dtype=torch.uint8, device="cuda")
+    args = (xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"])
+    kw = dict(initial_state=xc["initial_state"], final_state=fin, cu_seqlens=xc["cu_seqlens"])
+    F.fwd(*args, workspace=ws, **kw)
+    assert F.read_status(ws) == 0
+    o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                     initial_state=x["initial_state"], cu_seqlens=x["cu_seqlens"])
+    assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS and rel_fro(out.cpu(), o64) <= 1e-2
+    if fin is not None:
+        assert rel_fro(fin.cpu(), s64) <= STATE_REL
+    # and again through the plain call: same bits
+    first, first_fin = out.clone(), None if fin is None else fin.clone()
+    F.fwd(*args, **kw)
+    assert torch.equal(out.view(torch.int16), first.view(torch.int16)) and (fin is None or torch.equal(fin, first_fin))
