@@ -17,7 +17,7 @@ OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libfkda.so")
 HOST_SRC = os.path.join(CSRC, "fkda_host.cpp")
 HOST_EXT = os.path.join(HERE, "_fkda_host" + sysconfig.get_config_var("EXT_SUFFIX"))
-SOURCES = ["fkda_api.cu", "fkda_prepare.cu", "fkda_prepare_tc.cu", "fkda_scan.cu", "fkda_scan2.cu", "fkda_recur_split.cu", "fkda_recur.cu", "fkda_operands.cu", "fkda_scan_short.cu", "fkda_segscan.cu", "fkda_short16.cu", "fkda_refmode.cu", "fkda_aux.cu", "fkda_static_ws.cu"]
+SOURCES = ["fkda_api.cu", "fkda_prepare.cu", "fkda_prepare_tc.cu", "fkda_scan.cu", "fkda_scan2.cu", "fkda_recur_split.cu", "fkda_recur.cu", "fkda_operands.cu", "fkda_scan_short.cu", "fkda_segscan.cu", "fkda_short16.cu", "fkda_step.cu", "fkda_refmode.cu", "fkda_aux.cu", "fkda_static_ws.cu"]
 HEADERS = [os.path.join(CSRC, "fkda_common.cuh"), os.path.join(CSRC, "fkda_tma.cuh"), os.path.join(CSRC, "fkda_elem.cuh"), os.path.join(CSRC, "fkda_record.cuh"), os.path.join(os.path.dirname(HERE), "include", "fkda.h"),
            os.path.join(os.path.dirname(HERE), "include", "fkda_testing.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

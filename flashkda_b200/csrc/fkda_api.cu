@@ -11,7 +11,7 @@
 #include "fkda_common.cuh"
 
 namespace fkda {
-cudaError_t launch_chunk_prefix(const int64_t* cu, int N, int64_t T_total, int H, int n_segs, int* prefix, int* status,
+cudaError_t launch_chunk_prefix(const int64_t* cu, int N, int64_t T_total, int H, int n_segs, bool skip_short, int* prefix, int* status,
                                 cudaStream_t stream);
 cudaError_t launch_prepare(const PrepParams& p, cudaStream_t stream);
 cudaError_t launch_prepare_tc4(const PrepParams& p, cudaStream_t stream);
@@ -27,6 +27,7 @@ cudaError_t launch_short16(const __nv_bfloat16* q, const __nv_bfloat16* k, const
                            const __nv_bfloat16* beta, const float* A_log, const float* dt_bias, const void* initial_state,
                            void* final_state, __nv_bfloat16* out, int64_t N, int T, int H, int state_fp32, float scale,
                            float gate_scale, int* status, cudaStream_t stream);
+cudaError_t launch_step(const PrepParams& p, const ScanParams& s, cudaStream_t stream);
 cudaError_t launch_refmode(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* g,
                            const __nv_bfloat16* beta, const float* A_log, const float* dt_bias, const void* initial_state,
                            void* final_state, __nv_bfloat16* out, const int64_t* cu_seqlens, int64_t N, int64_t T, int64_t T_total,
@@ -210,7 +211,7 @@ int do_prepare(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, i
   cudaError_t e = p->cu_seqlens ? cudaSuccess : clear_status(p, stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(status)");
   if (p->cu_seqlens) {
-    e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), p->B * p->T, static_cast<int>(p->H), L.n_segs, prefix, status, stream);
+    e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), p->B * p->T, static_cast<int>(p->H), L.n_segs, false, prefix, status, stream);
     if (e != cudaSuccess) return cuda_fail(e, "chunk_prefix launch");
   }
   fkda::PrepParams q = prep_params(p, L);
@@ -341,7 +342,7 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   }
   cudaError_t e = cudaSuccess;
   if (p->cu_seqlens)
-    e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), T_total, static_cast<int>(p->H), runs,
+    e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), T_total, static_cast<int>(p->H), runs, true,
                                   reinterpret_cast<int*>(ws + L.prefix_off), status, stream);
   else e = clear_status(p, stream);
   if (e != cudaSuccess) return cuda_fail(e, "scheduling launch");
@@ -349,6 +350,7 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   if (e != cudaSuccess) return cuda_fail(e, "token-parallel launch");
   fkda::ScanParams s = scan_params(p, L);
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
+  s.skip_short = p->cu_seqlens != nullptr;
   if (runs > 1) {
     e = fkda::launch_scan_segmented(s, runs, run_len, reinterpret_cast<float*>(ws + L.seg_off), 0, v, stream);
   } else {
@@ -364,6 +366,9 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
     }
   }
   if (e != cudaSuccess) return cuda_fail(e, "recurrence launch");
+  // The sequences of a few tokens, decode steps among the prompts: a padded chunk each would cost several times their own work.
+  if (p->cu_seqlens) e = fkda::launch_step(prep_params(p, L), s, stream);
+  if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
   return FKDA_OK;
 }
 
@@ -451,6 +456,11 @@ int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
     // short fixed-length sequences (a continuation step): one fused kernel, no operand records
     cudaError_t e = clear_status(p, stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(status)");
+    if (p->T <= fkda::kStepMaxT && !(p->flags & FKDA_FLAG_FUSED_ANY_T)) {
+      e = fkda::launch_step(prep_params(p, L), scan_params(p, L), stream);
+      if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
+      return FKDA_OK;
+    }
     e = fkda::launch_short16(static_cast<const __nv_bfloat16*>(p->q), static_cast<const __nv_bfloat16*>(p->k),
                              static_cast<const __nv_bfloat16*>(p->v), static_cast<const __nv_bfloat16*>(p->g),
                              static_cast<const __nv_bfloat16*>(p->beta), p->A_log, p->dt_bias, p->initial_state, p->final_state,

@@ -385,6 +385,14 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
   return y;
 }
 
+// Fixed-length sequences of at most this many tokens take the fused short-sequence kernel (fkda_short16.cu).
+constexpr int64_t kFusedMaxT = 32;
+// ... and of at most this many tokens the per-token kernel (fkda_step.cu), in packed batches too.  It costs about 0.4 us per
+// token, chain and SM beside the stream over the states; the tile kernel's cost does not depend on the tokens.  64 x 32
+// chains, bf16 states: 25 us at one token, 47 against 45 at five; fp32: 44, and 59 against 63.
+constexpr int64_t kStepMaxT = 4;
+constexpr int kOrderMax = 4096;      // packed batches of more sequences keep the given order instead of longest first
+
 // ---- kernel parameter blocks ---------------------------------------------------------------
 struct PrepParams {
   const __nv_bfloat16* q;
@@ -437,6 +445,7 @@ struct ScanParams {
   const int* select;           // device word, or nullptr: the kernel runs only if *select == select_want
   int select_want;
   const int* seg_chunks_dev;   // varlen batches: run length decided on the device from the longest sequence (else nullptr)
+  int skip_short;              // packed batches: sequences of at most kStepMaxT tokens are somebody else's (no chunks, no state)
   int* next_walk;              // persistent recurrence kernel: device counter (zeroed) that hands out the walks, or nullptr (in turn)
   // Test aids of the look-ahead kernel's give-up path (both 0 in production): a wait limit in microseconds instead of
   // the default, and a number of records after which the copy producer stops issuing copies, so that the consumers'
@@ -500,9 +509,6 @@ inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned t
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
-
-// Fixed-length sequences of at most this many tokens take the fused short-sequence kernel (fkda_short16.cu).
-constexpr int64_t kFusedMaxT = 32;
 
 // Duration of a pass of `ctas` CTAs in hundredths of one chunk step of the look-ahead kernel, per chunk of run length,
 // and the kernel that achieves it: the look-ahead kernel runs one CTA per SM, the compact kernel two at 1.58 times the
@@ -583,7 +589,8 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
     cv.eos = cv.bos + p.T;
     cv.chunk_base = cv.n * static_cast<int>((p.T + kChunk - 1) / kChunk);
   }
-  cv.nchunks = static_cast<int>((cv.eos - cv.bos + kChunk - 1) / kChunk);
+  const bool skipped = p.skip_short && cv.eos - cv.bos <= kStepMaxT;
+  cv.nchunks = skipped ? 0 : static_cast<int>((cv.eos - cv.bos + kChunk - 1) / kChunk);
   {  // never read past the records of this head, whatever cu_seqlens claims
     const int avail = p.total_chunks > cv.chunk_base ? p.total_chunks - cv.chunk_base : 0;
     if (cv.nchunks > avail) cv.nchunks = avail;
@@ -626,6 +633,10 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
       cv.init_base = slots + (seg * 3 + 2) * kSegSlotFloats;
       if (seg != p.n_segs - 1) cv.fin_base = nullptr;
     }
+  }
+  if (skipped) {
+    cv.init_mode = 0;
+    cv.fin_base = nullptr;
   }
   cv.write_out = !kSeg || variant == 0;
   cv.zero_up = kSeg && variant == 2;

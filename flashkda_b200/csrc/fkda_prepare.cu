@@ -25,9 +25,10 @@ namespace fkda {
 // so it is chosen unless the longest sequence alone would then set the duration.
 // For batches with few chains that are walked in runs (n_segs > 1) it sets the run length, status[2]: the longest
 // sequence's chunks spread over the runs, at least 8 chunks.
-constexpr int kOrderMax = 4096;      // batches of more sequences keep the given order
-__global__ void chunk_prefix_kernel(const int64_t* __restrict__ cu, int N, int64_t T_total, int H, int n_segs, int sms,
+// skip_short: sequences of at most kStepMaxT tokens count no chunks (another kernel has them).
+__global__ void chunk_prefix_kernel(const int64_t* __restrict__ cu, int N, int64_t T_total, int H, int n_segs, int sms, int skip_short,
                                     int* __restrict__ prefix, int* __restrict__ status) {
+  grid_dependency_wait();
   __shared__ int warp_sums[32];
   __shared__ int carry;
   __shared__ int longest;
@@ -50,7 +51,7 @@ __global__ void chunk_prefix_kernel(const int64_t* __restrict__ cu, int N, int64
         a = a < 0 ? 0 : (a > T_total ? T_total : a);
         b = b < a ? a : (b > T_total ? T_total : b);
       }
-      cnt = static_cast<int>((b - a + kChunk - 1) / kChunk);
+      cnt = skip_short && b - a <= kStepMaxT ? 0 : static_cast<int>((b - a + kChunk - 1) / kChunk);
       atomicMax(&longest, cnt);
     }
     int x = cnt;
@@ -666,10 +667,10 @@ store_record:
   }
 }
 
-cudaError_t launch_chunk_prefix(const int64_t* cu, int N, int64_t T_total, int H, int n_segs, int* prefix, int* status,
+cudaError_t launch_chunk_prefix(const int64_t* cu, int N, int64_t T_total, int H, int n_segs, bool skip_short, int* prefix, int* status,
                                 cudaStream_t stream) {
-  chunk_prefix_kernel<<<1, N > 256 ? 1024 : 256, 0, stream>>>(cu, N, T_total, H, n_segs, device_sm_count(), prefix, status);
-  return cudaGetLastError();
+  return launch_after(chunk_prefix_kernel, 1, N > 256 ? 1024 : 256, 0, stream, cu, N, T_total, H, n_segs, device_sm_count(), skip_short ? 1 : 0, prefix,
+                      status);
 }
 
 cudaError_t launch_prepare(const PrepParams& p, cudaStream_t stream) {

@@ -72,7 +72,7 @@ struct Info {
   int pad[3];
 };
 static_assert(sizeof(Info) == 32, "info");
-enum { kFirst = 1, kLast = 2, kEmpty = 4 /* no tokens: the state is handed through */, kQuiet = 8 /* no outputs wanted */, kEnd = 16 };
+enum { kQuiet = 1 /* no outputs wanted */, kEnd = 2 };
 
 // The chunks of one walk on the recurrence warps, from stage s (phase par) on; ready: that stage is known to be full.  S: rows v = row0 + 16 vt + g (+ 8), columns 8 jt + 2 t, + 1.
 template <bool kOut>
@@ -341,16 +341,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       }
       const ChainView cv = chain_view<kSeg>(p, walk_index);
       load_state(S, cv, row0, lane);
-      if (cv.nchunks == 0) {             // an empty sequence: its one item has nothing to compute
-        if (!ready && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(bar(B_U + s));
-          mbar_arrive(bar(B_EMPTY + s));
-        }
-        if (++s == kStages) { s = 0; par ^= 1u; }
-        ready = false;
-        ++i;
+      if (cv.nchunks == 0) {
+        // (an empty run: its state is handed through)
       } else if (!kSeg || cv.write_out) {
         ok = walk<true>(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, false, row0, lane, abort_flag, s, par, ready);
       } else {
@@ -380,44 +372,47 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           cur.ended = true;
           return;
         }
-        const int base = cur.turn * static_cast<int>(gridDim.x);
-        const int walk = !kStream ? static_cast<int>(blockIdx.x) : p.next_walk != nullptr ? atomicAdd(p.next_walk, 1)
-                                                : base + ((cur.turn & 1) ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x));
-        ++cur.turn;
-        if (walk >= walks || walk < 0) {
-          // (the last round may be shorter than the grid: a CTA without a walk in it is done, there is no round after it)
-          cur.ended = true;
-          f->flags = kEnd;
-          mbar_arrive(bar(B_FULL + s));
-          if (++cs == kStages) cs = 0;
-          ++copied;
-          return;
+        for (;;) {
+          const int base = cur.turn * static_cast<int>(gridDim.x);
+          const int walk = !kStream ? static_cast<int>(blockIdx.x) : p.next_walk != nullptr ? atomicAdd(p.next_walk, 1)
+                           : base + ((cur.turn & 1) ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x));
+          ++cur.turn;
+          const bool past = walk >= walks || walk < 0;
+          ChainView cv{};
+          if (!past) cv = chain_view<kSeg>(p, walk);
+          if (past || (kStream && cv.nchunks == 0 && p.N <= kOrderMax)) {
+            // (The last round may be shorter than the grid: a CTA without a walk in it is done, there is no round after it.
+            // Skipped sequences come last in the order by length.)
+            cur.ended = true;
+            f->flags = kEnd;
+            mbar_arrive(bar(B_FULL + s));
+            if (++cs == kStages) cs = 0;
+            ++copied;
+            return;
+          }
+          if (kStream && cv.nchunks == 0) continue;
+          cur.walk = walk;
+          cur.h = cv.h;
+          cur.bos = cv.bos;
+          cur.eos = cv.eos;
+          cur.c = 0;
+          cur.n = cv.nchunks;
+          cur.flags = cv.write_out ? 0 : kQuiet;
+          cur.rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
+          if (copied > 0 && (cv.init_mode == 1 || cv.init_mode == 2)) bulk_prefetch_l2(cv.init_base, kD * kD * (cv.init_mode == 1 ? 4 : 2));
+          break;
         }
-        const ChainView cv = chain_view<kSeg>(p, walk);
-        cur.walk = walk;
-        cur.h = cv.h;
-        cur.bos = cv.bos;
-        cur.eos = cv.eos;
-        cur.c = 0;
-        cur.n = cv.nchunks > 0 ? cv.nchunks : 1;
-        cur.flags = (cv.nchunks > 0 ? 0 : kEmpty) | (cv.write_out ? 0 : kQuiet);
-        cur.rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
-        if (copied > 0 && (cv.init_mode == 1 || cv.init_mode == 2)) bulk_prefetch_l2(cv.init_base, kD * kD * (cv.init_mode == 1 ? 4 : 2));
       }
       const long long t0 = cur.bos + static_cast<long long>(cur.c) * kChunk;
       f->out_off = (t0 * p.H + cur.h) * kD;
       f->len = cur.eos - t0 < kChunk ? static_cast<int>(cur.eos - t0) : kChunk;
       f->walk = cur.walk;
-      f->flags = (cur.flags & (kEmpty | kQuiet)) | (cur.c == 0 ? kFirst : 0) | (cur.c + 1 == cur.n ? kLast : 0);
-      if (cur.flags & kEmpty) {
-        mbar_arrive(bar(B_FULL + s));
-      } else {
-        const uint32_t dst = sbase + s * kStageBytes;
-        mbar_arrive_expect_tx(bar(B_FULL + s), kCrBytes + 8192);
-        bulk_g2s(dst + 8192, cur.rec + static_cast<size_t>(cur.c) * kCrBytes, kCrBytes, bar(B_FULL + s));
-        tma_load_3d(dst, &tm_v, 0, cur.h, static_cast<int>(t0), bar(B_FULL + s));
-        tma_load_3d(dst + 4096, &tm_v, 64, cur.h, static_cast<int>(t0), bar(B_FULL + s));
-      }
+      f->flags = cur.flags;
+      const uint32_t dst = sbase + s * kStageBytes;
+      mbar_arrive_expect_tx(bar(B_FULL + s), kCrBytes + 8192);
+      bulk_g2s(dst + 8192, cur.rec + static_cast<size_t>(cur.c) * kCrBytes, kCrBytes, bar(B_FULL + s));
+      tma_load_3d(dst, &tm_v, 0, cur.h, static_cast<int>(t0), bar(B_FULL + s));
+      tma_load_3d(dst + 4096, &tm_v, 64, cur.h, static_cast<int>(t0), bar(B_FULL + s));
       ++cur.c;
       ++copied;
       if (++cs == kStages) cs = 0;
@@ -434,7 +429,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       if (++ps == kStages) { ps = 0; ps_par ^= 1u; }
       if (++po == kOBufs) { po = 0; po_par ^= 1u; }
       const int flags = static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags;
-      if (flags & (kEmpty | kQuiet | kEnd)) {
+      if (flags & (kQuiet | kEnd)) {
         mbar_arrive(bar(B_O + o));
         if (!(flags & kEnd)) mbar_arrive(bar(B_EMPTY + s));
         return true;
@@ -454,13 +449,11 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     };
 
     int n_one = 0;                     // (one walk per CTA) its items
-    if (!kStream) {
-      n_one = chain_view<kSeg>(p, static_cast<int>(blockIdx.x)).nchunks;
-      if (n_one == 0) n_one = 1;
-    }
-    if (w == 1 && lane == 0 && ok)
+    if (!kStream) n_one = chain_view<kSeg>(p, static_cast<int>(blockIdx.x)).nchunks;
+    const bool work = kStream || n_one > 0;
+    if (w == 1 && lane == 0 && ok && work)
       for (int k = 0; k < kStages && !cur.ended; ++k) copy();
-    if (w == 0 && lane == 0 && ok) ok = products(0);
+    if (w == 0 && lane == 0 && ok && work) ok = products(0);
     bool end_ahead = false;            // (first warp) the end of the stream has been passed on
     int i = 0, o = 0, es = 0;          // item; its output buffer and its stage with their phases
     uint32_t o_par = 0, es_par = 0;
@@ -478,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       const volatile Info* f = infos + (i & (kInfos - 1));
       const int flags = f->flags;
       if (flags & kEnd) break;
-      if (!(flags & (kEmpty | kQuiet))) {
+      if (!(flags & kQuiet)) {
         const long long off = f->out_off;
         const int len = f->len;
         tc_fence_after();

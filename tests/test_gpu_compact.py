@@ -45,3 +45,37 @@ def test_compact_path_matches_the_recurrence(name):
     first, first_fin = out.clone(), None if fin is None else fin.clone()
     F.fwd(*args, **kw)
     assert torch.equal(out.view(torch.int16), first.view(torch.int16)) and (fin is None or torch.equal(fin, first_fin))
+
+
+@pytest.mark.parametrize("state", [None, "bf16", "fp32"])
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 4), (2, 5), (5, 15), (5, 16), (3, 17), (2, 31), (2, 32), (400, 3)])
+def test_short_sequences_match_the_recurrence(B, T, state):
+    """The per-token kernel (quarters of a chain, whole chains) and the 16-token tile kernel (one block, two blocks) on either
+    side of the lines between them."""
+    w = Workload("s", H=2, B=B, T=T, state_in=state, state_out=state or "fp32", state_std=0.5, seed=B * 100 + T, lower_bound=-2.0)
+    x = make_inputs(w)
+    xc = to_cuda(x)
+    out = torch.full_like(xc["v"], float("nan"))
+    fin = torch.full_like(xc["final_state"], float("nan"))
+    F.fwd(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"],
+          initial_state=xc["initial_state"], final_state=fin)
+    o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                     initial_state=x["initial_state"])
+    assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS and rel_fro(out.cpu(), o64) <= 1e-2
+    assert rel_fro(fin.cpu(), s64) <= STATE_REL
+
+
+def test_decode_tokens_among_prompts():
+    """A packed batch that mixes sequences of a few tokens, which the per-token kernel takes, with prompts."""
+    lens = [1] * 7 + [40, 4, 5, 0, 300, 1, 3, 33]
+    w = Workload("m", H=12, seq_lens=lens, state_in="bf16", state_out="bf16", state_std=0.5, seed=77)
+    x = make_inputs(w)
+    xc = to_cuda(x)
+    out, fin = torch.full_like(xc["v"], float("nan")), torch.full_like(xc["final_state"], float("nan"))
+    F.fwd(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"],
+          initial_state=xc["initial_state"], final_state=fin, cu_seqlens=xc["cu_seqlens"])
+    o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                     initial_state=x["initial_state"], cu_seqlens=x["cu_seqlens"])
+    assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS
+    assert rel_fro(fin.cpu(), s64) <= STATE_REL
+    assert torch.equal(fin[lens.index(0)].cpu(), x["initial_state"][lens.index(0)])
