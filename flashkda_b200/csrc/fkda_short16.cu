@@ -1,57 +1,66 @@
 // Fused forward pass for batches of short fixed-length sequences: one CTA per (sequence, head) chain walks the
 // sequence in blocks of 16 tokens,
 // reads q, k, v, g, beta and the chain's state, and writes out and the new state - no operand record goes through
-// global memory, and between blocks the state stays in shared memory in fp32.  This is the shape of a continuation / decode step after a prefill: per chain 16 KB of inputs
-// against 128 KB of fp32 state in and out, so the kernel is a stream over the states.
+// global memory, and between blocks the state stays in shared memory in fp32.  This is the shape of a continuation step
+// after a prefill: per chain 16 KB of inputs against 128 KB of fp32 state in and out, so the kernel is a stream over the states.
 //
 // Replaces, for these shapes, both of the reference's kernels (csrc/smxx/fwd_kernel1.cuh:107-586 and
 // fwd_kernel2.cuh:115-839), whose K2 spends most of its time loading and converting states here.  The algebra is
 // the single sub-block case of the chunked form used by the other kernels:
 //     k+ = khat 2^G, q+ = scale qhat 2^G, k- = khat 2^-G, kr = k- 2^Gtot, e = 2^Gtot        (G: running log2 decay)
-//     A = tril(k+ k-^T, -1) diag_rows(beta),  M = tril(q+ k-^T),  T = (I + A)^-1,  w' = T diag(beta) k+,  u' = T diag(beta) v
-//     U = u' - w' S,   O = q+ S + M U,   S' = diag(e) S + kr^T U                              (S: [k][v], stored [v][k])
-// Every warp owns 16 rows v of the state as fp32 mma.sync accumulator fragments: the same registers, rounded to
-// bf16, are the B fragments of w' S and q+ S, and after scaling by e they are the accumulator of the update.  The
-// state rows travel as whole-row bulk copies (fully coalesced) through a padded staging buffer in shared memory:
-// the copy in is issued before anything else and lands while the operands are being formed; the copy out is issued
-// per warp as soon as its 16 rows are done.
+//     A = tril(k+ k-^T, -1) diag_rows(beta),  M = tril(q+ k-^T),  TB = (I + A)^-1 diag(beta)
+//     R = v - k+ S,   U = TB R,   O = q+ S + M U,   S' = diag(e) S + kr^T U                   (S: [k][v], stored [v][k])
+// Eight warps own 16 rows v of the state and 16 channels of the element-wise stage each (mma fragment layout, fkda_elem.cuh);
+// the state is the A operand of R^T = v^T - S^T k+^T and S^T q+^T and, scaled by e, the accumulator of the update, read
+// from shared memory both times so that few registers are held.  Neither product needs T, so a ninth warp works out A, T
+// and M meanwhile: three rendezvous per block.  The state rows travel as whole-row bulk copies (fully coalesced)
+// through a padded staging buffer: the copy in is issued right behind the inputs, the copy out per warp as soon as
+// its rows are done.
+//
+// What bounds it: HBM, as far as the CTAs of an SM cover each other's phases - two of them with fp32 state, three with bf16.
+// 512 x 32 chains of 16 tokens: 435 us with fp32 states (5.7 TB/s), 302 us with bf16 (4.7 TB/s); 506 and 350 with the states asked
+// for ahead of the inputs, whose 16 KB then queue behind them; 460 and 402 with w' = TB k+, u' = TB v formed before the state
+// was touched (a rendezvous more, and two CTAs per SM for either type).  Asking the L2 for the next chain's state: slower.
 #include "fkda_common.cuh"
+#include "fkda_elem.cuh"
+#include "fkda_tma.cuh"
 
 namespace fkda {
 namespace short16 {
 
 constexpr int kRows = 16;
-constexpr int kThreads = 256;
+constexpr int kThreads = 288;
 constexpr int kLdS = 20;                         // row stride (floats) of the 16x16 fp32 matrices
 // shared memory (byte offsets)
 constexpr int kStQ = 0;                          // staged q, k, g, v: [16 tok][256 B], 16-byte chunks XOR-swizzled by the row
 constexpr int kStK = kStQ + 4096;
 constexpr int kStG = kStK + 4096;
 constexpr int kStV = kStG + 4096;
-constexpr int kKP = kStV + 4096;                 // bf16 [16][128] tiles in the 8x8 core-matrix layout
-constexpr int kQP = kKP + 4096;
-constexpr int kKM = kQP + 4096;
-constexpr int kKR = kKM + 4096;
-constexpr int kWP = kKR + 4096;
-constexpr int kTB = kWP + 4096;                  // bf16 [16][16] T diag(beta), core layout
+constexpr int kKN = kStV + 4096;                 // bf16 [16][128] tiles in the 8x8 core-matrix layout: -k+, k-, q+, kr
+constexpr int kKM = kKN + 4096;
+constexpr int kQP = kKM + 4096;
+constexpr int kKR = kQP + 4096;
+constexpr int kTB = kKR + 4096;                  // bf16 [16][16] T diag(beta), core layout
 constexpr int kMQK = kTB + 512;                  // bf16 [16][16]
 constexpr int kA = kMQK + 512;                   // fp32 [16][20]
 constexpr int kT = kA + kRows * kLdS * 4;        // fp32 [16][20]
 constexpr int kE = kT + kRows * kLdS * 4;        // fp32 [128] decay of the whole block
-constexpr int kTot = kE + 512;                   // fp32 [2][128] log2 decay of rows 0-7 and of rows 8-15
-constexpr int kSsq = kTot + 1024;                // fp32 [2][16][4] partial sums of squares (q, k)
-constexpr int kBeta = kSsq + 512;                // fp32 [16]
+constexpr int kSsq = kE + 512;                   // fp32 [q|k][16 rows][8 warps] partial sums of squares
+constexpr int kBeta = kSsq + 1024;               // fp32 [16]
 constexpr int kBar = kBeta + 64;                 // mbarrier of the state copy, abort flag
 constexpr int kState = (kBar + 16 + 127) / 128 * 128;   // [128 v] state rows, padded: fragment reads hit 32 distinct banks
-constexpr int kStride32 = 512 + 32;              // fp32 rows: stride = 8 words mod 32 (8-byte reads by half-warps)
-constexpr int kStride16 = 256 + 16;              // bf16 rows: stride = 4 words mod 32 (4-byte reads)
-constexpr int kSmemBytes = kState + kD * kStride32;
-static_assert(2 * (kSmemBytes + 1024) <= 227 * 1024, "two CTAs per SM");
+constexpr int kStgStride = 48;                   // output staging (over the dead -k+ and k-): [16 tok][16 v] per warp
+static_assert(8 * kRows * kStgStride <= 8192, "output staging");
 
-__device__ __forceinline__ uint4 as_u4(const __nv_bfloat162 (&x)[4]) {
-  return make_uint4(*reinterpret_cast<const uint32_t*>(&x[0]), *reinterpret_cast<const uint32_t*>(&x[1]),
-                    *reinterpret_cast<const uint32_t*>(&x[2]), *reinterpret_cast<const uint32_t*>(&x[3]));
-}
+// State rows in shared memory: fp32 unless a bf16 state needs one block only.
+template <bool kWide>
+struct Rows {
+  static constexpr int kStride = kWide ? 512 + 32 : 256 + 16;      // 8 words mod 32 (8-byte reads), 4 words mod 32 (4-byte reads)
+  static constexpr int kSmemBytes = kState + kD * kStride;
+  static constexpr int kCtas = kWide ? 2 : 3;
+  static_assert(kCtas * (kSmemBytes + 1024) <= 227 * 1024, "CTAs per SM");
+};
+constexpr int kBf16Row = 256 + 16;               // where a bf16 row arrives inside a wide slot (its second half)
 
 struct Params {
   const __nv_bfloat16* q;
@@ -66,15 +75,17 @@ struct Params {
   __nv_bfloat16* out;
   int T;                 // tokens per sequence
   int H;
-  int state_fp32;
   float scale;
   float gate_scale;      // lower_bound * log2(e)
   int* status;           // device status word (a bounded wait that gives up is recorded there)
 };
 
-// kOneBlock: T <= 16, compiled without the block loop's bookkeeping
-template <bool kOneBlock>
-__global__ void __launch_bounds__(kThreads, 2) short16_kernel(const Params p) {
+// kFp32: type of the state tensors; kOneBlock: T <= 16, compiled without the block loop's bookkeeping
+template <bool kFp32, bool kOneBlock>
+__global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) short16_kernel(const Params p) {
+  using namespace elem;
+  constexpr bool kWide = kFp32 || !kOneBlock;
+  constexpr int kStride = Rows<kWide>::kStride;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -82,200 +93,224 @@ __global__ void __launch_bounds__(kThreads, 2) short16_kernel(const Params p) {
   const int n = chain / p.H, h = chain - n * p.H;       // consecutive CTAs: consecutive heads of the same tokens
   const int64_t t_seq0 = static_cast<int64_t>(n) * p.T;
   const int nblk = kOneBlock ? 1 : (p.T + kRows - 1) / kRows;
-
-  float* s_A = reinterpret_cast<float*>(smem + kA);
-  float* s_T = reinterpret_cast<float*>(smem + kT);
   float* s_e = reinterpret_cast<float*>(smem + kE);
-  float* s_tot = reinterpret_cast<float*>(smem + kTot);
   float* s_ssq = reinterpret_cast<float*>(smem + kSsq);
   float* s_beta = reinterpret_cast<float*>(smem + kBeta);
 
-  // ---- the state: one bulk copy per row into the padded staging buffer, issued before anything else --------------
   const uint32_t bar = sbase + kBar;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kBar + 8);
-  const int row_bytes = p.state_fp32 ? 512 : 256;
-  const int in_off = p.state_fp32 ? 0 : kStride16;     // bf16 rows arrive in the second half of their fp32 slot
+  constexpr int row_bytes = kFp32 ? 512 : 256;
+  constexpr int in_off = !kFp32 && kWide ? kBf16Row : 0;
   if (tid == 0) {
     *abort_flag = 0;
     mbar_init(bar, kD);
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_wait();
+  // ---- inputs: coalesced asynchronous loads, 16 lanes per 256-byte token row; those of the next block are requested as
+  // soon as the staging of the current block has been consumed
+  auto load_rows = [&](int blk, int dst, const __nv_bfloat16* src) {
+    const int lrow = tid >> 4, chunk = tid & 15;
+    const bool valid = kRows * blk + lrow < p.T;
+    const size_t off = (static_cast<size_t>(t_seq0 + (valid ? kRows * blk + lrow : 0)) * p.H + h) * kD + 8 * chunk;
+    cp_async16(sbase + dst + stage_off(lrow, chunk), src + off, valid ? 16u : 0u);
+  };
+  if (warp < 8) {
+    load_rows(0, kStQ, p.q);
+    load_rows(0, kStK, p.k);
+    load_rows(0, kStG, p.g);
+    load_rows(0, kStV, p.v);
+  }
+  // ---- the state: one bulk copy per row into the padded staging buffer, behind the inputs, which are needed first ----
   if (p.initial_state != nullptr && tid < kD) {
     mbar_arrive_expect_tx(bar, row_bytes);
-    bulk_g2s(sbase + kState + tid * kStride32 + in_off,
+    bulk_g2s(sbase + kState + tid * kStride + in_off,
              static_cast<const uint8_t*>(p.initial_state) + (static_cast<size_t>(chain) * kD + tid) * row_bytes, row_bytes, bar);
   }
-  // ---- inputs: coalesced asynchronous loads, 16 lanes per 256-byte token row; q, k, g and v of the next block are
-  // requested as soon as the staging of the current block has been consumed
-  auto load_qkg = [&](int blk) {
-    const int lrow = tid >> 4, chunk = tid & 15;
-    const bool valid = kRows * blk + lrow < p.T;
-    const size_t off = (static_cast<size_t>(t_seq0 + (valid ? kRows * blk + lrow : 0)) * p.H + h) * kD + 8 * chunk;
-    const uint32_t nbytes = valid ? 16u : 0u;
-    const uint32_t dst = sbase + stage_off(lrow, chunk);
-    cp_async16(dst + kStQ, p.q + off, nbytes);
-    cp_async16(dst + kStK, p.k + off, nbytes);
-    cp_async16(dst + kStG, p.g + off, nbytes);
-  };
-  auto load_v = [&](int blk) {
-    const int lrow = tid >> 4, chunk = tid & 15;
-    const bool valid = kRows * blk + lrow < p.T;
-    const size_t off = (static_cast<size_t>(t_seq0 + (valid ? kRows * blk + lrow : 0)) * p.H + h) * kD + 8 * chunk;
-    cp_async16(sbase + kStV + stage_off(lrow, chunk), p.v + off, valid ? 16u : 0u);
-  };
-  load_qkg(0);
-  load_v(0);
-  // thread -> one (row, 8-column) item: rows 0-7 in warps 0-3, rows 8-15 in warps 4-7
-  const int r8 = tid & 7;
-  const int j = (tid >> 3) & 15;
-  const int half = tid >> 7;
-  const int row = r8 + 8 * half;
-  const float ha = 0.5f * ex2f(__ldg(p.A_log + h) * kLog2e);
-  const float hgs = 0.5f * p.gate_scale;
-  float hab[8];
-  {
-    const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.dt_bias + h * kD + 8 * j));
-    const float4 b1 = __ldg(reinterpret_cast<const float4*>(p.dt_bias + h * kD + 8 * j + 4));
-    hab[0] = ha * b0.x; hab[1] = ha * b0.y; hab[2] = ha * b0.z; hab[3] = ha * b0.w;
-    hab[4] = ha * b1.x; hab[5] = ha * b1.y; hab[6] = ha * b1.z; hab[7] = ha * b1.w;
+  const int g = lane >> 2, t4 = lane & 3, mi = lane >> 3, r = lane & 7;
+  const float ha = 0.5f * ex2f(__ldg(p.A_log + h) * kLog2e), hgs = 0.5f * p.gate_scale;
+  float hab[2] = {0.f, 0.f};               // channels 16 warp + 8 nt + g
+  if (warp < 8) {
+    hab[0] = ha * __ldg(p.dt_bias + h * kD + 16 * warp + g);
+    hab[1] = ha * __ldg(p.dt_bias + h * kD + 16 * warp + 8 + g);
   }
-  const int g = lane >> 2, t4 = lane & 3;
-  const int mi = lane >> 3, r = lane & 7;
-  const int v0 = 16 * warp + g;
-  uint8_t* const srow = smem + kState + v0 * kStride32;
+  // a 16 x 16 triangle of ones as A fragments, and the gate's constant part (fkda_elem.cuh)
+  uint32_t tri[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = g + 8 * (i & 1), k0 = 2 * t4 + 8 * (i >> 1);
+    tri[i] = (k0 <= row ? 0x3c00u : 0u) | (k0 + 1 <= row ? 0x3c000000u : 0u);
+  }
+  uint8_t* const srow = smem + kState + (16 * (warp & 7) + g) * kStride;
   bool failed = false;
 
   for (int blk = 0; blk < nblk; ++blk) {
-  const int64_t t0 = t_seq0 + kRows * blk;
-  const int len = p.T - kRows * blk < kRows ? p.T - kRows * blk : kRows;
-  if (tid < kRows) {
-    float b = 0.f;
-    if (tid < len) b = sigmoid_fast(__bfloat162float(p.beta[static_cast<size_t>(t0 + tid) * p.H + h]));
-    s_beta[tid] = b;
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  if (*abort_flag) { failed = true; break; }
+    const int64_t t0 = t_seq0 + kRows * blk;
+    const int len = p.T - kRows * blk < kRows ? p.T - kRows * blk : kRows;
+    float beta = 0.f;
+    if (warp == 8 && lane < len) beta = sigmoid_fast(__bfloat162float(p.beta[static_cast<size_t>(t0 + lane) * p.H + h]));
+    cp_async_wait_all();
+    __syncthreads();
+    if (*abort_flag) { failed = true; break; }
 
-  // ---- norms, gate, running decay ---------------------------------------------------------------------------------
-  const uint4 qw = *reinterpret_cast<const uint4*>(smem + kStQ + stage_off(row, j));
-  const uint4 kw = *reinterpret_cast<const uint4*>(smem + kStK + stage_off(row, j));
-  float G[8];
-  {
-    float f[8], sq = 0.f, sk = 0.f;
-    unpack8(qw, f);
+    float R[2][4], O[2][4];                // [token tile]: rows v = 16 warp + g (+ 8), tokens 8 nt + 2 t4, + 1
+    if (warp < 8) {
+      // ---- element-wise stage: 16 channels of 16 tokens --------------------------------------------------------------
+      const uint32_t src = sbase + stage_off(8 * (mi & 1) + r, 2 * warp + (mi >> 1));
+      uint32_t q[4], k[4], gw[4];          // registers 2 nt + half: tokens g + 8 half, channels 8 nt + 2 t4, + 1
+      ldsm_x4(src + kStQ, q[0], q[1], q[2], q[3]);
+      ldsm_x4(src + kStK, k[0], k[1], k[2], k[3]);
+      ldsm_x4_trans(src + kStG, gw[0], gw[1], gw[2], gw[3]);
+      auto squares = [&](const uint32_t(&x)[4], float* dst) {
+        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16_16816(c0, x[0], x[1], x[2], x[3], x[0], x[2]);
+        mma_bf16_16816(c1, x[0], x[1], x[2], x[3], x[1], x[3]);
+        if (t4 == (g >> 1)) {
+          dst[g * 8] = (g & 1) ? c0[1] : c0[0];
+          dst[(8 + g) * 8] = (g & 1) ? c1[3] : c1[2];
+        }
+      };
+      squares(q, s_ssq + warp);
+      squares(k, s_ssq + 128 + warp);
+      f2 G[2][2], tot[2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sq = fmaf(f[i], f[i], sq);
-    unpack8(kw, f);
+      for (int nt = 0; nt < 2; ++nt) {
+        uint32_t hi[2], lo[2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sk = fmaf(f[i], f[i], sk);
-    sq += __shfl_xor_sync(0xffffffffu, sq, 8);
-    sk += __shfl_xor_sync(0xffffffffu, sk, 8);
-    sq += __shfl_xor_sync(0xffffffffu, sq, 16);
-    sk += __shfl_xor_sync(0xffffffffu, sk, 16);
-    if (lane < 8) {
-      s_ssq[(0 * kRows + row) * 4 + (warp & 3)] = sq;
-      s_ssq[(1 * kRows + row) * 4 + (warp & 3)] = sk;
-    }
-    const uint4 gw = *reinterpret_cast<const uint4*>(smem + kStG + stage_off(row, j));
-    unpack8(gw, f);
-    const bool valid = row < len;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float x = valid ? fmaf(tanh_approx(fmaf(f[i], ha, hab[i])), hgs, hgs) : 0.f;
-#pragma unroll
-      for (int d = 1; d < 8; d <<= 1) {          // inclusive scan over the 8 rows held by the 8 lanes of this group
-        const float y = __shfl_up_sync(0xffffffffu, x, d, 8);
-        if (r8 >= d) x += y;
+        for (int b = 0; b < 2; ++b) {
+          float x0 = tanh_approx(fmaf(bf_lo(gw[2 * nt + b]), ha, hab[nt])), x1 = tanh_approx(fmaf(bf_hi(gw[2 * nt + b]), ha, hab[nt]));
+          if (len < kRows) {               // tokens that are not there do not decay
+            if (8 * b + 2 * t4 >= len) x0 = -1.f;
+            if (8 * b + 2 * t4 + 1 >= len) x1 = -1.f;
+          }
+          const __half2 hh = __floats2half2_rn(x0, x1);
+          const float2 back = __half22float2(hh);
+          const __half2 ll = __floats2half2_rn(x0 - back.x, x1 - back.y);
+          hi[b] = *reinterpret_cast<const uint32_t*>(&hh);
+          lo[b] = *reinterpret_cast<const uint32_t*>(&ll);
+        }
+        const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
+        float d[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_f16_16816(d, tri, hi[0], hi[1]);
+        mma_f16_16816(s, ones, hi[0], hi[1]);
+        mma_f16_16816(d, tri, lo[0], lo[1]);
+        mma_f16_16816(s, ones, lo[0], lo[1]);
+        const float c0 = hgs * static_cast<float>(g + 1), c1 = hgs * static_cast<float>(g + 9);
+        G[nt][0] = fma2(pk(d[0], d[1]), pk(hgs, hgs), pk(c0, c0));
+        G[nt][1] = fma2(pk(d[2], d[3]), pk(hgs, hgs), pk(c1, c1));
+        tot[nt] = fma2(pk(s[0], s[1]), pk(hgs, hgs), pk(16.f * hgs, 16.f * hgs));
       }
-      G[i] = x;
-    }
-    float th[8];
+      asm volatile("bar.sync 1, 256;" ::: "memory");      // the partial sums of squares are complete
+      float rq[2], rk[2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) th[i] = __shfl_sync(0xffffffffu, G[i], 7, 8);
-    if (r8 == 0) {
-      *reinterpret_cast<float4*>(s_tot + half * kD + 8 * j) = make_float4(th[0], th[1], th[2], th[3]);
-      *reinterpret_cast<float4*>(s_tot + half * kD + 8 * j + 4) = make_float4(th[4], th[5], th[6], th[7]);
-    }
-  }
-  __syncthreads();
-
-  // ---- decayed operands ---------------------------------------------------------------------------------------------
-  {
-    const float4 a0 = *reinterpret_cast<const float4*>(s_tot + 8 * j);
-    const float4 a1 = *reinterpret_cast<const float4*>(s_tot + 8 * j + 4);
-    const float4 c0 = *reinterpret_cast<const float4*>(s_tot + kD + 8 * j);
-    const float4 c1 = *reinterpret_cast<const float4*>(s_tot + kD + 8 * j + 4);
-    const float lo[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-    const float hi[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    float fa[8];
+      for (int b = 0; b < 2; ++b) {
+        const float4* s = reinterpret_cast<const float4*>(s_ssq + (g + 8 * b) * 8);
+        float4 x = s[0], y = s[1];
+        rq[b] = rsqrtf(((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w)) + 1e-6f) * p.scale;
+        x = s[32];
+        y = s[33];
+        rk[b] = rsqrtf(((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w)) + 1e-6f);
+      }
+      uint32_t kn[4], qp[4], km[4], kr[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (half) G[i] += lo[i];
-      fa[i] = ex2f(lo[i] + hi[i]);
-    }
-    if (tid < 128 && r8 == 0) {
-      *reinterpret_cast<float4*>(s_e + 8 * j) = make_float4(fa[0], fa[1], fa[2], fa[3]);
-      *reinterpret_cast<float4*>(s_e + 8 * j + 4) = make_float4(fa[4], fa[5], fa[6], fa[7]);
-    }
-    const float4 sq4 = *reinterpret_cast<const float4*>(s_ssq + (0 * kRows + row) * 4);
-    const float4 sk4 = *reinterpret_cast<const float4*>(s_ssq + (1 * kRows + row) * 4);
-    const float rq = rsqrtf(sq4.x + sq4.y + sq4.z + sq4.w + 1e-6f) * p.scale;
-    const float rk = rsqrtf(sk4.x + sk4.y + sk4.z + sk4.w + 1e-6f);
-    const uint32_t qraw[4] = {qw.x, qw.y, qw.z, qw.w};
-    const uint32_t kraw[4] = {kw.x, kw.y, kw.z, kw.w};
-    __nv_bfloat162 kp[4], qp[4], km[4], kr[4];
+      for (int nt = 0; nt < 2; ++nt) {
+        const f2 e = exp2_pair(tot[nt]);
+        if (g == 0) *reinterpret_cast<f2*>(s_e + 16 * warp + 8 * nt + 2 * t4) = e;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const float pw0 = ex2f(G[2 * m]), pw1 = ex2f(G[2 * m + 1]);
-      const float ip0 = ex2f(-G[2 * m]), ip1 = ex2f(-G[2 * m + 1]);
-      const __nv_bfloat162 k2 = *reinterpret_cast<const __nv_bfloat162*>(&kraw[m]);
-      const __nv_bfloat162 q2 = *reinterpret_cast<const __nv_bfloat162*>(&qraw[m]);
-      kp[m] = __hmul2(k2, __floats2bfloat162_rn(rk * pw0, rk * pw1));
-      qp[m] = __hmul2(q2, __floats2bfloat162_rn(rq * pw0, rq * pw1));
-      km[m] = __hmul2(k2, __floats2bfloat162_rn(rk * ip0, rk * ip1));
-      kr[m] = __hmul2(km[m], __floats2bfloat162_rn(fa[2 * m], fa[2 * m + 1]));
-    }
-    *reinterpret_cast<uint4*>(smem + kKP + core_off(row, 8 * j, kD)) = as_u4(kp);
-    *reinterpret_cast<uint4*>(smem + kQP + core_off(row, 8 * j, kD)) = as_u4(qp);
-    *reinterpret_cast<uint4*>(smem + kKM + core_off(row, 8 * j, kD)) = as_u4(km);
-    *reinterpret_cast<uint4*>(smem + kKR + core_off(row, 8 * j, kD)) = as_u4(kr);
-  }
-  __syncthreads();
-  if (!kOneBlock && blk + 1 < nblk) load_qkg(blk + 1);
-
-  // ---- A, M (one warp each), then T = (I + A)^-1 and T diag(beta) inside warp 0 --------------------------------
-  if (warp < 2) {
-    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    const uint32_t a_lane = sbase + (warp == 0 ? kKP : kQP) + (mi & 1) * 2048 + (mi >> 1) * 128 + r * 16;
-    const uint32_t b_lane = sbase + kKM + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
-      ldsm_x4(a_lane + ks * 256, a0, a1, a2, a3);
-      ldsm_x4(b_lane + ks * 256, b0, b1, b2, b3);
-      mma_bf16_16816(acc[0], a0, a1, a2, a3, b0, b1);
-      mma_bf16_16816(acc[1], a0, a1, a2, a3, b2, b3);
-    }
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int lr = g + 8 * hh, lc = nt * 8 + 2 * t4;
-        float x0 = acc[nt][2 * hh], x1 = acc[nt][2 * hh + 1];
-        if (warp == 0) {                 // strictly lower triangle, rows scaled by beta
-          const float br = s_beta[lr];
-          x0 = (lc < lr) ? x0 * br : 0.f;
-          x1 = (lc + 1 < lr) ? x1 * br : 0.f;
-          *reinterpret_cast<float2*>(s_A + lr * kLdS + lc) = make_float2(x0, x1);
-        } else {                         // lower triangle with the diagonal
-          x0 = (lc <= lr) ? x0 : 0.f;
-          x1 = (lc + 1 <= lr) ? x1 : 0.f;
-          *reinterpret_cast<uint32_t*>(smem + kMQK + core_off(lr, lc, kRows)) = pack_bf16(x0, x1);
+        for (int b = 0; b < 2; ++b) {
+          const f2 kh = mul(unpack_bf(k[2 * nt + b]), pk(rk[b], rk[b])), qh = mul(unpack_bf(q[2 * nt + b]), pk(rq[b], rq[b]));
+          const f2 pw = exp2_pair(G[nt][b]), m = mul(kh, exp2_neg_pair(G[nt][b]));
+          kn[2 * nt + b] = round_bf(mul(kh, mul(pw, pk(-1.f, -1.f))));
+          qp[2 * nt + b] = round_bf(mul(qh, pw));
+          km[2 * nt + b] = round_bf(m);
+          kr[2 * nt + b] = round_bf(mul(m, e));
         }
       }
-    if (warp == 0) {
+      const uint32_t dst = sbase + (mi & 1) * 2048 + (2 * warp + (mi >> 1)) * 128 + r * 16;
+      stsm_x4(dst + kKN, kn[0], kn[1], kn[2], kn[3]);
+      stsm_x4(dst + kQP, qp[0], qp[1], qp[2], qp[3]);
+      stsm_x4(dst + kKM, km[0], km[1], km[2], km[3]);
+      stsm_x4(dst + kKR, kr[0], kr[1], kr[2], kr[3]);
+    } else if (lane < kRows) {
+      s_beta[lane] = beta;
+    }
+    __syncthreads();
+    if (!kOneBlock && blk + 1 < nblk && warp < 8) {
+      load_rows(blk + 1, kStQ, p.q);
+      load_rows(blk + 1, kStK, p.k);
+      load_rows(blk + 1, kStG, p.g);
+    }
+
+    const bool zero_state = blk == 0 && p.initial_state == nullptr;
+    if (warp < 8) {
+      // ---- R^T = v^T - S^T k+^T, O^T = S^T q+^T ---------------------------------------------------------------------------
+      {
+        uint32_t x[4];
+        ldsm_x4_trans(sbase + kStV + stage_off(8 * (mi & 1) + r, 2 * warp + (mi >> 1)), x[0], x[1], x[2], x[3]);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          R[nt][0] = bf_lo(x[nt]);
+          R[nt][1] = bf_hi(x[nt]);
+          R[nt][2] = bf_lo(x[2 + nt]);
+          R[nt][3] = bf_hi(x[2 + nt]);
+          O[nt][0] = O[nt][1] = O[nt][2] = O[nt][3] = 0.f;
+        }
+      }
+      if (!zero_state) {
+        if (blk == 0) mbar_wait(bar, 0, abort_flag);     // gives up after 2 s and raises the abort flag, seen at the next block top / the exit
+        const uint32_t b_lane = sbase + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          uint32_t a[4], b0, b1, b2, b3;
+          if (kWide && (kFp32 || blk > 0)) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {    // e & 1: rows + 8, e >> 1: columns + 8
+              const float2 s = *reinterpret_cast<const float2*>(srow + (e & 1) * 8 * kStride + (16 * ks + 8 * (e >> 1) + 2 * t4) * 4);
+              a[e] = pack_bf16(s.x, s.y);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              a[e] = *reinterpret_cast<const uint32_t*>(srow + in_off + (e & 1) * 8 * kStride + (16 * ks + 8 * (e >> 1) + 2 * t4) * 2);
+          }
+          ldsm_x4(b_lane + kKN + ks * 256, b0, b1, b2, b3);
+          mma_bf16_16816(R[0], a[0], a[1], a[2], a[3], b0, b1);
+          mma_bf16_16816(R[1], a[0], a[1], a[2], a[3], b2, b3);
+          ldsm_x4(b_lane + kQP + ks * 256, b0, b1, b2, b3);
+          mma_bf16_16816(O[0], a[0], a[1], a[2], a[3], b0, b1);
+          mma_bf16_16816(O[1], a[0], a[1], a[2], a[3], b2, b3);
+        }
+      }
+    } else {
+      // ---- ninth warp: A, T = (I + A)^-1, T diag(beta); tril(M) -----------------------------------------------------------
+      float* s_A = reinterpret_cast<float*>(smem + kA);
+      float* s_T = reinterpret_cast<float*>(smem + kT);
+      const uint32_t a_lane = sbase + (mi & 1) * 2048 + (mi >> 1) * 128 + r * 16;
+      const uint32_t b_lane = sbase + kKM + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
+      float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, mq[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+        ldsm_x4(b_lane + ks * 256, b0, b1, b2, b3);
+        ldsm_x4(a_lane + kKN + ks * 256, a0, a1, a2, a3);
+        mma_bf16_16816(acc[0], a0, a1, a2, a3, b0, b1);
+        mma_bf16_16816(acc[1], a0, a1, a2, a3, b2, b3);
+        ldsm_x4(a_lane + kQP + ks * 256, a0, a1, a2, a3);
+        mma_bf16_16816(mq[0], a0, a1, a2, a3, b0, b1);
+        mma_bf16_16816(mq[1], a0, a1, a2, a3, b2, b3);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const int lr = g + 8 * hh, lc = nt * 8 + 2 * t4;
+          const float br = -s_beta[lr];      // (the operand is -k+)
+          *reinterpret_cast<float2*>(s_A + lr * kLdS + lc) =
+              make_float2(lc < lr ? acc[nt][2 * hh] * br : 0.f, lc + 1 < lr ? acc[nt][2 * hh + 1] * br : 0.f);
+          *reinterpret_cast<uint32_t*>(smem + kMQK + core_off(lr, lc, kRows)) =
+              pack_bf16(lc <= lr ? mq[nt][2 * hh] : 0.f, lc + 1 <= lr ? mq[nt][2 * hh + 1] : 0.f);
+        }
       __syncwarp();
       if (lane < kRows) {
         // forward substitution, one column per lane: x_i = [i == c] - sum_{j<i} A_ij x_j
@@ -309,141 +344,71 @@ __global__ void __launch_bounds__(kThreads, 2) short16_kernel(const Params p) {
           const float4 tb = *reinterpret_cast<const float4*>(s_T + rr * kLdS + 8 * q8 + 4);
           const float4 ba = *reinterpret_cast<const float4*>(s_beta + 8 * q8);
           const float4 bb = *reinterpret_cast<const float4*>(s_beta + 8 * q8 + 4);
-          const float tv[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
-          const float bv[8] = {ba.x, ba.y, ba.z, ba.w, bb.x, bb.y, bb.z, bb.w};
-          uint32_t w[4];
-#pragma unroll
-          for (int e2 = 0; e2 < 4; ++e2) {
-            const int c = 8 * q8 + 2 * e2;
-            w[e2] = pack_bf16(c <= rr ? tv[2 * e2] * bv[2 * e2] : 0.f, c + 1 <= rr ? tv[2 * e2 + 1] * bv[2 * e2 + 1] : 0.f);
-          }
-          *reinterpret_cast<uint4*>(dst + q8 * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<uint4*>(dst + q8 * 128) = make_uint4(pack_bf16(ta.x * ba.x, ta.y * ba.y), pack_bf16(ta.z * ba.z, ta.w * ba.w),
+                                                                 pack_bf16(tb.x * bb.x, tb.y * bb.y), pack_bf16(tb.z * bb.z, tb.w * bb.w));
         }
       }
     }
-  }
-  __syncthreads();
+    __syncthreads();
+    if (!kOneBlock && blk + 1 < nblk && warp < 8) load_rows(blk + 1, kStV, p.v);
 
-  // ---- w' = TB k+ (this warp's 16 k-columns, to shared memory) and u' = TB v (this warp's 16 v, kept) ------------
-  float up[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-  {
-    uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
-    ldsm_x4(sbase + kTB + (mi & 1) * 256 + (mi >> 1) * 128 + r * 16, a0, a1, a2, a3);
-    float wp[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    ldsm_x4_trans(sbase + kKP + (mi & 1) * 2048 + (2 * warp + (mi >> 1)) * 128 + r * 16, b0, b1, b2, b3);
-    mma_bf16_16816(wp[0], a0, a1, a2, a3, b0, b1);
-    mma_bf16_16816(wp[1], a0, a1, a2, a3, b2, b3);
+    if (warp < 8) {
+      // ---- U^T = R^T TB^T, O^T += U^T mqk^T --------------------------------------------------------------------------------
+      uint32_t u[4], b0, b1, b2, b3;         // A fragments: e & 1 rows + 8, e >> 1 tokens + 8
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      const int c = 16 * warp + 8 * nt + 2 * t4;
-      *reinterpret_cast<uint32_t*>(smem + kWP + core_off(g, c, kD)) = pack_bf16(wp[nt][0], wp[nt][1]);
-      *reinterpret_cast<uint32_t*>(smem + kWP + core_off(g + 8, c, kD)) = pack_bf16(wp[nt][2], wp[nt][3]);
-    }
-    ldsm_x4_trans(sbase + kStV + stage_off(8 * (mi & 1) + r, 2 * warp + (mi >> 1)), b0, b1, b2, b3);
-    mma_bf16_16816(up[0], a0, a1, a2, a3, b0, b1);
-    mma_bf16_16816(up[1], a0, a1, a2, a3, b2, b3);
-  }
-  __syncthreads();
-  if (!kOneBlock && blk + 1 < nblk) load_v(blk + 1);
+      for (int e = 0; e < 4; ++e) u[e] = pack_bf16(R[e >> 1][2 * (e & 1)], R[e >> 1][2 * (e & 1) + 1]);
+      ldsm_x4(sbase + kTB + (mi >> 1) * 256 + (mi & 1) * 128 + r * 16, b0, b1, b2, b3);
+      float U[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      mma_bf16_16816(U[0], u[0], u[1], u[2], u[3], b0, b1);
+      mma_bf16_16816(U[1], u[0], u[1], u[2], u[3], b2, b3);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) u[e] = pack_bf16(U[e >> 1][2 * (e & 1)], U[e >> 1][2 * (e & 1) + 1]);
+      ldsm_x4(sbase + kMQK + (mi >> 1) * 256 + (mi & 1) * 128 + r * 16, b0, b1, b2, b3);
+      mma_bf16_16816(O[0], u[0], u[1], u[2], u[3], b0, b1);
+      mma_bf16_16816(O[1], u[0], u[1], u[2], u[3], b2, b3);
 
-  // ---- this warp's 16 rows of the state -> accumulator fragments -----------------------------------------------------
-  // tile jt covers state columns k = 8jt .. 8jt+7: S[jt][0,1] = row v0, columns 8jt + 2t, +1; S[jt][2,3] = row v0 + 8
-  float S[16][4];
-  if (blk == 0 && p.initial_state == nullptr) {
+      // ---- S^T = S^T diag(e) + U^T kr in place: fp32 between blocks, the caller's type at the end ------------------------
+      const bool last = kOneBlock || blk + 1 == nblk;
+      if (!last || p.final_state != nullptr) {
 #pragma unroll
-    for (int jt = 0; jt < 16; ++jt) S[jt][0] = S[jt][1] = S[jt][2] = S[jt][3] = 0.f;
-  } else {
-    if (blk == 0) mbar_wait(bar, 0, abort_flag);     // gives up after 2 s and raises the abort flag, seen at the next block top / the exit
-    if (blk > 0 || p.state_fp32) {
+        for (int jp = 0; jp < 8; ++jp) {     // two column tiles per transposed load
+          ldsm_x4_trans(sbase + kKR + (mi & 1) * 2048 + (2 * jp + (mi >> 1)) * 128 + r * 16, b0, b1, b2, b3);
 #pragma unroll
-      for (int jt = 0; jt < 16; ++jt) {
-        const float2 lo = *reinterpret_cast<const float2*>(srow + (8 * jt + 2 * t4) * 4);
-        const float2 hi = *reinterpret_cast<const float2*>(srow + 8 * kStride32 + (8 * jt + 2 * t4) * 4);
-        S[jt][0] = lo.x; S[jt][1] = lo.y; S[jt][2] = hi.x; S[jt][3] = hi.y;
+          for (int c = 0; c < 2; ++c) {
+            const int col = 8 * (2 * jp + c) + 2 * t4;
+            float S[4] = {0.f, 0.f, 0.f, 0.f};
+            if (!zero_state) {
+              if (kWide && (kFp32 || blk > 0)) {
+                const float2 lo = *reinterpret_cast<const float2*>(srow + col * 4), hi = *reinterpret_cast<const float2*>(srow + 8 * kStride + col * 4);
+                S[0] = lo.x; S[1] = lo.y; S[2] = hi.x; S[3] = hi.y;
+              } else {
+                const uint32_t lo = *reinterpret_cast<const uint32_t*>(srow + in_off + col * 2);
+                const uint32_t hi = *reinterpret_cast<const uint32_t*>(srow + in_off + 8 * kStride + col * 2);
+                S[0] = bf_lo(lo); S[1] = bf_hi(lo); S[2] = bf_lo(hi); S[3] = bf_hi(hi);
+              }
+              const float2 e2 = *reinterpret_cast<const float2*>(s_e + col);
+              S[0] *= e2.x; S[1] *= e2.y; S[2] *= e2.x; S[3] *= e2.y;
+            }
+            mma_bf16_16816(S, u[0], u[1], u[2], u[3], c ? b2 : b0, c ? b3 : b1);
+            if (kFp32 || !last) {
+              *reinterpret_cast<float2*>(srow + col * 4) = make_float2(S[0], S[1]);
+              *reinterpret_cast<float2*>(srow + 8 * kStride + col * 4) = make_float2(S[2], S[3]);
+            } else {
+              *reinterpret_cast<uint32_t*>(srow + col * 2) = pack_bf16(S[0], S[1]);
+              *reinterpret_cast<uint32_t*>(srow + 8 * kStride + col * 2) = pack_bf16(S[2], S[3]);
+            }
+          }
+        }
       }
-    } else {
-#pragma unroll
-      for (int jt = 0; jt < 16; ++jt) {
-        const uint32_t lo = *reinterpret_cast<const uint32_t*>(srow + kStride16 + (8 * jt + 2 * t4) * 2);
-        const uint32_t hi = *reinterpret_cast<const uint32_t*>(srow + 8 * kStride32 + kStride16 + (8 * jt + 2 * t4) * 2);
-        S[jt][0] = bf_lo(lo); S[jt][1] = bf_hi(lo); S[jt][2] = bf_lo(hi); S[jt][3] = bf_hi(hi);
-      }
+      // ---- out: [v][tok] -> [tok][v] by stmatrix, one 16-byte piece per lane -------------------------------------------------
+      const uint32_t stg = kKN + warp * kRows * kStgStride;
+      stsm_x4_trans(sbase + stg + (8 * (mi >> 1) + r) * kStgStride + (mi & 1) * 16, pack_bf16(O[0][0], O[0][1]), pack_bf16(O[0][2], O[0][3]),
+                    pack_bf16(O[1][0], O[1][1]), pack_bf16(O[1][2], O[1][3]));
+      __syncwarp();
+      if ((lane >> 1) < len)
+        *reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(t0 + (lane >> 1)) * p.H + h) * kD + 16 * warp + 8 * (lane & 1)) =
+            *reinterpret_cast<const uint4*>(smem + stg + (lane >> 1) * kStgStride + (lane & 1) * 16);
     }
-  }
-
-  // ---- W = w' S and O = q+ S on this warp's 16 v (B fragments = the state registers rounded to bf16) -------------
-  float Wa[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-  float Oa[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-  {
-    const uint32_t w_lane = sbase + kWP + (mi & 1) * 2048 + (mi >> 1) * 128 + r * 16;
-    const uint32_t q_lane = sbase + kQP + (mi & 1) * 2048 + (mi >> 1) * 128 + r * 16;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      uint32_t w0, w1, w2, w3, q0, q1, q2, q3;
-      ldsm_x4(w_lane + ks * 256, w0, w1, w2, w3);
-      ldsm_x4(q_lane + ks * 256, q0, q1, q2, q3);
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {     // v tile m: rows v0 (m = 0) or v0 + 8 (m = 1) of the state
-        const uint32_t b0 = pack_bf16(S[2 * ks][2 * m], S[2 * ks][2 * m + 1]);
-        const uint32_t b1 = pack_bf16(S[2 * ks + 1][2 * m], S[2 * ks + 1][2 * m + 1]);
-        mma_bf16_16816(Wa[m], w0, w1, w2, w3, b0, b1);
-        mma_bf16_16816(Oa[m], q0, q1, q2, q3, b0, b1);
-      }
-    }
-  }
-  // U = u' - W as bf16, then its four 8x8 tiles transposed: Ut[m][hh] = tile (tokens 8hh.., v tile m)^T,
-  // i.e. this thread holds U[token 8hh + 2t, +1][v = 8m + g]
-  uint32_t Ut[2][2];
-#pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    Ut[m][0] = movmatrix_trans(pack_bf16(up[m][0] - Wa[m][0], up[m][1] - Wa[m][1]));
-    Ut[m][1] = movmatrix_trans(pack_bf16(up[m][2] - Wa[m][2], up[m][3] - Wa[m][3]));
-  }
-  {  // O += M U
-    uint32_t a0, a1, a2, a3;
-    ldsm_x4(sbase + kMQK + (mi & 1) * 256 + (mi >> 1) * 128 + r * 16, a0, a1, a2, a3);
-    mma_bf16_16816(Oa[0], a0, a1, a2, a3, Ut[0][0], Ut[0][1]);
-    mma_bf16_16816(Oa[1], a0, a1, a2, a3, Ut[1][0], Ut[1][1]);
-  }
-#pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    const int vcol = 16 * warp + 8 * m + 2 * t4;
-    if (g < len)
-      *reinterpret_cast<uint32_t*>(p.out + (static_cast<size_t>(t0 + g) * p.H + h) * kD + vcol) = pack_bf16(Oa[m][0], Oa[m][1]);
-    if (g + 8 < len)
-      *reinterpret_cast<uint32_t*>(p.out + (static_cast<size_t>(t0 + g + 8) * p.H + h) * kD + vcol) = pack_bf16(Oa[m][2], Oa[m][3]);
-  }
-
-  // ---- S' = diag(e) S + U^T kr: A = U^T (rows v, K = tokens), B = kr read transposed, accumulators = the state ----
-  const bool last = kOneBlock || blk + 1 == nblk;
-  if (!last || p.final_state != nullptr) {
-#pragma unroll
-    for (int jp = 0; jp < 8; ++jp) {   // two column tiles per transposed load
-      uint32_t b0, b1, b2, b3;
-      ldsm_x4_trans(sbase + kKR + (mi & 1) * 2048 + (2 * jp + (mi >> 1)) * 128 + r * 16, b0, b1, b2, b3);
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int jt = 2 * jp + q;
-        const float2 e2 = *reinterpret_cast<const float2*>(s_e + 8 * jt + 2 * t4);
-        S[jt][0] *= e2.x; S[jt][1] *= e2.y; S[jt][2] *= e2.x; S[jt][3] *= e2.y;
-        mma_bf16_16816(S[jt], Ut[0][0], Ut[1][0], Ut[0][1], Ut[1][1], q ? b2 : b0, q ? b3 : b1);
-      }
-    }
-    // back into this warp's staging rows (nobody else touches them): fp32 between blocks, the caller's type at the end
-    if (!last || p.state_fp32) {
-#pragma unroll
-      for (int jt = 0; jt < 16; ++jt) {
-        *reinterpret_cast<float2*>(srow + (8 * jt + 2 * t4) * 4) = make_float2(S[jt][0], S[jt][1]);
-        *reinterpret_cast<float2*>(srow + 8 * kStride32 + (8 * jt + 2 * t4) * 4) = make_float2(S[jt][2], S[jt][3]);
-      }
-    } else {
-#pragma unroll
-      for (int jt = 0; jt < 16; ++jt) {
-        *reinterpret_cast<uint32_t*>(srow + (8 * jt + 2 * t4) * 2) = pack_bf16(S[jt][0], S[jt][1]);
-        *reinterpret_cast<uint32_t*>(srow + 8 * kStride32 + (8 * jt + 2 * t4) * 2) = pack_bf16(S[jt][2], S[jt][3]);
-      }
-    }
-  }
   }  // blocks
 
   if (failed || *abort_flag > 0) {
@@ -453,13 +418,13 @@ __global__ void __launch_bounds__(kThreads, 2) short16_kernel(const Params p) {
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusWaitTimeout);
     return;
   }
-  if (p.final_state != nullptr) {      // one bulk copy per row, per warp as soon as its rows are done
+  if (p.final_state != nullptr && warp < 8) {      // one bulk copy per row, per warp as soon as its rows are done
     fence_proxy_async_smem();
     __syncwarp();
     if (lane < 16) {
       const int vr = 16 * warp + lane;
       bulk_s2g(static_cast<uint8_t*>(p.final_state) + (static_cast<size_t>(chain) * kD + vr) * row_bytes,
-               sbase + kState + vr * kStride32, row_bytes);
+               sbase + kState + vr * kStride, row_bytes);
       bulk_commit();
       bulk_wait_read0();               // shared memory must outlive the copy's reads
     }
@@ -473,13 +438,15 @@ cudaError_t launch_short16(const __nv_bfloat16* q, const __nv_bfloat16* k, const
                            void* final_state, __nv_bfloat16* out, int64_t N, int T, int H, int state_fp32, float scale,
                            float gate_scale, int* status, cudaStream_t stream) {
   if (N * H == 0) return cudaSuccess;
-  short16::Params p{q, k, v, g, beta, A_log, dt_bias, initial_state, final_state, out, T, H, state_fp32, scale, gate_scale, status};
-  auto kernel = T <= short16::kRows ? short16::short16_kernel<true> : short16::short16_kernel<false>;
-  static SmemOptIn opt_in[2];
-  cudaError_t e = opt_in[T <= short16::kRows ? 1 : 0].ensure(kernel, short16::kSmemBytes);
+  using namespace short16;
+  const Params p{q, k, v, g, beta, A_log, dt_bias, initial_state, final_state, out, T, H, scale, gate_scale, status};
+  const int form = (state_fp32 ? 2 : 0) + (T <= kRows ? 1 : 0);
+  void (*const kernels[4])(Params) = {short16_kernel<false, false>, short16_kernel<false, true>, short16_kernel<true, false>, short16_kernel<true, true>};
+  const int smem = form == 1 ? Rows<false>::kSmemBytes : Rows<true>::kSmemBytes;
+  static SmemOptIn opt_in[4];
+  cudaError_t e = opt_in[form].ensure(kernels[form], smem);
   if (e != cudaSuccess) return e;
-  kernel<<<static_cast<unsigned>(N * H), short16::kThreads, short16::kSmemBytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_after(kernels[form], static_cast<unsigned>(N * H), kThreads, smem, stream, p);
 }
 
 }  // namespace fkda
