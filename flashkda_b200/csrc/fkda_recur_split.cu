@@ -7,7 +7,11 @@
 //     O^T = S^T q+^T + U^T mqk^T,
 // is done by a second warp per sixteen rows, which gets the bf16 copies of S^T and U^T through shared memory as the very
 // fragments it needs.  With 32 rows the two kinds of warp sit on different SM sub-partitions and the chain's warp has a
-// tensor pipe to itself: 70 mma.sync of 8 cycles per chunk and the latencies between them.
+// tensor pipe to itself: 70 mma.sync of 8 cycles per chunk and the latencies between them, which bound it.  Hence no wait
+// on the chain but the one for the record, looked at ahead (a second one, for a free box, cost 0.08 us per chunk although
+// it never had to wait), and the decay of the state under the latency of U^T (32 rows; with 64 the output warp of the same
+// sub-partition fills that time, and it gives nothing).  Per chunk, 8 heads of 4096 tokens: 0.73 -> 0.60 us.  Two warps per
+// sixteen rows with half of the channels each and an exchange of partial sums: 0.78.
 // Warps 0 .. NW-1: recurrence; NW .. 2 NW-1: output; 2 NW: copies.
 #include "fkda_common.cuh"
 #include "fkda_record.cuh"
@@ -22,15 +26,16 @@ struct Plan {
   static constexpr int kSplits = kD / kRows;              // CTAs per chain
   static constexpr int kStages = 4;
   static constexpr int kStageBytes = 33 * 1024;           // v box [32 tok][64 ch], 128-byte swizzle | record
-  static constexpr int kBoxBytes = 5 * 1024;              // fragments of S^T (4 KB) and U^T (1 KB) of one warp
+  static constexpr int kBoxBytes = 5 * 1024;              // fragments of S^T (4 KB) and U^T (1 KB) of one warp, one per stage
   static constexpr int kStgStride = 48;                   // output staging, bytes per token: conflict-free stmatrix
-  static constexpr int kSmBox = kStages * kStageBytes;    // [NW][2]
-  static constexpr int kSmStg = kSmBox + NW * 2 * kBoxBytes;
+  static constexpr int kSmBox = kStages * kStageBytes;    // [kStages][NW]
+  static constexpr int kSmStg = kSmBox + kStages * NW * kBoxBytes;
   static constexpr int kSmBars = kSmStg + NW * 32 * kStgStride;
   static constexpr int kSmMisc = kSmBars + 256;
   static constexpr int kSmem = kSmMisc + 16;
+  static constexpr int kDecayAhead = NW == 2 ? 16 : 0;  // column tiles of the state that are decayed while U^T is computed
   static constexpr int kThreads = 32 * (2 * NW + 1);
-  static constexpr int B_FULL = 0, B_EMPTY = kStages, B_BOX = 2 * kStages, B_BOX_FREE = B_BOX + 2 * NW, B_COUNT = B_BOX_FREE + 2 * NW;
+  static constexpr int B_FULL = 0, B_EMPTY = kStages, B_BOX = 2 * kStages, B_COUNT = B_BOX + kStages * NW;
   static_assert(kSmem <= 227 * 1024 && B_COUNT * 8 <= 256 && 4096 + kCrBytes <= kStageBytes, "shared memory plan");
 };
 
@@ -50,12 +55,9 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
     *abort_flag = (sbase & 1023u) != 0u ? 1 : 0;          // the swizzled tiles need this alignment: report instead of computing garbage
     for (int s = 0; s < P::kStages; ++s) {
       mbar_init(bar(P::B_FULL + s), 1);
-      mbar_init(bar(P::B_EMPTY + s), 2 * NW);
+      mbar_init(bar(P::B_EMPTY + s), 2 * NW);             // (a full stage's boxes are free too: their readers arrive here)
     }
-    for (int i = 0; i < 2 * NW; ++i) {
-      mbar_init(bar(P::B_BOX + i), 1);
-      mbar_init(bar(P::B_BOX_FREE + i), 1);
-    }
+    for (int i = 0; i < P::kStages * NW; ++i) mbar_init(bar(P::B_BOX + i), 1);
     fence_mbar_init();
   }
   __syncthreads();
@@ -97,8 +99,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
     bool ready = false;
     for (int c = 0; c < nchunks; ++c) {
       if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(P::B_FULL + s), par, abort_flag)) { ok = false; break; }
-      const int box_i = 2 * warp + (c & 1);
-      if (c >= 2 && !warp_wait(bar(P::B_BOX_FREE + box_i), ((c >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+      const int box_i = s * NW + warp;
       const uint32_t stage = sbase + s * P::kStageBytes;
       uint4* box = reinterpret_cast<uint4*>(smem + P::kSmBox + box_i * P::kBoxBytes) + lane;
 
@@ -151,6 +152,17 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
             u[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
       };
       as_operand(R);
+      const float2* e2 = reinterpret_cast<const float2*>(smem + s * P::kStageBytes + 4096 + kCrE) + t;
+      auto decay = [&](int jt) {
+        const float2 e = e2[4 * jt];
+        uint32_t y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[jt][k]);
+        mul2(y[0], y[1], e);
+        mul2(y[2], y[3], e);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) S[jt][k] = __uint_as_float(y[k]);
+      };
       {
         float U[4][4];
 #pragma unroll
@@ -161,6 +173,8 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
         mma_bf16_16816(U[1], u[0][0], u[0][1], u[0][2], u[0][3], l[2], l[3]);
         mma_bf16_16816(U[2], u[1][0], u[1][1], u[1][2], u[1][3], m[2], m[3]);
         mma_bf16_16816(U[3], u[1][0], u[1][1], u[1][2], u[1][3], n[2], n[3]);
+#pragma unroll
+        for (int jt = 0; jt < P::kDecayAhead; ++jt) decay(jt);   // while they are under way
         as_operand(U);
       }
       box[256] = make_uint4(u[0][0], u[0][1], u[0][2], u[0][3]);
@@ -168,7 +182,6 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(P::B_BOX + box_i));
       // S^T = S^T diag(e) + U^T kr; the next stage's barrier is looked at meanwhile
-      const float2* e2 = reinterpret_cast<const float2*>(smem + s * P::kStageBytes + 4096 + kCrE) + t;
       const int s1 = s + 1 == P::kStages ? 0 : s + 1;
       const uint32_t par1 = s1 == 0 ? par ^ 1u : par;
       ready = mbar_test(bar(P::B_FULL + s1), par1);
@@ -176,14 +189,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
       for (int jt = 0; jt < 16; ++jt) {
         uint32_t B[4];
         ldsm_x4_trans(stage + kr_lane + jt * 128, B[0], B[1], B[2], B[3]);
-        const float2 e = e2[4 * jt];
-        uint32_t y[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[jt][k]);
-        mul2(y[0], y[1], e);
-        mul2(y[2], y[3], e);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) S[jt][k] = __uint_as_float(y[k]);
+        if (jt >= P::kDecayAhead) decay(jt);
         mma_bf16_16816(S[jt], u[0][0], u[0][1], u[0][2], u[0][3], B[0], B[1]);
         mma_bf16_16816(S[jt], u[1][0], u[1][1], u[1][2], u[1][3], B[2], B[3]);
       }
@@ -217,9 +223,10 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
     const uint32_t q_lane = 4096 + kCrQP + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
     const uint32_t m_lane = 4096 + kCrMQK + r * 16;
     int s = 0;
+    uint32_t par = 0;
     for (int c = 0; c < nchunks; ++c) {
-      const int box_i = 2 * w + (c & 1);
-      if (!warp_wait(bar(P::B_BOX + box_i), (c >> 1) & 1, abort_flag)) { ok = false; break; }
+      const int box_i = s * NW + w;
+      if (!warp_wait(bar(P::B_BOX + box_i), par, abort_flag)) { ok = false; break; }
       const uint32_t stage = sbase + s * P::kStageBytes;
       const uint4* box = reinterpret_cast<const uint4*>(smem + P::kSmBox + box_i * P::kBoxBytes) + lane;
       float O[4][4];
@@ -248,10 +255,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
         mma_bf16_16816(O[3], u1.x, u1.y, u1.z, u1.w, n[2], n[3]);
       }
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(bar(P::B_BOX_FREE + box_i));
-        mbar_arrive(bar(P::B_EMPTY + s));
-      }
+      if (lane == 0) mbar_arrive(bar(P::B_EMPTY + s));
 #pragma unroll
       for (int k = 0; k < 2; ++k)
         stsm_x4_trans(stg + (8 * (2 * k + (mi >> 1)) + r) * P::kStgStride + (mi & 1) * 16, pack_bf16(O[2 * k][0], O[2 * k][1]),
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
               *reinterpret_cast<const uint4*>(stg_p + tok * P::kStgStride + piece * 16);
       }
       __syncwarp();
-      if (++s == P::kStages) s = 0;
+      if (++s == P::kStages) { s = 0; par ^= 1u; }
     }
   } else if (lane == 0) {
     // ===== copies: the record and this CTA's half of the v tile =========================================================
