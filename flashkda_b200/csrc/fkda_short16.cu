@@ -17,8 +17,10 @@
 // through a padded staging buffer: the copy in is issued right behind the inputs, the copy out per warp as soon as
 // its rows are done.
 //
-// What bounds it: HBM, as far as the CTAs of an SM cover each other's phases - two of them with fp32 state, three with bf16.
-// 512 x 32 chains of 16 tokens: 435 us with fp32 states (5.7 TB/s), 302 us with bf16 (4.7 TB/s); 506 and 350 with the states asked
+// What bounds it: HBM, as far as the CTAs of an SM cover each other's phases - two of them with fp32 state; four with bf16 and
+// one block, for which the operands lie over the staged inputs (three beside them: 302 us below).
+// 512 x 32 chains of 16 tokens: 435 us with fp32 states (5.7 TB/s), 270 us with bf16 (5.2 TB/s).  With fewer CTAs and the
+// earlier order of the phases: 506 and 350 with the states asked
 // for ahead of the inputs, whose 16 KB then queue behind them; 460 and 402 with w' = TB k+, u' = TB v formed before the state
 // was touched (a rendezvous more, and two CTAs per SM for either type).  Asking the L2 for the next chain's state: slower.
 #include "fkda_common.cuh"
@@ -36,28 +38,29 @@ constexpr int kStQ = 0;                          // staged q, k, g, v: [16 tok][
 constexpr int kStK = kStQ + 4096;
 constexpr int kStG = kStK + 4096;
 constexpr int kStV = kStG + 4096;
-constexpr int kKN = kStV + 4096;                 // bf16 [16][128] tiles in the 8x8 core-matrix layout: -k+, k-, q+, kr
-constexpr int kKM = kKN + 4096;
-constexpr int kQP = kKM + 4096;
-constexpr int kKR = kQP + 4096;
-constexpr int kTB = kKR + 4096;                  // bf16 [16][16] T diag(beta), core layout
-constexpr int kMQK = kTB + 512;                  // bf16 [16][16]
-constexpr int kA = kMQK + 512;                   // fp32 [16][20]
-constexpr int kT = kA + kRows * kLdS * 4;        // fp32 [16][20]
-constexpr int kE = kT + kRows * kLdS * 4;        // fp32 [128] decay of the whole block
-constexpr int kSsq = kE + 512;                   // fp32 [q|k][16 rows][8 warps] partial sums of squares
-constexpr int kBeta = kSsq + 1024;               // fp32 [16]
-constexpr int kBar = kBeta + 64;                 // mbarrier of the state copy, abort flag
-constexpr int kState = (kBar + 16 + 127) / 128 * 128;   // [128 v] state rows, padded: fragment reads hit 32 distinct banks
 constexpr int kStgStride = 48;                   // output staging (over the dead -k+ and k-): [16 tok][16 v] per warp
 static_assert(8 * kRows * kStgStride <= 8192, "output staging");
 
-// State rows in shared memory: fp32 unless a bf16 state needs one block only.
-template <bool kWide>
-struct Rows {
+// The rest.  A call of one block has no inputs of a next one to receive, so the operands lie over the staged inputs.
+// State rows are fp32 unless a bf16 state needs one block only.
+template <bool kWide, bool kOneBlock>
+struct Lay {
+  static constexpr int kKN = kOneBlock ? 0 : kStV + 4096;          // bf16 [16][128] tiles in the 8x8 core-matrix layout: -k+, k-, q+, kr
+  static constexpr int kKM = kKN + 4096;
+  static constexpr int kQP = kKM + 4096;
+  static constexpr int kKR = kQP + 4096;
+  static constexpr int kTB = kKR + 4096;                           // bf16 [16][16] T diag(beta), core layout
+  static constexpr int kMQK = kTB + 512;                           // bf16 [16][16]
+  static constexpr int kA = kMQK + 512;                            // fp32 [16][20]
+  static constexpr int kT = kA + kRows * kLdS * 4;                 // fp32 [16][20]
+  static constexpr int kE = kT + kRows * kLdS * 4;                 // fp32 [128] decay of the whole block
+  static constexpr int kSsq = kE + 512;                            // fp32 [q|k][16 rows][8 warps] partial sums of squares
+  static constexpr int kBeta = kSsq + 1024;                        // fp32 [16]
+  static constexpr int kBar = kBeta + 64;                          // mbarrier of the state copy, abort flag
+  static constexpr int kState = (kBar + 16 + 127) / 128 * 128;     // [128 v] state rows, padded: fragment reads hit 32 distinct banks
   static constexpr int kStride = kWide ? 512 + 32 : 256 + 16;      // 8 words mod 32 (8-byte reads), 4 words mod 32 (4-byte reads)
   static constexpr int kSmemBytes = kState + kD * kStride;
-  static constexpr int kCtas = kWide ? 2 : 3;
+  static constexpr int kCtas = kWide ? 2 : 4;
   static_assert(kCtas * (kSmemBytes + 1024) <= 227 * 1024, "CTAs per SM");
 };
 constexpr int kBf16Row = 256 + 16;               // where a bf16 row arrives inside a wide slot (its second half)
@@ -82,10 +85,11 @@ struct Params {
 
 // kFp32: type of the state tensors; kOneBlock: T <= 16, compiled without the block loop's bookkeeping
 template <bool kFp32, bool kOneBlock>
-__global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) short16_kernel(const Params p) {
+__global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>::kCtas) short16_kernel(const Params p) {
   using namespace elem;
   constexpr bool kWide = kFp32 || !kOneBlock;
-  constexpr int kStride = Rows<kWide>::kStride;
+  using L = Lay<kWide, kOneBlock>;
+  constexpr int kKN = L::kKN, kKM = L::kKM, kQP = L::kQP, kKR = L::kKR, kTB = L::kTB, kMQK = L::kMQK, kState = L::kState, kStride = L::kStride;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -93,12 +97,12 @@ __global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) sh
   const int n = chain / p.H, h = chain - n * p.H;       // consecutive CTAs: consecutive heads of the same tokens
   const int64_t t_seq0 = static_cast<int64_t>(n) * p.T;
   const int nblk = kOneBlock ? 1 : (p.T + kRows - 1) / kRows;
-  float* s_e = reinterpret_cast<float*>(smem + kE);
-  float* s_ssq = reinterpret_cast<float*>(smem + kSsq);
-  float* s_beta = reinterpret_cast<float*>(smem + kBeta);
+  float* s_e = reinterpret_cast<float*>(smem + L::kE);
+  float* s_ssq = reinterpret_cast<float*>(smem + L::kSsq);
+  float* s_beta = reinterpret_cast<float*>(smem + L::kBeta);
 
-  const uint32_t bar = sbase + kBar;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kBar + 8);
+  const uint32_t bar = sbase + L::kBar;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kBar + 8);
   constexpr int row_bytes = kFp32 ? 512 : 256;
   constexpr int in_off = !kFp32 && kWide ? kBf16Row : 0;
   if (tid == 0) {
@@ -155,6 +159,7 @@ __global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) sh
     if (*abort_flag) { failed = true; break; }
 
     float R[2][4], O[2][4];                // [token tile]: rows v = 16 warp + g (+ 8), tokens 8 nt + 2 t4, + 1
+    uint32_t x[4];                         // v^T of this warp's rows
     if (warp < 8) {
       // ---- element-wise stage: 16 channels of 16 tokens --------------------------------------------------------------
       const uint32_t src = sbase + stage_off(8 * (mi & 1) + r, 2 * warp + (mi >> 1));
@@ -162,6 +167,7 @@ __global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) sh
       ldsm_x4(src + kStQ, q[0], q[1], q[2], q[3]);
       ldsm_x4(src + kStK, k[0], k[1], k[2], k[3]);
       ldsm_x4_trans(src + kStG, gw[0], gw[1], gw[2], gw[3]);
+      if (kOneBlock) ldsm_x4_trans(src + kStV, x[0], x[1], x[2], x[3]);
       auto squares = [&](const uint32_t(&x)[4], float* dst) {
         float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
         mma_bf16_16816(c0, x[0], x[1], x[2], x[3], x[0], x[2]);
@@ -201,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) sh
         G[nt][1] = fma2(pk(d[2], d[3]), pk(hgs, hgs), pk(c1, c1));
         tot[nt] = fma2(pk(s[0], s[1]), pk(hgs, hgs), pk(16.f * hgs, 16.f * hgs));
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");      // the partial sums of squares are complete
+      asm volatile("bar.sync 1, 256;" ::: "memory");      // the partial sums of squares are complete, the staged inputs read
       float rq[2], rk[2];
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
@@ -246,8 +252,7 @@ __global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) sh
     if (warp < 8) {
       // ---- R^T = v^T - S^T k+^T, O^T = S^T q+^T ---------------------------------------------------------------------------
       {
-        uint32_t x[4];
-        ldsm_x4_trans(sbase + kStV + stage_off(8 * (mi & 1) + r, 2 * warp + (mi >> 1)), x[0], x[1], x[2], x[3]);
+        if (!kOneBlock) ldsm_x4_trans(sbase + kStV + stage_off(8 * (mi & 1) + r, 2 * warp + (mi >> 1)), x[0], x[1], x[2], x[3]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           R[nt][0] = bf_lo(x[nt]);
@@ -284,8 +289,8 @@ __global__ void __launch_bounds__(kThreads, Rows<kFp32 || !kOneBlock>::kCtas) sh
       }
     } else {
       // ---- ninth warp: A, T = (I + A)^-1, T diag(beta); tril(M) -----------------------------------------------------------
-      float* s_A = reinterpret_cast<float*>(smem + kA);
-      float* s_T = reinterpret_cast<float*>(smem + kT);
+      float* s_A = reinterpret_cast<float*>(smem + L::kA);
+      float* s_T = reinterpret_cast<float*>(smem + L::kT);
       const uint32_t a_lane = sbase + (mi & 1) * 2048 + (mi >> 1) * 128 + r * 16;
       const uint32_t b_lane = sbase + kKM + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
       float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, mq[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -442,7 +447,7 @@ cudaError_t launch_short16(const __nv_bfloat16* q, const __nv_bfloat16* k, const
   const Params p{q, k, v, g, beta, A_log, dt_bias, initial_state, final_state, out, T, H, scale, gate_scale, status};
   const int form = (state_fp32 ? 2 : 0) + (T <= kRows ? 1 : 0);
   void (*const kernels[4])(Params) = {short16_kernel<false, false>, short16_kernel<false, true>, short16_kernel<true, false>, short16_kernel<true, true>};
-  const int smem = form == 1 ? Rows<false>::kSmemBytes : Rows<true>::kSmemBytes;
+  const int smem = form == 0 || form == 2 ? Lay<true, false>::kSmemBytes : form == 1 ? Lay<false, true>::kSmemBytes : Lay<true, true>::kSmemBytes;
   static SmemOptIn opt_in[4];
   cudaError_t e = opt_in[form].ensure(kernels[form], smem);
   if (e != cudaSuccess) return e;
