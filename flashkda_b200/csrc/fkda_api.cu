@@ -294,9 +294,9 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
 // Runs per sequence for the walk over compact records (1: whole sequences), at most `most` of them, and their length.
 // Hundredths of a microsecond per chunk step, measured: a chain split over four or two CTAs (fkda_recur_split.cu) or in one
 // CTA (fkda_recur.cu), the latter with and without outputs; a pass costs about 8 us beside its steps, the chaining of
-// the maps 3 us per run and wave of its CTAs.
+// the maps 1.45 us per run and wave of its CTAs.
 int plan_runs(int64_t chains, int64_t chunks, int most, int sms, int* len) {
-  constexpr int64_t kQuad = 60, kHalf = 80, kOne = 132, kQuiet = 95;
+  constexpr int64_t kQuad = 58, kHalf = 90, kOne = 132, kQuiet = 95;
   const int64_t whole = (chains * 4 <= sms ? kQuad : chains * 2 <= sms ? kHalf : kOne * ((chains + sms - 1) / sms)) * chunks;
   int64_t best = whole;
   int best_n = 1;
@@ -306,7 +306,7 @@ int plan_runs(int64_t chains, int64_t chunks, int most, int sms, int* len) {
     if ((n - 1) * l >= chunks) continue;       // the last run would be empty
     const int64_t pass1 = (chains * (2 * n - 3) + sms - 1) / sms * kQuiet * l, run0 = kOne * l;
     const int64_t pass2 = (chains * (n - 1) + sms - 1) / sms * kOne * l;
-    const int64_t cost = (pass1 > run0 ? pass1 : run0) + pass2 + 1600 + 300 * (n - 2) * ((chains * 8 + sms - 1) / sms);
+    const int64_t cost = (pass1 > run0 ? pass1 : run0) + pass2 + 1600 + 145 * (n - 2) * ((chains * 16 + sms - 1) / sms);
     if (cost < best) {
       best = cost;
       best_n = static_cast<int>(n);

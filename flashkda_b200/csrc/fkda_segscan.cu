@@ -18,35 +18,63 @@ cudaError_t launch_scan(const ScanParams& p, cudaStream_t stream);
 
 namespace {
 
-constexpr int kCmbRows = 16;                              // state rows per CTA: one m16 tile
-constexpr int kMapStride = kSegMapStride;                 // floats per map row, in its slot and here (B fragments: bank 8 t + g)
+constexpr int kCmbRows = 8;                               // state rows per CTA: the n of an mma, whose m are columns of the map
+constexpr int kMapStride = kSegMapStride;                 // floats per map row, in its slot and here (fragments: bank 8 t + g)
 constexpr int kMapStg = kD * kMapStride * 4;
-constexpr int kZStride = 132;                             // floats per staged state row (A fragments: bank 4 g + t)
 constexpr int kMapBufs = 3;                               // maps in flight
 constexpr int kCmbM = 0;                                  // kMapBufs x [128][136] fp32: transition maps
-constexpr int kCmbZ = kCmbM + kMapBufs * kMapStg;         // [16][132] fp32: this CTA's rows of the state
-constexpr int kCmbBars = kCmbZ + kCmbRows * kZStride * 4;
+constexpr int kCmbZ = kCmbM + kMapBufs * kMapStg;         // [16 k-steps][32 lanes]: this CTA's rows of the state as B fragments, leading and trailing parts
+constexpr int kCmbPart = kCmbZ + 16 * 512;                // [8 warps][32 lanes][4] fp32: partial sums of the upper half of k
+constexpr int kCmbBars = kCmbPart + 8 * 512;
+constexpr int kCmbThreads = 512;
 constexpr int kCmbSmemBytes = kCmbBars + 64 + 128;
 static_assert(kCmbSmemBytes <= 227 * 1024, "map buffers fit one SM");
 
+// x = hi + lo, both tf32, hi rounded to nearest (away from zero on ties, as cvt.rna does) by integer arithmetic: the
+// conversion instruction issues at a fraction of that rate.  lo <= 2^-11 |x| is cut off 2^-21 below x.
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  lo = __float_as_uint(x - __uint_as_float(hi)) & 0xffffe000u;
+}
+
 // Z_start[run + 1] = Z_start[run] M[run] + N[run] for run = 1 .. n_segs-2; rows of Z are independent, so each CTA
-// carries sixteen of them through all runs.  The maps arrive by bulk copies (one per map: its slot holds it with padded
-// rows) three runs ahead, so the serial chain of runs sees shared-memory latency only.  The products run on the tensor cores in
-// tf32 with both operands split into a leading and a trailing part (three mma per tile: the error of the split, about
-// 2^-21 relative, is that of an fp32 product), fp32 accumulation on top of N.
-__global__ void __launch_bounds__(256) seg_combine_kernel(float* seg_buf, int n_segs, int* status) {
+// carries eight of them through all runs, as Z^T[run + 1] = M^T Z^T + N^T.  The maps arrive by bulk copies (one per map: its
+// slot holds it with padded rows) three runs ahead.  The products run on the tensor cores in tf32 with both operands split into a leading and a
+// trailing part (three mma per tile: the error of the split, about 2^-21 relative, is that of an fp32 product), fp32
+// accumulation on top of N.
+// What bounds it: the serial chain of runs.  So a run's map waits in registers, split, before the state that it is applied to
+// is there: each k-step's fragments are replaced by the next run's as soon as its products are issued, in the issue slots
+// that these leave.  What remains on the chain is 48 mma per warp and one exchange of the state through shared memory, split
+// once by its producer.  Per run: 3.2 us with sixteen rows per CTA and both operands read and split on the chain, 1.4 us now
+// (2 heads of 65536 tokens: 331 -> 274 us).  Sixteen warps, two per sixteen columns with half of k each: with eight the loop is 8 KB of code,
+// which the instruction caches no longer hold (1.7 us).
+__global__ void __launch_bounds__(kCmbThreads, 1) seg_combine_kernel(float* seg_buf, int n_segs, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   const uint32_t sbase = smem_u32(smem);
-  float* z = reinterpret_cast<float*>(smem + kCmbZ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kCmbBars + 32);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   float* slots = seg_buf + static_cast<size_t>(blockIdx.x) * n_segs * 3 * kSegSlotFloats;
   const int r_base = blockIdx.y * kCmbRows;
   auto load_map = [&](int run) {      // one thread: the whole slot, rows padded as the recurrence kernel left them
+    if (run + 1 >= n_segs) return;
     const int b = (run - 1) % kMapBufs;
     mbar_arrive_expect_tx(sbase + kCmbBars + 8 * b, kMapStg);
     bulk_g2s(sbase + kCmbM + b * kMapStg, slots + (run * 3 + 0) * kSegSlotFloats, kMapStg, sbase + kCmbBars + 8 * b);
+  };
+  auto wait_map = [&](int run) { return mbar_wait(sbase + kCmbBars + 8 * ((run - 1) % kMapBufs), ((run - 1) / kMapBufs) & 1, abort_flag); };
+  // rows g, g + 8 of an m-tile stand for the columns n0 + 2 g, + 1, so that two fragment registers are one 8-byte load;
+  // accumulators: rows 2 t, + 1 of the state (i & 1), those columns (i >> 1)
+  auto put_z = [&](int n0, const float(&x)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int col = n0 + 2 * g + (i >> 1), row = 2 * t + (i & 1);
+      uint32_t hi, lo;
+      split_tf32(x[i], hi, lo);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(smem + kCmbZ) + (col >> 3) * 128 + (4 * row + (col & 3)) * 4 + ((col >> 2) & 1);
+      dst[0] = hi;
+      dst[2] = lo;
+    }
   };
   if (tid == 0) {
     *abort_flag = 0;
@@ -54,44 +82,39 @@ __global__ void __launch_bounds__(256) seg_combine_kernel(float* seg_buf, int n_
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_wait();
   if (tid == 0)
-    for (int run = 1; run <= kMapBufs && run + 1 < n_segs; ++run) load_map(run);
-  {
-    // the state at the start of run 1: thread -> (row, eight columns)
-    const int r = tid >> 4, c = (tid & 15) * 8;
-    const float* src = slots + (1 * 3 + 2) * kSegSlotFloats + static_cast<size_t>(r_base + r) * kD + c;
-    const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src + 4));
-    *reinterpret_cast<float4*>(z + r * kZStride + c) = a;
-    *reinterpret_cast<float4*>(z + r * kZStride + c + 4) = b;
-  }
-  __syncthreads();
-  const int g = lane >> 2, t = lane & 3;
-  const int n0 = warp * 16;              // this warp's sixteen output columns
-  // N of a run: mma C layout, rows g and g + 8, columns n0 + 8 nt + 2 t + {0, 1}; fetched one run ahead (its latency
-  // would otherwise sit on the serial chain of runs)
-  auto load_n = [&](int run, float (&d)[2][4]) {
-    const float* N = slots + (run * 3 + 1) * kSegSlotFloats + static_cast<size_t>(r_base) * kD;
+    for (int run = 1; run <= kMapBufs; ++run) load_map(run);
+  const int n0 = (warp & 7) * 16, half = warp >> 3;        // this warp's sixteen output columns, its half of k
+  // a CTA's rows of a slot in the accumulators' layout
+  auto load_rows = [&](const float* slot, float (&d)[4]) {
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      const float2 lo = *reinterpret_cast<const float2*>(N + g * kD + n0 + 8 * nt + 2 * t);
-      const float2 hi = *reinterpret_cast<const float2*>(N + (g + 8) * kD + n0 + 8 * nt + 2 * t);
-      d[nt][0] = lo.x; d[nt][1] = lo.y; d[nt][2] = hi.x; d[nt][3] = hi.y;
+    for (int i = 0; i < 2; ++i) {
+      const float2 y = *reinterpret_cast<const float2*>(slot + static_cast<size_t>(r_base + 2 * t + i) * kD + n0 + 2 * g);
+      d[i] = y.x;
+      d[2 + i] = y.y;
     }
   };
-  float next_n[2][4];
-  if (n_segs > 2) load_n(1, next_n);
-  for (int run = 1; run + 1 < n_segs; ++run) {
-    const int b = (run - 1) % kMapBufs;
-    float acc[2][4];                  // accumulators start from N
+  float x[4], next_n[4];                 // N of a run is fetched one run ahead
+  load_rows(slots + (1 * 3 + 2) * kSegSlotFloats, x);      // the state at the start of run 1
+  if (half == 0) put_z(n0, x);
+  load_rows(slots + (1 * 3 + 1) * kSegSlotFloats, next_n);
+  // this warp's columns of a map, split: [k-step][leading, trailing part][A fragment]
+  uint32_t m[8][2][4];
+  auto load_m = [&](int run, int ks) {
+    const float* M = reinterpret_cast<const float*>(smem + kCmbM + ((run - 1) % kMapBufs) * kMapStg) + (64 * half + 8 * ks + t) * kMapStride + n0 + 2 * g;
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int e = 0; e < 2; ++e) {
+      const float2 y = *reinterpret_cast<const float2*>(M + 4 * e * kMapStride);
+      split_tf32(y.x, m[ks][0][2 * e], m[ks][1][2 * e]);
+      split_tf32(y.y, m[ks][0][2 * e + 1], m[ks][1][2 * e + 1]);
+    }
+  };
+  bool ok = wait_map(1);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[nt][i] = next_n[nt][i];
-    if (run + 2 < n_segs) load_n(run + 1, next_n);
-    if (tid < 64 && run + 5 < n_segs)     // and the lines of a later N into the L2: 16 rows of 512 bytes
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(slots + ((run + 4) * 3 + 1) * kSegSlotFloats +
-                                                     static_cast<size_t>(r_base + (tid >> 2)) * kD + (tid & 3) * 32));
-    const bool ok = mbar_wait(sbase + kCmbBars + 8 * b, ((run - 1) / kMapBufs) & 1, abort_flag, 32);
+  for (int ks = 0; ks < 8; ++ks) load_m(1, ks);
+  int run = 1;
+  for (;; ++run) {
     if (!__syncthreads_and(ok)) {
       if (tid == 0) {
         atomicCAS(status, kStatusOk, kStatusWaitTimeout);
@@ -104,56 +127,48 @@ __global__ void __launch_bounds__(256) seg_combine_kernel(float* seg_buf, int n_
       }
       break;
     }
-    const float* M = reinterpret_cast<const float*>(smem + kCmbM + b * kMapStg);
-    // four accumulators per tile, used in turn: the 48 mma of a tile would otherwise form one dependent chain
-    float part[2][3][4];
+    // here: z holds the state at the start of `run`, m its map, whose buffer is free
+    if (run + 1 >= n_segs) break;
+    if (tid == 0) load_map(run + kMapBufs);
+    float acc[3][4];                  // hi hi on top of N, lo hi, hi lo
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int i = 0; i < 4; ++i) {
+      acc[0][i] = half == 0 ? next_n[i] : 0.f;
+      acc[1][i] = acc[2][i] = 0.f;
+    }
+    if (run + 2 < n_segs) {
+      if (half == 0) load_rows(slots + ((run + 1) * 3 + 1) * kSegSlotFloats, next_n);
+      ok = wait_map(run + 1);
+    }
+    if (tid < 32 && run + 5 < n_segs)     // and the lines of a later N into the L2: 16 rows of 512 bytes
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(slots + ((run + 4) * 3 + 1) * kSegSlotFloats +
+                                                     static_cast<size_t>(r_base + (tid >> 2)) * kD + (tid & 3) * 32));
+    const uint4* z = reinterpret_cast<const uint4*>(smem + kCmbZ) + 256 * half + lane;
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) part[nt][q][i] = 0.f;
-#pragma unroll 2
-    for (int ks = 0; ks < kD / 8; ks += 2) {
-#pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        const int k0 = 8 * (ks + kk);
-        const float af[4] = {z[g * kZStride + k0 + t], z[(g + 8) * kZStride + k0 + t], z[g * kZStride + k0 + t + 4],
-                             z[(g + 8) * kZStride + k0 + t + 4]};
-        uint32_t ah[4], al[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          ah[i] = to_tf32(af[i]);
-          al[i] = to_tf32(af[i] - __uint_as_float(ah[i]));
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const float b0 = M[(k0 + t) * kMapStride + n0 + 8 * nt + g], b1 = M[(k0 + t + 4) * kMapStride + n0 + 8 * nt + g];
-          const uint32_t bh0 = to_tf32(b0), bh1 = to_tf32(b1);
-          const uint32_t bl0 = to_tf32(b0 - __uint_as_float(bh0)), bl1 = to_tf32(b1 - __uint_as_float(bh1));
-          mma_tf32_1688(part[nt][0], al[0], al[1], al[2], al[3], bh0, bh1);
-          mma_tf32_1688(part[nt][1], ah[0], ah[1], ah[2], ah[3], bl0, bl1);
-          if (kk == 0) mma_tf32_1688(part[nt][2], ah[0], ah[1], ah[2], ah[3], bh0, bh1);
-          else mma_tf32_1688(acc[nt], ah[0], ah[1], ah[2], ah[3], bh0, bh1);
-        }
-      }
+    for (int ks = 0; ks < 8; ++ks) {
+      const uint4 b = z[32 * ks];     // two registers of the leading part, two of the trailing one
+      mma_tf32_1688(acc[1], m[ks][1][0], m[ks][1][1], m[ks][1][2], m[ks][1][3], b.x, b.y);
+      mma_tf32_1688(acc[2], m[ks][0][0], m[ks][0][1], m[ks][0][2], m[ks][0][3], b.z, b.w);
+      mma_tf32_1688(acc[0], m[ks][0][0], m[ks][0][1], m[ks][0][2], m[ks][0][3], b.x, b.y);
+      load_m(run + 1, ks);            // (behind the last run: whatever the buffer holds, not used)
     }
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int i = 0; i < 4; ++i) x[i] = acc[0][i] + (acc[1][i] + acc[2][i]);
+    float4* part = reinterpret_cast<float4*>(smem + kCmbPart) + (warp & 7) * 32 + lane;
+    if (half == 1) *part = make_float4(x[0], x[1], x[2], x[3]);
+    __syncthreads();                  // every thread is done with z; the partial sums are there
+    if (half == 0) {
+      const float4 y = *part;
+      x[0] += y.x;
+      x[1] += y.y;
+      x[2] += y.z;
+      x[3] += y.w;
+      put_z(n0, x);
+      float* zs = slots + ((run + 1) * 3 + 2) * kSegSlotFloats;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[nt][i] += (part[nt][0][i] + part[nt][1][i]) + part[nt][2][i];
-    __syncthreads();                  // every thread is done with z and with map buffer b
-    if (tid == 0 && run + kMapBufs + 1 < n_segs) load_map(run + kMapBufs);
-    float* zs = slots + ((run + 1) * 3 + 2) * kSegSlotFloats + static_cast<size_t>(r_base) * kD;
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      const int c = n0 + 8 * nt + 2 * t;
-      *reinterpret_cast<float2*>(z + g * kZStride + c) = make_float2(acc[nt][0], acc[nt][1]);
-      *reinterpret_cast<float2*>(z + (g + 8) * kZStride + c) = make_float2(acc[nt][2], acc[nt][3]);
-      *reinterpret_cast<float2*>(zs + g * kD + c) = make_float2(acc[nt][0], acc[nt][1]);
-      *reinterpret_cast<float2*>(zs + (g + 8) * kD + c) = make_float2(acc[nt][2], acc[nt][3]);
+      for (int i = 0; i < 2; ++i)
+        *reinterpret_cast<float2*>(zs + static_cast<size_t>(r_base + 2 * t + i) * kD + n0 + 2 * g) = make_float2(x[i], x[2 + i]);
     }
-    __syncthreads();
   }
 }
 
@@ -181,8 +196,7 @@ cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_ch
     e = opt_in.ensure(seg_combine_kernel, kCmbSmemBytes);
     if (e != cudaSuccess) return e;
     const dim3 grid(static_cast<unsigned>(chains), kD / kCmbRows);
-    seg_combine_kernel<<<grid, 256, kCmbSmemBytes, stream>>>(seg_buf, n_segs, p.status);
-    e = cudaGetLastError();
+    e = launch_after(seg_combine_kernel, grid, kCmbThreads, kCmbSmemBytes, stream, seg_buf, n_segs, p.status);
     if (e != cudaSuccess) return e;
   }
   p.seg_pass = 2;
