@@ -351,6 +351,7 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   fkda::ScanParams s = scan_params(p, L);
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
   s.skip_short = p->cu_seqlens != nullptr;
+  s.release_next = p->cu_seqlens != nullptr && runs == 1;      // (to the step kernel below)
   if (runs > 1) {
     e = fkda::launch_scan_segmented(s, runs, run_len, reinterpret_cast<float*>(ws + L.seg_off), 0, v, stream);
   } else {

@@ -176,6 +176,8 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // is still running; everything up to this wait (barrier set-up, tensor-memory allocation) then overlaps with that
 // kernel's end.  Nothing that an earlier kernel writes or reads may be touched before it.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Once every CTA of this kernel has come here, the next kernel may start on the SMs that this one leaves free.
+__device__ __forceinline__ void grid_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- bulk async copies (the TMA engine, untiled form; 16-byte aligned addresses and sizes) ------
 __device__ __forceinline__ void bulk_g2s(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
@@ -446,6 +448,7 @@ struct ScanParams {
   int select_want;
   const int* seg_chunks_dev;   // varlen batches: run length decided on the device from the longest sequence (else nullptr)
   int skip_short;              // packed batches: sequences of at most kStepMaxT tokens are somebody else's (no chunks, no state)
+  int release_next;            // the next kernel needs nothing of this one's results and may start beside it
   int* next_walk;              // persistent recurrence kernel: device counter (zeroed) that hands out the walks, or nullptr (in turn)
   // Test aids of the look-ahead kernel's give-up path (both 0 in production): a wait limit in microseconds instead of
   // the default, and a number of records after which the copy producer stops issuing copies, so that the consumers'

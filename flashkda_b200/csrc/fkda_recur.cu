@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
   const uint32_t tmem = *tmem_slot;
   bool ok = *abort_flag == 0;
   grid_dependency_wait();
+  if (p.release_next) grid_release_next();
 
   if (warp < 4) {
     // ===== recurrence ================================================================================================

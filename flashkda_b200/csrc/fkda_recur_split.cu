@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
   __syncthreads();
   bool ok = *abort_flag == 0;
   grid_dependency_wait();
+  if (p.release_next) grid_release_next();
   const ChainView cv = chain_view<false>(p, blockIdx.x / P::kSplits);
   const int cta_row = static_cast<int>(blockIdx.x % P::kSplits) * P::kRows;
   const int nchunks = ok ? cv.nchunks : 0;

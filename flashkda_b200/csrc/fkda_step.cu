@@ -10,6 +10,10 @@
 // products of a token fold into one value per lane on the way through the reduction.  Every CTA works out the tokens'
 // vectors for itself (a few hundred elements) while its rows of the state arrive.
 //
+// In a packed batch it runs beside the recurrence over the longer sequences, on the SMs that this leaves free: it reads none of
+// the call's intermediate results, and when the recurrence starts, all that came before the call is complete.  One CTA waits for
+// the recurrence at its end, so that a kernel that waits for this one waits for both.
+//
 // What bounds it: the stream over the states at one token (512 x 32 chains: 171 us with bf16 states, 323 with fp32: 97 and
 // 102 % of the measured copy rate; the tile kernel takes 330 and 470), then the shared-memory pipe: 840 cycles per token,
 // chain and SM, 512 of them the reads of the vectors, 230 the shuffles.  Above kStepMaxT the tile form
@@ -79,7 +83,7 @@ __global__ void __launch_bounds__(kThreads, kWhole ? 5 : 6) step_kernel(const Pa
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chain = static_cast<int>(kWhole ? blockIdx.x : blockIdx.x >> 2), row0 = kWhole ? 0 : static_cast<int>(blockIdx.x & 3) * kRows;
   const int n = chain / p.H, h = chain - n * p.H;
-  grid_dependency_wait();
+  if (!kPacked) grid_dependency_wait();
   int T = p.T;
   int64_t bos = static_cast<int64_t>(n) * p.T;
   if constexpr (kPacked) {
@@ -87,7 +91,10 @@ __global__ void __launch_bounds__(kThreads, kWhole ? 5 : 6) step_kernel(const Pa
     bos = p.cu_seqlens[n];
     bos = bos < 0 ? 0 : (bos > p.T_total ? p.T_total : bos);
     eos = eos < bos ? bos : (eos > p.T_total ? p.T_total : eos);
-    if (eos - bos > kStepMaxT) return;
+    if (eos - bos > kStepMaxT) {
+      if (blockIdx.x == 0) grid_dependency_wait();
+      return;
+    }
     T = static_cast<int>(eos - bos);
   }
   float4(*const s_vec)[4][kD / 4] = reinterpret_cast<float4(*)[4][kD / 4]>(smem);
@@ -226,6 +233,7 @@ __global__ void __launch_bounds__(kThreads, kWhole ? 5 : 6) step_kernel(const Pa
     const int t = i / kPieces, c = (i % kPieces) * 8;
     *reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(bos + t) * p.H + h) * kD + row0 + c) = *reinterpret_cast<const uint4*>(&s_out[t][c]);
   }
+  if (kPacked && blockIdx.x == 0) grid_dependency_wait();
 }
 
 }  // namespace step
