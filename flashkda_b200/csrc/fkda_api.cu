@@ -199,6 +199,7 @@ fkda::PrepParams prep_params(const fkda_fwd_params* p, const Layout& L) {
   q.H = static_cast<int>(p->H);
   q.N = static_cast<int>(p->N);
   q.total_chunks = static_cast<int>(L.chunks_per_head);
+  q.seq_chunks = q.slice_chunks = static_cast<int>((p->T + fkda::kChunk - 1) / fkda::kChunk);
   q.scale = p->scale;
   q.gate_scale = static_cast<float>(static_cast<double>(p->lower_bound) * 1.4426950408889634);
   return q;
@@ -317,6 +318,21 @@ int plan_runs(int64_t chains, int64_t chunks, int most, int sms, int* len) {
   return best_n;
 }
 
+// Where fewer chains than SMs have a CTA each, the SMs beyond them can work out operands meanwhile.  The call is then cut in two
+// time slices, and the second one's operands are computed beside the first one's recurrence, by kSliceWaves waves of two
+// CTAs on each free SM that end with it.  A chunk of the recurrence takes 1.32 us; a CTA of the token-parallel stage 3.7 us per item
+// and 5 us to fill and drain its pipeline.  Returns the chunks of the first slice, or 0 where the stage is not shortened by
+// 40 us: the second pair of launches and the stage's share of the recurrence's bandwidth cost about 30.  96 heads of 8192 tokens:
+// 628 -> 576 us; 75 of 16384: 1121 -> 989; 128 chains, whose 20 free SMs would gain nothing, stay in one piece.
+constexpr int kSliceWaves = 2;
+int plan_slice(int64_t chains, int64_t chunks, int sms) {
+  if (chains >= sms || chunks < 16) return 0;
+  const double c = static_cast<double>(chunks), per_us = 2.0 * kSliceWaves * static_cast<double>(sms - chains) / (3.7 * static_cast<double>(chains));
+  const double second = per_us * (1.32 / kSliceWaves * c - 5.0) / (1.0 + 1.32 / kSliceWaves * per_us);
+  if (second * 0.0118 * static_cast<double>(chains) < 40.0) return 0;
+  return static_cast<int>(c - second);
+}
+
 // The forward pass over compact records (fkda_record.cuh): token-parallel stage, then the recurrence in the form that suits
 // the number of chains.
 int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
@@ -346,7 +362,14 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
                                   reinterpret_cast<int*>(ws + L.prefix_off), status, stream);
   else e = clear_status(p, stream);
   if (e != cudaSuccess) return cuda_fail(e, "scheduling launch");
-  e = fkda::launch_operands(prep_params(p, L), (p->flags & FKDA_FLAG_PREPARE_TCGEN05) != 0, stream);
+  // Fewer chains than a quarter or half of the SMs: a chain's time is what counts, it is split over four or two CTAs.
+  // (FKDA_FLAG_SCAN_NO_SEGMENTS: one CTA walks the whole chain.)
+  const bool whole = (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS) != 0, one_item = (p->flags & FKDA_FLAG_PREPARE_TCGEN05) != 0;
+  const int rows = runs > 1 || whole ? 0 : chains * 4 <= sms ? 32 : chains * 2 <= sms ? 64 : 0;
+  fkda::PrepParams q = prep_params(p, L);
+  const int slice = p->cu_seqlens || runs > 1 || rows || whole || one_item ? 0 : plan_slice(chains, q.seq_chunks, sms);
+  if (slice) q.slice_chunks = slice;
+  e = fkda::launch_operands(q, one_item, stream);
   if (e != cudaSuccess) return cuda_fail(e, "token-parallel launch");
   fkda::ScanParams s = scan_params(p, L);
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
@@ -356,13 +379,24 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
     e = fkda::launch_scan_segmented(s, runs, run_len, reinterpret_cast<float*>(ws + L.seg_off), 0, v, stream);
   } else {
     s.seg_chunks_dev = nullptr;
-    // Fewer chains than a quarter or half of the SMs: a chain's time is what counts, it is split over four or two CTAs.
-    // (FKDA_FLAG_SCAN_NO_SEGMENTS: one CTA walks the whole chain.)
-    const bool split = (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS) == 0;
-    if (split && chains * 4 <= sms) e = fkda::launch_recur_split(s, v, 32, stream);
-    else if (split && chains * 2 <= sms) e = fkda::launch_recur_split(s, v, 64, stream);
-    else {
-      s.next_walk = p->cu_seqlens ? status + 3 : nullptr;
+    s.next_walk = p->cu_seqlens ? status + 3 : nullptr;
+    if (rows) {
+      e = fkda::launch_recur_split(s, v, rows, stream);
+    } else if (slice) {
+      s.slice_end = slice;
+      s.release_next = 1;
+      e = fkda::launch_recur(s, v, stream);
+      if (e != cudaSuccess) return cuda_fail(e, "recurrence launch");
+      q.slice_begin = slice;
+      q.slice_chunks = q.seq_chunks - slice;
+      q.beside = 2 * kSliceWaves * (sms - static_cast<int>(chains));
+      e = fkda::launch_operands(q, false, stream);
+      if (e != cudaSuccess) return cuda_fail(e, "token-parallel launch");
+      s.slice_begin = slice;
+      s.slice_end = q.seq_chunks;
+      s.release_next = 0;
+      e = fkda::launch_recur(s, v, stream);
+    } else {
       e = fkda::launch_recur(s, v, stream);
     }
   }

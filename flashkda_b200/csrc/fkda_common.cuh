@@ -34,6 +34,7 @@ constexpr int kRecWP = 10752;
 constexpr int kRecQP = 18944;
 constexpr int kRecUP = 27136;
 constexpr int kRecBytes = 35328;
+constexpr int kCompactRecBytes = 29184;          // of fkda_record.cuh
 
 // workspace header (bytes): [0,64) status words, [256, 256+4*(N+1)) chunk prefix, records after
 constexpr int kWsHeaderBytes = 256;
@@ -418,6 +419,10 @@ struct PrepParams {
   int dbg;                     // tuning aid: bit mask of phases to skip (0 in production)
   int wait_limit_us;           // 0: the waits give up after kWaitLimitNs; else after this many microseconds (test aid)
   int first_load_only;         // 0: normal; 1: a CTA of the pipelined kernel loads the tiles of its first item only (test aid)
+  int seq_chunks;              // compact records of equal lengths: chunks of a sequence
+  int slice_begin;             // ... of which the call works out slice_chunks, from slice_begin on
+  int slice_chunks;
+  int beside;                  // ... beside the kernel before, none of whose results it needs, with so many CTAs; the last one waits for that kernel
 };
 
 struct ScanParams {
@@ -455,6 +460,10 @@ struct ScanParams {
   // next wait runs out with nothing in flight.
   int wait_limit_us;
   int stop_copies_after;
+  // Equal lengths in two time slices: the chunks [slice_begin, slice_end) of every sequence (slice_end 0: all of them), the state
+  // between the slices in fp32 over the chain's first records, which nobody reads any more.
+  int slice_begin;
+  int slice_end;
 };
 
 constexpr int kSegMapStride = 136;             // floats per row of a transition map M in its slot: the map chaining reads
@@ -564,7 +573,7 @@ struct ChainView {
   int fin_stride;              // elements per row there (128; a transition map's slot: kSegMapStride)
   bool write_out, zero_up;
 };
-template <bool kSeg>
+template <bool kSeg, bool kSlice = false>   // kSlice: minds the time slice of ScanParams
 __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) {
   ChainView cv;
   int chain = block, seg = 0, variant = 0;
@@ -635,6 +644,24 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
       cv.init_mode = 1;
       cv.init_base = slots + (seg * 3 + 2) * kSegSlotFloats;
       if (seg != p.n_segs - 1) cv.fin_base = nullptr;
+    }
+  }
+  if constexpr (kSlice) {
+    if (p.slice_end > 0) {
+      uint8_t* between = const_cast<uint8_t*>(p.records) + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCompactRecBytes;
+      if (p.slice_end < cv.nchunks) {
+        cv.eos = cv.bos + static_cast<int64_t>(p.slice_end) * kChunk;
+        cv.nchunks = p.slice_end;
+        cv.fin_base = between;
+        cv.fin_fp32 = 1;
+      }
+      if (p.slice_begin > 0) {
+        cv.bos += static_cast<int64_t>(p.slice_begin) * kChunk;
+        cv.chunk_base += p.slice_begin;
+        cv.nchunks -= p.slice_begin;
+        cv.init_base = between;
+        cv.init_mode = 1;
+      }
     }
   }
   if (skipped) {

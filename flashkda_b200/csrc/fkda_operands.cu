@@ -61,6 +61,7 @@ struct Info {
 };
 static_assert(sizeof(Info) == 32, "info");
 
+template <bool kSlice>
 __device__ __forceinline__ Info decode(const PrepParams& p, unsigned item) {
   Info r;
   r.h = static_cast<int>(item % static_cast<unsigned>(p.H));        // consecutive items: consecutive heads of a chunk, adjacent in memory
@@ -80,8 +81,9 @@ __device__ __forceinline__ Info decode(const PrepParams& p, unsigned item) {
     const long long rem = eos - r.t0;
     r.len = rem < kChunk ? static_cast<int>(rem) : kChunk;
   } else {
-    const unsigned cps = static_cast<unsigned>((p.T + kChunk - 1) / kChunk);
-    const unsigned n = static_cast<unsigned>(r.gc) / cps, lc = static_cast<unsigned>(r.gc) - n * cps;
+    const unsigned cps = kSlice ? static_cast<unsigned>(p.slice_chunks) : static_cast<unsigned>((p.T + kChunk - 1) / kChunk);
+    const unsigned n = static_cast<unsigned>(r.gc) / cps, lc = static_cast<unsigned>(r.gc) - n * cps + (kSlice ? static_cast<unsigned>(p.slice_begin) : 0u);
+    if (kSlice) r.gc = static_cast<int>(n * static_cast<unsigned>(p.seq_chunks) + lc);
     r.t0 = static_cast<long long>(n) * p.T + static_cast<long long>(lc) * kChunk;
     const long long rem = p.T - static_cast<long long>(lc) * kChunk;
     r.len = rem < kChunk ? static_cast<int>(rem) : kChunk;
@@ -300,6 +302,7 @@ __device__ __forceinline__ bool inverse_role(const PrepParams& p, uint8_t* smem,
 }
 
 // Loads, stores and tril(M).
+template <bool kSlice>
 __device__ __forceinline__ bool copy_role(const PrepParams& p, const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tg, uint8_t* smem,
                                           uint32_t sbase, uint32_t tmem, int n_it, int lane, volatile int* abort_flag) {
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
@@ -319,7 +322,7 @@ __device__ __forceinline__ bool copy_role(const PrepParams& p, const CUtensorMap
   };
   // decode an item and ask the L2 for its tiles, an item before they are loaded
   auto look_ahead = [&](int i) {
-    const Info f = decode(p, blockIdx.x + static_cast<unsigned>(i) * gridDim.x);
+    const Info f = decode<kSlice>(p, blockIdx.x + static_cast<unsigned>(i) * gridDim.x);
     infos[i & (kInfos - 1)] = f;
     if (i < 2) return;
     const int tc = static_cast<int>(f.t0);
@@ -448,6 +451,8 @@ __device__ __forceinline__ bool product_role(const PrepParams& p, uint8_t* smem,
   return ok;
 }
 
+// kSlice: a time slice of equal-length sequences (PrepParams::slice_*); the other form has fewer registers to hold
+template <bool kSlice>
 __global__ void __launch_bounds__(kThreads, 2)
 operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_g,
                 const PrepParams p) {
@@ -478,13 +483,13 @@ operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   bool ok = *abort_flag == 0;
-  grid_dependency_wait();
-  const unsigned items = static_cast<unsigned>(p.cu_seqlens != nullptr ? p.chunk_prefix[p.N] : p.total_chunks) * static_cast<unsigned>(p.H);
+  if (!kSlice || !p.beside) grid_dependency_wait();
+  const unsigned items = static_cast<unsigned>(p.cu_seqlens != nullptr ? p.chunk_prefix[p.N] : kSlice ? p.N * p.slice_chunks : p.total_chunks) * static_cast<unsigned>(p.H);
   const int n_it = !ok || blockIdx.x >= items ? 0 : static_cast<int>((items - blockIdx.x + gridDim.x - 1) / gridDim.x);
   if (warp < 8) {
     if (!element_role(p, smem, sbase, n_it, warp, lane, abort_flag)) ok = false;
   } else if (warp == 9) {
-    if (!copy_role(p, &tm_q, &tm_k, &tm_g, smem, sbase, tmem, n_it, lane, abort_flag)) ok = false;
+    if (!copy_role<kSlice>(p, &tm_q, &tm_k, &tm_g, smem, sbase, tmem, n_it, lane, abort_flag)) ok = false;
   } else if (warp == 11) {
     if (!product_role(p, smem, sbase, tmem, n_it, lane, abort_flag)) ok = false;
   } else {
@@ -497,6 +502,7 @@ operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem, kTmemCols);
   }
+  if (kSlice && p.beside && blockIdx.x == gridDim.x - 1) grid_dependency_wait();
 }
 
 }  // namespace operands
@@ -506,11 +512,14 @@ cudaError_t launch_operands(const PrepParams& p, bool one_per_cta, cudaStream_t 
   if (p.total_chunks == 0 || p.H == 0 || p.T_total == 0) return cudaSuccess;
   CUtensorMap tq, tk, tg;
   if (!make_map(&tq, p.q, p.T_total, p.H) || !make_map(&tk, p.k, p.T_total, p.H) || !make_map(&tg, p.g, p.T_total, p.H)) return cudaErrorInvalidValue;
-  static SmemOptIn opt_in;
-  cudaError_t e = opt_in.ensure(operands::operands_kernel, operands::kSmemBytes);
+  const bool slice = p.slice_chunks != p.seq_chunks;
+  auto kernel = slice ? operands::operands_kernel<true> : operands::operands_kernel<false>;
+  static SmemOptIn opt_in[2];
+  cudaError_t e = opt_in[slice].ensure(kernel, operands::kSmemBytes);
   if (e != cudaSuccess) return e;
-  const long long items = static_cast<long long>(p.total_chunks) * p.H, slots = one_per_cta ? items : 2ll * device_sm_count();
-  return launch_after(operands::operands_kernel, static_cast<unsigned>(items < slots ? items : slots), operands::kThreads, operands::kSmemBytes,
+  const long long items = (slice ? static_cast<long long>(p.N) * p.slice_chunks : static_cast<long long>(p.total_chunks)) * p.H;
+  const long long slots = one_per_cta ? items : p.beside ? p.beside : 2ll * device_sm_count();
+  return launch_after(kernel, static_cast<unsigned>(items < slots ? items : slots), operands::kThreads, operands::kSmemBytes,
                       stream, tq, tk, tg, p);
 }
 

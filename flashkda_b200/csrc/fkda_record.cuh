@@ -14,5 +14,6 @@
 
 namespace fkda {
 constexpr int kCrKN = 0, kCrQP = 8192, kCrKR = 16384, kCrTB = 24576, kCrMQK = 26624, kCrE = 28672, kCrBytes = 29184;
+static_assert(kCrBytes == kCompactRecBytes);
 static_assert(kCrBytes <= kRecBytes, "the workspace is sized for the larger record");
 }  // namespace fkda

@@ -285,7 +285,8 @@ __device__ __forceinline__ void store_state(const float (&S)[2][16][4], const Ch
 // are computed.  Equal lengths: walks in turn, every other round backwards; packed batches take the next longest
 // sequence from a device counter.  Otherwise one walk per CTA: a chunk costs 8 % less (2470 against 2680 cycles: the loop
 // has no registers to spare and every value kept for the stream is felt), a walk 3 us more.
-template <bool kSeg, bool kStream>
+// kSlice: one walk per CTA, a time slice of it (ScanParams::slice_*).
+template <bool kSeg, bool kStream, bool kSlice>
 __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constant__ CUtensorMap tm_v, const ScanParams p, const int walks) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           break;
         }
       }
-      const ChainView cv = chain_view<kSeg>(p, walk_index);
+      const ChainView cv = chain_view<kSeg, kSlice>(p, walk_index);
       load_state(S, cv, row0, lane);
       if (cv.nchunks == 0) {
         // (an empty run: its state is handed through)
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           ++cur.turn;
           const bool past = walk >= walks || walk < 0;
           ChainView cv{};
-          if (!past) cv = chain_view<kSeg>(p, walk);
+          if (!past) cv = chain_view<kSeg, kSlice>(p, walk);
           if (past || (kStream && cv.nchunks == 0 && p.N <= kOrderMax)) {
             // (The last round may be shorter than the grid: a CTA without a walk in it is done, there is no round after it.
             // Skipped sequences come last in the order by length.)
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     };
 
     int n_one = 0;                     // (one walk per CTA) its items
-    if (!kStream) n_one = chain_view<kSeg>(p, static_cast<int>(blockIdx.x)).nchunks;
+    if (!kStream) n_one = chain_view<kSeg, kSlice>(p, static_cast<int>(blockIdx.x)).nchunks;
     const bool work = kStream || n_one > 0;
     if (w == 1 && lane == 0 && ok && work)
       for (int k = 0; k < kStages && !cur.ended; ++k) copy();
@@ -553,9 +554,13 @@ cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream
   // in a CTA of its own are what the tighter chunk loop saves.)
   const int64_t sms = device_sm_count();
   const bool stream_form = p.seg_chunks == 0 && walks > sms && (p.T_total + static_cast<int64_t>(p.N) * (kChunk / 2)) / kChunk <= 24 * static_cast<int64_t>(p.N);
-  auto kernel = p.seg_chunks > 0 ? recur::recur_kernel<true, false> : stream_form ? recur::recur_kernel<false, true> : recur::recur_kernel<false, false>;
-  static SmemOptIn opt_in[3];
-  cudaError_t e = opt_in[p.seg_chunks > 0 ? 1 : stream_form ? 2 : 0].ensure(kernel, recur::kSmem);
+  // (a time slice is for fewer walks than SMs; its own form, as what it looks up costs the others 0.8 %)
+  void (*const kernels[4])(CUtensorMap, ScanParams, int) = {recur::recur_kernel<false, false, false>, recur::recur_kernel<true, false, false>,
+                                                            recur::recur_kernel<false, true, false>, recur::recur_kernel<false, false, true>};
+  const int form = p.seg_chunks > 0 ? 1 : p.slice_end > 0 ? 3 : stream_form ? 2 : 0;
+  const auto kernel = kernels[form];
+  static SmemOptIn opt_in[4];
+  cudaError_t e = opt_in[form].ensure(kernel, recur::kSmem);
   if (e != cudaSuccess) return e;
   return launch_after(kernel, static_cast<unsigned>(stream_form ? sms : walks), recur::kThreads, recur::kSmem, stream, tv, p, static_cast<int>(walks));
 }

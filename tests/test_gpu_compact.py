@@ -1,6 +1,6 @@
 """GPU: the forward pass over compact records at the sizes where its kernels can go wrong - around the 32-token chunk, its
 16-token halves and the rings of the copies; batches on either side of the lines between the forms of the recurrence (a chain
-split over four or two CTAs, one CTA per chain, the persistent form, runs); empty sequences; every state form."""
+split over four or two CTAs, one CTA per chain, two time slices, the persistent form, runs); empty sequences; every state form."""
 import pytest
 import torch
 
@@ -19,6 +19,8 @@ CASES = {
     "one_cta_no_state": Workload("c", H=100, B=1, T=48),
     "persistent_two_rounds": Workload("c", H=50, B=6, T=70, state_in="bf16", state_out="bf16"),
     "persistent_packed_with_empty": Workload("c", H=16, seq_lens=[0, 5, 33, 0, 64, 1, 31, 32, 100, 0, 2, 47], state_in="fp32", state_out="fp32"),
+    "two_slices": Workload("c", H=30, B=3, T=32 * 140 + 7, state_in="fp32", state_out="fp32"),
+    "two_slices_no_state": Workload("c", H=80, B=1, T=32 * 150),
     "runs": Workload("c", H=2, B=1, T=32 * 700 + 9, state_in="fp32", state_out="fp32", lower_bound=-1.0),
 }
 
