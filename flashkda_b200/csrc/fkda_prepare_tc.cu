@@ -5,7 +5,7 @@
 // two of eight warps, a one-warp inverse) and writes the same operand record as fkda_prepare.cu (fkda_common.cuh),
 // so every recurrence kernel consumes its output unchanged.  An item is one (32-token chunk, head) pair.  Two kernels:
 //
-//   prepare_pipe_kernel (default)   three CTAs per SM, each a loop over items with two operand buffers: eight element
+//   prepare_pipe_kernel             three CTAs per SM, each a loop over items with two operand buffers: eight element
 //                                   warps work on item i while a ninth warp does the serial part of item i - 1
 //   prepare_tc4_kernel              one CTA of eight warps per item, four CTAs per SM, phases separated by CTA-wide
 //                                   barriers; other resident CTAs fill the waits of the serial part
