@@ -17,8 +17,10 @@ OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libfkda.so")
 HOST_SRC = os.path.join(CSRC, "fkda_host.cpp")
 HOST_EXT = os.path.join(HERE, "_fkda_host" + sysconfig.get_config_var("EXT_SUFFIX"))
+HOST_STAMP = os.path.join(OBJ_DIR, "fkda_host.command")
+PUBLIC_HEADER = os.path.join(os.path.dirname(HERE), "include", "fkda.h")
 SOURCES = ["fkda_api.cu", "fkda_prepare.cu", "fkda_prepare_tc.cu", "fkda_scan.cu", "fkda_scan2.cu", "fkda_recur_split.cu", "fkda_recur.cu", "fkda_operands.cu", "fkda_scan_short.cu", "fkda_segscan.cu", "fkda_short16.cu", "fkda_step.cu", "fkda_refmode.cu", "fkda_aux.cu", "fkda_static_ws.cu"]
-HEADERS = [os.path.join(CSRC, "fkda_common.cuh"), os.path.join(CSRC, "fkda_tma.cuh"), os.path.join(CSRC, "fkda_elem.cuh"), os.path.join(CSRC, "fkda_record.cuh"), os.path.join(os.path.dirname(HERE), "include", "fkda.h"),
+HEADERS = [os.path.join(CSRC, "fkda_common.cuh"), os.path.join(CSRC, "fkda_tma.cuh"), os.path.join(CSRC, "fkda_elem.cuh"), os.path.join(CSRC, "fkda_record.cuh"), PUBLIC_HEADER,
            os.path.join(os.path.dirname(HERE), "include", "fkda_testing.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -40,21 +42,37 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def _build_host(force):
-    """The host path of `fwd` (checks, scratch memory, launch), a CPython extension on top of libfkda.so and torch."""
-    if not force and not _stale(HOST_EXT, [HOST_SRC, LIB] + HEADERS[4:5]):
-        return ""
+def _host_command():
     import torch
     tdir = os.path.dirname(os.path.abspath(torch.__file__))
     inc, libdir = os.path.join(tdir, "include"), os.path.join(tdir, "lib")
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"),
-           "-isystem", sysconfig.get_paths()["include"], HOST_SRC, "-o", HOST_EXT, LIB, "-Wl,-rpath,$ORIGIN", f"-L{libdir}",
-           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f'-DFKDA_TORCH_VERSION="{torch.__version__}"',
+            "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"),
+            "-isystem", sysconfig.get_paths()["include"], HOST_SRC, "-o", HOST_EXT, LIB, "-Wl,-rpath,$ORIGIN", f"-L{libdir}",
+            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
+def _host_stale(cmd):
+    """Whether the extension has to be built: its sources are newer, or it was built by another command (another torch,
+    another Python)."""
+    if _stale(HOST_EXT, [HOST_SRC, LIB, PUBLIC_HEADER]) or not os.path.exists(HOST_STAMP):
+        return True
+    with open(HOST_STAMP) as f:
+        return f.read() != "\n".join(cmd)
+
+
+def _build_host(force):
+    """The host path of `fwd` (checks, scratch memory, launch), a CPython extension on top of libfkda.so and torch."""
+    cmd = _host_command()
+    if not force and not _host_stale(cmd):
+        return ""
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    with open(HOST_STAMP, "w") as f:
+        f.write("\n".join(cmd))
     return r.stderr
 
 

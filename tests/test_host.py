@@ -133,6 +133,17 @@ def test_flag_constants_match_the_header():
     assert F.FLAG_SEGMENTS(5) == 5 << 8 and "FKDA_FLAG_SEGMENTS(n)" in text
 
 
+def test_the_host_extension_is_rebuilt_when_torch_changes(monkeypatch, tmp_path):
+    from flashkda_b200 import build as B
+    monkeypatch.setattr(B, "_stale", lambda target, deps: False)          # (sources older than the extension)
+    monkeypatch.setattr(B, "HOST_STAMP", str(tmp_path / "command"))
+    assert B._host_stale(B._host_command())                               # nobody knows how it was built
+    (tmp_path / "command").write_text("\n".join(B._host_command()))
+    assert not B._host_stale(B._host_command())
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    assert B._host_stale(B._host_command())
+
+
 def test_new_entry_points_reject_bad_arguments_without_a_gpu():
     L = ctypes.CDLL(F.lib_path())
     i64, ci = ctypes.c_int64, ctypes.c_int
