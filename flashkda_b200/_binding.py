@@ -7,6 +7,7 @@ into `out` / `final_state`, the call returns None and does not synchronise.
 """
 import ctypes
 import os
+import warnings
 
 import torch
 
@@ -89,16 +90,27 @@ def lib():
 
 
 def _load_host():
-    """The native host path (csrc/fkda_host.cpp), loaded with the library on the first call."""
+    """The native host path (csrc/fkda_host.cpp), loaded with the library on the first call.  It is compiled against one
+    torch and one Python; where it cannot be used the checks below do its work through ctypes: the same launches, some
+    20 us more per call."""
     global _fwd_fast
     lib()
     try:
         from . import _fkda_host
+        built_for = getattr(_fkda_host, "torch_version", "another version")
+        if built_for != torch.__version__:
+            raise ImportError(f"built for torch {built_for}, running with {torch.__version__}")
+        _fwd_fast = _fkda_host.fwd_fast
     except ImportError as e:
-        raise RuntimeError(f"the native host path of flash_kda cannot be loaded ({e}): build it with "
-                           "`python -m flashkda_b200.build`") from e
-    _fwd_fast = _fkda_host.fwd_fast
+        warnings.warn(f"the native host path of flash_kda is not used ({e}): every call takes some 20 us longer; "
+                      "`python -m flashkda_b200.build` rebuilds it", RuntimeWarning, stacklevel=3)
+        _fwd_fast = _decline
     return _fwd_fast
+
+
+def _decline(*args):
+    """Stands in for the native host path: not handled, take the Python checks."""
+    return False
 
 
 def last_error() -> str:

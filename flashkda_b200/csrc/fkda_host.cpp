@@ -124,4 +124,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fkda_host", nullptr, -1, methods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fkda_host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__fkda_host(void) {
+  PyObject* m = PyModule_Create(&module);
+  // the torch whose headers this was compiled against: another one may lay out a tensor differently (checked by the loader)
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", FKDA_TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}

@@ -513,6 +513,23 @@ def test_runs_on_the_current_stream():
     assert torch.equal(o0.view(torch.int16), o1.view(torch.int16)) and torch.equal(f0, f1)
 
 
+def test_without_the_native_host_path_the_call_gives_the_same_bits(monkeypatch):
+    """The plain call through the Python checks and ctypes: a decode step, a prefill, a packed batch."""
+    from flashkda_b200 import _binding
+    for w in (Workload("h1", H=4, B=2, T=1, state_in="fp32", state_out="fp32", seed=1), Workload("h2", H=4, B=2, T=100, state_in="bf16", state_out="bf16", seed=2),
+              Workload("h3", H=2, seq_lens=[1, 70, 33], state_out="fp32", seed=3)):
+        x = to_cuda(make_inputs(w))
+        got = []
+        for fast in (_binding._load_host(), _binding._decline):
+            monkeypatch.setattr(_binding, "_fwd_fast", fast)
+            out, fin = torch.full_like(x["v"], float("nan")), torch.full_like(x["final_state"], float("nan"))
+            flash_kda.fwd(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], out, x["A_log"], x["dt_bias"], x["lower_bound"],
+                          initial_state=x["initial_state"], final_state=fin, cu_seqlens=x["cu_seqlens"])
+            got.append((out, fin))
+        assert not torch.isnan(got[0][0].float()).any()
+        assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("name", golden_names())
 def test_reference_rounding_mode_reproduces_golden_vectors(name):
     """With FLAG_REFERENCE_ROUNDING the forward pass uses the reference's tile size, bf16 state and rounding points

@@ -80,6 +80,26 @@ def test_cpu_tensors_are_rejected_not_computed():
         flash_kda.fwd(**_cpu_args())
 
 
+@pytest.mark.parametrize("why", ["cannot be imported", "built for another torch"])
+def test_a_host_path_that_does_not_fit_leaves_the_python_checks(why, monkeypatch):
+    """The native host path belongs to one torch and one Python.  Where it does not load or was built for another torch the
+    call says so once and goes through the Python checks, whose message a CPU tensor then gets."""
+    import sys
+    import types
+
+    from flashkda_b200 import _binding
+    other = None if why == "cannot be imported" else types.SimpleNamespace(torch_version="0.0", fwd_fast=None)
+    monkeypatch.setattr(_binding, "_fwd_fast", None)
+    monkeypatch.setitem(sys.modules, "flashkda_b200._fkda_host", other)
+    monkeypatch.delattr(F, "_fkda_host", raising=False)
+    if other is not None:
+        monkeypatch.setattr(F, "_fkda_host", other, raising=False)
+    with pytest.warns(RuntimeWarning, match="native host path"), pytest.raises(RuntimeError, match="must be on CUDA"):
+        flash_kda.fwd(**_cpu_args())
+    with pytest.raises(RuntimeError, match="must be on CUDA"):
+        flash_kda.fwd(**_cpu_args())
+
+
 def test_c_abi_rejects_bad_params_without_a_gpu():
     from flashkda_b200._binding import FwdParams
     L = F.lib()
