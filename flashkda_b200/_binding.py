@@ -25,6 +25,7 @@ FLAG_REFERENCE_ROUNDING = 0x20
 FLAG_FUSED_ANY_T = 0x40
 FLAG_PREPARE_TCGEN05 = 0x80
 FLAG_PREPARE_MMA_SYNC = 0x20000
+FLAG_OPERANDS_PER_ITEM = 0x80000
 
 
 def FLAG_SEGMENTS(n: int) -> int:

@@ -364,7 +364,7 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   if (e != cudaSuccess) return cuda_fail(e, "scheduling launch");
   // Fewer chains than a quarter or half of the SMs: a chain's time is what counts, it is split over four or two CTAs.
   // (FKDA_FLAG_SCAN_NO_SEGMENTS: one CTA walks the whole chain.)
-  const bool whole = (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS) != 0, one_item = (p->flags & FKDA_FLAG_PREPARE_TCGEN05) != 0;
+  const bool whole = (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS) != 0, one_item = (p->flags & FKDA_FLAG_OPERANDS_PER_ITEM) != 0;
   const int rows = runs > 1 || whole ? 0 : chains * 4 <= sms ? 32 : chains * 2 <= sms ? 64 : 0;
   fkda::PrepParams q = prep_params(p, L);
   const int slice = p->cu_seqlens || runs > 1 || rows || whole || one_item ? 0 : plan_slice(chains, q.seq_chunks, sms);
@@ -510,7 +510,7 @@ int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
   // two-stage form: the whole walk on kernels that share nothing with the runs it is compared against.)
   const bool cross_check = p->cu_seqlens != nullptr && (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS);
   if (p->B * p->T > 0 && !cross_check && (p->flags & ~static_cast<uint32_t>(FKDA_FLAG_STATUS_UNREAD | FKDA_FLAG_SCAN_NO_SEGMENTS | FKDA_FLAG_NO_FUSED_SHORT |
-                                                            FKDA_FLAG_PREPARE_TCGEN05)) == 0)
+                                                            FKDA_FLAG_OPERANDS_PER_ITEM)) == 0)
     return do_compact(p, L, stream);
   rc = do_prepare(p, L, stream);
   if (rc != FKDA_OK) return rc;

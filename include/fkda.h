@@ -47,17 +47,21 @@ typedef enum fkda_state_dtype { FKDA_STATE_NONE = 0, FKDA_STATE_BF16 = 1, FKDA_S
  * complete forward pass, just slower than the two-kernel path beyond that; the flag exists so that tests can walk
  * many blocks with it). */
 #define FKDA_FLAG_FUSED_ANY_T 0x40u
-/* The token-parallel stage runs on the pipelined TMA + tcgen05 kernel (csrc/fkda_prepare_tc.cu: tile loads by TMA, the
- * intra-chunk products on tcgen05 with accumulators in tensor memory; three CTAs per SM, each a loop over (chunk, head)
- * items with the serial part of an item on a ninth warp while the other eight are on the next item).  This flag selects
- * the one-CTA-per-item form of that kernel instead (four CTAs per SM; at most 65535 sequences of at most 65535 chunks
- * each for equal lengths, else the call fails).  Same operand records. */
+/* Selects the two-stage form (fkda_prepare, fkda_scan) with its token-parallel stage on prepare_tc4_kernel, the
+ * one-CTA-per-item form of the pipelined TMA + tcgen05 kernel that fkda_prepare runs without a flag
+ * (csrc/fkda_prepare_tc.cu; same operand records; at most 65535 sequences of at most 65535 chunks each for equal lengths,
+ * else the call fails). */
 #define FKDA_FLAG_PREPARE_TCGEN05 0x80u
-/* The same stage on the earlier kernel (vectorised global loads, mma.sync products).  Same operand records. */
+/* The two-stage form with its token-parallel stage on prepare_kernel (vectorised global loads, mma.sync products).  Same
+ * operand records. */
 #define FKDA_FLAG_PREPARE_MMA_SYNC 0x20000u
 /* Nobody will read the status word of this call's workspace (scratch memory that the caller of the caller never sees): it
  * is left uninitialised where no kernel needs it, which saves a memset node in front of a call of a few microseconds. */
 #define FKDA_FLAG_STATUS_UNREAD 0x40000u
+/* The token-parallel stage of the default path (operands_kernel, csrc/fkda_operands.cu) with one CTA per (chunk, head) item,
+ * so that no CTA reuses a buffer, an accumulator or a barrier phase: slower, the same bits (verification aid; no effect on
+ * calls that take another path). */
+#define FKDA_FLAG_OPERANDS_PER_ITEM 0x80000u
 /* Cut every sequence of the batch into n (2..255) runs walked in parallel, whatever the planner would
  * choose; the workspace must then be sized with fkda_get_workspace_size_flags.  Together with FKDA_FLAG_SCAN_PLAIN or
  * FKDA_FLAG_SCAN_LOOKAHEAD both passes over the runs use that recurrence kernel (otherwise each pass picks the faster

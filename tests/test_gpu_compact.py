@@ -49,6 +49,36 @@ def test_compact_path_matches_the_recurrence(name):
     assert torch.equal(out.view(torch.int16), first.view(torch.int16)) and (fin is None or torch.equal(fin, first_fin))
 
 
+@pytest.mark.parametrize("case", ["fixed_many_items", "packed_many_sequences", "tails"])
+def test_operands_kernel_gives_the_bits_of_its_one_item_per_cta_form(case):
+    """A CTA of the token-parallel kernel reuses tile slots, operands, accumulators, staging and barrier phases over many items;
+    with one item per CTA nothing is reused.  A stale tile, a buffer overwritten too early or a lost phase would show in the
+    results of the call: up to 74 items per CTA, ragged sequences, repeated calls."""
+    if case == "fixed_many_items":
+        w = Workload("o1", H=32, B=4, T=5400, state_out="fp32", seed=21)
+    elif case == "packed_many_sequences":
+        import random
+        rnd = random.Random(5)
+        w = Workload("o2", H=8, seq_lens=[rnd.choice([0, 1, 7, 31, 32, 33, 63, 64, 65, 100, 257, 1000]) for _ in range(300)], state_out="fp32", seed=22)
+    else:
+        w = Workload("o3", H=5, B=7, T=32 * 40 + 3, state_in="bf16", state_out="bf16", seed=23)
+    x = make_inputs(w, device="cuda")
+
+    def call(flags):
+        out, fin = torch.full_like(x["v"], float("nan")), torch.full_like(x["final_state"], float("nan"))
+        ws = torch.empty(F.get_workspace_size(x["q"].shape[0] * x["q"].shape[1], w.H, w.N), dtype=torch.uint8, device="cuda")
+        F.fwd(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], out, x["A_log"], x["dt_bias"], x["lower_bound"],
+              initial_state=x["initial_state"], final_state=fin, cu_seqlens=x["cu_seqlens"], workspace=ws, flags=flags)
+        assert F.read_status(ws) == 0
+        return out, fin
+
+    out, fin = call(F.FLAG_OPERANDS_PER_ITEM)
+    assert not torch.isnan(out.float()).any() and not torch.isnan(fin.float()).any()
+    for _ in range(3):
+        o, f = call(0)
+        assert torch.equal(o.view(torch.int16), out.view(torch.int16)) and torch.equal(f, fin)
+
+
 @pytest.mark.parametrize("state", [None, "bf16", "fp32"])
 @pytest.mark.parametrize("B,T", [(1, 1), (3, 4), (2, 5), (5, 15), (5, 16), (3, 17), (2, 31), (2, 32), (400, 3)])
 def test_short_sequences_match_the_recurrence(B, T, state):

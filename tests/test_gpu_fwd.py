@@ -40,6 +40,22 @@ def run_gpu(x, fin_dtype, flags=0, check_status=True):
     return out.cpu(), None if fin is None else fin.cpu()
 
 
+def run_two_stage(x, fin_dtype, flags=0):
+    """The same call stage by stage: without flags on the pipelined token-parallel kernel and the recurrence that fkda_scan
+    chooses."""
+    xc = to_cuda(x)
+    out = torch.full_like(xc["v"], float("nan"))
+    B, T, H = x["q"].shape[:3]
+    N = x["cu_seqlens"].numel() - 1 if x["cu_seqlens"] is not None else B
+    fin = None if fin_dtype is None else torch.full((N, H, 128, 128), float("nan"), dtype=fin_dtype, device="cuda")
+    args = (xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"])
+    kw = dict(initial_state=xc["initial_state"], final_state=fin, cu_seqlens=xc["cu_seqlens"], flags=flags)
+    ws = F.prepare(*args, **kw)
+    F.scan(*args, workspace=ws, **kw)
+    assert F.read_status(ws) == 0
+    return out.cpu(), None if fin is None else fin.cpu()
+
+
 def check_against_f64(x, out, fin, tag, big_state=False):
     o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"],
                                      x["dt_bias"], x["lower_bound"], initial_state=x["initial_state"],
@@ -73,27 +89,38 @@ def test_golden_cases(name, flags):
     assert d_out <= (1e-2 if big else OUT_MAX_ABS) and d_st <= STATE_REL
 
 
-OTHER_PREPARE_KERNELS = {"mma_sync": F.FLAG_PREPARE_MMA_SYNC, "tcgen05_cta_per_item": F.FLAG_PREPARE_TCGEN05}
+TWO_STAGE_KERNELS = {"mma_sync": F.FLAG_PREPARE_MMA_SYNC, "tcgen05_cta_per_item": F.FLAG_PREPARE_TCGEN05, "tcgen05_pipelined": None}
 
 
-@pytest.mark.parametrize("kernel", list(OTHER_PREPARE_KERNELS))
+def run_on(kernel, x, fin_dtype):
+    """The two-stage form with its token-parallel stage on one of its three kernels: the pipelined one is fkda_prepare
+    without flags, the other two have a flag that fkda_fwd takes."""
+    flags = TWO_STAGE_KERNELS[kernel]
+    return run_two_stage(x, fin_dtype) if flags is None else run_gpu(x, fin_dtype, flags | F.FLAG_NO_FUSED_SHORT)
+
+
+@pytest.mark.parametrize("kernel", list(TWO_STAGE_KERNELS))
 @pytest.mark.parametrize("name", golden_names())
 def test_golden_cases_on_the_other_token_parallel_kernels(name, kernel):
-    """The token-parallel stage on the mma.sync kernel and on the one-CTA-per-item form of the TMA + tcgen05 kernel
-    (the default is the pipelined TMA + tcgen05 kernel): same golden cases."""
+    """The two-stage form on each of its three token-parallel kernels: same golden cases."""
     x, ref_out, ref_fin = load_golden(name)
     fin_dtype = None if ref_fin is None else ref_fin.dtype
-    out, fin = run_gpu(x, fin_dtype, OTHER_PREPARE_KERNELS[kernel] | F.FLAG_NO_FUSED_SHORT)
+    out, fin = run_on(kernel, x, fin_dtype)
     big = x["initial_state"] is not None and x["initial_state"].float().abs().max() > 100
     check_against_f64(x, out, fin, f"{name}[{kernel} prepare]", big_state=big)
 
 
 def test_the_two_tcgen05_kernels_write_the_same_bits():
-    """The pipelined kernel and the one-CTA-per-item kernel do the same arithmetic in the same order."""
+    """The pipelined kernel and the one-CTA-per-item kernel do the same arithmetic in the same order; and the flag that
+    selects the latter selects the two-stage form (the default path rounds elsewhere: its bits are others)."""
     x = make_inputs(Workload("req", H=4, B=2, T=300, state_in="fp32", state_out="fp32", seed=65))
-    o0, s0 = run_gpu(x, torch.float32)
-    o1, s1 = run_gpu(x, torch.float32, F.FLAG_PREPARE_TCGEN05)
+    o0, s0 = run_on("tcgen05_pipelined", x, torch.float32)
+    o1, s1 = run_on("tcgen05_cta_per_item", x, torch.float32)
     assert torch.equal(o0.view(torch.int16), o1.view(torch.int16)) and torch.equal(s0, s1)
+    o2, s2 = run_two_stage(x, torch.float32, F.FLAG_PREPARE_TCGEN05)
+    assert torch.equal(o0.view(torch.int16), o2.view(torch.int16)) and torch.equal(s0, s2)
+    o3, _ = run_gpu(x, torch.float32)
+    assert not torch.equal(o0.view(torch.int16), o3.view(torch.int16)), "the flag does not change the path"
 
 
 @pytest.mark.parametrize("kernel", ["tcgen05_pipelined", "tcgen05_cta_per_item"])
@@ -102,7 +129,6 @@ def test_tma_tcgen05_token_parallel_kernel_shapes(case, kernel):
     """Shapes that stress the TMA + tcgen05 kernels: ragged last chunks, many short sequences (items of every
     length), more items than one pass of the CTAs holds, and repeated calls that must be bit-reproducible; each
     against the fp64 oracle and against the mma.sync kernel."""
-    tc_flag = {"tcgen05_pipelined": 0, "tcgen05_cta_per_item": F.FLAG_PREPARE_TCGEN05}[kernel]
     if case == "fixed_tails":
         w = Workload("tc1", H=3, B=5, T=32 * 3 + 17, state_in="fp32", state_out="fp32", state_std=0.5, seed=61)
     elif case == "varlen_ragged":
@@ -113,13 +139,13 @@ def test_tma_tcgen05_token_parallel_kernel_shapes(case, kernel):
         w = Workload("tc4", H=16, B=2, T=1024, state_in="fp32", state_out="fp32", seed=64)
     x = make_inputs(w)
     dt = torch.bfloat16 if w.state_in == "bf16" else torch.float32
-    out, fin = run_gpu(x, dt, tc_flag)
+    out, fin = run_on(kernel, x, dt)
     check_against_f64(x, out, fin, f"{kernel} prepare, {case}")
     o0, s0 = run_gpu(x, dt, F.FLAG_PREPARE_MMA_SYNC)
     assert max_abs(out, o0) <= 1e-2 and rel_fro(fin, s0) <= (2e-2 if dt == torch.bfloat16 else 5e-3)
     if case == "long_repeat":
         for _ in range(4):
-            o2, s2 = run_gpu(x, dt, tc_flag)
+            o2, s2 = run_on(kernel, x, dt)
             assert torch.equal(o2.view(torch.int16), out.view(torch.int16)) and torch.equal(s2, fin)
 
 

@@ -87,6 +87,7 @@ FORMS = {
     "simt": F.FLAG_SCAN_SIMT,
     "mma_sync_prepare": F.FLAG_PREPARE_MMA_SYNC,
     "tcgen05_cta_per_item_prepare": F.FLAG_PREPARE_TCGEN05,
+    "operands_per_item": F.FLAG_OPERANDS_PER_ITEM,
     "reference_rounding": F.FLAG_REFERENCE_ROUNDING,
 }
 
