@@ -136,8 +136,8 @@ def get_workspace_size(T_total: int, H: int, N: int = 1, flags: int = 0) -> int:
 
 
 def plan_segments(chains: int, chunks_per_sequence: int):
-    """(runs per sequence, chunks per run) the recurrence uses for a batch of `chains` chains of that many chunks (varlen: the
-    average sequence length; the run length then follows the longest sequence); (1, 0) = whole sequences."""
+    """(runs per sequence, chunks per run) the recurrence uses for a batch of `chains` chains of that many chunks (varlen: a
+    third more than the average; the run length then follows the longest sequence); (1, 0) = whole sequences."""
     a, b = ctypes.c_int(0), ctypes.c_int(0)
     _check(lib().fkda_plan_segments(chains, chunks_per_sequence, ctypes.byref(a), ctypes.byref(b)))
     return a.value, b.value

@@ -75,43 +75,85 @@ struct Layout {
   int64_t total_bytes;
 };
 
+// How many runs to cut each sequence of a batch into (1 = walk whole sequences), at most `most` of them, and their length in
+// chunks.  Pass 1 holds chains * (2 n - 3) CTAs and pass 2 chains * (n - 1), both walking ceil(chunks / n) chunks.  The one
+// planner: the workspace size, the launch and fkda_plan_segments ask here.  Its costs are those of the default path's kernels,
+// in hundredths of a microsecond, fitted to 124 calls of 1 to 40 heads and 129 to 4096 chunks, each cut in up to thirteen ways
+// (1.1 % off on average, 4.6 % at most): a chunk step of a chain split over four or two CTAs (fkda_recur_split.cu) or in one
+// CTA (fkda_recur.cu), the latter with and without outputs; what the two passes cost beside their steps, and every round of
+// CTAs after the first; the chaining of the maps per run and round of its CTAs.  (The two-stage form walks its runs by the same
+// plan.)  With more chains than a third of the SMs pass 1 alone would take more than one round; below 48 chunks the fixed costs
+// are all there is.
+int plan_runs(int64_t chains, int64_t chunks, int64_t most, int sms, int* len) {
+  constexpr int64_t kQuad = 58, kHalf = 87, kOne = 132, kQuiet = 88, kPasses = 1100, kRound = 640, kChaining = 165, kMostRuns = 160;
+  *len = 0;
+  if (chains <= 0 || chains * 3 > sms || chunks < 48) return 1;
+  const int64_t whole = (chains * 4 <= sms ? kQuad : kHalf) * chunks;
+  auto rounds = [&](int64_t ctas) { return (ctas + sms - 1) / sms; };
+  int64_t best = whole;
+  int best_n = 1;
+  for (int64_t n = 3; n <= (most < kMostRuns ? most : kMostRuns); ++n) {
+    const int64_t l = (chunks + n - 1) / n;
+    if (l < 8) break;
+    if ((n - 1) * l >= chunks) continue;       // the last run would be empty
+    const int64_t r1 = rounds(chains * (2 * n - 3)), r2 = rounds(chains * (n - 1));
+    // run 0, the first CTA of a chain, has outputs: with the last chain's in the last round that round is a slow one
+    const bool slow_end = (chains - 1) * (2 * n - 3) >= (r1 - 1) * sms;
+    const int64_t pass1 = (slow_end ? (r1 - 1) * kQuiet + kOne : r1 * kQuiet) * l, pass2 = r2 * kOne * l;
+    const int64_t cost = pass1 + pass2 + kPasses + (r1 + r2 - 2) * kRound + kChaining * (n - 2) * rounds(chains * 16);
+    if (cost < best) {
+      best = cost;
+      best_n = static_cast<int>(n);
+    }
+  }
+  if (best_n == 1 || best * 100 > whole * 97) return 1;       // (closer than the fit)
+  *len = static_cast<int>((chunks + best_n - 1) / best_n);
+  return best_n;
+}
+
 // Runs per sequence under `flags`: forced by FKDA_FLAG_SEGMENTS(n), switched off by the
 // kernel-selection flags, else planned from the sizes.
-int segments_for(int64_t chains, int64_t chunks_per_seq, int64_t flags, int* seg_chunks) {
+int segments_for(int64_t chains, int64_t chunks_per_seq, int64_t planned_chunks, int64_t most, int64_t flags, int* seg_chunks) {
   *seg_chunks = 0;
   if (flags & (FKDA_FLAG_SCAN_SIMT | FKDA_FLAG_SCAN_NO_SEGMENTS)) return 1;
   const int64_t forced = (flags >> 8) & 0xff;
   if ((flags & FKDA_FLAG_SCAN_PLAIN) && forced < 2) return 1;
   if (forced >= 2) {
-    if (chunks_per_seq < forced) return 1;
+    if (chunks_per_seq < forced || forced > most) return 1;
     *seg_chunks = static_cast<int>((chunks_per_seq + forced - 1) / forced);
     return static_cast<int>(forced);
   }
   if (flags & FKDA_FLAG_SCAN_LOOKAHEAD) return 1;
   // The planner tries up to 158 run counts with a dozen 64-bit divisions each (several microseconds), and a call asks
-  // twice; it is a pure function of these three numbers, so each thread keeps its last answer.
-  thread_local struct { int64_t chains = -1, chunks = -1; int sms = -1, n = 1, len = 0; } last;
+  // twice; it is a pure function of these four numbers, so each thread keeps its last answer.
+  thread_local struct { int64_t chains = -1, chunks = -1, most = -1; int sms = -1, n = 1, len = 0; } last;
   const int sms = fkda::device_sm_count();
-  if (last.chains != chains || last.chunks != chunks_per_seq || last.sms != sms) {
-    last.n = fkda::plan_segments(chains, chunks_per_seq, &last.len, sms);
+  if (last.chains != chains || last.chunks != planned_chunks || last.most != most || last.sms != sms) {
+    last.n = plan_runs(chains, planned_chunks, most, sms, &last.len);
     last.chains = chains;
-    last.chunks = chunks_per_seq;
+    last.chunks = planned_chunks;
+    last.most = most;
     last.sms = sms;
   }
   *seg_chunks = last.len;
   return last.n;
 }
 
-// `varlen` < 0: size for whichever mode needs more (the upper bound T_total/32 + N covers both).
-bool make_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t flags, Layout* L) {
+constexpr int64_t kAnyRoom = INT64_MAX;
+
+// `varlen` < 0: size for whichever mode needs more (the upper bound T_total/32 + N covers both).  `room`: no more runs are
+// planned than fit a workspace of so many bytes.
+bool make_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t flags, Layout* L, int64_t room = kAnyRoom) {
   if (T_total < 0 || H <= 0 || N <= 0) return false;
   int64_t chunks;
   if (varlen == 0) chunks = N * ((T_per_seq + fkda::kChunk - 1) / fkda::kChunk);
   else chunks = T_total / fkda::kChunk + N;
+  bool fixed = varlen == 0;
   if (varlen < 0) {
     int64_t fixed_ub = (T_total + fkda::kChunk - 1) / fkda::kChunk + N;
     chunks = fixed_ub > chunks ? fixed_ub : chunks;
-    if (T_total % N == 0) T_per_seq = T_total / N; else varlen = 1;   // a fixed-length call has T_total = N T
+    fixed = T_total % N == 0;                                         // a fixed-length call has T_total = N T
+    if (fixed) T_per_seq = T_total / N;
   }
   L->prefix_off = fkda::kWsHeaderBytes;
   int64_t prefix_bytes = ((2 * N + 1) * 4 + 255) / 256 * 256;   // chunk prefix [N+1] followed by the chain order [N]
@@ -121,11 +163,21 @@ bool make_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_pe
   L->n_segs = 1;
   L->seg_chunks = 0;
   if (N * H <= 0x7fffffffLL) {
-    // Fixed-length: planned from the sequence length.  Varlen: the lengths are on the device, so the number of runs is
-    // planned for sequences of the average length and the run length follows the longest sequence, on the device.
-    // (A size query, varlen < 0, gets the same plan either way: both use T_total / N.)
-    const int64_t per_seq = varlen > 0 ? (T_total / N + fkda::kChunk - 1) / fkda::kChunk : (T_per_seq + fkda::kChunk - 1) / fkda::kChunk;
-    L->n_segs = segments_for(N * H, per_seq, flags, &L->seg_chunks);
+    const int64_t run_bytes = N * H * 3 * fkda::kSegSlotFloats * 4;
+    const int64_t most = room == kAnyRoom ? room : room > L->seg_off ? (room - L->seg_off) / run_bytes : 0;
+    auto chunks_of = [](int64_t tokens) { return (tokens + fkda::kChunk - 1) / fkda::kChunk; };
+    // Fixed-length: planned from the sequence length.  Packed batches: the lengths are on the device.  The longest sequence sets
+    // the time, one a third above the average is planned for, and the run length follows the longest one on the device.  (A
+    // size query, varlen < 0, has room for either plan.)
+    if (fixed) L->n_segs = segments_for(N * H, chunks_of(T_per_seq), chunks_of(T_per_seq), most, flags, &L->seg_chunks);
+    if (varlen != 0) {
+      int len = 0;
+      const int n = segments_for(N * H, chunks_of(T_total / N), chunks_of(N > 1 ? T_total * 4 / (N * 3) : T_total), most, flags, &len);
+      if (n > L->n_segs) {
+        L->n_segs = n;
+        L->seg_chunks = len;
+      }
+    }
   }
   L->seg_bytes = L->n_segs > 1 ? N * H * L->n_segs * 3 * fkda::kSegSlotFloats * 4 : 0;
   L->total_bytes = L->seg_off + L->seg_bytes;
@@ -140,8 +192,8 @@ bool fused_short(const fkda_fwd_params* p) {
   return p->cu_seqlens == nullptr && p->T > 0 && (any_t || (p->T <= fkda::kFusedMaxT && (p->flags & 0xff57u) == 0));
 }
 
-// `whole_call`: the operator (fkda_fwd) rather than one of its stages
-int validate(const fkda_fwd_params* p, Layout* L, bool whole_call = false) {
+// `whole_call`: the operator (fkda_fwd) rather than one of its stages; `fit`: its plan keeps to the given workspace
+int validate(const fkda_fwd_params* p, Layout* L, bool whole_call = false, bool fit = false) {
   if (!p) return fail(FKDA_ERR_INVALID_ARGUMENT, "params is NULL");
   if (!p->q || !p->k || !p->v || !p->g || !p->beta || !p->out) return fail(FKDA_ERR_INVALID_ARGUMENT, "q, k, v, g, beta and out must be non-NULL");
   if (!p->A_log || !p->dt_bias) return fail(FKDA_ERR_INVALID_ARGUMENT, "A_log and dt_bias must be non-NULL");
@@ -163,7 +215,7 @@ int validate(const fkda_fwd_params* p, Layout* L, bool whole_call = false) {
   const int64_t T_total = p->B * p->T;
   if (p->H > 65535) return fail(FKDA_ERR_INVALID_ARGUMENT, "H must be at most 65535");
   if (p->N * p->H > 0x7fffffffLL) return fail(FKDA_ERR_INVALID_ARGUMENT, "N*H exceeds 2^31-1 chains");
-  if (!make_layout(T_total, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
+  if (!make_layout(T_total, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, L, fit ? p->workspace_bytes : kAnyRoom)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
   if (L->chunks_per_head * p->H > 0x7fffffffLL) return fail(FKDA_ERR_INVALID_ARGUMENT, "too many (chunk, head) pairs for one call");
   if (!p->workspace) return fail(FKDA_ERR_INVALID_ARGUMENT, "workspace is NULL");
   if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return fail(FKDA_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
@@ -292,32 +344,6 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   return FKDA_OK;
 }
 
-// Runs per sequence for the walk over compact records (1: whole sequences), at most `most` of them, and their length.
-// Hundredths of a microsecond per chunk step, measured: a chain split over four or two CTAs (fkda_recur_split.cu) or in one
-// CTA (fkda_recur.cu), the latter with and without outputs; a pass costs about 8 us beside its steps, the chaining of
-// the maps 1.45 us per run and wave of its CTAs.
-int plan_runs(int64_t chains, int64_t chunks, int most, int sms, int* len) {
-  constexpr int64_t kQuad = 58, kHalf = 90, kOne = 132, kQuiet = 95;
-  const int64_t whole = (chains * 4 <= sms ? kQuad : chains * 2 <= sms ? kHalf : kOne * ((chains + sms - 1) / sms)) * chunks;
-  int64_t best = whole;
-  int best_n = 1;
-  for (int64_t n = 3; n <= most; ++n) {
-    const int64_t l = (chunks + n - 1) / n;
-    if (l < 8) break;
-    if ((n - 1) * l >= chunks) continue;       // the last run would be empty
-    const int64_t pass1 = (chains * (2 * n - 3) + sms - 1) / sms * kQuiet * l, run0 = kOne * l;
-    const int64_t pass2 = (chains * (n - 1) + sms - 1) / sms * kOne * l;
-    const int64_t cost = (pass1 > run0 ? pass1 : run0) + pass2 + 1600 + 145 * (n - 2) * ((chains * 16 + sms - 1) / sms);
-    if (cost < best) {
-      best = cost;
-      best_n = static_cast<int>(n);
-    }
-  }
-  if (best * 10 > whole * 9) best_n = 1;
-  *len = static_cast<int>((chunks + best_n - 1) / best_n);
-  return best_n;
-}
-
 // Where fewer chains than SMs have a CTA each, the SMs beyond them can work out operands meanwhile.  The call is then cut in two
 // time slices, and the second one's operands are computed beside the first one's recurrence, by kSliceWaves waves of two
 // CTAs on each free SM that end with it.  A chunk of the recurrence takes 1.32 us; a CTA of the token-parallel stage 3.7 us per item
@@ -340,22 +366,7 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   int* status = reinterpret_cast<int*>(ws);
   const int64_t chains = p->N * p->H, T_total = p->B * p->T;
   const int sms = fkda::device_sm_count();
-  int runs = 1, run_len = 0;
-  if (L.n_segs > 1) {
-    thread_local struct { int64_t chains = -1, chunks = -1; int most = 0, sms = 0, n = 1, len = 0; } last;
-    // (packed batches: the longest sequence sets the time either way; its length is on the device, a third above the average is assumed)
-    const int64_t tokens = p->cu_seqlens ? (p->N > 1 ? T_total * 4 / (p->N * 3) : T_total) : p->T;
-    const int64_t chunks = (tokens + fkda::kChunk - 1) / fkda::kChunk;
-    if (last.chains != chains || last.chunks != chunks || last.most != L.n_segs || last.sms != sms) {
-      last.n = plan_runs(chains, chunks, L.n_segs, sms, &last.len);
-      last.chains = chains;
-      last.chunks = chunks;
-      last.most = L.n_segs;
-      last.sms = sms;
-    }
-    runs = last.n;
-    run_len = last.len;
-  }
+  const int runs = L.n_segs, run_len = L.seg_chunks;
   cudaError_t e = cudaSuccess;
   if (p->cu_seqlens)
     e = fkda::launch_chunk_prefix(p->cu_seqlens, static_cast<int>(p->N), T_total, static_cast<int>(p->H), runs, true,
@@ -407,71 +418,9 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   return FKDA_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-int fkda_get_workspace_size_flags(int64_t T_total, int64_t H, int64_t N, int64_t flags, int64_t* bytes) {
+int do_fwd(const fkda_fwd_params* p, void* cuda_stream, bool fit) {
   Layout L;
-  if (!bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "bytes is NULL");
-  if (!make_layout(T_total, H, N, -1, 0, flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "T_total >= 0, H > 0 and N > 0 required");
-  *bytes = L.total_bytes;
-  return FKDA_OK;
-}
-
-int fkda_get_workspace_size(int64_t T_total, int64_t H, int64_t N, int64_t* bytes) {
-  return fkda_get_workspace_size_flags(T_total, H, N, 0, bytes);
-}
-
-int fkda_plan_segments(int64_t chains, int64_t chunks_per_sequence, int* segments, int* chunks_per_segment) {
-  if (!segments || !chunks_per_segment) return fail(FKDA_ERR_INVALID_ARGUMENT, "NULL pointer");
-  *segments = fkda::plan_segments(chains, chunks_per_sequence, chunks_per_segment, fkda::device_sm_count());
-  return FKDA_OK;
-}
-
-int fkda_workspace_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t* records_offset,
-                          int64_t* record_bytes, int64_t* chunks_per_head) {
-  Layout L;
-  if (!make_layout(T_total, H, N, varlen ? 1 : 0, T_per_seq, 0, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
-  if (records_offset) *records_offset = L.records_off;
-  if (record_bytes) *record_bytes = fkda::kRecBytes;
-  if (chunks_per_head) *chunks_per_head = L.chunks_per_head;
-  return FKDA_OK;
-}
-
-int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t flags, int64_t* bytes) {
-  Layout L;
-  if (!bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "bytes is NULL");
-  if (!make_layout(T_total, H, N, varlen ? 1 : 0, T_per_seq, flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
-  *bytes = L.total_bytes;
-  return FKDA_OK;
-}
-
-int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes) {
-  Layout L;
-  if (!p || !bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "NULL pointer");
-  if (!make_layout(p->B * p->T, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
-  *bytes = (p->flags & FKDA_FLAG_STATUS_UNREAD) && fused_short(p) ? fkda::kWsHeaderBytes : L.total_bytes;
-  return FKDA_OK;
-}
-
-int fkda_prepare(const fkda_fwd_params* p, void* cuda_stream) {
-  Layout L;
-  int rc = validate(p, &L);
-  if (rc != FKDA_OK) return rc;
-  return do_prepare(p, L, static_cast<cudaStream_t>(cuda_stream));
-}
-
-int fkda_scan(const fkda_fwd_params* p, void* cuda_stream) {
-  Layout L;
-  int rc = validate(p, &L);
-  if (rc != FKDA_OK) return rc;
-  return do_scan(p, L, static_cast<cudaStream_t>(cuda_stream));
-}
-
-int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
-  Layout L;
-  int rc = validate(p, &L, true);
+  int rc = validate(p, &L, true, fit);
   if (rc != FKDA_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   if (p->flags & FKDA_FLAG_REFERENCE_ROUNDING) {
@@ -516,6 +465,74 @@ int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) {
   if (rc != FKDA_OK) return rc;
   return do_scan(p, L, stream);
 }
+
+}  // namespace
+
+namespace fkda {
+int fwd_within(const fkda_fwd_params* p, void* cuda_stream) { return do_fwd(p, cuda_stream, true); }
+}  // namespace fkda
+
+extern "C" {
+
+int fkda_get_workspace_size_flags(int64_t T_total, int64_t H, int64_t N, int64_t flags, int64_t* bytes) {
+  Layout L;
+  if (!bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "bytes is NULL");
+  if (!make_layout(T_total, H, N, -1, 0, flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "T_total >= 0, H > 0 and N > 0 required");
+  *bytes = L.total_bytes;
+  return FKDA_OK;
+}
+
+int fkda_get_workspace_size(int64_t T_total, int64_t H, int64_t N, int64_t* bytes) {
+  return fkda_get_workspace_size_flags(T_total, H, N, 0, bytes);
+}
+
+int fkda_plan_segments(int64_t chains, int64_t chunks_per_sequence, int* segments, int* chunks_per_segment) {
+  if (!segments || !chunks_per_segment) return fail(FKDA_ERR_INVALID_ARGUMENT, "NULL pointer");
+  *segments = plan_runs(chains, chunks_per_sequence, kAnyRoom, fkda::device_sm_count(), chunks_per_segment);
+  return FKDA_OK;
+}
+
+int fkda_workspace_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t* records_offset,
+                          int64_t* record_bytes, int64_t* chunks_per_head) {
+  Layout L;
+  if (!make_layout(T_total, H, N, varlen ? 1 : 0, T_per_seq, 0, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
+  if (records_offset) *records_offset = L.records_off;
+  if (record_bytes) *record_bytes = fkda::kRecBytes;
+  if (chunks_per_head) *chunks_per_head = L.chunks_per_head;
+  return FKDA_OK;
+}
+
+int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_per_seq, int64_t flags, int64_t* bytes) {
+  Layout L;
+  if (!bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "bytes is NULL");
+  if (!make_layout(T_total, H, N, varlen ? 1 : 0, T_per_seq, flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
+  *bytes = L.total_bytes;
+  return FKDA_OK;
+}
+
+int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes) {
+  Layout L;
+  if (!p || !bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "NULL pointer");
+  if (!make_layout(p->B * p->T, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
+  *bytes = (p->flags & FKDA_FLAG_STATUS_UNREAD) && fused_short(p) ? fkda::kWsHeaderBytes : L.total_bytes;
+  return FKDA_OK;
+}
+
+int fkda_prepare(const fkda_fwd_params* p, void* cuda_stream) {
+  Layout L;
+  int rc = validate(p, &L);
+  if (rc != FKDA_OK) return rc;
+  return do_prepare(p, L, static_cast<cudaStream_t>(cuda_stream));
+}
+
+int fkda_scan(const fkda_fwd_params* p, void* cuda_stream) {
+  Layout L;
+  int rc = validate(p, &L);
+  if (rc != FKDA_OK) return rc;
+  return do_scan(p, L, static_cast<cudaStream_t>(cuda_stream));
+}
+
+int fkda_fwd(const fkda_fwd_params* p, void* cuda_stream) { return do_fwd(p, cuda_stream, false); }
 
 int fkda_prologue(const void* q, const void* k, const void* g, const void* beta, const float* A_log, const float* dt_bias,
                   float lower_bound, int64_t T_total, int64_t H, void* qn, void* kn, float* gate, float* beta_act,

@@ -522,42 +522,6 @@ inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned t
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
-// Duration of a pass of `ctas` CTAs in hundredths of one chunk step of the look-ahead kernel, per chunk of run length,
-// and the kernel that achieves it: the look-ahead kernel runs one CTA per SM, the compact kernel two at 1.58 times the
-// step (measured).
-inline int64_t pass_cost_x100(int64_t ctas, bool* compact, int64_t sms, int64_t la_step_x100 = 100) {
-  const int64_t la = (ctas + sms - 1) / sms * la_step_x100, co = (ctas + 2 * sms - 1) / (2 * sms) * 158;
-  *compact = co < la;
-  return co < la ? co : la;
-}
-
-// How many runs to cut each sequence of a batch into (1 = walk whole sequences), and their length in chunks (varlen
-// batches: called with the average sequence length; the run length is then set on the device from the longest one).  Pass 1 holds chains * (2 n - 3) CTAs and pass 2 chains * (n - 1), both walking ceil(chunks / n) chunks, each
-// on whichever recurrence kernel gets that many CTAs through faster; chaining the maps costs about three chunk steps
-// per run.  The plan is a pure function of the sizes and the device's SM count, so that the workspace size and the
-// launch agree.
-inline int plan_segments(int64_t chains, int64_t chunks, int* seg_chunks, int64_t sms) {
-  *seg_chunks = 0;
-  if (chains <= 0 || chains * 3 > sms || chunks < 48) return 1;
-  bool c;
-  const int64_t whole = pass_cost_x100(chains, &c, sms) * chunks;
-  int64_t best = whole, best_n = 1;
-  for (int64_t n = 3; n <= 160; ++n) {
-    const int64_t len = (chunks + n - 1) / n;
-    if (len < 8) break;
-    if ((n - 1) * len >= chunks) continue;       // the last run would be empty
-    // (a run walks its chunks about a tenth more slowly than a whole sequence; each pass costs about ten chunk steps of
-    // launch, set-up and state traffic; a step of the map chaining about two and a half, per wave of its chains x 8 CTAs)
-    const int64_t cmb_waves = (chains * 8 + sms - 1) / sms;
-    const int64_t cost = (pass_cost_x100(chains * (2 * n - 3), &c, sms, 110) + pass_cost_x100(chains * (n - 1), &c, sms, 110)) * len + 100 * 20 +
-                         250 * (n - 2) * cmb_waves;
-    if (cost < best) { best = cost; best_n = n; }
-  }
-  if (best_n == 1 || best * 4 > whole * 3) return 1;
-  *seg_chunks = static_cast<int>((chunks + best_n - 1) / best_n);
-  return static_cast<int>(best_n);
-}
-
 // What one CTA of a recurrence kernel walks: a whole (sequence, head) chain, or, in the segment-parallel form (kSeg), one
 // run of it in one of three variants - 0: the recurrence proper; 1: offset half of the run's affine map (zero state in, no
 // output); 2: transition half (identity in, u' taken as zero, no output).  Pass 1 holds, per chain, run 0 (variant 0)

@@ -18,6 +18,12 @@ cudaError_t launch_scan(const ScanParams& p, cudaStream_t stream);
 
 namespace {
 
+// Two-stage form: whether a pass of `ctas` CTAs takes less time on the compact kernel (two CTAs per SM at 1.58 times the
+// chunk step, measured) than on the look-ahead kernel (one).
+bool compact_is_faster(int64_t ctas, int64_t sms) {
+  return (ctas + 2 * sms - 1) / (2 * sms) * 158 < (ctas + sms - 1) / sms * 100;
+}
+
 constexpr int kCmbRows = 8;                               // state rows per CTA: the n of an mma, whose m are columns of the map
 constexpr int kMapStride = kSegMapStride;                 // floats per map row, in its slot and here (fragments: bank 8 t + g)
 constexpr int kMapStg = kD * kMapStride * 4;
@@ -181,12 +187,9 @@ cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_ch
   p.seg_chunks = seg_chunks;
   p.n_segs = n_segs;
   p.seg_buf = seg_buf;
-  // either recurrence kernel can walk the runs: whichever gets the pass's CTAs through in less time
   const int64_t chains = static_cast<int64_t>(p.N) * p.H;
-  bool compact1, compact2;
   const int sms = device_sm_count();
-  pass_cost_x100(chains * (2 * n_segs - 3), &compact1, sms);
-  pass_cost_x100(chains * (n_segs - 1), &compact2, sms);
+  bool compact1 = compact_is_faster(chains * (2 * n_segs - 3), sms), compact2 = compact_is_faster(chains * (n_segs - 1), sms);
   if (kernel_choice) compact1 = compact2 = kernel_choice == 1;   // forced: 1 compact, 2 look-ahead
   p.seg_pass = 1;
   cudaError_t e = v != nullptr ? launch_recur(p, v, stream) : compact1 ? launch_scan(p, stream) : launch_scan2(p, stream);

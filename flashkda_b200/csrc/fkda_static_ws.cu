@@ -28,6 +28,10 @@
 #include "../../include/fkda.h"
 #include "fkda_common.cuh"
 
+namespace fkda {
+int fwd_within(const fkda_fwd_params* p, void* cuda_stream);      // fkda_fwd with a plan that keeps to the workspace
+}
+
 namespace {
 
 constexpr int64_t kStaticWsBytes = 64ll << 20;
@@ -91,16 +95,8 @@ int fkda_fwd_static_ws(const fkda_fwd_params* p, void* cuda_stream) {
   fkda_fwd_params q = *p;
   q.workspace = ws;
   q.workspace_bytes = kStaticWsBytes;
-  {
-    // few long chains would be cut into runs, which needs room beyond the records: where that room is missing the
-    // sequences are walked whole instead (slower, same result) rather than refused.  Decided on this call's exact
-    // layout, not on the upper bound that a size query gives.
-    int64_t exact = 0;
-    if (fkda_workspace_bytes_exact(p->B * p->T, p->H, p->N, p->cu_seqlens != nullptr, p->T, p->flags, &exact) == FKDA_OK &&
-        exact > kStaticWsBytes)
-      q.flags |= FKDA_FLAG_SCAN_NO_SEGMENTS;
-  }
-  const int rc = fkda_fwd(&q, cuda_stream);
+  // (few long chains are cut into runs, which needs room beyond the records: into no more than there is room for)
+  const int rc = fkda::fwd_within(&q, cuda_stream);
   if (rc != FKDA_OK) snprintf(g_msg, sizeof(g_msg), "%s", fkda_last_error());
   return rc;
 }

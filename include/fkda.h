@@ -111,10 +111,12 @@ int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen
  * `workspace_bytes` and the data pointers other than cu_seqlens are not looked at). */
 int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes);
 
-/* The planner of the segment-parallel recurrence: into how many runs (1 = none) a batch with `chains`
- * = N*H chains of `chunks_per_sequence` 32-token chunks is cut, and the run length in chunks.  (For a varlen batch the call plans with the average sequence length and
- * sets the run length on the device from the longest sequence.)  The reference has no
- * counterpart: its recurrence kernel always walks a whole sequence per CTA (csrc/smxx/fwd_kernel2.cuh:434-742). */
+/* The plan of the recurrence over long sequences: into how many runs (1 = none), walked in parallel, fkda_fwd cuts the
+ * sequences of a batch with `chains` = N*H chains of `chunks_per_sequence` 32-token chunks, and the run length in chunks
+ * (0 with one run).  fkda_scan and the workspace size follow the same plan.  For a packed batch the lengths are on the device:
+ * the call plans for sequences a third longer than the average and sets the run length on the device from the longest one.
+ * The reference has no counterpart: its recurrence kernel always walks a whole sequence per CTA
+ * (csrc/smxx/fwd_kernel2.cuh:434-742). */
 int fkda_plan_segments(int64_t chains, int64_t chunks_per_sequence, int* segments, int* chunks_per_segment);
 
 /* The whole operator (replaces fwd(), csrc/flash_kda.cpp:28-217), enqueued on `stream`: a token-parallel stage and a

@@ -79,6 +79,29 @@ def test_operands_kernel_gives_the_bits_of_its_one_item_per_cta_form(case):
         assert torch.equal(o.view(torch.int16), out.view(torch.int16)) and torch.equal(f, fin)
 
 
+@pytest.mark.parametrize("H,T,packed", [(24, 8192, False), (8, 8192, False), (4, 20000, False), (2, 12000, True)])
+def test_the_call_walks_the_runs_that_the_planner_reports(H, T, packed):
+    """The slots behind the records show how many runs a call has made: the state at the start of every run but the first is in
+    its slot, and nothing is written behind the slots of the reported number of runs.  (Packed: two sequences of T tokens,
+    planned for a third more.)"""
+    N = 2 if packed else 1
+    w = Workload("plan", H=H, T=T, seq_lens=[T, T] if packed else None, state_out="fp32", seed=H)
+    x = make_inputs(w, device="cuda")
+    runs, _ = F.plan_segments(N * H, ((T * 4 // 3 if packed else T) + 31) // 32)
+    off, rec, per_head = F.workspace_layout(N * T, H, N, packed, T)
+    slots, slot = off + rec * per_head * H, 3 * 128 * 136 * 4
+    size = max(F.get_workspace_size(N * T, H, N), slots) + 2 * N * H * slot
+    ws = torch.full((size,), 0x5A, dtype=torch.uint8, device="cuda")
+    F.fwd(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"],
+          final_state=x["final_state"], cu_seqlens=x["cu_seqlens"], workspace=ws)
+    assert F.read_status(ws) == 0
+    used = runs if runs > 1 else 0
+    assert bool((ws[slots + used * N * H * slot:] == 0x5A).all()), "more runs than reported"
+    if used:
+        states = ws[slots:slots + used * N * H * slot].view(N * H, used, 3, 128 * 136 * 4)[:, 1:, 2, :128 * 128 * 4]
+        assert bool((states != 0x5A).any(-1).all()), "fewer runs than reported"
+
+
 @pytest.mark.parametrize("state", [None, "bf16", "fp32"])
 @pytest.mark.parametrize("B,T", [(1, 1), (3, 4), (2, 5), (5, 15), (5, 16), (3, 17), (2, 31), (2, 32), (400, 3)])
 def test_short_sequences_match_the_recurrence(B, T, state):

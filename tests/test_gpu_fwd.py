@@ -424,17 +424,18 @@ def test_segment_parallel_scan_on_either_recurrence_kernel(kernel):
     assert max_abs(o_seg, o_ref) <= 1e-2 and rel_fro(s_seg, s_ref) <= 5e-3
 
 
-def test_segment_parallel_scan_planned_many_chains():
-    """Twenty-four chains of 256 chunks: the planner cuts them, the first pass has more CTAs than SMs and runs on the
-    compact kernel, the second on the look-ahead kernel."""
+def test_segment_parallel_scan_on_both_recurrence_kernels():
+    """Two-stage form, twenty-four chains in seven runs: the first pass has more CTAs than SMs and runs on the compact
+    kernel, the second on the look-ahead kernel."""
     w = Workload("segmany", H=12, B=2, T=8192 - 13, state_in="bf16", state_out="bf16", state_std=0.5, seed=9)
-    runs, run_chunks = F.plan_segments(w.H * w.B, (w.T + 31) // 32)
-    assert runs >= 3 and w.H * w.B * (2 * runs - 3) > 148 >= w.H * w.B * (runs - 1), (runs, run_chunks)
+    runs = 7
+    assert w.H * w.B * (2 * runs - 3) > 148 >= w.H * w.B * (runs - 1)
     x = make_inputs(w)
-    o1, s1 = run_gpu(x, torch.bfloat16)
-    check_against_f64(x, o1, s1, f"planned runs={runs}x{run_chunks}, 24 chains")
-    o0, s0 = run_gpu(x, torch.bfloat16, F.FLAG_SCAN_NO_SEGMENTS)
+    o1, s1 = run_two_stage(x, torch.bfloat16, F.FLAG_SEGMENTS(runs))
+    check_against_f64(x, o1, s1, f"{runs} runs, 24 chains")
+    o0, s0 = run_two_stage(x, torch.bfloat16, F.FLAG_SCAN_NO_SEGMENTS)
     assert max_abs(o1, o0) <= 1e-2 and rel_fro(s1, s0) <= 2e-2
+    assert not torch.equal(o1.view(torch.int16), o0.view(torch.int16)), "the two paths round differently: equal outputs mean the runs were not used"
 
 
 @pytest.mark.parametrize("kernel", ["compact", "lookahead"])

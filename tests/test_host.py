@@ -127,7 +127,8 @@ def test_segment_planner_is_consistent_with_the_workspace_size():
     import flashkda_b200 as F
     assert F.plan_segments(128, 256) == (1, 0)          # one chain per SM already
     assert F.plan_segments(8, 16) == (1, 0)             # too short to be worth it
-    for chains, chunks in [(8, 4096), (16, 256), (1, 4096), (4, 129), (36, 1000)]:
+    assert F.plan_segments(36, 1000) == (1, 0)          # split over four CTAs each instead: the SMs are full without runs
+    for chains, chunks in [(8, 4096), (16, 256), (1, 4096), (4, 129)]:
         runs, per = F.plan_segments(chains, chunks)
         assert runs >= 3 and per * runs >= chunks and (runs - 1) * per < chunks, (chains, chunks, runs, per)
         H, N, T = chains, 1, chunks * 32

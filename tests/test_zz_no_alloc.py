@@ -81,10 +81,12 @@ def test_static_scratch_entry_point_matches_fkda_fwd_twice_in_a_row():
     assert float(out.float().abs().max()) == 0.0
 
 
-def test_static_scratch_walks_whole_sequences_when_the_runs_do_not_fit():
+@pytest.mark.parametrize("T", [57600, 60400], ids=["fewer_runs", "no_runs"])
+def test_static_scratch_serves_a_long_chain_whose_runs_do_not_fit(T):
     """One long chain: the planner would cut it into runs, whose scratch does not fit the built-in array beside the
-    records; the call is then served by the walk over whole sequences instead of being refused."""
-    w = Workload("long", H=1, B=1, T=57600, state_in="fp32", state_out="fp32", seed=34)
-    runs, _ = F.plan_segments(1, w.T // 32)
-    assert runs > 1 and F.get_workspace_size(w.T, 1, 1) > (64 << 20) >= F.get_workspace_size(w.T, 1, 1, F.FLAG_SCAN_NO_SEGMENTS)
+    records; the call is then served by fewer runs, or by the walk over the whole sequence, instead of being refused."""
+    w = Workload("long", H=1, B=1, T=T, state_in="fp32", state_out="fp32", seed=34)
+    runs, _ = F.plan_segments(1, (w.T + 31) // 32)
+    whole = F.get_workspace_size(w.T, 1, 1, F.FLAG_SCAN_NO_SEGMENTS)
+    assert runs > 1 and F.get_workspace_size(w.T, 1, 1) > (64 << 20) >= whole
     _run_both(w)
