@@ -347,15 +347,19 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
 // Where fewer chains than SMs have a CTA each, the SMs beyond them can work out operands meanwhile.  The call is then cut in two
 // time slices, and the second one's operands are computed beside the first one's recurrence, by kSliceWaves waves of two
 // CTAs on each free SM that end with it.  A chunk of the recurrence takes 1.32 us; a CTA of the token-parallel stage 3.7 us per item
-// and 5 us to fill and drain its pipeline.  Returns the chunks of the first slice, or 0 where the stage is not shortened by
-// 40 us: the second pair of launches and the stage's share of the recurrence's bandwidth cost about 30.  96 heads of 8192 tokens:
-// 628 -> 576 us; 75 of 16384: 1121 -> 989; 128 chains, whose 20 free SMs would gain nothing, stay in one piece.
+// and 5 us to fill and drain its pipeline.  Returns the chunks of the first slice, or 0 where what the stage is shortened by is
+// not worth it: the second pair of launches costs about 20 us and the stage's share of the recurrence's bandwidth about 4 % of the
+// call.  Gains measured against one piece, chains x chunks: 75 x 512 13 %, 96 x 256 10 %, 110 x 256 7 %, 120 x 512 3 %, 124 x 1024
+// 1.5 %, 128 x 512 and 128 x 1024 nothing to 1 %, 130 x 1024 -0.4 %, 134 x 1024 -3 %, 140 x 2048 -5 %: the line at 5 % of the
+// call lies at 129 chains.  Equal lengths only: a packed batch's lengths, which the slices would have to follow, are on the
+// device.  Chains split over CTAs leave too few SMs free beside them (20 at 32 chains, none at 37 or 74).
 constexpr int kSliceWaves = 2;
 int plan_slice(int64_t chains, int64_t chunks, int sms) {
   if (chains >= sms || chunks < 16) return 0;
-  const double c = static_cast<double>(chunks), per_us = 2.0 * kSliceWaves * static_cast<double>(sms - chains) / (3.7 * static_cast<double>(chains));
+  const double c = static_cast<double>(chunks), n = static_cast<double>(chains), per_us = 2.0 * kSliceWaves * (sms - n) / (3.7 * n);
   const double second = per_us * (1.32 / kSliceWaves * c - 5.0) / (1.0 + 1.32 / kSliceWaves * per_us);
-  if (second * 0.0118 * static_cast<double>(chains) < 40.0) return 0;
+  const double saved = second * 0.0118 * n, call = c * (0.0118 * n + 1.32);
+  if (saved < 40.0 || saved < 0.05 * call) return 0;
   return static_cast<int>(c - second);
 }
 
@@ -567,6 +571,10 @@ int fkda_selftest_umma(const void* A, const void* B, float* D, int mode, int rep
                                              reps, status, static_cast<cudaStream_t>(cuda_stream));
   if (e != cudaSuccess) return cuda_fail(e, "selftest launch");
   return FKDA_OK;
+}
+
+int fkda_debug_plan_slice(int64_t chains, int64_t chunks_per_sequence) {
+  return chains > 0 ? plan_slice(chains, chunks_per_sequence, fkda::device_sm_count()) : 0;
 }
 
 int fkda_debug_scan_giveup(const fkda_fwd_params* p, int stop_copies_after, int wait_limit_us, void* cuda_stream) {

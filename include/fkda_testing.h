@@ -24,6 +24,10 @@ int fkda_selftest_umma(const void* A, const void* B, float* D, int mode, int rep
  * through the 32x32b shape (see tmem_layout_probe_kernel).  One warp, a few microseconds. */
 int fkda_debug_tmem_layout_probe(void* out, void* cuda_stream);
 
+/* Chunks of the first of the two time slices in which fkda_fwd works a batch of `chains` equal-length chains, one CTA each,
+ * through, or 0 where it goes through in one piece. */
+int fkda_debug_plan_slice(int64_t chains, int64_t chunks_per_sequence);
+
 /* The give-up path of the bounded waits, provoked without a fault: fkda_prepare followed by the
  * look-ahead recurrence kernel on whole sequences, in which the copy producer of every chain stops
  * issuing copies after `stop_copies_after` records and every wait gives up after `wait_limit_us`

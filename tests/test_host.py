@@ -139,6 +139,17 @@ def test_segment_planner_is_consistent_with_the_workspace_size():
             == 2 * 4 * 3 * 128 * 136 * 4)
 
 
+def test_time_slices_where_they_were_measured_to_gain():
+    """Two slices pay where many SMs are free beside a long recurrence: not for few free SMs (from 130 chains on they cost up
+    to 5 % of the call), not for a CTA per SM or more, not for short sequences."""
+    L = ctypes.CDLL(F.lib_path())
+    L.fkda_debug_plan_slice.argtypes = [ctypes.c_int64, ctypes.c_int64]
+    for chains, chunks in [(75, 512), (80, 128), (96, 256), (110, 256), (120, 256), (124, 1024)]:
+        assert 0 < L.fkda_debug_plan_slice(chains, chunks) < chunks, (chains, chunks)
+    for chains, chunks in [(130, 1024), (140, 1024), (140, 2048), (146, 4096), (147, 32768), (148, 4096), (1000, 4096), (75, 64), (96, 100), (0, 100), (128, 256)]:
+        assert L.fkda_debug_plan_slice(chains, chunks) == 0, (chains, chunks)
+
+
 def test_flag_constants_match_the_header():
     text = open(os.path.join(ROOT, "include", "fkda.h")).read()
     values = {m.group(1): int(m.group(2), 16) for m in re.finditer(r"#define\s+(FKDA_FLAG_\w+)\s+(0x[0-9a-fA-F]+)u", text)}
