@@ -78,6 +78,8 @@ def lib():
         L.fkda_debug_scan_giveup.restype = ci
         L.fkda_debug_prepare_giveup.argtypes = [ctypes.POINTER(FwdParams), ci, vp]
         L.fkda_debug_prepare_giveup.restype = ci
+        L.fkda_debug_operands.argtypes = [ctypes.POINTER(FwdParams), ci, vp]
+        L.fkda_debug_operands.restype = ci
         if hasattr(L, "fkda_debug_umma_bench"):        # builds made with -DFKDA_TUNING only
             L.fkda_debug_umma_bench.argtypes = [ci, ci, ci, ci, ci, vp, vp, vp]
             L.fkda_debug_umma_bench.restype = ci
@@ -348,6 +350,16 @@ def prepare_giveup(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, cu
     p, ws = _params(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, None, None, cu_seqlens, workspace, 0)
     with torch.cuda.device(q.device):
         _check(lib().fkda_debug_prepare_giveup(ctypes.byref(p), int(wait_limit_us), _stream(q)))
+
+
+def operands(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, cu_seqlens=None, *, workspace=None, flags=0, wait_limit_us=0):
+    """Test and measuring aid: the token-parallel stage of the default path alone; fills and returns the workspace.  With
+    `wait_limit_us` its CTAs load the tiles of their first item only and their waits give up after that time
+    (include/fkda_testing.h)."""
+    p, ws = _params(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, None, None, cu_seqlens, workspace, flags)
+    with torch.cuda.device(q.device):
+        _check(lib().fkda_debug_operands(ctypes.byref(p), int(wait_limit_us), _stream(q)))
+    return ws
 
 
 def umma_bench(issuers=1, reps=64, ksteps=8, n=64, a_in_tmem=True, device="cuda"):

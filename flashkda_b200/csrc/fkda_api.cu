@@ -363,9 +363,15 @@ int plan_slice(int64_t chains, int64_t chunks, int sms) {
   return static_cast<int>(c - second);
 }
 
+// What the test entry points ask of do_compact: to end behind the token-parallel stage, and a wait that nothing completes.
+struct TestAid {
+  bool operands_only;
+  int wait_limit_us;       // 0: nothing is held back
+};
+
 // The forward pass over compact records (fkda_record.cuh): token-parallel stage, then the recurrence in the form that suits
 // the number of chains.
-int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
+int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, const TestAid* aid = nullptr) {
   uint8_t* ws = static_cast<uint8_t*>(p->workspace);
   int* status = reinterpret_cast<int*>(ws);
   const int64_t chains = p->N * p->H, T_total = p->B * p->T;
@@ -384,8 +390,14 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
   fkda::PrepParams q = prep_params(p, L);
   const int slice = p->cu_seqlens || runs > 1 || rows || whole || one_item ? 0 : plan_slice(chains, q.seq_chunks, sms);
   if (slice) q.slice_chunks = slice;
+  if (aid != nullptr && aid->operands_only) {
+    q.slice_chunks = q.seq_chunks;
+    q.wait_limit_us = aid->wait_limit_us;
+    q.first_load_only = aid->wait_limit_us > 0;
+  }
   e = fkda::launch_operands(q, one_item, stream);
   if (e != cudaSuccess) return cuda_fail(e, "token-parallel launch");
+  if (aid != nullptr && aid->operands_only) return FKDA_OK;
   fkda::ScanParams s = scan_params(p, L);
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
   s.skip_short = p->cu_seqlens != nullptr;
@@ -603,6 +615,15 @@ int fkda_debug_prepare_giveup(const fkda_fwd_params* p, int wait_limit_us, void*
   if (p->flags & (FKDA_FLAG_PREPARE_TCGEN05 | FKDA_FLAG_PREPARE_MMA_SYNC))
     return fail(FKDA_ERR_INVALID_ARGUMENT, "the give-up aid drives the pipelined kernel: no kernel-selection flag");
   return do_prepare(p, L, static_cast<cudaStream_t>(cuda_stream), wait_limit_us, 1);
+}
+
+int fkda_debug_operands(const fkda_fwd_params* p, int wait_limit_us, void* cuda_stream) {
+  Layout L;
+  int rc = validate(p, &L);
+  if (rc != FKDA_OK) return rc;
+  if (wait_limit_us < 0 || wait_limit_us > 1000000) return fail(FKDA_ERR_INVALID_ARGUMENT, "0 <= wait_limit_us <= 1000000 required");
+  const TestAid aid{true, wait_limit_us};
+  return do_compact(p, L, static_cast<cudaStream_t>(cuda_stream), &aid);
 }
 
 #ifdef FKDA_TUNING

@@ -275,9 +275,10 @@ __device__ __forceinline__ bool element_role(const PrepParams& p, uint8_t* smem,
 __device__ __forceinline__ bool inverse_role(const PrepParams& p, uint8_t* smem, uint32_t sbase, uint32_t tmem, int n_it, int b, int lane,
                                              volatile int* abort_flag) {
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+  bool ok = true;
   for (int i = b; i < n_it; i += 2) {
     // (only this barrier: it cannot run a phase ahead of a warp that frees its result)
-    if (!warp_wait(bar(B_D1 + b), (i >> 1) & 1, abort_flag)) return false;
+    if (!warp_wait(bar(B_D1 + b), (i >> 1) & 1, abort_flag)) { ok = false; break; }
     const int h = reinterpret_cast<const Info*>(smem + kSmInfo)[i & (kInfos - 1)].h, gc = reinterpret_cast<const Info*>(smem + kSmInfo)[i & (kInfos - 1)].gc;
     const float* s_beta = reinterpret_cast<const float*>(smem + kSmBeta + (i & 3) * 128);
     tc_fence_after();
@@ -297,8 +298,8 @@ __device__ __forceinline__ bool inverse_role(const PrepParams& p, uint8_t* smem,
       bulk_commit();
     }
   }
-  if (lane == 0) bulk_wait_read0();
-  return true;
+  if (lane == 0) bulk_wait_read0();                  // giving up too: the store reads this CTA's shared memory
+  return ok;
 }
 
 // Loads, stores and tril(M).
@@ -338,6 +339,7 @@ __device__ __forceinline__ bool copy_role(const PrepParams& p, const CUtensorMap
   if (lane == 0) {
     for (int i = 0; i < 2 && i < n_it; ++i) {
       look_ahead(i);
+      if (i == 1 && p.first_load_only) break;        // test aid: a wait that nothing completes
       load(i);
       ++loaded;
     }
@@ -356,7 +358,7 @@ __device__ __forceinline__ bool copy_role(const PrepParams& p, const CUtensorMap
       bulk_commit();
       if (i + 3 < n_it) look_ahead(i + 3);
       bulk_wait_read0();             // (also the tril(M) of the item before)
-      if (i + 2 < n_it) {
+      if (i + 2 < n_it && !p.first_load_only) {
         load(i + 2);
         ++loaded;
       }
@@ -463,7 +465,8 @@ operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kSmMisc);
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
   if (tid == 0) {
-    *abort_flag = (sbase & 1023u) != 0u ? 1 : 0;       // the swizzled tiles need this alignment: report instead of computing garbage
+    // the swizzled tiles need this alignment: report instead of computing garbage (below zero: a wait limit, test aid)
+    *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(B_IN + i), 1);
       mbar_init(bar(B_NORMP + i), 8);
@@ -482,7 +485,7 @@ operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  bool ok = *abort_flag == 0;
+  bool ok = *abort_flag <= 0;
   if (!kSlice || !p.beside) grid_dependency_wait();
   const unsigned items = static_cast<unsigned>(p.cu_seqlens != nullptr ? p.chunk_prefix[p.N] : kSlice ? p.N * p.slice_chunks : p.total_chunks) * static_cast<unsigned>(p.H);
   const int n_it = !ok || blockIdx.x >= items ? 0 : static_cast<int>((items - blockIdx.x + gridDim.x - 1) / gridDim.x);

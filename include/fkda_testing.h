@@ -42,6 +42,12 @@ int fkda_debug_scan_giveup(const fkda_fwd_params* p, int stop_copies_after, int 
  * memory and return.  (A CTA has a second item once the call has more than three (chunk, head) items per SM.) */
 int fkda_debug_prepare_giveup(const fkda_fwd_params* p, int wait_limit_us, void* cuda_stream);
 
+/* The token-parallel stage of the default path alone (operands_kernel): its compact records (29184 bytes each, layout in
+ * csrc/fkda_record.cuh) lie head by head from the records offset of fkda_workspace_layout on.  With wait_limit_us > 0 every
+ * CTA loads the tiles of its first item only and every wait gives up after so many microseconds, as in
+ * fkda_debug_prepare_giveup (a CTA has a second item once the call has more than two items per SM). */
+int fkda_debug_operands(const fkda_fwd_params* p, int wait_limit_us, void* cuda_stream);
+
 #ifdef FKDA_TUNING
 /* The following exist only in builds made with -DFKDA_TUNING (FKDA_NVCC_EXTRA=-DFKDA_TUNING python -m
  * flashkda_b200.build --force). */

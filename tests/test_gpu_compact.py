@@ -79,6 +79,30 @@ def test_operands_kernel_gives_the_bits_of_its_one_item_per_cta_form(case):
         assert torch.equal(o.view(torch.int16), out.view(torch.int16)) and torch.equal(f, fin)
 
 
+def test_a_wait_in_operands_kernel_gives_up_and_the_context_stays_usable():
+    """Every CTA loads the tiles of its first item only and the waits are given three milliseconds.  With 600 items some CTAs
+    have a second one whose tiles never come: the call must return with status 2 and its tensor memory released, which the
+    ordinary call behind it needs.  With an item per CTA nobody meets the missing load.  Nothing faults, and what a CTA has in
+    flight when it gives up (its first item's products and stores) has ended before it leaves."""
+    for T, status in ((32 * 600, 2), (32 * 200, 0)):
+        w = Workload("g", H=1, T=T, state_out="fp32", seed=6)
+        x = make_inputs(w, device="cuda")
+        args = (x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"])
+        ws = torch.empty(F.get_workspace_size(T, 1, 1), dtype=torch.uint8, device="cuda")
+        F.fwd(*args, final_state=x["final_state"], workspace=ws)
+        assert F.read_status(ws) == 0
+        out, fin = x["out"].clone(), x["final_state"].clone()
+        F.operands(*args, workspace=ws, wait_limit_us=3000)
+        if status:
+            with pytest.raises(RuntimeError, match="bounded wait"):
+                F.read_status(ws)
+        else:
+            assert F.read_status(ws) == 0
+        F.fwd(*args, final_state=x["final_state"], workspace=ws)
+        assert F.read_status(ws) == 0
+        assert torch.equal(x["out"].view(torch.int16), out.view(torch.int16)) and torch.equal(x["final_state"], fin)
+
+
 @pytest.mark.parametrize("H,T,packed", [(24, 8192, False), (8, 8192, False), (4, 20000, False), (2, 12000, True)])
 def test_the_call_walks_the_runs_that_the_planner_reports(H, T, packed):
     """The slots behind the records show how many runs a call has made: the state at the start of every run but the first is in
