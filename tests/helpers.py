@@ -82,5 +82,19 @@ def decode_record(rec_u8):
     return out
 
 
+# ---- compact records (layout in flashkda_b200/csrc/fkda_record.cuh) ----
+COMPACT = dict(KN=0, QP=8192, KR=16384, TB=24576, MQK=26624, E=28672, BYTES=29184)
+
+
+def decode_compact(rec_u8):
+    """rec_u8: CPU uint8 tensor of one 29184-byte record -> dict of float64 matrices."""
+    out = {}
+    for name, rows, cols in (("KN", 32, 128), ("QP", 32, 128), ("KR", 32, 128), ("TB", 32, 32), ("MQK", 32, 32)):
+        raw = rec_u8[COMPACT[name]:COMPACT[name] + rows * cols * 2].view(torch.bfloat16)
+        out[name.lower()] = raw[_core_index(rows, cols)].double()
+    out["ec"] = rec_u8[COMPACT["E"]:COMPACT["E"] + 512].view(torch.float32).double()
+    return out
+
+
 def to_cuda(x):
     return {k: (v.cuda() if isinstance(v, torch.Tensor) else v) for k, v in x.items()}

@@ -8,7 +8,7 @@ import torch
 import flashkda_b200 as F
 import oracle
 from flashkda_b200.workloads import Workload, make_inputs
-from helpers import decode_record, to_cuda
+from helpers import COMPACT, decode_compact, decode_record, to_cuda
 
 pytestmark = pytest.mark.gpu
 
@@ -94,6 +94,55 @@ def test_prepare_records_match_fp64_operands(case, kernel):
     # with packed bf16 multiplies (two and three roundings of 2^-9 each).
     assert worst["qp"] < 8e-3 and worst["kr"] < 1.2e-2 and worst["ec"] < 2e-3, worst
     assert worst["mqk"] < 2e-2 and worst["wp"] < 3e-2 and worst["up"] < 3e-2, worst
+
+
+@pytest.mark.parametrize("case", ["fixed", "varlen", "strong_decay"])
+def test_compact_records_match_fp64_operands(case):
+    """Records of the default token-parallel kernel against the fp64 chunk operands of the oracle: k+ (negated), q+, kr, the
+    chunk's decay and tril(q+ k-^T) as such, T diag(beta) by what it is for, its products with k+ and v.  Bounds relative to
+    the largest entry: one bf16 rounding (2^-9) of an operand whose factors carry the gate's error (tanh.approx, 2^-11 of a
+    sigmoid, on |G| <= 231 log2 units per chunk, of which a factor that is not vanishing has seen a few); products of two or
+    three such operands twice to three times that."""
+    if case == "fixed":
+        w = Workload("f", H=2, B=2, T=80, seed=11)
+    elif case == "varlen":
+        w = Workload("v", H=2, seq_lens=[17, 33, 64, 5], seed=12)
+    else:
+        w = Workload("s", H=2, B=1, T=64, seed=13)
+    x = make_inputs(w)
+    if case == "strong_decay":
+        x["g"] = torch.full_like(x["g"], 8.0)
+        x["A_log"] = torch.full_like(x["A_log"], 2.0)
+    xc = to_cuda(x)
+    ws = F.operands(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], xc["scale"], xc["out"], xc["A_log"], xc["dt_bias"],
+                    xc["lower_bound"], cu_seqlens=xc["cu_seqlens"])
+    assert F.read_status(ws) == 0
+    ws = ws.cpu()
+    T_total, H = x["q"].shape[0] * x["q"].shape[1], w.H
+    off, _, per_head = F.workspace_layout(T_total, H, w.N, x["cu_seqlens"] is not None, x["q"].shape[1])
+    flat = {k: x[k].reshape(1, T_total, *x[k].shape[2:]).contiguous() for k in ("q", "k", "v", "g", "beta")}
+    worst = {}
+    gc, t_seq = 0, 0
+    for L in (w.seq_lens if w.seq_lens is not None else [w.T] * w.B):
+        for t0 in range(0, L, 32):
+            n = min(32, L - t0)
+            for h in range(H):
+                o = off + (h * per_head + gc) * COMPACT["BYTES"]
+                got = decode_compact(ws[o:o + COMPACT["BYTES"]])
+                exp = oracle.chunk_operands(flat["q"], flat["k"], flat["v"], flat["g"], flat["beta"], x["scale"],
+                                            x["A_log"], x["dt_bias"], x["lower_bound"], h, t_seq + t0, n, 32)
+                v = torch.zeros(32, 128, dtype=torch.float64)
+                v[:n] = flat["v"][0, t_seq + t0:t_seq + t0 + n, h].double()
+                assert torch.equal(got["mqk"], got["mqk"].tril()) and torch.equal(got["tb"], got["tb"].tril())
+                for key, a, e in (("kn", got["kn"], -exp["kpp"]), ("qp", got["qp"], exp["qpp"]), ("kr", got["kr"], exp["kr"]),
+                                  ("mqk", got["mqk"], exp["mqk"]), ("ec", got["ec"], exp["ec"]),
+                                  ("wp", got["tb"] @ exp["kpp"], exp["wp"]), ("up", got["tb"] @ v, exp["up"])):
+                    worst[key] = max(worst.get(key, 0.0), (a - e).abs().max().item() / max(e.abs().max().item(), 1e-3))
+            gc += 1
+        t_seq += L
+    print("operands", case, {k: f"{v:.2e}" for k, v in worst.items()})
+    assert worst["kn"] < 8e-3 and worst["qp"] < 8e-3 and worst["kr"] < 8e-3 and worst["ec"] < 2e-3, worst
+    assert worst["mqk"] < 1.6e-2 and worst["wp"] < 1.6e-2 and worst["up"] < 1.6e-2, worst
 
 
 @pytest.mark.parametrize("case", ["fixed_many_iterations", "varlen_many_sequences", "tails"])
