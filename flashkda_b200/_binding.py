@@ -80,6 +80,8 @@ def lib():
         L.fkda_debug_prepare_giveup.restype = ci
         L.fkda_debug_operands.argtypes = [ctypes.POINTER(FwdParams), ci, vp]
         L.fkda_debug_operands.restype = ci
+        L.fkda_debug_recurrence_giveup.argtypes = [ctypes.POINTER(FwdParams), ci, ci, vp]
+        L.fkda_debug_recurrence_giveup.restype = ci
         if hasattr(L, "fkda_debug_umma_bench"):        # builds made with -DFKDA_TUNING only
             L.fkda_debug_umma_bench.argtypes = [ci, ci, ci, ci, ci, vp, vp, vp]
             L.fkda_debug_umma_bench.restype = ci
@@ -360,6 +362,16 @@ def operands(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, cu_seqle
     with torch.cuda.device(q.device):
         _check(lib().fkda_debug_operands(ctypes.byref(p), int(wait_limit_us), _stream(q)))
     return ws
+
+
+def recurrence_giveup(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state=None, final_state=None,
+                      cu_seqlens=None, *, workspace, stop_copies_after=1, wait_limit_us=3000):
+    """Test aid: the default path with a recurrence whose copies stop after `stop_copies_after` records per CTA (negative: a
+    chaining of runs whose copies stop after so many maps) and whose waits give up after `wait_limit_us` microseconds
+    (include/fkda_testing.h)."""
+    p, ws = _params(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state, final_state, cu_seqlens, workspace, 0)
+    with torch.cuda.device(q.device):
+        _check(lib().fkda_debug_recurrence_giveup(ctypes.byref(p), int(stop_copies_after), int(wait_limit_us), _stream(q)))
 
 
 def umma_bench(issuers=1, reps=64, ksteps=8, n=64, a_in_tmem=True, device="cuda"):

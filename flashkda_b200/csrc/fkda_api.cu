@@ -367,6 +367,7 @@ int plan_slice(int64_t chains, int64_t chunks, int sms) {
 struct TestAid {
   bool operands_only;
   int wait_limit_us;       // 0: nothing is held back
+  int stop_copies_after;   // records per CTA of the recurrence, or (negative) maps of the chaining of runs
 };
 
 // The forward pass over compact records (fkda_record.cuh): token-parallel stage, then the recurrence in the form that suits
@@ -400,6 +401,11 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, c
   if (aid != nullptr && aid->operands_only) return FKDA_OK;
   fkda::ScanParams s = scan_params(p, L);
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
+  if (aid != nullptr) {
+    (aid->stop_copies_after > 0 ? s.wait_limit_us : s.map_wait_limit_us) = aid->wait_limit_us;
+    s.stop_copies_after = aid->stop_copies_after > 0 ? aid->stop_copies_after : 0;
+    s.stop_maps_after = aid->stop_copies_after < 0 ? -aid->stop_copies_after : 0;
+  }
   s.skip_short = p->cu_seqlens != nullptr;
   s.release_next = p->cu_seqlens != nullptr && runs == 1;      // (to the step kernel below)
   if (runs > 1) {
@@ -622,7 +628,17 @@ int fkda_debug_operands(const fkda_fwd_params* p, int wait_limit_us, void* cuda_
   int rc = validate(p, &L);
   if (rc != FKDA_OK) return rc;
   if (wait_limit_us < 0 || wait_limit_us > 1000000) return fail(FKDA_ERR_INVALID_ARGUMENT, "0 <= wait_limit_us <= 1000000 required");
-  const TestAid aid{true, wait_limit_us};
+  const TestAid aid{true, wait_limit_us, 0};
+  return do_compact(p, L, static_cast<cudaStream_t>(cuda_stream), &aid);
+}
+
+int fkda_debug_recurrence_giveup(const fkda_fwd_params* p, int stop_copies_after, int wait_limit_us, void* cuda_stream) {
+  Layout L;
+  int rc = validate(p, &L);
+  if (rc != FKDA_OK) return rc;
+  if (stop_copies_after == 0 || wait_limit_us < 1 || wait_limit_us > 1000000)
+    return fail(FKDA_ERR_INVALID_ARGUMENT, "stop_copies_after != 0 and 1 <= wait_limit_us <= 1000000 required");
+  const TestAid aid{false, wait_limit_us, stop_copies_after};
   return do_compact(p, L, static_cast<cudaStream_t>(cuda_stream), &aid);
 }
 

@@ -455,11 +455,13 @@ struct ScanParams {
   int skip_short;              // packed batches: sequences of at most kStepMaxT tokens are somebody else's (no chunks, no state)
   int release_next;            // the next kernel needs nothing of this one's results and may start beside it
   int* next_walk;              // persistent recurrence kernel: device counter (zeroed) that hands out the walks, or nullptr (in turn)
-  // Test aids of the look-ahead kernel's give-up path (both 0 in production): a wait limit in microseconds instead of
-  // the default, and a number of records after which the copy producer stops issuing copies, so that the consumers'
-  // next wait runs out with nothing in flight.
+  // Test aids of the give-up path (0 in production): a wait limit in microseconds instead of the default, and a number of
+  // records after which a CTA's copies stop, so that the next wait for one runs out with nothing in flight; the same for the
+  // maps of the kernel that chains runs.
   int wait_limit_us;
   int stop_copies_after;
+  int map_wait_limit_us;
+  int stop_maps_after;
   // Equal lengths in two time slices: the chunks [slice_begin, slice_end) of every sequence (slice_end 0: all of them), the state
   // between the slices in fp32 over the chain's first records, which nobody reads any more.
   int slice_begin;

@@ -296,7 +296,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
   Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
   if (tid == 0) {
-    *abort_flag = (sbase & 1023u) != 0u ? 1 : 0;       // the swizzled tiles need this alignment: report instead of computing garbage
+    // the swizzled tiles need this alignment: report instead of computing garbage (below zero: a wait limit, test aid)
+    *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar(B_FULL + s), 1);
       mbar_init(bar(B_EMPTY + s), 4 + 1);              // recurrence warps + commit of the output products
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  bool ok = *abort_flag == 0;
+  bool ok = *abort_flag <= 0;
   grid_dependency_wait();
   if (p.release_next) grid_release_next();
 
@@ -368,6 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     int cs = 0;                        // stage of the next item
     auto copy = [&]() {
       const int s = cs;
+      if (p.stop_copies_after > 0 && copied >= p.stop_copies_after) return;      // test aid: the next wait for a record runs out
       Info* f = infos + (copied & (kInfos - 1));
       if (cur.c == cur.n) {            // the next walk
         if (!kStream && cur.turn > 0) {

@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + P::kSmMisc);
   auto bar = [&](int i) { return sbase + P::kSmBars + 8 * i; };
   if (tid == 0) {
-    *abort_flag = (sbase & 1023u) != 0u ? 1 : 0;          // the swizzled tiles need this alignment: report instead of computing garbage
+    // the swizzled tiles need this alignment: report instead of computing garbage (below zero: a wait limit, test aid)
+    *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
     for (int s = 0; s < P::kStages; ++s) {
       mbar_init(bar(P::B_FULL + s), 1);
       mbar_init(bar(P::B_EMPTY + s), 2 * NW);             // (a full stage's boxes are free too: their readers arrive here)
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
     fence_mbar_init();
   }
   __syncthreads();
-  bool ok = *abort_flag == 0;
+  bool ok = *abort_flag <= 0;
   grid_dependency_wait();
   if (p.release_next) grid_release_next();
   const ChainView cv = chain_view<false>(p, blockIdx.x / P::kSplits);
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(Plan<NW>::kThreads, 1) recur_split_kernel(cons
     int issued = 0;
     for (int c = 0; c < nchunks; ++c) {
       const int s = c % P::kStages;
+      if (p.stop_copies_after > 0 && c >= p.stop_copies_after) break;            // test aid: the next wait for a record runs out
       if (c >= P::kStages && !mbar_wait_parked(bar(P::B_EMPTY + s), (c / P::kStages - 1) & 1, abort_flag)) { ok = false; break; }
       const uint32_t dst = sbase + s * P::kStageBytes, full = bar(P::B_FULL + s);
       mbar_arrive_expect_tx(full, kCrBytes + 4096);

@@ -54,7 +54,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
 // once by its producer.  Per run: 3.2 us with sixteen rows per CTA and both operands read and split on the chain, 1.4 us now
 // (2 heads of 65536 tokens: 331 -> 274 us).  Sixteen warps, two per sixteen columns with half of k each: with eight the loop is 8 KB of code,
 // which the instruction caches no longer hold (1.7 us).
-__global__ void __launch_bounds__(kCmbThreads, 1) seg_combine_kernel(float* seg_buf, int n_segs, int* status) {
+__global__ void __launch_bounds__(kCmbThreads, 1) seg_combine_kernel(float* seg_buf, int n_segs, int* status, int wait_limit_us, int stop_maps_after) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   const uint32_t sbase = smem_u32(smem);
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kCmbThreads, 1) seg_combine_kernel(float* seg_
   float* slots = seg_buf + static_cast<size_t>(blockIdx.x) * n_segs * 3 * kSegSlotFloats;
   const int r_base = blockIdx.y * kCmbRows;
   auto load_map = [&](int run) {      // one thread: the whole slot, rows padded as the recurrence kernel left them
-    if (run + 1 >= n_segs) return;
+    if (run + 1 >= n_segs || (stop_maps_after > 0 && run > stop_maps_after)) return;     // (test aid: the next wait for a map runs out)
     const int b = (run - 1) % kMapBufs;
     mbar_arrive_expect_tx(sbase + kCmbBars + 8 * b, kMapStg);
     bulk_g2s(sbase + kCmbM + b * kMapStg, slots + (run * 3 + 0) * kSegSlotFloats, kMapStg, sbase + kCmbBars + 8 * b);
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kCmbThreads, 1) seg_combine_kernel(float* seg_
     }
   };
   if (tid == 0) {
-    *abort_flag = 0;
+    *abort_flag = -wait_limit_us;       // (below zero: a wait limit, test aid)
     for (int i = 0; i < kMapBufs; ++i) mbar_init(sbase + kCmbBars + 8 * i, 1);
     fence_mbar_init();
   }
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kCmbThreads, 1) seg_combine_kernel(float* seg_
       if (half == 0) load_rows(slots + ((run + 1) * 3 + 1) * kSegSlotFloats, next_n);
       ok = wait_map(run + 1);
     }
-    if (tid < 32 && run + 5 < n_segs)     // and the lines of a later N into the L2: 16 rows of 512 bytes
+    if (tid < 32 && run + 5 < n_segs)     // and the lines of a later N into the L2: eight rows of 512 bytes
       asm volatile("prefetch.global.L2 [%0];" ::"l"(slots + ((run + 4) * 3 + 1) * kSegSlotFloats +
                                                      static_cast<size_t>(r_base + (tid >> 2)) * kD + (tid & 3) * 32));
     const uint4* z = reinterpret_cast<const uint4*>(smem + kCmbZ) + 256 * half + lane;
@@ -199,7 +199,7 @@ cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_ch
     e = opt_in.ensure(seg_combine_kernel, kCmbSmemBytes);
     if (e != cudaSuccess) return e;
     const dim3 grid(static_cast<unsigned>(chains), kD / kCmbRows);
-    e = launch_after(seg_combine_kernel, grid, kCmbThreads, kCmbSmemBytes, stream, seg_buf, n_segs, p.status);
+    e = launch_after(seg_combine_kernel, grid, kCmbThreads, kCmbSmemBytes, stream, seg_buf, n_segs, p.status, p.map_wait_limit_us, p.stop_maps_after);
     if (e != cudaSuccess) return e;
   }
   p.seg_pass = 2;

@@ -103,6 +103,41 @@ def test_a_wait_in_operands_kernel_gives_up_and_the_context_stays_usable():
         assert torch.equal(x["out"].view(torch.int16), out.view(torch.int16)) and torch.equal(x["final_state"], fin)
 
 
+GIVEUP = {
+    "split4": (Workload("g", H=3, B=2, T=200, state_in="fp32", state_out="fp32", seed=1), 2),
+    "split2": (Workload("g", H=25, B=2, T=200, state_out="fp32", seed=2), 3),
+    "one_cta": (Workload("g", H=50, B=2, T=300, state_in="bf16", state_out="bf16", seed=3), 4),
+    "persistent": (Workload("g", H=50, B=6, T=200, state_out="fp32", seed=4), 9),
+    "packed_with_decode": (Workload("g", H=40, seq_lens=[1, 200, 40, 3, 300, 64], state_in="fp32", state_out="fp32", seed=5), 1),
+    "slices": (Workload("g", H=80, T=32 * 128, state_out="fp32", seed=6), 7),
+    "runs": (Workload("g", H=2, T=32 * 700, state_out="fp32", lower_bound=-1.0, seed=7), 6),
+    "chaining": (Workload("g", H=2, T=32 * 700, state_out="fp32", lower_bound=-1.0, seed=7), -4),
+}
+
+
+@pytest.mark.parametrize("form", list(GIVEUP))
+def test_a_wait_in_the_recurrence_gives_up_and_the_context_stays_usable(form):
+    """Each form of the recurrence with copies that stop in the middle of a walk and waits of three milliseconds: the call must
+    return with status 2, and the ordinary call behind it, which needs all of the tensor memory, gives the bits of the one
+    before.  Nothing faults and nothing is in flight when a wait runs out."""
+    w, stop = GIVEUP[form]
+    x = make_inputs(w, device="cuda")
+    args = (x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"])
+    kw = dict(initial_state=x["initial_state"], final_state=x["final_state"], cu_seqlens=x["cu_seqlens"])
+    ws = torch.empty(F.get_workspace_size(x["q"].shape[0] * x["q"].shape[1], w.H, w.N), dtype=torch.uint8, device="cuda")
+    F.fwd(*args, workspace=ws, **kw)
+    assert F.read_status(ws) == 0
+    out, fin = x["out"].clone(), x["final_state"].clone()
+    F.recurrence_giveup(*args, workspace=ws, stop_copies_after=stop, **kw)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        F.read_status(ws)
+    F.recurrence_giveup(*args, workspace=ws, stop_copies_after=1000000 if stop > 0 else -1000000, wait_limit_us=1000000, **kw)     # (held back by nothing)
+    assert F.read_status(ws) == 0
+    F.fwd(*args, workspace=ws, **kw)
+    assert F.read_status(ws) == 0
+    assert torch.equal(x["out"].view(torch.int16), out.view(torch.int16)) and torch.equal(x["final_state"], fin)
+
+
 @pytest.mark.parametrize("H,T,packed", [(24, 8192, False), (8, 8192, False), (4, 20000, False), (2, 12000, True)])
 def test_the_call_walks_the_runs_that_the_planner_reports(H, T, packed):
     """The slots behind the records show how many runs a call has made: the state at the start of every run but the first is in
