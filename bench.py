@@ -21,7 +21,9 @@ The JSON line carries:
                copies of q,k,v,g,beta,state and device->host copies of out and final_state
                inside the timed region (fixed-length batches: one call per sequence, so that the
                copies of neighbouring sequences overlap with the forward pass; `mode` says which)
-  roofline     dominant kernel: the algorithmic bytes that kernel itself moves / its mean duration,
+  kernels_ms   the stages of the path that the timed call takes, each alone, back to back
+  gpu_launches kernels of the timed region: those of one call, counted in a graph captured around it, times the calls
+  roofline     dominant stage: the algorithmic bytes that it moves itself / its mean duration,
                against the measured HBM copy bandwidth; `roofline_call` (the headline) is the
                call's algorithmic bytes over the whole call (all kernels)
   parity       a sample of (sequence, head) chains of the timed call's result against the fp64
@@ -181,6 +183,28 @@ def time_cuda(fn, steps, stream):
     b.record(stream)
     torch.cuda.synchronize()
     return a.elapsed_time(b) / steps
+
+
+def kernels_per_call(call):
+    """Kernels that one call launches, all of them this repository's own: the kernel nodes of a CUDA graph captured around it."""
+    import ctypes
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):      # (NCCL's watchdog thread may go on)
+        call()
+    cu = ctypes.CDLL("libcuda.so.1")
+    handle, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    if cu.cuGraphGetNodes(handle, None, ctypes.byref(n)) != 0:
+        raise RuntimeError("cuGraphGetNodes failed")
+    nodes = (ctypes.c_void_p * n.value)()
+    if cu.cuGraphGetNodes(handle, nodes, ctypes.byref(n)) != 0:
+        raise RuntimeError("cuGraphGetNodes failed")
+    kernels = 0
+    for node in nodes:
+        kind = ctypes.c_int(-1)
+        if cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) != 0:
+            raise RuntimeError("cuGraphNodeGetType failed")
+        kernels += kind.value == 0          # CU_GRAPH_NODE_TYPE_KERNEL
+    return kernels
 
 
 def bind_near_gpu(local_rank, local_world):
@@ -418,10 +442,21 @@ def main():
               flags=args.flags)
     pos = (x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"])
     ksteps = max(3, min(args.steps, 10))
-    # short fixed-length sequences take one fused kernel: the call is the kernel
-    fused = x["cu_seqlens"] is None and 0 < T <= 32 and (args.flags & 0xFF57) == 0
-    ms_prepare = 0.0 if fused else time_cuda(lambda: F.prepare(*pos, **kw), ksteps, stream)
-    ms_scan = 0.0 if fused else time_cuda(lambda: F.scan(*pos, **kw), ksteps, stream)
+    # The stages of the path that the call takes.  Short fixed-length sequences: one kernel, which is the call.  Else the two
+    # stages of the default path, each alone over the workspace of a whole call, or of the two-stage form where a flag selects it.
+    varlen = x["cu_seqlens"] is not None
+    fused = not varlen and 0 < T <= 32 and (args.flags & 0xFF57) == 0
+    one_kernel = "refmode" if args.flags & F.FLAG_REFERENCE_ROUNDING else ("step" if T <= 4 else "short16") if fused else None
+    two_stage = args.flags & ~(F.FLAG_SCAN_NO_SEGMENTS | F.FLAG_NO_FUSED_SHORT | F.FLAG_OPERANDS_PER_ITEM) or \
+        (varlen and args.flags & F.FLAG_SCAN_NO_SEGMENTS)
+    stages = []
+    if one_kernel is None and two_stage:
+        stages = [("prepare", lambda: F.prepare(*pos, **kw)), ("scan", lambda: F.scan(*pos, **kw))]
+    elif one_kernel is None:
+        kw_in = {n: v for n, v in kw.items() if n not in ("initial_state", "final_state")}
+        stages = [("operands", lambda: F.operands(*pos, **kw_in)), ("recurrence", lambda: F.recurrence(*pos, **kw))]
+    ms_stage = [time_cuda(fn, ksteps, stream) for _, fn in stages] or [0.0, 0.0]
+    launches_per_call = kernels_per_call(call_ws)
     call_ws()                      # leave the results of a complete call in out / final_state for the checks below
     torch.cuda.synchronize()
 
@@ -509,8 +544,8 @@ def main():
         e2e = (ms_e2e_local, h2d, d2h, e2e_mode, ms_copy_local)
 
     # ---- reduce over ranks: max time -------------------------------------------------------------------
-    ms, ms_ws, ms_prepare, ms_scan, ms_e2e, ms_copy = reduce_max_ms(
-        [ms, ms_ws, ms_prepare, ms_scan, e2e[0] if e2e else 0.0, e2e[4] if e2e else 0.0], world, dev)
+    ms, ms_ws, *ms_stage, ms_e2e, ms_copy = reduce_max_ms(
+        [ms, ms_ws, *ms_stage, e2e[0] if e2e else 0.0, e2e[4] if e2e else 0.0], world, dev)
 
     strong = None
     if world > 1 and not args.no_strong and args.config == 1 and not args.shape:
@@ -519,37 +554,17 @@ def main():
             if baseline_workload(cfg).H % world == 0:
                 strong.append(strong_scaling(F, flash_kda, cfg, world, rank, dev, stream, max(3, min(args.steps, 10)), args.flags, dist))
 
-    # kernels per call: prepare, the recurrence (one launch, or pass 1 + map chaining + pass 2 when sequences are cut
-    # into runs), plus the chunk prefix for varlen
-    runs = 1
-    varlen = x["cu_seqlens"] is not None
-    chains = N * H_local
-    per_seq_chunks = ((B * T) // N + 31) // 32 if varlen else (T + 31) // 32     # varlen: planned for the average length
-    forced = (args.flags >> 8) & 0xFF
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    if not (args.flags & 0x9) and not ((args.flags & 0x2) and forced < 2):
-        runs = forced if forced >= 2 else (1 if args.flags & 0x4 else F.plan_segments(chains, per_seq_chunks)[0])
-    if not varlen and 0 < T <= 64 and not (args.flags & 0x4):
-        runs = 1
-    if chains > sms and not (args.flags & 0x7):
-        runs = 1                      # more chains than SMs: the compact kernel on whole sequences
-    recurrence = 1 if runs == 1 else 2 + (1 if runs > 2 else 0)
-    if varlen and sms < chains <= 1024 and not (args.flags & 0x7):
-        recurrence = 2                # both recurrence kernels are launched; the one not chosen on the device leaves at once
-    launches_per_call = 1 + (1 if varlen else 0) + recurrence
-    if fused:
-        launches_per_call = 1
-
     if rank == 0:
         peak, peak_kind = measured_peaks()
         alg = algorithmic_bytes(B * T, H_local, N, w.state_in, w.state_out)      # per rank, per call
-        # what each kernel moves of those bytes: the token-parallel kernel reads q, k, v, g, beta; the recurrence writes
-        # out and moves the states (its other input, the operand records, is not algorithmic)
-        alg_prepare = 1026 * B * T * H_local
-        alg_scan = alg - alg_prepare
-        dom_name, dom_ms, dom_alg = ("scan", ms_scan, alg_scan) if ms_scan >= ms_prepare else ("prepare", ms_prepare, alg_prepare)
-        if fused:
-            dom_name, dom_ms, dom_alg = "short16", ms_ws, alg
+        # What each stage moves of those bytes.  Default path: the token-parallel stage reads q, k, g, beta; the recurrence
+        # reads v, writes out and moves the states.  Two-stage form: v is read by the first stage.  (The operand records
+        # between the stages are not algorithmic.)
+        first = (1026 if two_stage else 770) * B * T * H_local
+        if one_kernel:
+            dom_name, dom_ms, dom_alg = one_kernel, ms_ws, alg
+        else:
+            dom_name, dom_ms, dom_alg = max(((stages[0][0], ms_stage[0], first), (stages[1][0], ms_stage[1], alg - first)), key=lambda d: d[1])
         ach = dom_alg / (dom_ms * 1e-3) / 1e9
         ach_call = alg / (ms * 1e-3) / 1e9
         line = {
@@ -563,12 +578,12 @@ def main():
             "gpu_launches": launches_per_call * args.steps,
             "preallocated_workspace": {"ms_per_step": ms_ws, "value": tokens_global / (ms_ws * 1e-3)},
             "sustained": sustained,
-            "kernels_ms": {"short16": ms_ws} if fused else {"prepare": ms_prepare, "scan": ms_scan},
+            "kernels_ms": {one_kernel: ms_ws} if one_kernel else {name: t for (name, _), t in zip(stages, ms_stage)},
             "roofline": {"bound": "hbm", "kernel": dom_name, "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak, "peak_source": peak_kind, "algorithmic_bytes": dom_alg,
                          "call_algorithmic_bytes": alg,
                          "traffic": (SHORT16_TRAFFIC_BYTES_PER_CHAIN * N * H_local
-                                     if fused and T == 16 and w.state_in == "fp32" and w.state_out == "fp32" else
+                                     if one_kernel == "short16" and T == 16 and w.state_in == "fp32" and w.state_out == "fp32" else
                                      TRAFFIC_BYTES_PER_TOKEN_HEAD.get(dom_name) and
                                      TRAFFIC_BYTES_PER_TOKEN_HEAD[dom_name] * B * T * H_local)},
             "roofline_call": {"achieved": ach_call, "peak": peak, "unit": "GB/s", "frac": ach_call / peak,
@@ -602,12 +617,12 @@ def main():
         dist.destroy_process_group()
 
 
-# DRAM bytes per token-head of each kernel, from ncu captures summarised under profiles/
-# (dram__bytes_read.sum + dram__bytes_write.sum per launch / token-heads of the captured case).
-SHORT16_TRAFFIC_BYTES_PER_CHAIN = 140_400   # profiles/short16_kernel_B128xT16xH32.md (T = 16, fp32 state in and out), scaled by chains
-# ncu dram bytes per token-head: profiles/prepare_pipe_kernel_prepare_tc4_kernel_B8xT1024xH16.md (prepare) and
-# profiles/prepare_kernel_scan2_kernel_B8xT1024xH16.md (scan), scaled by token-heads
-TRAFFIC_BYTES_PER_TOKEN_HEAD = {"prepare": 1774, "scan": 1313}
+# DRAM bytes from ncu captures summarised under profiles/ (dram__bytes_read.sum + dram__bytes_write.sum of one launch), scaled by
+# chains or token-heads; on these small cases part of what a stage has written is still in the L2 when it ends.
+SHORT16_TRAFFIC_BYTES_PER_CHAIN = 140_100   # profiles/short16_kernel_B128xT16xH32.md (T = 16, fp32 state in and out)
+# operands, recurrence: profiles/operands_kernel_recur_kernel_B8xT1024xH16.md; prepare, scan (two-stage form):
+# profiles/prepare_pipe_kernel_prepare_tc4_kernel_B8xT1024xH16.md, profiles/prepare_kernel_scan2_kernel_B8xT1024xH16.md
+TRAFFIC_BYTES_PER_TOKEN_HEAD = {"operands": 1287, "recurrence": 1352, "prepare": 1774, "scan": 1313}
 
 if __name__ == "__main__":
     main()

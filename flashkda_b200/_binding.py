@@ -80,6 +80,8 @@ def lib():
         L.fkda_debug_prepare_giveup.restype = ci
         L.fkda_debug_operands.argtypes = [ctypes.POINTER(FwdParams), ci, vp]
         L.fkda_debug_operands.restype = ci
+        L.fkda_debug_recurrence.argtypes = [ctypes.POINTER(FwdParams), vp]
+        L.fkda_debug_recurrence.restype = ci
         L.fkda_debug_recurrence_giveup.argtypes = [ctypes.POINTER(FwdParams), ci, ci, vp]
         L.fkda_debug_recurrence_giveup.restype = ci
         if hasattr(L, "fkda_debug_umma_bench"):        # builds made with -DFKDA_TUNING only
@@ -362,6 +364,14 @@ def operands(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, cu_seqle
     with torch.cuda.device(q.device):
         _check(lib().fkda_debug_operands(ctypes.byref(p), int(wait_limit_us), _stream(q)))
     return ws
+
+
+def recurrence(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state=None, final_state=None, cu_seqlens=None, *,
+               workspace, flags=0):
+    """Test and measuring aid: what follows `operands` in a call of the default path, over the records it left in `workspace`."""
+    p, ws = _params(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state, final_state, cu_seqlens, workspace, flags)
+    with torch.cuda.device(q.device):
+        _check(lib().fkda_debug_recurrence(ctypes.byref(p), _stream(q)))
 
 
 def recurrence_giveup(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state=None, final_state=None,

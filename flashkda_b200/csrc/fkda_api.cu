@@ -363,9 +363,9 @@ int plan_slice(int64_t chains, int64_t chunks, int sms) {
   return static_cast<int>(c - second);
 }
 
-// What the test entry points ask of do_compact: to end behind the token-parallel stage, and a wait that nothing completes.
+// What the test entry points ask of do_compact: one of its stages alone, and a wait that nothing completes.
 struct TestAid {
-  bool operands_only;
+  bool operands, recurrence;
   int wait_limit_us;       // 0: nothing is held back
   int stop_copies_after;   // records per CTA of the recurrence, or (negative) maps of the chaining of runs
 };
@@ -389,20 +389,20 @@ int do_compact(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream, c
   const bool whole = (p->flags & FKDA_FLAG_SCAN_NO_SEGMENTS) != 0, one_item = (p->flags & FKDA_FLAG_OPERANDS_PER_ITEM) != 0;
   const int rows = runs > 1 || whole ? 0 : chains * 4 <= sms ? 32 : chains * 2 <= sms ? 64 : 0;
   fkda::PrepParams q = prep_params(p, L);
-  const int slice = p->cu_seqlens || runs > 1 || rows || whole || one_item ? 0 : plan_slice(chains, q.seq_chunks, sms);
+  const bool one_stage = aid != nullptr && !(aid->operands && aid->recurrence);
+  const int slice = p->cu_seqlens || runs > 1 || rows || whole || one_item || one_stage ? 0 : plan_slice(chains, q.seq_chunks, sms);
   if (slice) q.slice_chunks = slice;
-  if (aid != nullptr && aid->operands_only) {
-    q.slice_chunks = q.seq_chunks;
+  if (aid != nullptr && !aid->recurrence) {
     q.wait_limit_us = aid->wait_limit_us;
     q.first_load_only = aid->wait_limit_us > 0;
   }
-  e = fkda::launch_operands(q, one_item, stream);
+  if (aid == nullptr || aid->operands) e = fkda::launch_operands(q, one_item, stream);
   if (e != cudaSuccess) return cuda_fail(e, "token-parallel launch");
-  if (aid != nullptr && aid->operands_only) return FKDA_OK;
+  if (aid != nullptr && !aid->recurrence) return FKDA_OK;
   fkda::ScanParams s = scan_params(p, L);
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p->v);
   if (aid != nullptr) {
-    (aid->stop_copies_after > 0 ? s.wait_limit_us : s.map_wait_limit_us) = aid->wait_limit_us;
+    (aid->stop_copies_after < 0 ? s.map_wait_limit_us : s.wait_limit_us) = aid->wait_limit_us;
     s.stop_copies_after = aid->stop_copies_after > 0 ? aid->stop_copies_after : 0;
     s.stop_maps_after = aid->stop_copies_after < 0 ? -aid->stop_copies_after : 0;
   }
@@ -628,7 +628,15 @@ int fkda_debug_operands(const fkda_fwd_params* p, int wait_limit_us, void* cuda_
   int rc = validate(p, &L);
   if (rc != FKDA_OK) return rc;
   if (wait_limit_us < 0 || wait_limit_us > 1000000) return fail(FKDA_ERR_INVALID_ARGUMENT, "0 <= wait_limit_us <= 1000000 required");
-  const TestAid aid{true, wait_limit_us, 0};
+  const TestAid aid{true, false, wait_limit_us, 0};
+  return do_compact(p, L, static_cast<cudaStream_t>(cuda_stream), &aid);
+}
+
+int fkda_debug_recurrence(const fkda_fwd_params* p, void* cuda_stream) {
+  Layout L;
+  int rc = validate(p, &L);
+  if (rc != FKDA_OK) return rc;
+  const TestAid aid{false, true, 0, 0};
   return do_compact(p, L, static_cast<cudaStream_t>(cuda_stream), &aid);
 }
 
@@ -638,7 +646,7 @@ int fkda_debug_recurrence_giveup(const fkda_fwd_params* p, int stop_copies_after
   if (rc != FKDA_OK) return rc;
   if (stop_copies_after == 0 || wait_limit_us < 1 || wait_limit_us > 1000000)
     return fail(FKDA_ERR_INVALID_ARGUMENT, "stop_copies_after != 0 and 1 <= wait_limit_us <= 1000000 required");
-  const TestAid aid{false, wait_limit_us, stop_copies_after};
+  const TestAid aid{true, true, wait_limit_us, stop_copies_after};
   return do_compact(p, L, static_cast<cudaStream_t>(cuda_stream), &aid);
 }
 

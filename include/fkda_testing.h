@@ -48,6 +48,10 @@ int fkda_debug_prepare_giveup(const fkda_fwd_params* p, int wait_limit_us, void*
  * fkda_debug_prepare_giveup (a CTA has a second item once the call has more than two items per SM). */
 int fkda_debug_operands(const fkda_fwd_params* p, int wait_limit_us, void* cuda_stream);
 
+/* The rest of the default path alone, over the records that fkda_debug_operands left in the workspace: the recurrence and, in
+ * packed batches, what goes with it.  (In one piece also where the whole call goes through in two time slices.) */
+int fkda_debug_recurrence(const fkda_fwd_params* p, void* cuda_stream);
+
 /* The give-up path of the default path's recurrence, in whichever form the sizes select: the whole call, in which the copies of
  * every CTA of the recurrence stop after `stop_copies_after` records (negative: those of the kernel that chains the maps of
  * runs after -stop_copies_after maps) and the waits of that kernel give up after `wait_limit_us` microseconds. */

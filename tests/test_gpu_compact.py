@@ -43,8 +43,13 @@ def test_compact_path_matches_the_recurrence(name):
     assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS and rel_fro(out.cpu(), o64) <= 1e-2
     if fin is not None:
         assert rel_fro(fin.cpu(), s64) <= STATE_REL
-    # and again through the plain call: same bits
+    # and again through the plain call, and stage by stage: same bits
     first, first_fin = out.clone(), None if fin is None else fin.clone()
+    out.fill_(float("nan"))
+    F.operands(*args, cu_seqlens=xc["cu_seqlens"], workspace=ws)
+    F.recurrence(*args, workspace=ws, **kw)
+    assert F.read_status(ws) == 0
+    assert torch.equal(out.view(torch.int16), first.view(torch.int16)) and (fin is None or torch.equal(fin, first_fin))
     F.fwd(*args, **kw)
     assert torch.equal(out.view(torch.int16), first.view(torch.int16)) and (fin is None or torch.equal(fin, first_fin))
 
@@ -101,6 +106,19 @@ def test_a_wait_in_operands_kernel_gives_up_and_the_context_stays_usable():
         F.fwd(*args, final_state=x["final_state"], workspace=ws)
         assert F.read_status(ws) == 0
         assert torch.equal(x["out"].view(torch.int16), out.view(torch.int16)) and torch.equal(x["final_state"], fin)
+
+
+def test_benchmark_counts_the_kernels_that_a_call_launches():
+    """bench.py's count, from a graph captured around a call: one kernel for a step of a few tokens, two for a prefill, four with
+    runs (two passes and the chaining of their maps), three in a packed batch plus the one for its decode tokens."""
+    from bench import kernels_per_call, make_caller
+    for w, n in ((Workload("k", H=4, B=3, T=1, state_out="fp32"), 1), (Workload("k", H=4, B=3, T=300, state_out="fp32"), 2),
+                 (Workload("k", H=2, T=32 * 700, state_out="fp32"), 4), (Workload("k", H=4, seq_lens=[300, 1, 70], state_out="fp32"), 4)):
+        x = make_inputs(w, device="cuda")
+        ws = torch.empty(F.get_workspace_size(x["q"].shape[0] * x["q"].shape[1], w.H, w.N), dtype=torch.uint8, device="cuda")
+        call = make_caller(F, x, ws, 0)
+        call()
+        assert kernels_per_call(call) == n, w
 
 
 GIVEUP = {
