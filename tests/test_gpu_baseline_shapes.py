@@ -76,11 +76,12 @@ def test_config4_short_B512_T16_H32():
     run_and_sample(w, [(0, 0), (255, 13), (511, 31)])
 
 
-def test_many_equal_chains_take_the_compact_kernel_by_default():
-    """Fixed-length batch with more chains than SMs and T > 160: the automatic choice of the two-CTAs-per-SM
-    recurrence kernel, on default flags and the default per-call workspace allocation."""
+@pytest.mark.parametrize("flags", [0, F.FLAG_PREPARE_MMA_SYNC], ids=["default", "two_stage"])
+def test_many_equal_chains(flags):
+    """Fixed-length batch with more chains than SMs and more than 24 chunks each: by default one CTA per chain in more than
+    one round, on the default per-call workspace allocation; in the two-stage form the two-CTAs-per-SM recurrence kernel."""
     w = Workload("many", H=32, B=6, T=1024 + 19, state_in="bf16", state_out="bf16", seed=41)
-    run_and_sample(w, [(0, 0), (5, 31), (3, 9)], default_alloc=True)
+    run_and_sample(w, [(0, 0), (5, 31), (3, 9)], flags=flags, default_alloc=flags == 0)
 
 
 def test_H96_T8192():

@@ -179,32 +179,35 @@ def test_varlen_matrix(seq_lens, state):
     check_against_f64(x, out, fin, f"varlen{seq_lens}-{state}")
 
 
-@pytest.mark.parametrize("kernel", ["default", "short", "lookahead", "plain"])
+@pytest.mark.parametrize("kernel", ["default", "compact_records", "short", "lookahead", "plain"])
 @pytest.mark.parametrize("B,T,state", [(300, 16, "fp32"), (37, 33, "bf16"), (5, 64, "fp32"), (200, 1, None), (3, 32, "bf16"),
                                        (70, 9, "bf16"), (33, 16, None)])
 def test_short_chains_all_scan_kernels(B, T, state, kernel):
-    """By default sequences of at most 16 tokens go to the fused short-sequence kernel and those of at most two
-    chunks to the persistent short-chain kernel; the other recurrence kernels must give the same answers on the
-    same shapes ("short": the two-kernel path with the persistent short-chain kernel also for T <= 16)."""
-    flags = {"default": 0, "short": F.FLAG_NO_FUSED_SHORT, "lookahead": F.FLAG_SCAN_LOOKAHEAD, "plain": F.FLAG_SCAN_PLAIN}[kernel]
+    """By default sequences of at most 32 tokens go to the per-token or the tile kernel; the two kernels of the default path
+    and the recurrence kernels of the two-stage form must give the same answers on the same shapes ("short": stage by stage,
+    where sequences of at most two chunks go to the persistent short-chain kernel)."""
+    flags = {"default": 0, "compact_records": F.FLAG_NO_FUSED_SHORT, "lookahead": F.FLAG_SCAN_LOOKAHEAD, "plain": F.FLAG_SCAN_PLAIN}.get(kernel)
     w = Workload("s", H=3, B=B, T=T, state_in=state, state_out=state or "fp32", state_std=0.5, seed=B + T)
     x = make_inputs(w)
     fin_dtype = torch.bfloat16 if state == "bf16" else torch.float32
-    out, fin = run_gpu(x, fin_dtype, flags)
+    out, fin = run_two_stage(x, fin_dtype) if flags is None else run_gpu(x, fin_dtype, flags)
     check_against_f64(x, out, fin, f"short-B{B}xT{T}-{state}-{kernel}")
 
 
 @pytest.mark.parametrize("T,state", [(65, "fp32"), (96, "bf16"), (129, "fp32"), (160, None)])
 def test_many_chains_of_up_to_five_chunks(T, state):
-    """More chains than SMs and at most five chunks each: the persistent short-chain kernel takes these too; same
-    answers as the look-ahead kernel and the fp64 recurrence."""
+    """More chains than SMs and at most five chunks each: the persistent form of the default recurrence, and stage by stage
+    the persistent short-chain kernel; same answers as the look-ahead kernel and the fp64 recurrence."""
     w = Workload("s5", H=4, B=40, T=T, state_in=state, state_out=state or "fp32", state_std=0.5, seed=T, lower_bound=-1.0)
     x = make_inputs(w)
     dt = torch.bfloat16 if state == "bf16" else torch.float32
     o1, s1 = run_gpu(x, dt)
     check_against_f64(x, o1, s1, f"160 chains of T={T}, {state} state")
+    o2, s2 = run_two_stage(x, dt)
+    check_against_f64(x, o2, s2, f"160 chains of T={T}, {state} state, stage by stage")
     o0, s0 = run_gpu(x, dt, F.FLAG_SCAN_LOOKAHEAD)
-    assert max_abs(o1, o0) <= 1e-2 and rel_fro(s1, s0) <= (2e-2 if state == "bf16" else 5e-3)
+    for o, s in ((o1, s1), (o2, s2)):
+        assert max_abs(o, o0) <= 1e-2 and rel_fro(s, s0) <= (2e-2 if state == "bf16" else 5e-3)
 
 
 @pytest.mark.parametrize("B,T", [(2, 64), (2, 1024), (4, 256), (8, 128), (64, 16)])
@@ -253,11 +256,11 @@ def test_state_handoff_split_equals_unsplit():
     assert rel_fro(s2, s_all) <= 2e-3
 
 
-@pytest.mark.parametrize("flags", [F.FLAG_SCAN_NO_SEGMENTS, 0], ids=["whole_sequences", "planned_runs"])
+@pytest.mark.parametrize("flags", [F.FLAG_SCAN_LOOKAHEAD, F.FLAG_SEGMENTS(5), F.FLAG_SCAN_NO_SEGMENTS, 0],
+                         ids=["lookahead", "two_stage_runs", "one_cta_per_chain", "chain_split_over_four"])
 def test_long_chains_repeated_calls_stay_in_step(flags):
-    """Long chains exercise every barrier of the look-ahead kernel thousands of times; repeated calls must never
-    trip a bounded wait (status 0) and must be bit-reproducible (no race on tensor- or shared memory).  With 32
-    chains the planner would cut the sequences into runs: both forms are walked."""
+    """Long chains exercise every barrier of a recurrence kernel thousands of times; repeated calls must never
+    trip a bounded wait (status 0) and must be bit-reproducible (no race on tensor- or shared memory)."""
     w = Workload("long", H=16, B=2, T=4096, state_in="fp32", state_out="fp32", seed=99)
     x = make_inputs(w)
     ref = None

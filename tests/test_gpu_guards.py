@@ -100,11 +100,17 @@ def test_varlen_tail_rows_and_guard_bands(seq_lens, form):
     run_guarded(w, surplus_rows=41, flags=FORMS[form])
 
 
-@pytest.mark.parametrize("B,T,flags", [(5, 16, 0), (7, 23, 0), (4, 9, F.FLAG_NO_FUSED_SHORT), (9, 50, 0), (3, 33, 0), (40, 129, 0),
-                                       (200, 150, 0), (2, 300, 0)],
-                         ids=["fused16", "fused23", "short9", "short50", "short33", "fixed129", "manyshort150", "fixed300"])
+MMA = F.FLAG_PREPARE_MMA_SYNC          # the two-stage form
+
+
+@pytest.mark.parametrize("B,T,flags", [(5, 3, 0), (100, 3, 0), (5, 16, 0), (7, 23, 0), (4, 9, F.FLAG_NO_FUSED_SHORT), (9, 50, 0), (30, 33, 0),
+                                       (60, 129, 0), (40, 900, 0), (1, 6000, 0), (4, 9, MMA | F.FLAG_NO_FUSED_SHORT), (9, 50, MMA),
+                                       (200, 150, MMA), (2, 300, MMA)],
+                         ids=["step_quarters", "step_whole", "fused16", "fused23", "split4_9", "split4_50", "split2_33", "persistent129", "one_cta900",
+                              "runs6000", "two_stage_short9", "two_stage_short50", "two_stage_manyshort150", "two_stage_fixed300"])
 def test_fixed_length_guard_bands(B, T, flags):
-    """Fixed-length forms (fused short-sequence kernel, persistent short-chain kernel, short-chunk prepare, plain path)
-    with partial last chunks: guard bands around out, final state and workspace stay untouched."""
+    """Fixed-length forms (per-token and tile kernel, split, persistent and one-CTA recurrence, runs; in the two-stage form the
+    short-chunk prepare and the persistent short-chain kernel) with partial last chunks: guard bands around out, final state and
+    workspace stay untouched."""
     w = Workload("guardf", H=3, B=B, T=T, state_in="fp32", state_out="fp32", state_std=0.5, seed=B * 1000 + T)
     run_guarded(w, surplus_rows=0, flags=flags)

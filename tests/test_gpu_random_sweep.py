@@ -2,8 +2,8 @@
 
 Complements the fixed matrices of test_gpu_fwd.py (which follow the reference's tests/test_fwd_full.py:48-205): every
 case draws batch / length / heads / varlen mix / state dtypes / lower bound / gate scale at random, so that kernel
-selection (fused short-sequence kernel, persistent short-chain scan, look-ahead scan, segment-parallel scan, short-chunk
-prepare) and ragged edges meet in combinations nobody wrote down."""
+selection (per-token and tile kernel, split and persistent recurrence, runs; stage by stage the scan kernels) and ragged edges meet
+in combinations nobody wrote down."""
 import random
 
 import pytest
@@ -11,7 +11,7 @@ import torch
 
 import flashkda_b200 as F
 from flashkda_b200.workloads import Workload, make_inputs
-from test_gpu_fwd import check_against_f64, run_gpu
+from test_gpu_fwd import check_against_f64, run_gpu, run_two_stage
 
 pytestmark = pytest.mark.gpu
 
@@ -28,7 +28,7 @@ def draw_case(seed):
     elif kind == "fixed":
         B, T, seq = rng.randint(1, 6), rng.randint(71, 700), None
     elif kind == "fixed_long":
-        B, T, seq = 1, rng.randint(1536, 2600), None            # few long chains: the planner cuts them into runs
+        B, T, seq = 1, rng.randint(3072, 5200), None            # few long chains: the planner cuts them into runs
         H = rng.choice([1, 2, 4])
     elif kind == "varlen":
         seq = [rng.randint(1, 400) for _ in range(rng.randint(1, 6))]
@@ -41,13 +41,16 @@ def draw_case(seed):
     return w, rng
 
 
+@pytest.mark.parametrize("form", ["whole_call", "stage_by_stage"])
 @pytest.mark.parametrize("seed", range(48))
-def test_random_case(seed):
+def test_random_case(seed, form):
     w, rng = draw_case(seed)
+    if w.name.endswith("fixed_long"):
+        assert F.plan_segments(w.H, (w.T + 31) // 32)[0] > 1
     x = make_inputs(w)
     if rng.random() < 0.3:       # gates near the ends of their range
         x["g"] = torch.full_like(x["g"], rng.choice([-6.0, 6.0]))
     fin_dtype = {None: None, "bf16": torch.bfloat16, "fp32": torch.float32}[w.state_out]
-    out, fin = run_gpu(x, fin_dtype)
+    out, fin = (run_gpu if form == "whole_call" else run_two_stage)(x, fin_dtype)
     big = x["initial_state"] is not None and w.state_std > 0.1
     check_against_f64(x, out, fin, w.name, big_state=big and x["initial_state"].float().abs().max() > 100)

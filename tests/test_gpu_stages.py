@@ -50,7 +50,7 @@ def test_prologue_kernel():
 @pytest.mark.parametrize("kernel", ["mma_sync", "tcgen05_cta_per_item", "tcgen05_pipelined"])
 @pytest.mark.parametrize("case", ["fixed", "varlen", "strong_decay"])
 def test_prepare_records_match_fp64_operands(case, kernel):
-    """Operand records of the three token-parallel kernels (the default pipelined TMA + tcgen05 one, its
+    """Operand records of the two-stage form's three token-parallel kernels (the pipelined TMA + tcgen05 one, its
     one-CTA-per-item form and the mma.sync one) against the fp64 chunk operands of the oracle."""
     flags = {"mma_sync": F.FLAG_PREPARE_MMA_SYNC, "tcgen05_cta_per_item": F.FLAG_PREPARE_TCGEN05, "tcgen05_pipelined": 0}[kernel]
     if case == "fixed":
