@@ -2,7 +2,9 @@
 
 Python host side of the drop-in boundary: mirrors flash_kda/__init__.py:5-41 and the argument
 checks of csrc/flash_kda.cpp:44-174 of the reference, then calls the C-ABI library
-(include/fkda.h) through ctypes with raw device pointers and torch's current CUDA stream.
+(include/fkda.h) with raw device pointers and torch's current CUDA stream: an ordinary call through a
+small CPython extension (csrc/fkda_host.cpp), every other one, and all of them where that extension
+does not fit the running torch, through ctypes.
 There is no CPU or PyTorch fallback: without the compiled library, or without a CUDA device,
 `fwd` raises.
 """

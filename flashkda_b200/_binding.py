@@ -1,4 +1,4 @@
-"""ctypes binding of libfkda.so and the torch-facing wrappers.
+"""Binding of libfkda.so (native host path for the ordinary call, ctypes for the rest) and the torch-facing wrappers.
 
 `fwd` keeps the reference's Python signature (flash_kda/__init__.py:5) and error behaviour:
 every argument problem raises RuntimeError before anything is launched (the reference's

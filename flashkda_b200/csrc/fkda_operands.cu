@@ -7,11 +7,15 @@
 //   warp  9      loads of the next item, stores of the record, tril(M)
 //   warp  11     row norms from the partial sums of the element warps; first products [A; M] = [k+; q+] k-^T on tcgen05
 //
-// 770 bytes read and 912 written per token-head: 0.27 ms of HBM time on a million token-heads.  It takes 0.374 ms
-// (4.7 TB/s), where the kernel of the larger record (fkda_prepare_tc.cu, 2130 bytes) takes 0.489.  What bounds it is
-// instruction issue: 6.6 thousand warp instructions per item at two per cycle and SM.  The sixteen element warps of
-// an SM run the same 6 KB of code, which the sub-partitions' instruction caches hold; the long straight-line inverse is kept
-// to one warp per item and spread over two sub-partitions.
+// 770 bytes read and 912 written per token-head: 0.27 ms of HBM time on a million token-heads.  Alone it takes 0.384 ms
+// in a burst of calls (4.6 TB/s) and 0.410 kept up under the power cap, where the kernel of the larger record
+// (fkda_prepare_tc.cu, 2130 bytes) takes 0.489.  What bounds it is latency: no unit of the SM is full (8 x 1024 tokens x
+// 16 heads: issue slots 49 %, shared-memory pipe 38, special functions 27, tensor cores 16), and with six warps to a scheduler
+// one on average has something to issue.  A warp spends a third of its time in waits for hand-offs and tiles - an
+// element warp has three rendezvous per item: tiles, norms, the first products of the item before - and a seventh in the
+// latencies of dependent instructions.  The sixteen element warps of an SM run the same 6 KB of code, which the
+// sub-partitions' instruction caches hold; the long straight-line inverse is kept to one warp per item and spread over two
+// sub-partitions.
 //
 // Decay ranges: with G the running log2 decay inside the chunk and P its value after the first 16 tokens, the first products
 // use k+ = khat 2^(G - P) and k- = khat 2^(P - G): both stay inside 2^(+-115.4) for lower_bound >= -5 (16 tokens x 5 x

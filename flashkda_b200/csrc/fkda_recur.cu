@@ -19,7 +19,7 @@
 // which keeps the tensor cores from them for about 50 cycles, and the latencies in between: 2470 cycles per chunk (1720
 // with the output products left out).  Two warps of 16 rows per sub-partition read every operand twice as often and end at
 // the shared-memory pipe (2650); the output products on mma.sync in the output warps: 2700.  4 x 8192 tokens x 32 heads, fp32
-// state: 0.340 ms over records of 0.96 GB (4.4 TB/s).
+// state, over records of 0.96 GB: 0.357 ms in a burst of calls (4.2 TB/s), 0.382 kept up under the power cap.
 //
 // Warps 0-3: recurrence; 4-7: output, and one of them each the output products and the copies.  The code of a
 // recurrence warp and of the output warp on the same SM sub-partition together stay near 8 KB: beyond that a sub-partition's

@@ -3,10 +3,10 @@
 // The reference walks every (sequence, head) chain with one CTA from the first chunk to the last
 // (csrc/smxx/fwd_kernel2.cuh:434-742), so a call with fewer chains than SMs leaves most of the GPU idle.  A run
 // of chunks acts on the state Z = S^T ([v][k]) as an affine map, Z_end = Z_start M + N, because every chunk does
-//     Z' = Z (diag(e) - w'^T kr) + u'^T kr .
-// Here each sequence is cut into runs; a recurrence kernel itself (the look-ahead or the compact one, whichever gets
-// the pass's CTAs through faster) produces M (walk from the identity with u' = 0) and N (walk from zero) of the inner
-// runs in parallel, this file chains them into the state at the start of every run, and a second launch of a
+//     Z' = Z (diag(e) - w'^T kr) + u'^T kr ,          w' = T diag(beta) k+,  u' = T diag(beta) v .
+// Here each sequence is cut into runs; a recurrence kernel itself (recur_kernel over compact records; in the two-stage form
+// the look-ahead or the compact one, whichever gets the pass's CTAs through faster) produces M (walk from the identity with
+// v = 0) and N (walk from zero) of the inner runs in parallel, this file chains them into the state at the start of every run, and a second launch of a
 // recurrence kernel walks all runs in parallel from those states.
 #include "fkda_common.cuh"
 

@@ -19,8 +19,8 @@
 //
 // What bounds it: HBM, as far as the CTAs of an SM cover each other's phases - two of them with fp32 state; four with bf16 and
 // one block, for which the operands lie over the staged inputs (three beside them: 302 us below).
-// 512 x 32 chains of 16 tokens: 435 us with fp32 states (5.7 TB/s), 270 us with bf16 (5.2 TB/s).  With fewer CTAs and the
-// earlier order of the phases: 506 and 350 with the states asked
+// 512 x 32 chains of 16 tokens, twenty calls in a row: 436 us with fp32 states (5.7 TB/s), 273 us with bf16 (5.2 TB/s); kept
+// up under the power cap 465 and 305.  In a row too, with fewer CTAs and the earlier order of the phases: 506 and 350 with the states asked
 // for ahead of the inputs, whose 16 KB then queue behind them; 460 and 402 with w' = TB k+, u' = TB v formed before the state
 // was touched (a rendezvous more, and two CTAs per SM for either type).  Asking the L2 for the next chain's state: slower.
 #include "fkda_common.cuh"

@@ -14,8 +14,8 @@
 // the call's intermediate results, and when the recurrence starts, all that came before the call is complete.  One CTA waits for
 // the recurrence at its end, so that a kernel that waits for this one waits for both.
 //
-// What bounds it: the stream over the states at one token (512 x 32 chains: 171 us with bf16 states, 323 with fp32: 97 and
-// 102 % of the measured copy rate; the tile kernel takes 330 and 470), then the shared-memory pipe: 840 cycles per token,
+// What bounds it: the stream over the states at one token (512 x 32 chains: 173 us with bf16 states, 324 with fp32:
+// 6.3 and 6.7 TB/s, the measured copy rate; the tile kernel, whose time hardly depends on the tokens, 273 and 425), then the shared-memory pipe: 840 cycles per token,
 // chain and SM, 512 of them the reads of the vectors, 230 the shuffles.  Above kStepMaxT the tile form
 // (fkda_short16.cu) takes over.
 #include "fkda_common.cuh"
