@@ -121,6 +121,33 @@ def test_benchmark_counts_the_kernels_that_a_call_launches():
         assert kernels_per_call(call) == n, w
 
 
+@pytest.mark.parametrize("w", [Workload("d", H=4, B=3, T=1, state_in="fp32", state_out="fp32"), Workload("p", H=3, B=2, T=300, state_out="fp32"),
+                               Workload("s", H=80, T=32 * 128, state_out="fp32"), Workload("r", H=2, T=32 * 700, state_out="fp32"),
+                               Workload("v", H=12, seq_lens=[1, 40, 4, 300, 1, 33], state_in="bf16", state_out="bf16")],
+                         ids=["decode", "prefill", "two_slices", "runs", "packed_with_decode"])
+def test_captured_call_replays_on_new_inputs(w):
+    """The plain call in a CUDA graph (scratch memory from the graph's pool, kernels that start beside their predecessors):
+    replays on other inputs in the same buffers give the bits of ordinary calls."""
+    x = make_inputs(w, device="cuda")
+    args = (x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"])
+    kw = dict(initial_state=x["initial_state"], final_state=x["final_state"], cu_seqlens=x["cu_seqlens"])
+    F.fwd(*args, **kw)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        F.fwd(*args, **kw)
+    for seed in (1, 2):
+        gen = torch.Generator(device="cuda").manual_seed(seed)
+        for name in ("q", "k", "v", "g", "beta"):
+            x[name].copy_(torch.randn(x[name].shape, generator=gen, device="cuda"))
+        F.fwd(*args, **kw)
+        out, fin = x["out"].clone(), x["final_state"].clone()
+        x["out"].fill_(float("nan"))
+        x["final_state"].fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(x["out"].view(torch.int16), out.view(torch.int16)) and torch.equal(x["final_state"], fin)
+
+
 GIVEUP = {
     "split4": (Workload("g", H=3, B=2, T=200, state_in="fp32", state_out="fp32", seed=1), 2),
     "split2": (Workload("g", H=25, B=2, T=200, state_out="fp32", seed=2), 3),
