@@ -42,6 +42,15 @@ __device__ __forceinline__ uint32_t round_bf(f2 x) {
   return pack_bf16(a, b);
 }
 
+// x0, x1 = hi + lo, both fp16 pairs (22 bits of a tanh)
+__device__ __forceinline__ void split_f16(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 back = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x0 - back.x, x1 - back.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
 // D(16x8,f32) += A(16x16,f16,row) * B(16x8,f16,col)
 __device__ __forceinline__ void mma_f16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -108,11 +117,7 @@ __device__ __forceinline__ void gate_sums(const uint32_t (&gw)[4], const Const& 
       if (8 * b + 2 * t >= len) x0 = -1.f;
       if (8 * b + 2 * t + 1 >= len) x1 = -1.f;
     }
-    const __half2 h = __floats2half2_rn(x0, x1);
-    const float2 back = __half22float2(h);
-    const __half2 l = __floats2half2_rn(x0 - back.x, x1 - back.y);
-    hi[b] = *reinterpret_cast<const uint32_t*>(&h);
-    lo[b] = *reinterpret_cast<const uint32_t*>(&l);
+    split_f16(x0, x1, hi[b], lo[b]);
   }
   const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
   const f2 h2 = pk(hgs, hgs);

@@ -190,11 +190,7 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
             if (8 * b + 2 * t4 >= len) x0 = -1.f;
             if (8 * b + 2 * t4 + 1 >= len) x1 = -1.f;
           }
-          const __half2 hh = __floats2half2_rn(x0, x1);
-          const float2 back = __half22float2(hh);
-          const __half2 ll = __floats2half2_rn(x0 - back.x, x1 - back.y);
-          hi[b] = *reinterpret_cast<const uint32_t*>(&hh);
-          lo[b] = *reinterpret_cast<const uint32_t*>(&ll);
+          split_f16(x0, x1, hi[b], lo[b]);
         }
         const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
         float d[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};

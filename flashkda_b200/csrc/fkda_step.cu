@@ -19,6 +19,7 @@
 // chain and SM, 512 of them the reads of the vectors, 230 the shuffles.  Above kStepMaxT the tile form
 // (fkda_short16.cu) takes over.
 #include "fkda_common.cuh"
+#include "fkda_elem.cuh"
 
 namespace fkda {
 namespace step {
@@ -47,26 +48,14 @@ struct Params {
   float gate_scale;      // lower_bound * log2(e)
 };
 
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
+using elem::f2;
+using elem::fma2;
+using elem::mul;
+using elem::pk;
 __device__ __forceinline__ float sum2(f2 x) {
   float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+  elem::upk(x, a, b);
   return a + b;
-}
-__device__ __forceinline__ f2 mul(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
