@@ -50,7 +50,8 @@ typedef enum fkda_state_dtype { FKDA_STATE_NONE = 0, FKDA_STATE_BF16 = 1, FKDA_S
 /* Selects the two-stage form (fkda_prepare, fkda_scan) with its token-parallel stage on prepare_tc4_kernel, the
  * one-CTA-per-item form of the pipelined TMA + tcgen05 kernel that fkda_prepare runs without a flag
  * (csrc/fkda_prepare_tc.cu; same operand records; at most 65535 sequences of at most 65535 chunks each for equal lengths,
- * else the call fails). */
+ * else the call fails).  This flag and the next leave fixed lengths of at most 32 tokens to the fused kernels unless
+ * FKDA_FLAG_NO_FUSED_SHORT is given too. */
 #define FKDA_FLAG_PREPARE_TCGEN05 0x80u
 /* The two-stage form with its token-parallel stage on prepare_kernel (vectorised global loads, mma.sync products).  Same
  * operand records. */
