@@ -7,8 +7,7 @@
 //   * running sums of the gate: a product with a triangle of ones.  The summand is tanh in [-1, 1], split into two fp16
 //     parts (22 bits, products exact, fp32 accumulation), read by a transposing ldmatrix in the B-fragment layout.
 // In the row-per-lane layout these took 19 instructions per element (3 shuffles and 3 predicated adds per element for the
-// sums alone); here the whole stage is about 19 instructions per element, counting six decayed operands formed in fp32 with
-// packed arithmetic and rounded once.
+// sums alone).
 #pragma once
 #include <cuda_fp16.h>
 
@@ -58,27 +57,64 @@ __device__ __forceinline__ void mma_f16_16816(float (&c)[4], const uint32_t (&a)
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// What a thread keeps over all chunks: the triangle of ones as A fragments, one sign per sub-block.  Exponents are relative
-// to the boundary between the two 16-token sub-blocks: G_i = -sum of the tokens behind i up to the boundary in sub-block
-// 0, +sum of the tokens from the boundary up to i in sub-block 1.
+// The same onto zero (no registers to clear).
+__device__ __forceinline__ void mma_f16_16816_zero(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// D(16x8,f32) = A(16x8,bf16,row) * B(8x8,bf16,col), then D += ...
+__device__ __forceinline__ void mma_bf16_1688_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+}
+__device__ __forceinline__ void mma_bf16_1688(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(b));
+}
+
+// What a thread keeps over all chunks: the triangle of ones as A fragments, and the gate's constant part of the running sums.
+// (Opaque to the compiler, which would otherwise work them out again in every chunk to save the registers.)
 struct Const {
-  uint32_t tri[2][4];
-  float hc[4];              // gate_scale / 2 times the number of summands of token row g + 8 b (signed)
+  uint32_t tri[4];
+  float hc[2];              // gate_scale / 2 times the number of summands of row g + 8 b of a sub-block
   __device__ __forceinline__ Const(int lane, float hgs) {
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = g + 8 * (i & 1), k0 = 2 * t + 8 * (i >> 1);
-      tri[0][i] = (k0 > row ? 0xbc00u : 0u) | (k0 + 1 > row ? 0xbc000000u : 0u);       // -1
-      tri[1][i] = (k0 <= row ? 0x3c00u : 0u) | (k0 + 1 <= row ? 0x3c000000u : 0u);     // +1
+      tri[i] = (k0 <= row ? 0x3c00u : 0u) | (k0 + 1 <= row ? 0x3c000000u : 0u);
+      asm volatile("" : "+r"(tri[i]));
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int row = g + 8 * (b & 1);
-      hc[b] = hgs * static_cast<float>(b < 2 ? row - 15 : row + 1);
+    for (int b = 0; b < 2; ++b) {
+      hc[b] = hgs * static_cast<float>(g + 8 * b + 1);
+      asm volatile("" : "+f"(hc[b]));
     }
   }
 };
+
+// Shared memory by 32-bit address.
+__device__ __forceinline__ void sts_f32(uint32_t addr, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory"); }
+__device__ __forceinline__ void sts_f2(uint32_t addr, f2 x) { asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(x) : "memory"); }
+__device__ __forceinline__ float lds_f32(uint32_t addr) {
+  float x;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr) : "memory");
+  return x;
+}
+__device__ __forceinline__ int lds_s32(uint32_t addr) {
+  int x;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(x) : "r"(addr) : "memory");
+  return x;
+}
+__device__ __forceinline__ void sts_u4(uint32_t addr, uint32_t x) { asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(x) : "memory"); }
+__device__ __forceinline__ float4 lds_f4(uint32_t addr) {
+  float4 x;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(addr) : "memory");
+  return x;
+}
 
 // byte offset, inside a [32 tok][128 ch] tile of two 128-byte-swizzled [32 tok][64 ch] boxes, of the row that this lane
 // addresses in a ldmatrix.x4 over channel block cb (8 channels) and all 32 tokens
@@ -88,55 +124,68 @@ __device__ __forceinline__ uint32_t tile_off(int lane, int cb) {
 // the same in a core-matrix [32][128] operand
 __device__ __forceinline__ uint32_t core_row(int lane, int cb) { return static_cast<uint32_t>((lane >> 3) * 2048 + cb * 128 + (lane & 7) * 16); }
 
-// Partial sums of squares of the rows over this warp's channels: dst[row * 8], row = g + 8 b, written by one thread per row.
-__device__ __forceinline__ void row_squares(const uint32_t (&x)[2][4], float* dst, int lane) {
+// Partial sums of squares of the rows over this warp's channels, fp32 at dst + 32 row, row = g + 8 b, written by one thread per row.
+// (Products of depth 8: their operands are the registers as ldmatrix leaves them.)
+__device__ __forceinline__ void row_squares(const uint32_t (&x)[2][4], uint32_t dst, int lane) {
   const int g = lane >> 2;
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
-    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-    mma_bf16_16816(c0, x[0][2 * m], x[0][2 * m + 1], x[1][2 * m], x[1][2 * m + 1], x[0][2 * m], x[1][2 * m]);
-    mma_bf16_16816(c1, x[0][2 * m], x[0][2 * m + 1], x[1][2 * m], x[1][2 * m + 1], x[0][2 * m + 1], x[1][2 * m + 1]);
+    float c0[4], c1[4];
+    mma_bf16_1688_zero(c0, x[0][2 * m], x[0][2 * m + 1], x[0][2 * m]);
+    mma_bf16_1688_zero(c1, x[0][2 * m], x[0][2 * m + 1], x[0][2 * m + 1]);
+    mma_bf16_1688(c0, x[1][2 * m], x[1][2 * m + 1], x[1][2 * m]);
+    mma_bf16_1688(c1, x[1][2 * m], x[1][2 * m + 1], x[1][2 * m + 1]);
     if ((lane & 3) == (g >> 1)) {          // this thread holds the diagonal elements of rows g and g + 8
-      dst[(16 * m + g) * 8] = (g & 1) ? c0[1] : c0[0];
-      dst[(16 * m + 8 + g) * 8] = (g & 1) ? c1[3] : c1[2];
+      sts_f32(dst + (16 * m + g) * 32, (g & 1) ? c0[1] : c0[0]);
+      sts_f32(dst + (16 * m + 8 + g) * 32, (g & 1) ? c1[3] : c1[2]);
     }
   }
 }
 
 // Gate of one channel tile and its running sums: gw = transposed fragments (register b = tokens 8 b + 2 t, + 1 of channel g),
-// ha = exp(A_log) / 2, hab = ha * dt_bias of that channel.  G[b] = exponents of token g + 8 b, channels 2 t, + 1;
-// tot[m] = log2 decay of the whole sub-block m for those channels.  Tokens from `len` on do not decay.
-__device__ __forceinline__ void gate_sums(const uint32_t (&gw)[4], const Const& k, float ha, float hab, float hgs, int len, int lane, f2 (&G)[4],
+// ha = exp(A_log) / 2, hab = ha * dt_bias of that channel.  G[b] = exponents of token g + 8 b, channels 2 t, + 1, relative to
+// the boundary between the two 16-token sub-blocks (minus the sum of the tokens behind in sub-block 0, plus the sum up to it in
+// sub-block 1); tot[m] = log2 decay of the whole sub-block m for those channels.
+__device__ __forceinline__ void gate_sums(const uint32_t (&gw)[4], const Const& k, float ha, float hab, float hgs, int lane, f2 (&G)[4],
                                           f2 (&tot)[2]) {
-  const int t = lane & 3;
-  uint32_t hi[4], lo[4];
+  float th[8];
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
-    float x0 = tanh_approx(fmaf(bf_lo(gw[b]), ha, hab)), x1 = tanh_approx(fmaf(bf_hi(gw[b]), ha, hab));
-    if (len < kChunk) {
-      if (8 * b + 2 * t >= len) x0 = -1.f;
-      if (8 * b + 2 * t + 1 >= len) x1 = -1.f;
-    }
-    split_f16(x0, x1, hi[b], lo[b]);
+    th[2 * b] = tanh_approx(fmaf(bf_lo(gw[b]), ha, hab));
+    th[2 * b + 1] = tanh_approx(fmaf(bf_hi(gw[b]), ha, hab));
   }
-  const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
-  const f2 h2 = pk(hgs, hgs);
+  uint32_t hi[4], lo[4];
 #pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    float d[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
-    mma_f16_16816(d, k.tri[m], hi[2 * m], hi[2 * m + 1]);
-    mma_f16_16816(s, ones, hi[2 * m], hi[2 * m + 1]);
-    mma_f16_16816(d, k.tri[m], lo[2 * m], lo[2 * m + 1]);
-    mma_f16_16816(s, ones, lo[2 * m], lo[2 * m + 1]);
-    G[2 * m] = fma2(pk(d[0], d[1]), h2, pk(k.hc[2 * m], k.hc[2 * m]));
-    G[2 * m + 1] = fma2(pk(d[2], d[3]), h2, pk(k.hc[2 * m + 1], k.hc[2 * m + 1]));
-    tot[m] = fma2(pk(s[0], s[1]), h2, pk(16.f * hgs, 16.f * hgs));
-  }
+  for (int b = 0; b < 4; ++b) split_f16(th[2 * b], th[2 * b + 1], hi[b], lo[b]);
+  float d[2][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) mma_f16_16816_zero(d[m], k.tri, hi[2 * m], hi[2 * m + 1]);
+#pragma unroll
+  for (int m = 0; m < 2; ++m) mma_f16_16816(d[m], k.tri, lo[2 * m], lo[2 * m + 1]);
+  float x[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = fmaf(d[e >> 2][e & 3], hgs, k.hc[(e >> 1) & 1]);
+  const int last = lane | 28;              // the thread that holds the sums at token 15 of a sub-block for these channels
+  const float t0 = __shfl_sync(0xffffffffu, x[2], last), t1 = __shfl_sync(0xffffffffu, x[3], last);
+  tot[1] = pk(__shfl_sync(0xffffffffu, x[6], last), __shfl_sync(0xffffffffu, x[7], last));
+  tot[0] = pk(t0, t1);
+  G[0] = pk(x[0] - t0, x[1] - t1);
+  G[1] = pk(x[2] - t0, x[3] - t1);
+  G[2] = pk(x[4], x[5]);
+  G[3] = pk(x[6], x[7]);
 }
 __device__ __forceinline__ f2 exp2_pair(f2 x) {
   float a, b;
   upk(x, a, b);
   return pk(ex2f(a), ex2f(b));
+}
+// 1 / x for powers of two inside the operands' range: no negated exponent to form
+__device__ __forceinline__ f2 rcp_pair(f2 x) {
+  float a, b;
+  upk(x, a, b);
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(a));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(b));
+  return pk(a, b);
 }
 __device__ __forceinline__ f2 exp2_neg_pair(f2 x) {
   float a, b;

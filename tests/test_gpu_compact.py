@@ -238,3 +238,51 @@ def test_decode_tokens_among_prompts():
     assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS
     assert rel_fro(fin.cpu(), s64) <= STATE_REL
     assert torch.equal(fin[lens.index(0)].cpu(), x["initial_state"][lens.index(0)])
+
+
+@pytest.mark.parametrize("lens", [[33, 40, 1, 20, 97, 31], [47, 5, 63, 70, 16, 100, 17]])
+def test_rows_past_a_sequence_end_do_not_matter(lens):
+    """The last tile of a sequence holds the first rows of the next one: whatever these are, not-a-number included, the results of
+    the sequence are the same bits.  (Every other sequence is spoilt in turn.)"""
+    w = Workload("n", H=6, seq_lens=lens, state_in="fp32", state_out="fp32", seed=31)
+    x = make_inputs(w, device="cuda")
+
+    def call(q, k, v, g, beta):
+        out, fin = torch.zeros_like(x["v"]), torch.zeros_like(x["final_state"])
+        F.fwd(q, k, v, g, beta, x["scale"], out, x["A_log"], x["dt_bias"], x["lower_bound"], initial_state=x["initial_state"],
+              final_state=fin, cu_seqlens=x["cu_seqlens"], flags=F.FLAG_NO_FUSED_SHORT)
+        return out, fin
+
+    out, fin = call(*(x[n] for n in ("q", "k", "v", "g", "beta")))
+    ends = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    for spoilt in (0, 1):
+        bad = {n: x[n].clone() for n in ("q", "k", "v", "g", "beta")}
+        for i in range(spoilt, len(lens), 2):
+            for n in bad:
+                bad[n][:, ends[i]:ends[i + 1]] = float("nan") if i % 4 < 2 else float("inf")
+        o, f = call(*bad.values())
+        for i in range(1 - spoilt, len(lens), 2):
+            assert torch.equal(o[:, ends[i]:ends[i + 1]].view(torch.int16), out[:, ends[i]:ends[i + 1]].view(torch.int16)), (spoilt, i)
+            assert torch.equal(f[i], fin[i]), (spoilt, i)
+
+
+@pytest.mark.parametrize("T", [64, 75])
+def test_gate_parameters_at_the_ends_of_their_range(T):
+    """A gate whose slope underflows or overflows and biases that saturate it, in whole chunks and in the last one of a sequence
+    (whose absent tokens the kernel stands for by a gate input of minus infinity)."""
+    w = Workload("e", H=4, T=T, state_in="fp32", state_out="fp32", seed=32)
+    x = make_inputs(w)
+    x["A_log"] = torch.tensor([-100.0, 60.0, 1.0, 0.0])
+    x["dt_bias"][2, ::2] = 1e30
+    x["dt_bias"][2, 1::2] = -1e30
+    x["dt_bias"][3, ::2] = float("inf")
+    x["dt_bias"][3, 1::2] = -float("inf")
+    xc = to_cuda(x)
+    out, fin = torch.full_like(xc["v"], float("nan")), torch.full_like(xc["final_state"], float("nan"))
+    F.fwd(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"],
+          initial_state=xc["initial_state"], final_state=fin)
+    o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                     initial_state=x["initial_state"])
+    assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS
+    for h in range(4):
+        assert rel_fro(fin.cpu()[:, h], s64[:, h]) <= STATE_REL, h
