@@ -76,38 +76,49 @@ struct Layout {
 };
 
 // How many runs to cut each sequence of a batch into (1 = walk whole sequences), at most `most` of them, and their length in
-// chunks.  Pass 1 holds chains * (2 n - 3) CTAs and pass 2 chains * (n - 1), both walking ceil(chunks / n) chunks.  The one
-// planner: the workspace size, the launch and fkda_plan_segments ask here.  Its costs are those of the default path's kernels,
-// in hundredths of a microsecond, fitted to 124 calls of 1 to 40 heads and 129 to 4096 chunks, each cut in up to thirteen ways
-// (1.1 % off on average, 4.6 % at most): a chunk step of a chain split over four or two CTAs (fkda_recur_split.cu) or in one
-// CTA (fkda_recur.cu), the latter with and without outputs; what the two passes cost beside their steps, and every round of
-// CTAs after the first; the chaining of the maps per run and round of its CTAs.  (The two-stage form walks its runs by the same
-// plan.)  With more chains than a third of the SMs pass 1 alone would take more than one round; below 48 chunks the fixed costs
-// are all there is.
+// chunks.  The first pass has a CTA for every run but the last, which works out the run's map M and offset N; the second one a CTA
+// per run.  Where the gates' decay makes M vanish, which the first pass finds out (fkda_recur.cu), its two walks are a few chunks
+// long; where it does not, they are as long as the run and the maps are chained.  The plan is made for the former, among those that cost in the
+// latter at most a tenth more than whole sequences and a twelfth more than the best plan for it; of plans within 6 % and 3 us,
+// which is what the costs are off by, the one with the fewest runs.  The one planner: the workspace size, the launch and fkda_plan_segments ask here.
+// Its costs are those of the default path's kernels, in hundredths of a microsecond, fitted to 150 timed calls of 1 to 48
+// heads and 64 to 4096 chunks, half of them without decay: a chunk step of a chain split over four or two CTAs (fkda_recur_split.cu) or
+// in one CTA (fkda_recur.cu), the latter with and without outputs; the chunks that a map takes to vanish; what the passes cost
+// beside their steps, and every round of CTAs after the first; the chaining of the maps per run and round of its CTAs.  (The
+// two-stage form walks its runs by the same plan.)
 int plan_runs(int64_t chains, int64_t chunks, int64_t most, int sms, int* len) {
-  constexpr int64_t kQuad = 58, kHalf = 87, kOne = 132, kQuiet = 88, kPasses = 1100, kRound = 640, kChaining = 165, kMostRuns = 160;
+  constexpr int64_t kQuad = 59, kHalf = 87, kOne = 135, kQuiet = 95, kVanish = 9, kPasses = 1300, kRound = 640, kChaining = 160, kMostRuns = 160, kLeast = 10;
   *len = 0;
   if (chains <= 0 || chains * 3 > sms || chunks < 48) return 1;
   const int64_t whole = (chains * 4 <= sms ? kQuad : kHalf) * chunks;
   auto rounds = [&](int64_t ctas) { return (ctas + sms - 1) / sms; };
-  int64_t best = whole;
+  struct Cost { int64_t vanishing, lasting; };
+  auto cost = [&](int64_t n, int64_t l) {
+    const int64_t r1 = rounds(chains * (n - 1)), r2 = rounds(chains * n), common = r2 * kOne * l + kPasses + (r1 + r2 - 2) * kRound;
+    return Cost{common + r1 * 2 * kQuiet * (l < kVanish ? l : kVanish), common + r1 * 2 * kQuiet * l + kChaining * (n - 1) * rounds(chains * 16)};
+  };
+  int64_t least_lasting = INT64_MAX, best = INT64_MAX;
   int best_n = 1;
-  for (int64_t n = 3; n <= (most < kMostRuns ? most : kMostRuns); ++n) {
-    const int64_t l = (chunks + n - 1) / n;
-    if (l < 8) break;
-    if ((n - 1) * l >= chunks) continue;       // the last run would be empty
-    const int64_t r1 = rounds(chains * (2 * n - 3)), r2 = rounds(chains * (n - 1));
-    // run 0, the first CTA of a chain, has outputs: with the last chain's in the last round that round is a slow one
-    const bool slow_end = (chains - 1) * (2 * n - 3) >= (r1 - 1) * sms;
-    const int64_t pass1 = (slow_end ? (r1 - 1) * kQuiet + kOne : r1 * kQuiet) * l, pass2 = r2 * kOne * l;
-    const int64_t cost = pass1 + pass2 + kPasses + (r1 + r2 - 2) * kRound + kChaining * (n - 2) * rounds(chains * 16);
-    if (cost < best) {
-      best = cost;
-      best_n = static_cast<int>(n);
+  for (int pass = 0; pass < 3; ++pass) {
+    for (int64_t n = 3; n <= (most < kMostRuns ? most : kMostRuns); ++n) {
+      const int64_t l = (chunks + n - 1) / n;
+      if (l < kLeast) break;
+      if ((n - 1) * l >= chunks) continue;     // the last run would be empty
+      const Cost c = cost(n, l);
+      if (pass == 0) {
+        if (c.lasting < least_lasting) least_lasting = c.lasting;
+        continue;
+      }
+      if (c.lasting * 12 > least_lasting * 13 || c.lasting * 100 > whole * 110 || c.vanishing * 100 > whole * 97) continue;
+      if (pass == 1) {
+        if (c.vanishing < best) best = c.vanishing;
+      } else if (c.vanishing * 1000 <= best * 1058 && c.vanishing <= best + 300) {
+        best_n = static_cast<int>(n);
+        break;
+      }
     }
   }
-  if (best_n == 1 || best * 100 > whole * 97) return 1;       // (closer than the fit)
-  *len = static_cast<int>((chunks + best_n - 1) / best_n);
+  if (best_n > 1) *len = static_cast<int>((chunks + best_n - 1) / best_n);
   return best_n;
 }
 
@@ -125,18 +136,25 @@ int segments_for(int64_t chains, int64_t chunks_per_seq, int64_t planned_chunks,
   }
   if (flags & FKDA_FLAG_SCAN_LOOKAHEAD) return 1;
   // The planner tries up to 158 run counts with a dozen 64-bit divisions each (several microseconds), and a call asks
-  // twice; it is a pure function of these four numbers, so each thread keeps its last answer.
-  thread_local struct { int64_t chains = -1, chunks = -1, most = -1; int sms = -1, n = 1, len = 0; } last;
+  // twice, a packed one for two lengths; it is a pure function of these four numbers, so each thread keeps its last two answers.
+  struct Answer { int64_t chains = -1, chunks = -1, most = -1; int sms = -1, n = 1, len = 0; };
+  thread_local Answer kept[2];
+  thread_local int newest = 0;
   const int sms = fkda::device_sm_count();
-  if (last.chains != chains || last.chunks != planned_chunks || last.most != most || last.sms != sms) {
-    last.n = plan_runs(chains, planned_chunks, most, sms, &last.len);
-    last.chains = chains;
-    last.chunks = planned_chunks;
-    last.most = most;
-    last.sms = sms;
-  }
-  *seg_chunks = last.len;
-  return last.n;
+  for (const Answer& a : kept)
+    if (a.chains == chains && a.chunks == planned_chunks && a.most == most && a.sms == sms) {
+      *seg_chunks = a.len;
+      return a.n;
+    }
+  newest ^= 1;
+  Answer& a = kept[newest];
+  a.n = plan_runs(chains, planned_chunks, most, sms, &a.len);
+  a.chains = chains;
+  a.chunks = planned_chunks;
+  a.most = most;
+  a.sms = sms;
+  *seg_chunks = a.len;
+  return a.n;
 }
 
 constexpr int64_t kAnyRoom = INT64_MAX;
@@ -167,13 +185,16 @@ bool make_layout(int64_t T_total, int64_t H, int64_t N, int varlen, int64_t T_pe
     const int64_t most = room == kAnyRoom ? room : room > L->seg_off ? (room - L->seg_off) / run_bytes : 0;
     auto chunks_of = [](int64_t tokens) { return (tokens + fkda::kChunk - 1) / fkda::kChunk; };
     // Fixed-length: planned from the sequence length.  Packed batches: the lengths are on the device.  The longest sequence sets
-    // the time, one a third above the average is planned for, and the run length follows the longest one on the device.  (A
-    // size query, varlen < 0, has room for either plan.)
-    if (fixed) L->n_segs = segments_for(N * H, chunks_of(T_per_seq), chunks_of(T_per_seq), most, flags, &L->seg_chunks);
-    if (varlen != 0) {
+    // the time, one a third above the average is planned for, and the run length follows the longest one on the device; no more
+    // runs than sequences of the average length would have, so that a size query, which does not know the mode, needs one plan.
+    if (fixed) {
+      L->n_segs = segments_for(N * H, chunks_of(T_per_seq), chunks_of(T_per_seq), most, flags, &L->seg_chunks);
+    } else if (varlen != 0) {
+      const int64_t average = chunks_of(T_total / N);
+      L->n_segs = segments_for(N * H, average, chunks_of(N > 1 ? T_total * 4 / (N * 3) : T_total), most, flags, &L->seg_chunks);
       int len = 0;
-      const int n = segments_for(N * H, chunks_of(T_total / N), chunks_of(N > 1 ? T_total * 4 / (N * 3) : T_total), most, flags, &len);
-      if (n > L->n_segs) {
+      const int n = N > 1 ? segments_for(N * H, average, average, most, flags, &len) : L->n_segs;
+      if (n < L->n_segs) {
         L->n_segs = n;
         L->seg_chunks = len;
       }

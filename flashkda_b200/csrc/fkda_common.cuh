@@ -428,15 +428,16 @@ struct ScanParams {
   int N;
   int total_chunks;
   int state_fp32;              // dtype of both state tensors: 1 = fp32, 0 = bf16
-  // Segment-parallel form (batches with few chains): every sequence is cut into n_segs runs of
-  // seg_chunks chunks (varlen: of *seg_chunks_dev chunks, runs beyond a sequence's end being empty) and each CTA walks one run.  Pass 1 walks run 0 from the caller's state (its outputs are
-  // final) and, for the runs 1 .. n_segs-2, the two halves of the affine map  Z_end = Z_start M + N  that a run
-  // applies to the state Z = S^T: N from a zero state, M from the identity with u' taken as zero.  A small kernel
-  // chains the maps into the state at the start of every run; pass 2 walks runs 1 .. n_segs-1 from those.
+  // Segment-parallel form (batches with few chains): every sequence is cut into n_segs runs of seg_chunks chunks (varlen: of
+  // *seg_chunks_dev chunks, runs beyond a sequence's end being empty) and each CTA walks one run.  A run applies an affine map
+  // Z_end = Z_start M + N to the state Z = S^T.  Over compact records kSegMaps gives M and N of the runs 0 .. n_segs-2 and kSegWalks
+  // walks all runs.  In the two-stage form pass 1 walks run 0 from the caller's state (its outputs are final) and, for the runs 1 ..
+  // n_segs-2, N from a zero state and M from the identity with u' taken as zero; pass 2 walks the runs 1 .. n_segs-1.  Between
+  // the passes a small kernel chains the maps into the state at the start of every run.
   int seg_chunks;              // 0: one CTA per whole sequence
   int n_segs;
-  int seg_pass;                // 1 or 2
-  float* seg_buf;              // fp32 [(n*H + h)][n_segs][3][128][128]: 0 = M, 1 = N, 2 = state at the start of the run
+  int seg_pass;                // 1 or 2; over compact records kSegMaps or kSegWalks
+  float* seg_buf;              // fp32 [(n*H + h)][n_segs][3] slots: 0 = M, 1 = N, 2 = state at the start of the run
   const int* select;           // device word, or nullptr: the kernel runs only if *select == select_want
   int select_want;
   const int* seg_chunks_dev;   // varlen batches: run length decided on the device from the longest sequence (else nullptr)
@@ -459,6 +460,11 @@ struct ScanParams {
 constexpr int kSegMapStride = 136;             // floats per row of a transition map M in its slot: the map chaining reads
                                                // whole slots into shared memory, where this stride keeps its fragment loads conflict-free
 constexpr int64_t kSegSlotFloats = 128 * kSegMapStride;   // every slot has room for the padded form
+// Passes over runs on the compact records (ScanParams::seg_pass; 1 and 2 are the two-stage form's): maps of all runs but the last,
+// walks of all runs.
+constexpr int kSegMaps = 3, kSegWalks = 4;
+// Whether the map of a run is zero to the last bit: behind its offset's rows.
+__device__ __forceinline__ int* seg_zero_word(float* slots, int run) { return reinterpret_cast<int*>(slots + (run * 3 + 1) * kSegSlotFloats + kD * kD); }
 constexpr int kDefaultSms = 148;       // SMs of a B200: assumed where no device can be asked
 
 // SM count of the current device, asked once per device and cached; the kernel-selection rules, the planner of the
@@ -532,13 +538,13 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
   ChainView cv;
   int chain = block, seg = 0, variant = 0;
   if constexpr (kSeg) {
-    const int per = p.seg_pass == 1 ? 2 * p.n_segs - 3 : p.n_segs - 1;
+    const int per = p.seg_pass == 1 ? 2 * p.n_segs - 3 : p.seg_pass == kSegWalks ? p.n_segs : p.n_segs - 1;
     chain = block / per;
     const int j = block - chain * per;
     if (p.seg_pass == 1) {
       if (j > 0) { seg = 1 + ((j - 1) >> 1); variant = 1 + ((j - 1) & 1); }
     } else {
-      seg = 1 + j;
+      seg = p.seg_pass == 2 ? 1 + j : j;
     }
   }
   const int slot = chain / p.H;
@@ -595,8 +601,10 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
       }
       cv.fin_fp32 = 1;
     } else {
-      cv.init_mode = 1;
-      cv.init_base = slots + (seg * 3 + 2) * kSegSlotFloats;
+      if (seg > 0) {
+        cv.init_mode = 1;
+        cv.init_base = slots + (seg * 3 + 2) * kSegSlotFloats;
+      }
       if (seg != p.n_segs - 1) cv.fin_base = nullptr;
     }
   }

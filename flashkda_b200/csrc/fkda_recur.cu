@@ -72,104 +72,121 @@ struct Info {
   int pad[3];
 };
 static_assert(sizeof(Info) == 32, "info");
-enum { kQuiet = 1 /* no outputs wanted */, kEnd = 2 };
+enum { kEnd = 1 };
 
-// The chunks of one walk on the recurrence warps, from stage s (phase par) on; ready: that stage is known to be full.  S: rows v = row0 + 16 vt + g (+ 8), columns 8 jt + 2 t, + 1.
-template <bool kOut>
-__device__ __forceinline__ bool walk(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int nchunks, int64_t tokens, bool zero_v,
-                                     int row0, int lane, volatile int* abort_flag, int& s, uint32_t& par, bool& ready) {
-  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+// One chunk on the recurrence warps, from stage s.  S: rows v = row0 + 16 vt + g (+ 8), columns 8 jt + 2 t, + 1.  `ready`: whether the
+// next stage is full already.
+// kOut: copies of S and U for the output products.  kBack: the transposed step, S^T Phi^T with Phi = diag(e) + kn^T TB^T kr the
+// chunk's transition and no v: the same products with k+ and kr exchanged and TB transposed.
+template <bool kOut, bool kBack>
+__device__ __forceinline__ void step(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int s, int len, int row0, int lane, uint32_t next_full,
+                                     uint32_t next_par, bool& ready) {
   const int mi = lane >> 3, r = lane & 7, t = lane & 3;
-  const uint32_t kn_lane = 8192 + kCrKN + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
-  const uint32_t kr_lane = 8192 + kCrKR + mi * 2048 + r * 16;
+  const uint32_t kn_lane = 8192 + (kBack ? kCrKR : kCrKN) + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
+  const uint32_t kr_lane = 8192 + (kBack ? kCrKN : kCrKR) + mi * 2048 + r * 16;
   const uint32_t v_lane = (row0 >> 6) * 4096 + lane * 128;
   const uint32_t tb_lane = 8192 + kCrTB + r * 16;
-  for (int c = 0; c < nchunks; ++c) {
-    if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) return false;
-    const uint32_t stage = sbase + s * kStageBytes;
+  const uint32_t stage = sbase + s * kStageBytes;
 
-    // R^T = v^T - S^T k+^T: the accumulators start from v^T; operands of a k-step are loaded during the one before
-    float R[2][4][4];
-    {
-      uint32_t x[4][4];              // v^T: channel blocks of 8 rows; register = token block
+  // R^T = v^T - S^T k+^T: the accumulators start from v^T; operands of a k-step are loaded during the one before
+  float R[2][4][4];
+  if (kBack) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ldsm_x4_trans(stage + v_lane + ((((row0 >> 3) + i) & 7) ^ r) * 16, x[i][0], x[i][1], x[i][2], x[i][3]);
-      const int64_t left = tokens - static_cast<int64_t>(c) * kChunk;
-      if (left < kChunk || zero_v) {   // rows past the sequence end belong to somebody else
-        const int len = zero_v ? 0 : static_cast<int>(left);
+    for (int vt = 0; vt < 2; ++vt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const uint32_t keep = (8 * nt + 2 * t < len ? 0xffffu : 0u) | (8 * nt + 2 * t + 1 < len ? 0xffff0000u : 0u);
+      for (int nt = 0; nt < 4; ++nt) R[vt][nt][0] = R[vt][nt][1] = R[vt][nt][2] = R[vt][nt][3] = 0.f;
+  } else {
+    uint32_t x[4][4];              // v^T: channel blocks of 8 rows; register = token block
 #pragma unroll
-          for (int i = 0; i < 4; ++i) x[i][nt] &= keep;
-        }
-      }
+    for (int i = 0; i < 4; ++i) ldsm_x4_trans(stage + v_lane + ((((row0 >> 3) + i) & 7) ^ r) * 16, x[i][0], x[i][1], x[i][2], x[i][3]);
+    if (len < kChunk) {            // rows past the sequence end belong to somebody else
 #pragma unroll
-      for (int vt = 0; vt < 2; ++vt)
+      for (int nt = 0; nt < 4; ++nt) {
+        const uint32_t keep = (8 * nt + 2 * t < len ? 0xffffu : 0u) | (8 * nt + 2 * t + 1 < len ? 0xffff0000u : 0u);
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          R[vt][nt][0] = bf_lo(x[2 * vt][nt]);
-          R[vt][nt][1] = bf_hi(x[2 * vt][nt]);
-          R[vt][nt][2] = bf_lo(x[2 * vt + 1][nt]);
-          R[vt][nt][3] = bf_hi(x[2 * vt + 1][nt]);
-        }
-    }
-    uint32_t bb[2][8];
-    ldsm_x4(stage + kn_lane, bb[0][0], bb[0][1], bb[0][2], bb[0][3]);
-    ldsm_x4(stage + kn_lane + 4096, bb[0][4], bb[0][5], bb[0][6], bb[0][7]);
-    if (kOut) tc_fence_after();
-    const uint32_t sb = tq + kColSb + 64 * s;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t a[2][16];               // bf16 copy of the state: A fragments of four k-steps, and 32 columns of tensor memory
-#pragma unroll
-      for (int vt = 0; vt < 2; ++vt) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          a[vt][2 * j] = pack_bf16(S[vt][8 * half + j][0], S[vt][8 * half + j][1]);
-          a[vt][2 * j + 1] = pack_bf16(S[vt][8 * half + j][2], S[vt][8 * half + j][3]);
-        }
-        if (kOut) tmem_st_16x128b_x8(sb + (static_cast<uint32_t>(16 * vt) << 16) + 32 * half, a[vt]);
-      }
-#pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4) {
-        const int ks = 4 * half + k4;
-        const uint32_t(&B)[8] = bb[ks & 1];
-        if (ks < 7) {
-          uint32_t(&N)[8] = bb[(ks + 1) & 1];
-          ldsm_x4(stage + kn_lane + (ks + 1) * 256, N[0], N[1], N[2], N[3]);
-          ldsm_x4(stage + kn_lane + 4096 + (ks + 1) * 256, N[4], N[5], N[6], N[7]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-          for (int vt = 0; vt < 2; ++vt)
-            mma_bf16_16816(R[vt][nt], a[vt][4 * k4], a[vt][4 * k4 + 1], a[vt][4 * k4 + 2], a[vt][4 * k4 + 3], B[2 * nt], B[2 * nt + 1]);
+        for (int i = 0; i < 4; ++i) x[i][nt] &= keep;
       }
     }
-    // U^T = R^T (T diag(beta))^T
-    uint32_t l[4], m[4], n[4];       // T diag(beta): token tiles 0 and 1 (tokens 0-15 only: lower triangle), 2, 3
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        R[vt][nt][0] = bf_lo(x[2 * vt][nt]);
+        R[vt][nt][1] = bf_hi(x[2 * vt][nt]);
+        R[vt][nt][2] = bf_lo(x[2 * vt + 1][nt]);
+        R[vt][nt][3] = bf_hi(x[2 * vt + 1][nt]);
+      }
+  }
+  uint32_t bb[2][8];
+  ldsm_x4(stage + kn_lane, bb[0][0], bb[0][1], bb[0][2], bb[0][3]);
+  ldsm_x4(stage + kn_lane + 4096, bb[0][4], bb[0][5], bb[0][6], bb[0][7]);
+  if (kOut) tc_fence_after();
+  const uint32_t sb = tq + kColSb + 64 * s;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t a[2][16];               // bf16 copy of the state: A fragments of four k-steps, and 32 columns of tensor memory
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        a[vt][2 * j] = pack_bf16(S[vt][8 * half + j][0], S[vt][8 * half + j][1]);
+        a[vt][2 * j + 1] = pack_bf16(S[vt][8 * half + j][2], S[vt][8 * half + j][3]);
+      }
+      if (kOut) tmem_st_16x128b_x8(sb + (static_cast<uint32_t>(16 * vt) << 16) + 32 * half, a[vt]);
+    }
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+      const int ks = 4 * half + k4;
+      const uint32_t(&B)[8] = bb[ks & 1];
+      if (ks < 7) {
+        uint32_t(&N)[8] = bb[(ks + 1) & 1];
+        ldsm_x4(stage + kn_lane + (ks + 1) * 256, N[0], N[1], N[2], N[3]);
+        ldsm_x4(stage + kn_lane + 4096 + (ks + 1) * 256, N[4], N[5], N[6], N[7]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+          mma_bf16_16816(R[vt][nt], a[vt][4 * k4], a[vt][4 * k4 + 1], a[vt][4 * k4 + 2], a[vt][4 * k4 + 3], B[2 * nt], B[2 * nt + 1]);
+    }
+  }
+  // U^T = R^T (T diag(beta))^T
+  uint32_t l[4], m[4], n[4];       // T diag(beta): token tiles 0 and 1 (tokens 0-15 only: lower triangle), 2, 3; transposed: 0, 1, 2 and 3 (16-31 only)
+  if (kBack) {
+    ldsm_x4_trans(stage + tb_lane + mi * 512, l[0], l[1], l[2], l[3]);
+    ldsm_x4_trans(stage + tb_lane + mi * 512 + 128, m[0], m[1], m[2], m[3]);
+    ldsm_x4_trans(stage + tb_lane + 1024 + (mi & 1) * 512 + 256 + (mi >> 1) * 128, n[0], n[1], n[2], n[3]);
+  } else {
     ldsm_x4(stage + tb_lane + (mi >> 1) * 512 + (mi & 1) * 128, l[0], l[1], l[2], l[3]);
     ldsm_x4(stage + tb_lane + 1024 + mi * 128, m[0], m[1], m[2], m[3]);
     ldsm_x4(stage + tb_lane + 1536 + mi * 128, n[0], n[1], n[2], n[3]);
-    uint32_t kr[2][4];
-    ldsm_x4_trans(stage + kr_lane, kr[0][0], kr[0][1], kr[0][2], kr[0][3]);
-    uint32_t u[2][2][4];             // A fragments, k-step = 16 tokens: first of R^T, then of U^T
-    auto as_operand = [&](uint32_t(&d)[2][4], const float(&x)[4][4]) {
+  }
+  uint32_t kr[2][4];
+  ldsm_x4_trans(stage + kr_lane, kr[0][0], kr[0][1], kr[0][2], kr[0][3]);
+  uint32_t u[2][2][4];             // A fragments, k-step = 16 tokens: first of R^T, then of U^T
+  auto as_operand = [&](uint32_t(&d)[2][4], const float(&x)[4][4]) {
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks)
+    for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)  // e & 1: rows + 8, e >> 1: tokens + 8
-          d[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
-    };
+      for (int e = 0; e < 4; ++e)  // e & 1: rows + 8, e >> 1: tokens + 8
+        d[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
+  };
 #pragma unroll
-    for (int vt = 0; vt < 2; ++vt) as_operand(u[vt], R[vt]);
-    {
-      float U[2][4][4];
+  for (int vt = 0; vt < 2; ++vt) as_operand(u[vt], R[vt]);
+  {
+    float U[2][4][4];
 #pragma unroll
-      for (int vt = 0; vt < 2; ++vt) {
+    for (int vt = 0; vt < 2; ++vt) {
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) U[vt][nt][0] = U[vt][nt][1] = U[vt][nt][2] = U[vt][nt][3] = 0.f;
+      for (int nt = 0; nt < 4; ++nt) U[vt][nt][0] = U[vt][nt][1] = U[vt][nt][2] = U[vt][nt][3] = 0.f;
+      if (kBack) {
+        mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
+        mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
+        mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[0], n[1]);
+        mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
+        mma_bf16_16816(U[vt][0], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], l[2], l[3]);
+        mma_bf16_16816(U[vt][1], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
+      } else {
         mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
         mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[2], l[3]);
         mma_bf16_16816(U[vt][2], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
@@ -177,48 +194,59 @@ __device__ __forceinline__ bool walk(float (&S)[2][16][4], uint8_t* smem, uint32
         mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
         mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
       }
+    }
 #pragma unroll
-      for (int vt = 0; vt < 2; ++vt) {
-        as_operand(u[vt], U[vt]);
-        if (kOut) {
-          const uint32_t ut = tq + (static_cast<uint32_t>(16 * vt) << 16) + kColUt + 16 * s;
-          tmem_st_16x128b_x4(ut, u[vt][0], u[vt][1]);
-        }
+    for (int vt = 0; vt < 2; ++vt) {
+      as_operand(u[vt], U[vt]);
+      if (kOut) {
+        const uint32_t ut = tq + (static_cast<uint32_t>(16 * vt) << 16) + kColUt + 16 * s;
+        tmem_st_16x128b_x4(ut, u[vt][0], u[vt][1]);
       }
     }
-    // S^T = S^T diag(e) + U^T kr; the next stage's barrier is looked at meanwhile
-    const float2* e2 = reinterpret_cast<const float2*>(smem + s * kStageBytes + 8192 + kCrE) + t;
+  }
+  // S^T = S^T diag(e) + U^T kr; the next stage's barrier is looked at meanwhile
+  const float2* e2 = reinterpret_cast<const float2*>(smem + s * kStageBytes + 8192 + kCrE) + t;
+  ready = mbar_test(next_full, next_par);
+#pragma unroll
+  for (int jt = 0; jt < 16; ++jt) {
+    const uint32_t(&B)[4] = kr[jt & 1];
+    if (jt < 15) {
+      uint32_t(&N)[4] = kr[(jt + 1) & 1];
+      ldsm_x4_trans(stage + kr_lane + (jt + 1) * 128, N[0], N[1], N[2], N[3]);
+    }
+    const float2 e = e2[4 * jt];
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt) {
+      uint32_t y[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[vt][jt][k]);
+      mul2(y[0], y[1], e);
+      mul2(y[2], y[3], e);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) S[vt][jt][k] = __uint_as_float(y[k]);
+    }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt)
+        mma_bf16_16816(S[vt][jt], u[vt][ks][0], u[vt][ks][1], u[vt][ks][2], u[vt][ks][3], B[2 * ks], B[2 * ks + 1]);
+  }
+  if (kOut) {
+    tmem_wait_st();
+    tc_fence_before();
+  }
+}
+
+// The chunks of one walk on the recurrence warps, from stage s (phase par) on; ready: that stage is known to be full.
+__device__ __forceinline__ bool walk(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int nchunks, int64_t tokens, int row0, int lane,
+                                     volatile int* abort_flag, int& s, uint32_t& par, bool& ready) {
+  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+  for (int c = 0; c < nchunks; ++c) {
+    if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) return false;
+    const int64_t left = tokens - static_cast<int64_t>(c) * kChunk;
     const int s1 = s + 1 == kStages ? 0 : s + 1;
     const uint32_t par1 = s1 == 0 ? par ^ 1u : par;
-    ready = mbar_test(bar(B_FULL + s1), par1);
-#pragma unroll
-    for (int jt = 0; jt < 16; ++jt) {
-      const uint32_t(&B)[4] = kr[jt & 1];
-      if (jt < 15) {
-        uint32_t(&N)[4] = kr[(jt + 1) & 1];
-        ldsm_x4_trans(stage + kr_lane + (jt + 1) * 128, N[0], N[1], N[2], N[3]);
-      }
-      const float2 e = e2[4 * jt];
-#pragma unroll
-      for (int vt = 0; vt < 2; ++vt) {
-        uint32_t y[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[vt][jt][k]);
-        mul2(y[0], y[1], e);
-        mul2(y[2], y[3], e);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) S[vt][jt][k] = __uint_as_float(y[k]);
-      }
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-        for (int vt = 0; vt < 2; ++vt)
-          mma_bf16_16816(S[vt][jt], u[vt][ks][0], u[vt][ks][1], u[vt][ks][2], u[vt][ks][3], B[2 * ks], B[2 * ks + 1]);
-    }
-    if (kOut) {
-      tmem_wait_st();
-      tc_fence_before();
-    }
+    step<true, false>(S, smem, sbase, tq, s, left < kChunk ? static_cast<int>(left) : kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
     __syncwarp();
     if (lane == 0) {
       mbar_arrive(bar(B_U + s));
@@ -344,13 +372,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       }
       const ChainView cv = chain_view<kSeg, kSlice>(p, walk_index);
       load_state(S, cv, row0, lane);
-      if (cv.nchunks == 0) {
-        // (an empty run: its state is handed through)
-      } else if (!kSeg || cv.write_out) {
-        ok = walk<true>(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, false, row0, lane, abort_flag, s, par, ready);
-      } else {
-        ok = walk<false>(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, cv.zero_up, row0, lane, abort_flag, s, par, ready);
-      }
+      // (an empty run hands its state through)
+      if (cv.nchunks > 0) ok = walk(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, row0, lane, abort_flag, s, par, ready);
       if (ok && cv.fin_base != nullptr) store_state(S, cv, row0, lane);
       if (!kStream) break;
       i += cv.nchunks;
@@ -364,7 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     const size_t step = static_cast<size_t>(8) * p.H * kD;      // eight tokens on
 
     // ===== one lane of the second warp: the stream of chunks into the ring ==========================================
-    struct { long long bos, eos; const uint8_t* rec; int walk, h, c, n, flags, turn; bool ended; } cur{};
+    struct { long long bos, eos; const uint8_t* rec; int walk, h, c, n, turn; bool ended; } cur{};
     int copied = 0;
     int cs = 0;                        // stage of the next item
     auto copy = [&]() {
@@ -401,7 +424,6 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           cur.eos = cv.eos;
           cur.c = 0;
           cur.n = cv.nchunks;
-          cur.flags = cv.write_out ? 0 : kQuiet;
           cur.rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
           if (copied > 0 && (cv.init_mode == 1 || cv.init_mode == 2)) bulk_prefetch_l2(cv.init_base, kD * kD * (cv.init_mode == 1 ? 4 : 2));
           break;
@@ -411,7 +433,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       f->out_off = (t0 * p.H + cur.h) * kD;
       f->len = cur.eos - t0 < kChunk ? static_cast<int>(cur.eos - t0) : kChunk;
       f->walk = cur.walk;
-      f->flags = cur.flags;
+      f->flags = 0;
       const uint32_t dst = sbase + s * kStageBytes;
       mbar_arrive_expect_tx(bar(B_FULL + s), kCrBytes + 8192);
       bulk_g2s(dst + 8192, cur.rec + static_cast<size_t>(cur.c) * kCrBytes, kCrBytes, bar(B_FULL + s));
@@ -432,10 +454,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       if (i >= kOBufs && !mbar_wait_parked(bar(B_O_FREE + o), po_par, abort_flag)) return false;
       if (++ps == kStages) { ps = 0; ps_par ^= 1u; }
       if (++po == kOBufs) { po = 0; po_par ^= 1u; }
-      const int flags = static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags;
-      if (flags & (kQuiet | kEnd)) {
+      if (kStream && (static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags & kEnd)) {
         mbar_arrive(bar(B_O + o));
-        if (!(flags & kEnd)) mbar_arrive(bar(B_EMPTY + s));
         return true;
       }
       tc_fence_after();
@@ -473,9 +493,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       if (!__all_sync(0xffffffffu, mbar_wait_parked(bar(B_O + o), o_par, abort_flag))) { ok = false; break; }
       const volatile Info* f = infos + (i & (kInfos - 1));
-      const int flags = f->flags;
-      if (flags & kEnd) break;
-      if (!(flags & kQuiet)) {
+      if (kStream && (f->flags & kEnd)) break;
+      {
         const long long off = f->out_off;
         const int len = f->len;
         tc_fence_after();
@@ -502,9 +521,6 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           dst += step;
         }
         __syncwarp();
-      } else {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(B_O_FREE + o));
       }
       if (w == 1 && lane == 0 && !cur.ended) {
         if (!mbar_wait_parked(bar(B_EMPTY + es), es_par, abort_flag)) ok = false;
@@ -543,15 +559,198 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
   }
 }
 
+// ---- maps of runs (fkda_segscan.cu) ---------------------------------------------------------------------------------------
+// A CTA per (chain, run but the last): first the run's transition map M, from its last chunk to its first, then its offset N,
+// the walk from a zero state.  Walked backwards, Q <- Q Phi^T from the identity, the rows of M^T = Q never meet each other either, and
+// after c chunks Q is the map of the run's last c chunks: once it is zero to the last bit (103 nats of decay; a few hundred
+// tokens of ordinary gates), so is M, and nothing in front of those chunks can be seen behind the run.  Both walks then end there:
+// what they cost is a handful of chunks instead of two runs, and chaining such runs costs nothing at all.  A run
+// whose gates hold some channel to the end costs what it always did, a walk each for M and N, plus the test for zero (a hundred
+// cycles in the first sixteen chunks and then in every eighth).
+// 8 heads of 131072 tokens (lower_bound -2), recurrence with all its passes: 820 -> 340 us, 795 with gates that never decay; 16
+// heads of 32768 tokens, the whole call: 619 -> 365 us (610).  Few chains lose a tenth where nothing decays (1 head of 131072 tokens 338
+// -> 379 us, against 132 otherwise), as M and N had a CTA each.
+__device__ __forceinline__ bool is_zero(const float (&S)[2][16][4]) {
+  uint32_t any = 0;
+#pragma unroll
+  for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+    for (int jt = 0; jt < 16; ++jt)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) any |= __float_as_uint(S[vt][jt][k]);
+  return !__any_sync(0xffffffffu, (any << 1) != 0u);
+}
+
+__global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant__ CUtensorMap tm_v, const ScanParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sbase = smem_u32(smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kSmMisc + 4);
+  int* zeros = reinterpret_cast<int*>(smem + kSmMisc + 8);       // warps whose rows of the map are zero ...
+  int* longest = reinterpret_cast<int*>(smem + kSmMisc + 12);    // ... after so many chunks
+  Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
+  constexpr int B_TURN = B_U;                                    // M is done, N may be fetched
+  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+  if (tid == 0) {
+    *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
+    *zeros = 0;
+    *longest = 0;
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(bar(B_FULL + s), 1);
+      mbar_init(bar(B_EMPTY + s), 4);
+    }
+    mbar_init(bar(B_TURN), 4);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  bool ok = *abort_flag <= 0;
+  grid_dependency_wait();
+  const ChainView cv = chain_view<true>(p, static_cast<int>(blockIdx.x));
+  const int n = ok ? cv.nchunks : 0, run = static_cast<int>(blockIdx.x) % (p.n_segs - 1);
+  if (warp < 4) {
+    float* slots = p.seg_buf + (static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 * kSegSlotFloats;
+    const int row0 = 32 * warp, g = lane >> 2, t = lane & 3;
+    float S[2][16][4];
+    auto fill = [&](float diagonal) {
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+        for (int jt = 0; jt < 16; ++jt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) S[vt][jt][i] = 8 * jt + 2 * t + (i & 1) == row0 + 16 * vt + g + 8 * (i >> 1) ? diagonal : 0.f;
+    };
+    int s = 0;
+    uint32_t par = 0;
+    bool ready = false, zero = false;
+    auto next = [&](int& s1, uint32_t& par1) {
+      s1 = s + 1 == kStages ? 0 : s + 1;
+      par1 = s1 == 0 ? par ^ 1u : par;
+    };
+    auto release = [&](int s1, uint32_t par1) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(B_EMPTY + s));
+      s = s1;
+      par = par1;
+    };
+    fill(1.f);
+    for (int c = 0; ok; ++c) {
+      if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
+      int s1;
+      uint32_t par1;
+      next(s1, par1);
+      ready = false;
+      const bool end = static_cast<const volatile Info*>(infos)[c & (kInfos - 1)].flags & kEnd;
+      if (!end && !zero) {
+        step<false, true>(S, smem, sbase, 0, s, kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
+        if ((c < 16 || (c & 7) == 7) && is_zero(S)) {
+          zero = true;
+          if (lane == 0) {
+            atomicMax(longest, c + 1);
+            __threadfence_block();
+            atomicAdd(zeros, 1);
+          }
+        }
+      }
+      release(s1, par1);
+      if (end) break;
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const bool all_zero = *static_cast<volatile int*>(zeros) == 4;
+    const int first = all_zero ? n - *static_cast<volatile int*>(longest) : 0;
+    if (ok) {
+      if (!all_zero) {           // M, transposed back
+        float* M = slots + (run * 3 + 0) * kSegSlotFloats;
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+          for (int jt = 0; jt < 16; ++jt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) M[(8 * jt + 2 * t + (i & 1)) * kSegMapStride + row0 + 16 * vt + g + 8 * (i >> 1)] = S[vt][jt][i];
+      }
+      if (tid == 0) *seg_zero_word(slots, run) = all_zero;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(B_TURN));
+      fill(0.f);
+      ready = false;
+      for (int c = first; c < n; ++c) {
+        if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
+        int s1;
+        uint32_t par1;
+        next(s1, par1);
+        const int64_t left = cv.eos - cv.bos - static_cast<int64_t>(c) * kChunk;
+        step<false, false>(S, smem, sbase, 0, s, left < kChunk ? static_cast<int>(left) : kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
+        release(s1, par1);
+      }
+      if (ok) {
+        // behind a map of zero the offset is the state at the start of the next run
+        float* N = all_zero ? slots + ((run + 1) * 3 + 2) * kSegSlotFloats : slots + (run * 3 + 1) * kSegSlotFloats;
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+          for (int jt = 0; jt < 16; ++jt)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              *reinterpret_cast<float2*>(N + (row0 + 16 * vt + g + 8 * i) * kD + 8 * jt + 2 * t) = make_float2(S[vt][jt][2 * i], S[vt][jt][2 * i + 1]);
+      }
+    }
+  } else if (warp == 5 && lane == 0 && ok) {
+    const uint8_t* rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
+    int item = 0;
+    // an item of the ring: a chunk of the backward or of the forward walk, or (c < 0) the end of the backward one
+    auto put = [&](int c, bool with_v) -> bool {
+      const int s = item % kStages;
+      if (p.stop_copies_after > 0 && item >= p.stop_copies_after) return false;      // test aid: the next wait for a record runs out
+      if (item >= kStages && !mbar_wait_parked(bar(B_EMPTY + s), (item / kStages - 1) & 1, abort_flag)) { ok = false; return false; }
+      infos[item & (kInfos - 1)].flags = c < 0 ? kEnd : 0;
+      if (c < 0) {
+        mbar_arrive(bar(B_FULL + s));
+      } else {
+        const uint32_t dst = sbase + s * kStageBytes, full = bar(B_FULL + s);
+        mbar_arrive_expect_tx(full, kCrBytes + (with_v ? 8192 : 0));
+        bulk_g2s(dst + 8192, rec + static_cast<size_t>(c) * kCrBytes, kCrBytes, full);
+        if (with_v) {
+          const int t0 = static_cast<int>(cv.bos + static_cast<int64_t>(c) * kChunk);
+          tma_load_3d(dst, &tm_v, 0, cv.h, t0, full);
+          tma_load_3d(dst + 4096, &tm_v, 64, cv.h, t0, full);
+        }
+      }
+      ++item;
+      return true;
+    };
+    bool more = true;
+    for (int c = n - 1; more && c >= 0 && *static_cast<volatile int*>(zeros) < 4; --c) more = put(c, false);
+    more = more && put(-1, false);
+    if (more && !mbar_wait_parked(bar(B_TURN), 0, abort_flag)) more = ok = false;
+    if (more)
+      for (int c = *static_cast<volatile int*>(zeros) == 4 ? n - *static_cast<volatile int*>(longest) : 0; more && c < n; ++c) more = put(c, true);
+    if (!ok || *abort_flag > 0 || !more) {
+      // (giving up) copies in flight must land before the CTA's shared memory goes away
+      for (int c = item > kStages ? item - kStages : 0; c < item; ++c) {
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(bar(B_FULL + c % kStages), (c / kStages) & 1))
+          if (globaltimer_ns() - t0 > 20000000ull) break;
+      }
+    }
+  }
+  if (!ok || *abort_flag > 0) atomicCAS(p.status, kStatusOk, kStatusWaitTimeout);
+  __syncthreads();
+}
+
 }  // namespace recur
 
 // v: the value tensor [T_total][H][128]
 cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream_t stream) {
   int64_t walks = static_cast<int64_t>(p.N) * p.H;
-  if (p.seg_chunks > 0) walks *= p.seg_pass == 1 ? 2 * p.n_segs - 3 : p.n_segs - 1;
+  if (p.seg_chunks > 0) walks *= p.seg_pass == kSegMaps ? p.n_segs - 1 : p.n_segs;
   if (walks <= 0) return cudaSuccess;
   CUtensorMap tv;
   if (!make_map(&tv, v, p.T_total, p.H)) return cudaErrorInvalidValue;
+  if (p.seg_chunks > 0 && p.seg_pass == kSegMaps) {
+    static SmemOptIn opt_in;
+    cudaError_t e = opt_in.ensure(recur::maps_kernel, recur::kSmem);
+    if (e != cudaSuccess) return e;
+    return launch_after(recur::maps_kernel, static_cast<unsigned>(walks), recur::kThreads, recur::kSmem, stream, tv, p);
+  }
   // More walks than SMs and short ones on average: one persistent CTA per SM.  (At 24 chunks the 3 us a walk costs more
   // in a CTA of its own are what the tighter chunk loop saves.)
   const int64_t sms = device_sm_count();

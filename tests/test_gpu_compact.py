@@ -286,3 +286,39 @@ def test_gate_parameters_at_the_ends_of_their_range(T):
     assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS
     for h in range(4):
         assert rel_fro(fin.cpu()[:, h], s64[:, h]) <= STATE_REL, h
+
+
+@pytest.mark.parametrize("state", [None, "bf16", "fp32"])
+@pytest.mark.parametrize("packed", [False, True], ids=["equal", "packed"])
+@pytest.mark.parametrize("lasting", ["all", "none", "first", "odd", "pairs"])
+def test_runs_whose_maps_last_or_vanish(lasting, packed, state):
+    """The transition map of a run is found to be zero, or is chained: runs of tokens without any decay (the state at their start
+    reaches through them) among runs with ordinary gates, in every order; the packed batch has an empty sequence and one shorter
+    than the runs."""
+    H, lens = 2, [32 * 200 + 9, 0, 32 * 180, 32 * 3 + 1] if packed else None
+    w = Workload("m", H=H, T=0 if packed else 32 * 200 + 9, seq_lens=lens, state_in=state, state_out=state or "fp32", state_std=0.5, seed=61, lower_bound=-2.0)
+    chunks = (sum(lens) * 4 // (len(lens) * 3) if packed else w.T) // 32 + 1
+    average = (sum(lens) // len(lens) if packed else w.T) // 32 + 1
+    runs = min(F.plan_segments(w.N * H, chunks)[0], F.plan_segments(w.N * H, average)[0])
+    assert runs >= 5
+    x = make_inputs(w)
+    ends = [sum(lens[:i]) for i in range(len(lens) + 1)] if packed else [0, w.T]
+    per = 32 * max(8, -(-(200 + 1) // runs))
+    chosen = {"all": lambda r: True, "none": lambda r: False, "first": lambda r: r == 0, "odd": lambda r: r % 2 == 1, "pairs": lambda r: r % 4 >= 2}[lasting]
+    for a, b in zip(ends, ends[1:]):
+        for r in range(runs):
+            if chosen(r):
+                x["g"][:, min(a + r * per, b):min(a + (r + 1) * per, b)] = -12.0
+    x["A_log"].fill_(0.5)
+    xc = to_cuda(x)
+    out, fin = torch.full_like(xc["v"], float("nan")), torch.full_like(xc["final_state"], float("nan"))
+    ws = torch.empty(F.get_workspace_size(x["q"].shape[1], H, w.N), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        F.fwd(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"],
+              initial_state=xc["initial_state"], final_state=fin, cu_seqlens=xc["cu_seqlens"], workspace=ws)
+        assert F.read_status(ws) == 0
+        ws.fill_(0xFF)                   # (not-a-number in whatever the second call should not read)
+    o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                     initial_state=x["initial_state"], cu_seqlens=x["cu_seqlens"])
+    assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS and rel_fro(out.cpu(), o64) <= 1e-2
+    assert rel_fro(fin.cpu(), s64) <= STATE_REL
