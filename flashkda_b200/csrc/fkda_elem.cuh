@@ -34,7 +34,6 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ f2 unpack_bf(uint32_t w) { return pk(bf_lo(w), bf_hi(w)); }
 __device__ __forceinline__ uint32_t round_bf(f2 x) {
   float a, b;
   upk(x, a, b);
@@ -186,11 +185,6 @@ __device__ __forceinline__ f2 rcp_pair(f2 x) {
   asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(a));
   asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(b));
   return pk(a, b);
-}
-__device__ __forceinline__ f2 exp2_neg_pair(f2 x) {
-  float a, b;
-  upk(x, a, b);
-  return pk(ex2f(-a), ex2f(-b));
 }
 
 }  // namespace elem

@@ -57,9 +57,12 @@ struct Lay {
   static constexpr int kSsq = kE + 512;                            // fp32 [q|k][16 rows][8 warps] partial sums of squares
   static constexpr int kBeta = kSsq + 1024;                        // fp32 [16]
   static constexpr int kBar = kBeta + 64;                          // mbarrier of the state copy, abort flag
-  static constexpr int kState = (kBar + 16 + 127) / 128 * 128;     // [128 v] state rows, padded: fragment reads hit 32 distinct banks
-  static constexpr int kStride = kWide ? 512 + 32 : 256 + 16;      // 8 words mod 32 (8-byte reads), 4 words mod 32 (4-byte reads)
-  static constexpr int kSmemBytes = kState + kD * kStride;
+  // State: [128 v] fp32 rows, padded by eight words (8-byte fragment reads hit 32 distinct banks); or two halves of 64 columns of
+  // bf16 rows with the 128-byte swizzle, as the tensor copies bring them and ldmatrix wants them.
+  static constexpr int kAlign = kWide ? 128 : 1024;
+  static constexpr int kState = (kBar + 16 + kAlign - 1) / kAlign * kAlign;
+  static constexpr int kStride = 512 + 32;
+  static constexpr int kSmemBytes = kState + (kWide ? kD * kStride : kD * 256);
   static constexpr int kCtas = kWide ? 2 : 4;
   static_assert(kCtas * (kSmemBytes + 1024) <= 227 * 1024, "CTAs per SM");
 };
@@ -85,12 +88,13 @@ struct Params {
 
 // kFp32: type of the state tensors; kOneBlock: T <= 16, compiled without the block loop's bookkeeping
 template <bool kFp32, bool kOneBlock>
-__global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>::kCtas) short16_kernel(const Params p) {
+__global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>::kCtas)
+short16_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out, const Params p) {
   using namespace elem;
   constexpr bool kWide = kFp32 || !kOneBlock;
   using L = Lay<kWide, kOneBlock>;
   constexpr int kKN = L::kKN, kKM = L::kKM, kQP = L::kQP, kKR = L::kKR, kTB = L::kTB, kMQK = L::kMQK, kState = L::kState, kStride = L::kStride;
-  extern __shared__ __align__(128) uint8_t smem[];
+  extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chain = blockIdx.x;
@@ -104,10 +108,11 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
   const uint32_t bar = sbase + L::kBar;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kBar + 8);
   constexpr int row_bytes = kFp32 ? 512 : 256;
-  constexpr int in_off = !kFp32 && kWide ? kBf16Row : 0;
+  constexpr int in_off = kFp32 ? 0 : kBf16Row;
   if (tid == 0) {
-    *abort_flag = 0;
-    mbar_init(bar, kD);
+    // (the swizzled state needs this alignment: report instead of computing garbage)
+    *abort_flag = !kWide && (sbase & 1023u) != 0u ? 1 : 0;
+    mbar_init(bar, kWide ? kD : 1);
     fence_mbar_init();
   }
   __syncthreads();
@@ -126,8 +131,15 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
     load_rows(0, kStG, p.g);
     load_rows(0, kStV, p.v);
   }
-  // ---- the state: one bulk copy per row into the padded staging buffer, behind the inputs, which are needed first ----
-  if (p.initial_state != nullptr && tid < kD) {
+  // ---- the state, behind the inputs, which are needed first: one bulk copy per row into the padded staging buffer, or two
+  // tensor copies (a copy per row costs a dozen instructions, as the threads of a warp issue theirs one by one) ----
+  if (!kWide) {
+    if (p.initial_state != nullptr && tid == 0 && *abort_flag == 0) {
+      mbar_arrive_expect_tx(bar, kD * 256);
+      tma_load_3d(sbase + kState, &tm_in, 0, 0, chain, bar);
+      tma_load_3d(sbase + kState + 16384, &tm_in, 64, 0, chain, bar);
+    }
+  } else if (p.initial_state != nullptr && tid < kD) {
     mbar_arrive_expect_tx(bar, row_bytes);
     bulk_g2s(sbase + kState + tid * kStride + in_off,
              static_cast<const uint8_t*>(p.initial_state) + (static_cast<size_t>(chain) * kD + tid) * row_bytes, row_bytes, bar);
@@ -139,14 +151,10 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
     hab[0] = ha * __ldg(p.dt_bias + h * kD + 16 * warp + g);
     hab[1] = ha * __ldg(p.dt_bias + h * kD + 16 * warp + 8 + g);
   }
-  // a 16 x 16 triangle of ones as A fragments, and the gate's constant part (fkda_elem.cuh)
-  uint32_t tri[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = g + 8 * (i & 1), k0 = 2 * t4 + 8 * (i >> 1);
-    tri[i] = (k0 <= row ? 0x3c00u : 0u) | (k0 + 1 <= row ? 0x3c000000u : 0u);
-  }
   uint8_t* const srow = smem + kState + (16 * (warp & 7) + g) * kStride;
+  // (bf16 halves) the row this lane addresses in a ldmatrix.x4 over a 16 x 16 tile of this warp's rows, and its column tile's position
+  const uint32_t hrow = sbase + kState + (16 * (warp & 7) + 8 * (mi & 1) + r) * 128, hcol = static_cast<uint32_t>(((mi >> 1) ^ r) << 4);
+  auto half_tile = [&](int ks) { return hrow + (ks >> 2) * 16384 + (hcol ^ (32u * (ks & 3))); };
   bool failed = false;
 
   for (int blk = 0; blk < nblk; ++blk) {
@@ -168,17 +176,21 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
       ldsm_x4(src + kStK, k[0], k[1], k[2], k[3]);
       ldsm_x4_trans(src + kStG, gw[0], gw[1], gw[2], gw[3]);
       if (kOneBlock) ldsm_x4_trans(src + kStV, x[0], x[1], x[2], x[3]);
-      auto squares = [&](const uint32_t(&x)[4], float* dst) {
-        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_bf16_16816(c0, x[0], x[1], x[2], x[3], x[0], x[2]);
-        mma_bf16_16816(c1, x[0], x[1], x[2], x[3], x[1], x[3]);
+      const int part = 4 * (warp ^ (g & 4));   // (rows 4-7 of eight have the halves exchanged: sixteen-byte reads by row do not conflict)
+      auto squares = [&](const uint32_t(&x)[4], uint32_t dst) {
+        float c0[4], c1[4];
+        mma_bf16_1688_zero(c0, x[0], x[1], x[0]);
+        mma_bf16_1688_zero(c1, x[0], x[1], x[1]);
+        mma_bf16_1688(c0, x[2], x[3], x[2]);
+        mma_bf16_1688(c1, x[2], x[3], x[3]);
         if (t4 == (g >> 1)) {
-          dst[g * 8] = (g & 1) ? c0[1] : c0[0];
-          dst[(8 + g) * 8] = (g & 1) ? c1[3] : c1[2];
+          sts_f32(dst + g * 32, (g & 1) ? c0[1] : c0[0]);
+          sts_f32(dst + (8 + g) * 32, (g & 1) ? c1[3] : c1[2]);
         }
       };
-      squares(q, s_ssq + warp);
-      squares(k, s_ssq + 128 + warp);
+      squares(q, sbase + L::kSsq + part);
+      squares(k, sbase + L::kSsq + 512 + part);
+      const Const kc(lane, hgs);            // a 16 x 16 triangle of ones as A fragments, and the gate's constant part
       f2 G[2][2], tot[2];
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
@@ -192,27 +204,27 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
           }
           split_f16(x0, x1, hi[b], lo[b]);
         }
-        const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
-        float d[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_f16_16816(d, tri, hi[0], hi[1]);
-        mma_f16_16816(s, ones, hi[0], hi[1]);
-        mma_f16_16816(d, tri, lo[0], lo[1]);
-        mma_f16_16816(s, ones, lo[0], lo[1]);
-        const float c0 = hgs * static_cast<float>(g + 1), c1 = hgs * static_cast<float>(g + 9);
-        G[nt][0] = fma2(pk(d[0], d[1]), pk(hgs, hgs), pk(c0, c0));
-        G[nt][1] = fma2(pk(d[2], d[3]), pk(hgs, hgs), pk(c1, c1));
-        tot[nt] = fma2(pk(s[0], s[1]), pk(hgs, hgs), pk(16.f * hgs, 16.f * hgs));
+        float d[4];
+        mma_f16_16816_zero(d, kc.tri, hi[0], hi[1]);
+        mma_f16_16816(d, kc.tri, lo[0], lo[1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[e] = fmaf(d[e], hgs, kc.hc[e >> 1]);
+        G[nt][0] = pk(d[0], d[1]);
+        G[nt][1] = pk(d[2], d[3]);
+        tot[nt] = pk(__shfl_sync(0xffffffffu, d[2], lane | 28), __shfl_sync(0xffffffffu, d[3], lane | 28));     // token 15
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");      // the partial sums of squares are complete, the staged inputs read
       float rq[2], rk[2];
+      {
+        // lanes 0-15: rows of q, 16-31: rows of k
+        const uint32_t at = sbase + L::kSsq + lane * 32 + (lane & 4) * 4;
+        const float4 x = lds_f4(at), y = lds_f4(at ^ 16);
+        const float n = rsqrtf(((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w)) + 1e-6f) * (lane < 16 ? p.scale : 1.f);
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const float4* s = reinterpret_cast<const float4*>(s_ssq + (g + 8 * b) * 8);
-        float4 x = s[0], y = s[1];
-        rq[b] = rsqrtf(((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w)) + 1e-6f) * p.scale;
-        x = s[32];
-        y = s[33];
-        rk[b] = rsqrtf(((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w)) + 1e-6f);
+        for (int b = 0; b < 2; ++b) {
+          rq[b] = __shfl_sync(0xffffffffu, n, g + 8 * b);
+          rk[b] = __shfl_sync(0xffffffffu, n, 16 + g + 8 * b);
+        }
       }
       uint32_t kn[4], qp[4], km[4], kr[4];
 #pragma unroll
@@ -221,9 +233,10 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
         if (g == 0) *reinterpret_cast<f2*>(s_e + 16 * warp + 8 * nt + 2 * t4) = e;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
-          const f2 kh = mul(unpack_bf(k[2 * nt + b]), pk(rk[b], rk[b])), qh = mul(unpack_bf(q[2 * nt + b]), pk(rq[b], rq[b]));
-          const f2 pw = exp2_pair(G[nt][b]), m = mul(kh, exp2_neg_pair(G[nt][b]));
-          kn[2 * nt + b] = round_bf(mul(kh, mul(pw, pk(-1.f, -1.f))));
+          const uint32_t kw = k[2 * nt + b], qw = q[2 * nt + b];
+          const f2 kh = pk(bf_lo(kw) * rk[b], bf_hi(kw) * rk[b]), qh = pk(bf_lo(qw) * rq[b], bf_hi(qw) * rq[b]);
+          const f2 pw = exp2_pair(G[nt][b]), m = mul(kh, rcp_pair(pw));
+          kn[2 * nt + b] = round_bf(mul(kh, pw)) ^ 0x80008000u;
           qp[2 * nt + b] = round_bf(mul(qh, pw));
           km[2 * nt + b] = round_bf(m);
           kr[2 * nt + b] = round_bf(mul(m, e));
@@ -270,10 +283,12 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
               const float2 s = *reinterpret_cast<const float2*>(srow + (e & 1) * 8 * kStride + (16 * ks + 8 * (e >> 1) + 2 * t4) * 4);
               a[e] = pack_bf16(s.x, s.y);
             }
-          } else {
+          } else if (kWide) {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               a[e] = *reinterpret_cast<const uint32_t*>(srow + in_off + (e & 1) * 8 * kStride + (16 * ks + 8 * (e >> 1) + 2 * t4) * 2);
+          } else {
+            ldsm_x4(half_tile(ks), a[0], a[1], a[2], a[3]);
           }
           ldsm_x4(b_lane + kKN + ks * 256, b0, b1, b2, b3);
           mma_bf16_16816(R[0], a[0], a[1], a[2], a[3], b0, b1);
@@ -374,31 +389,39 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
 #pragma unroll
         for (int jp = 0; jp < 8; ++jp) {     // two column tiles per transposed load
           ldsm_x4_trans(sbase + kKR + (mi & 1) * 2048 + (2 * jp + (mi >> 1)) * 128 + r * 16, b0, b1, b2, b3);
+          uint32_t half[4] = {0u, 0u, 0u, 0u};       // (bf16 halves) the tile: c = 0 rows g, rows g + 8, c = 1 the same
+          if (!kWide && !zero_state) ldsm_x4(half_tile(jp), half[0], half[1], half[2], half[3]);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int col = 8 * (2 * jp + c) + 2 * t4;
-            float S[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t S[4] = {0u, 0u, 0u, 0u};
             if (!zero_state) {
               if (kWide && (kFp32 || blk > 0)) {
-                const float2 lo = *reinterpret_cast<const float2*>(srow + col * 4), hi = *reinterpret_cast<const float2*>(srow + 8 * kStride + col * 4);
+                const uint2 lo = *reinterpret_cast<const uint2*>(srow + col * 4), hi = *reinterpret_cast<const uint2*>(srow + 8 * kStride + col * 4);
                 S[0] = lo.x; S[1] = lo.y; S[2] = hi.x; S[3] = hi.y;
               } else {
-                const uint32_t lo = *reinterpret_cast<const uint32_t*>(srow + in_off + col * 2);
-                const uint32_t hi = *reinterpret_cast<const uint32_t*>(srow + in_off + 8 * kStride + col * 2);
-                S[0] = bf_lo(lo); S[1] = bf_hi(lo); S[2] = bf_lo(hi); S[3] = bf_hi(hi);
+                const uint32_t lo = kWide ? *reinterpret_cast<const uint32_t*>(srow + in_off + col * 2) : half[2 * c];
+                const uint32_t hi = kWide ? *reinterpret_cast<const uint32_t*>(srow + in_off + 8 * kStride + col * 2) : half[2 * c + 1];
+                S[0] = lo << 16; S[1] = lo & 0xffff0000u; S[2] = hi << 16; S[3] = hi & 0xffff0000u;
               }
               const float2 e2 = *reinterpret_cast<const float2*>(s_e + col);
-              S[0] *= e2.x; S[1] *= e2.y; S[2] *= e2.x; S[3] *= e2.y;
+              mul2(S[0], S[1], e2);
+              mul2(S[2], S[3], e2);
             }
-            mma_bf16_16816(S, u[0], u[1], u[2], u[3], c ? b2 : b0, c ? b3 : b1);
+            float Z[4] = {__uint_as_float(S[0]), __uint_as_float(S[1]), __uint_as_float(S[2]), __uint_as_float(S[3])};
+            mma_bf16_16816(Z, u[0], u[1], u[2], u[3], c ? b2 : b0, c ? b3 : b1);
             if (kFp32 || !last) {
-              *reinterpret_cast<float2*>(srow + col * 4) = make_float2(S[0], S[1]);
-              *reinterpret_cast<float2*>(srow + 8 * kStride + col * 4) = make_float2(S[2], S[3]);
+              *reinterpret_cast<float2*>(srow + col * 4) = make_float2(Z[0], Z[1]);
+              *reinterpret_cast<float2*>(srow + 8 * kStride + col * 4) = make_float2(Z[2], Z[3]);
+            } else if (kWide) {
+              *reinterpret_cast<uint32_t*>(srow + col * 2) = pack_bf16(Z[0], Z[1]);
+              *reinterpret_cast<uint32_t*>(srow + 8 * kStride + col * 2) = pack_bf16(Z[2], Z[3]);
             } else {
-              *reinterpret_cast<uint32_t*>(srow + col * 2) = pack_bf16(S[0], S[1]);
-              *reinterpret_cast<uint32_t*>(srow + 8 * kStride + col * 2) = pack_bf16(S[2], S[3]);
+              half[2 * c] = pack_bf16(Z[0], Z[1]);
+              half[2 * c + 1] = pack_bf16(Z[2], Z[3]);
             }
           }
+          if (!kWide) stsm_x4(half_tile(jp), half[0], half[1], half[2], half[3]);
         }
       }
       // ---- out: [v][tok] -> [tok][v] by stmatrix, one 16-byte piece per lane -------------------------------------------------
@@ -415,14 +438,21 @@ __global__ void __launch_bounds__(kThreads, Lay<kFp32 || !kOneBlock, kOneBlock>:
   if (failed || *abort_flag > 0) {
     // the state copy may still be landing: give it a moment before this CTA's shared memory goes away
     const uint64_t t_begin = globaltimer_ns();
-    while (!mbar_try_wait(bar, 0) && globaltimer_ns() - t_begin < 20000000ull) {}
+    while (p.initial_state != nullptr && !mbar_try_wait(bar, 0) && globaltimer_ns() - t_begin < 20000000ull) {}
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusWaitTimeout);
     return;
   }
   if (p.final_state != nullptr && warp < 8) {      // one bulk copy per row, per warp as soon as its rows are done
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane < 16) {
+    if (!kWide) {
+      if (lane == 0) {
+        tma_store_3d(&tm_out, sbase + kState + warp * 2048, 0, 16 * warp, chain);
+        tma_store_3d(&tm_out, sbase + kState + 16384 + warp * 2048, 64, 16 * warp, chain);
+        bulk_commit();
+        bulk_wait_read0();
+      }
+    } else if (lane < 16) {
       const int vr = 16 * warp + lane;
       bulk_s2g(static_cast<uint8_t*>(p.final_state) + (static_cast<size_t>(chain) * kD + vr) * row_bytes,
                sbase + kState + vr * kStride, row_bytes);
@@ -442,12 +472,16 @@ cudaError_t launch_short16(const __nv_bfloat16* q, const __nv_bfloat16* k, const
   using namespace short16;
   const Params p{q, k, v, g, beta, A_log, dt_bias, initial_state, final_state, out, T, H, scale, gate_scale, status};
   const int form = (state_fp32 ? 2 : 0) + (T <= kRows ? 1 : 0);
-  void (*const kernels[4])(Params) = {short16_kernel<false, false>, short16_kernel<false, true>, short16_kernel<true, false>, short16_kernel<true, true>};
+  void (*const kernels[4])(CUtensorMap, CUtensorMap, Params) = {short16_kernel<false, false>, short16_kernel<false, true>, short16_kernel<true, false>, short16_kernel<true, true>};
   const int smem = form == 0 || form == 2 ? Lay<true, false>::kSmemBytes : form == 1 ? Lay<false, true>::kSmemBytes : Lay<true, true>::kSmemBytes;
   static SmemOptIn opt_in[4];
   cudaError_t e = opt_in[form].ensure(kernels[form], smem);
   if (e != cudaSuccess) return e;
-  return launch_after(kernels[form], static_cast<unsigned>(N * H), kThreads, smem, stream, p);
+  CUtensorMap in{}, fin{};
+  if (form == 1 && ((initial_state != nullptr && !make_state_map(&in, initial_state, N * H, kD)) ||
+                    (final_state != nullptr && !make_state_map(&fin, final_state, N * H, 16))))
+    return cudaErrorInvalidValue;
+  return launch_after(kernels[form], static_cast<unsigned>(N * H), kThreads, smem, stream, in, fin, p);
 }
 
 }  // namespace fkda
