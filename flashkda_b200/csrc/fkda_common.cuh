@@ -380,7 +380,8 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
 constexpr int64_t kFusedMaxT = 32;
 // ... and of at most this many tokens the per-token kernel (fkda_step.cu), in packed batches too.  It costs about 0.4 us per
 // token, chain and SM beside the stream over the states; the tile kernel's cost does not depend on the tokens.  64 x 32
-// chains, bf16 states: 25 us at one token, 47 against 42 at five; fp32: 44, and 59 against 63.
+// chains, fp32 states: 52 us at four tokens against 60; bf16: 38 against 31, but the per-token kernel computes in fp32
+// throughout and the tile kernel on bf16 operands, so the line is not moved down to where the times cross.
 constexpr int64_t kStepMaxT = 4;
 constexpr int kOrderMax = 4096;      // packed batches of more sequences keep the given order instead of longest first
 

@@ -62,7 +62,18 @@ __device__ __forceinline__ void mma_f16_16816_zero(float (&c)[4], const uint32_t
                : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
-// D(16x8,f32) = A(16x8,bf16,row) * B(8x8,bf16,col), then D += ...
+// D(16x8,f32) = A(16x8,f16,row) * B(8x8,f16,col), then D += ...
+__device__ __forceinline__ void mma_f16_1688_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+}
+__device__ __forceinline__ void mma_f16_1688(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(b));
+}
+// The same with bf16 operands.
 __device__ __forceinline__ void mma_bf16_1688_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])

@@ -224,6 +224,23 @@ def test_short_sequences_match_the_recurrence(B, T, state):
     assert rel_fro(fin.cpu(), s64) <= STATE_REL
 
 
+@pytest.mark.parametrize("state", [None, "bf16", "fp32"])
+@pytest.mark.parametrize("B,T", [(3, 5), (3, 6), (5, 7), (3, 8), (3, 9), (300, 8)])
+def test_eight_token_tiles_match_the_recurrence(B, T, state):
+    """The eight-token form of the tile kernel, around its edges, with and without a final state."""
+    w = Workload("e", H=2, B=B, T=T, state_in=state, state_out=state or "fp32", state_std=0.5, seed=B * 100 + T, lower_bound=-2.0)
+    x = make_inputs(w)
+    xc = to_cuda(x)
+    out, fin = torch.full_like(xc["v"], float("nan")), torch.full_like(xc["final_state"], float("nan"))
+    for final in (fin, None):
+        F.fwd(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], out, xc["A_log"], xc["dt_bias"], x["lower_bound"],
+              initial_state=xc["initial_state"], final_state=final)
+        o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                         initial_state=x["initial_state"])
+        assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS and rel_fro(out.cpu(), o64) <= 1e-2
+    assert rel_fro(fin.cpu(), s64) <= STATE_REL
+
+
 def test_decode_tokens_among_prompts():
     """A packed batch that mixes sequences of a few tokens, which the per-token kernel takes, with prompts."""
     lens = [1] * 7 + [40, 4, 5, 0, 300, 1, 3, 33]
