@@ -1,27 +1,28 @@
 // Inter-chunk recurrence of the KDA prefill over compact records: the state of a (sequence, head) chain in registers, the
-// output products on tcgen05.
+// products on its copy on tcgen05.
 //
 // Replaces the reference's K2 (csrc/smxx/fwd_kernel2.cuh:115-839).  The rows v of S^T never meet each other in the
-// recurrence, so four warps hold 32 rows each as fp32 mma.sync accumulator fragments, and everything on the serial chain
-// stays in the fragment layout:
-//     R^T = v^T - S^T k+^T     A = the state registers rounded to bf16, B = -k+ rows by ldmatrix; the accumulators start
-//                              from v^T, which a transposing ldmatrix brings from its TMA tile     [32 v x 32 tok]
-//     U^T = R^T (T diag(beta))^T
-//     S^T = S^T diag(e) + U^T kr      A = U^T, the packed accumulators of the line above; accumulators = the state
-// No trip through tensor memory or shared memory lies on that chain and no rendezvous between warps; a chunk waits for its
-// record only.  (With the state in tensor memory, fkda_scan2.cu, a chunk costs a commit, a read, a decay and a write of the
-// whole state per step.)
-//     O^T = S^T q+^T + U^T mqk^T
-// is off the chain: the bf16 copies of S^T and U^T are left in tensor memory, one thread issues the ten products, four
-// other warps write the result.
+// recurrence, so four warps hold 32 rows each as fp32 mma.sync accumulator fragments:
+//     R^T = v^T - S^T k+^T                     on tcgen05, together with S^T q+^T: A = the bf16 copy of the state in tensor
+//                                              memory, B = k+ | q+ of the record                  [128 v x 64]
+//     U^T = R^T (T diag(beta))^T               mma.sync; R^T is read from tensor memory in fragment layout
+//     S^T = S^T diag(e) + U^T kr               mma.sync; A = U^T, the packed accumulators of the line above
+//     O^T = S^T q+^T + U^T mqk^T               the second product on top of the first, tcgen05; four other warps write it
+// With k+ and q+ in one operand the product on the chain costs the tensor cores no more than the output's alone, and it replaces
+// nearly half of a warp's mma.sync.  What made it pay (4 x 8192 tokens x 32 heads, cycles per chunk by clock64):
+//   * all of it on mma.sync but the output, which interrupts it: 2700 cycles, 0.342 ms; R^T on tcgen05 at first 2680;
+//   * no wait for a store to tensor memory right behind it (200 cycles each): 2530;
+//   * the products issued by a whole warp with operands that the compiler can see to be uniform (elect.sync) instead of from one
+//     lane's branch, where each costs 75 cycles: 2230;
+//   * one accumulator for both halves of k: 2140;
+//   * the state's decay while the product on its copy is under way, not between the mma.sync of the update: 2040;
+//   * the first half of the copy announced three quarters through the update: 2010.  0.280 ms in a burst of calls, 0.323 -
+//     0.335 kept up under the power cap (0.342 and 0.372 - 0.378 before).
+// Eight recurrence warps of 16 rows: 2700 (every operand is read twice as often); three groups of k instead of two: 0.325 ms; a
+// part of the decay left in the update: 0.297.  What bounds it now is the chain itself, of which a warp works 1900 cycles: update 1090,
+// the product's way through tensor memory 470, R and U 360.
 //
-// What bounds it: a warp's 140 mma.sync of 8 cycles on its sub-partition (1120 cycles per chunk), the ten tcgen05.mma, each of
-// which keeps the tensor cores from them for about 50 cycles, and the latencies in between: 2470 cycles per chunk (1720
-// with the output products left out).  Two warps of 16 rows per sub-partition read every operand twice as often and end at
-// the shared-memory pipe (2650); the output products on mma.sync in the output warps: 2700.  4 x 8192 tokens x 32 heads, fp32
-// state, over records of 0.96 GB: 0.357 ms in a burst of calls (4.2 TB/s), 0.382 kept up under the power cap.
-//
-// Warps 0-3: recurrence; 4-7: output, and one of them each the output products and the copies.  The code of a
+// Warps 0-3: recurrence; 4-7: output, and one of them each the tcgen05 products and the copies.  The code of a
 // recurrence warp and of the output warp on the same SM sub-partition together stay near 8 KB: beyond that a sub-partition's
 // instruction cache misses and straight-line code runs at three cycles per instruction and warp at best.
 #include "fkda_common.cuh"
@@ -43,15 +44,14 @@ constexpr int kSmBars = kSmInfo + kInfos * 32;
 constexpr int kSmMisc = kSmBars + 256;
 constexpr int kSmem = kSmMisc + 16;
 static_assert(kSmem <= 227 * 1024, "shared memory plan");
-// tensor memory columns.  The copies of S and U follow the stages: a stage is refilled only once the output products of
-// its chunk, which read both, are complete, so a full stage means that its copies may be written over.
-constexpr uint32_t kTmemCols = 512;
-constexpr int kOBufs = 3;
-constexpr uint32_t kColSb = 0;                     // kStages x 64: bf16 copy of S^T [v][k], two k per column
-constexpr uint32_t kColUt = kColSb + 64 * kStages; // kStages x 16: bf16 U^T [v][tok]
-constexpr uint32_t kColO = kColUt + 16 * kStages;  // kOBufs x 32: O^T [v][tok]
-static_assert(kColO + 32 * kOBufs <= kTmemCols, "tensor memory plan");
-enum { B_FULL = 0, B_EMPTY = kStages, B_U = 2 * kStages, B_O = 3 * kStages, B_O_FREE = B_O + kOBufs, B_COUNT = B_O_FREE + kOBufs };
+// tensor memory columns.  One copy of S and of U each: when the products of a chunk on S are complete, those of the chunk
+// before on U are too (one thread issues both), and the state's copy may be written over.
+constexpr uint32_t kTmemCols = 256;
+constexpr uint32_t kColSb = 0;                     // 64: bf16 copy of S^T [v][k], two k per column
+constexpr uint32_t kColUt = kColSb + 64;           // 16: bf16 U^T [v][tok]
+constexpr uint32_t kColD = 128;                    // two chunks x 64: S^T k+^T | S^T q+^T [v][tok], O^T on top of the latter
+static_assert(kColUt + 16 <= kColD && kColD + 128 <= kTmemCols, "tensor memory plan");
+enum { B_FULL = 0, B_EMPTY = kStages, B_S = 2 * kStages /*[2] halves of k*/, B_R = B_S + 2, B_U = B_R + 1, B_O = B_U + 1 /*[2]*/, B_O_FREE = B_O + 2 /*[2]*/, B_LAST = B_O_FREE + 2, B_COUNT };
 static_assert(B_COUNT * 8 <= 256, "barrier area");
 
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -74,119 +74,124 @@ struct Info {
 static_assert(sizeof(Info) == 32, "info");
 enum { kEnd = 1 };
 
-// One chunk on the recurrence warps, from stage s.  S: rows v = row0 + 16 vt + g (+ 8), columns 8 jt + 2 t, + 1.  `ready`: whether the
-// next stage is full already.
-// kOut: copies of S and U for the output products.  kBack: the transposed step, S^T Phi^T with Phi = diag(e) + kn^T TB^T kr the
-// chunk's transition and no v: the same products with k+ and kr exchanged and TB transposed.
-template <bool kOut, bool kBack>
-__device__ __forceinline__ void step(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int s, int len, int row0, int lane, uint32_t next_full,
-                                     uint32_t next_par, bool& ready) {
+// The bf16 copy of half of the state's columns into tensor memory.
+__device__ __forceinline__ void put_copy(const float (&S)[2][16][4], uint32_t tq, int half, int vt) {
+  uint32_t a[16];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    a[2 * j] = pack_bf16(S[vt][8 * half + j][0], S[vt][8 * half + j][1]);
+    a[2 * j + 1] = pack_bf16(S[vt][8 * half + j][2], S[vt][8 * half + j][3]);
+  }
+  tmem_st_16x128b_x8(tq + (static_cast<uint32_t>(16 * vt) << 16) + kColSb + 32 * half, a);
+}
+
+// The chunks of one walk on the recurrence warps, from stage s (phase par) on; ready: that stage is known to be full; item: its index in the
+// CTA's stream.  S: rows v = row0 + 16 vt + g (+ 8), columns 8 jt + 2 t, + 1.
+__device__ __forceinline__ bool walk(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int nchunks, int64_t tokens, int row0, int lane,
+                                     volatile int* abort_flag, int& s, uint32_t& par, bool& ready, uint32_t item) {
+  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
   const int mi = lane >> 3, r = lane & 7, t = lane & 3;
-  const uint32_t kn_lane = 8192 + (kBack ? kCrKR : kCrKN) + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
-  const uint32_t kr_lane = 8192 + (kBack ? kCrKN : kCrKR) + mi * 2048 + r * 16;
+  const uint32_t kr_lane = 8192 + kCrKR + mi * 2048 + r * 16;
   const uint32_t v_lane = (row0 >> 6) * 4096 + lane * 128;
   const uint32_t tb_lane = 8192 + kCrTB + r * 16;
-  const uint32_t stage = sbase + s * kStageBytes;
-
-  // R^T = v^T - S^T k+^T: the accumulators start from v^T; operands of a k-step are loaded during the one before
-  float R[2][4][4];
-  if (kBack) {
-#pragma unroll
-    for (int vt = 0; vt < 2; ++vt)
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) R[vt][nt][0] = R[vt][nt][1] = R[vt][nt][2] = R[vt][nt][3] = 0.f;
-  } else {
-    uint32_t x[4][4];              // v^T: channel blocks of 8 rows; register = token block
-#pragma unroll
-    for (int i = 0; i < 4; ++i) ldsm_x4_trans(stage + v_lane + ((((row0 >> 3) + i) & 7) ^ r) * 16, x[i][0], x[i][1], x[i][2], x[i][3]);
-    if (len < kChunk) {            // rows past the sequence end belong to somebody else
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const uint32_t keep = (8 * nt + 2 * t < len ? 0xffffu : 0u) | (8 * nt + 2 * t + 1 < len ? 0xffff0000u : 0u);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i][nt] &= keep;
-      }
-    }
-#pragma unroll
-    for (int vt = 0; vt < 2; ++vt)
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        R[vt][nt][0] = bf_lo(x[2 * vt][nt]);
-        R[vt][nt][1] = bf_hi(x[2 * vt][nt]);
-        R[vt][nt][2] = bf_lo(x[2 * vt + 1][nt]);
-        R[vt][nt][3] = bf_hi(x[2 * vt + 1][nt]);
-      }
-  }
-  uint32_t bb[2][8];
-  ldsm_x4(stage + kn_lane, bb[0][0], bb[0][1], bb[0][2], bb[0][3]);
-  ldsm_x4(stage + kn_lane + 4096, bb[0][4], bb[0][5], bb[0][6], bb[0][7]);
-  if (kOut) tc_fence_after();
-  const uint32_t sb = tq + kColSb + 64 * s;
+  auto arrive_after_st = [&](int b) {
+    tmem_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(b));
+  };
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
-    uint32_t a[2][16];               // bf16 copy of the state: A fragments of four k-steps, and 32 columns of tensor memory
-#pragma unroll
-    for (int vt = 0; vt < 2; ++vt) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        a[vt][2 * j] = pack_bf16(S[vt][8 * half + j][0], S[vt][8 * half + j][1]);
-        a[vt][2 * j + 1] = pack_bf16(S[vt][8 * half + j][2], S[vt][8 * half + j][3]);
-      }
-      if (kOut) tmem_st_16x128b_x8(sb + (static_cast<uint32_t>(16 * vt) << 16) + 32 * half, a[vt]);
-    }
-#pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4) {
-      const int ks = 4 * half + k4;
-      const uint32_t(&B)[8] = bb[ks & 1];
-      if (ks < 7) {
-        uint32_t(&N)[8] = bb[(ks + 1) & 1];
-        ldsm_x4(stage + kn_lane + (ks + 1) * 256, N[0], N[1], N[2], N[3]);
-        ldsm_x4(stage + kn_lane + 4096 + (ks + 1) * 256, N[4], N[5], N[6], N[7]);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int vt = 0; vt < 2; ++vt)
-          mma_bf16_16816(R[vt][nt], a[vt][4 * k4], a[vt][4 * k4 + 1], a[vt][4 * k4 + 2], a[vt][4 * k4 + 3], B[2 * nt], B[2 * nt + 1]);
-    }
+    put_copy(S, tq, half, 0);
+    put_copy(S, tq, half, 1);
+    arrive_after_st(B_S + half);
   }
-  // U^T = R^T (T diag(beta))^T
-  uint32_t l[4], m[4], n[4];       // T diag(beta): token tiles 0 and 1 (tokens 0-15 only: lower triangle), 2, 3; transposed: 0, 1, 2 and 3 (16-31 only)
-  if (kBack) {
-    ldsm_x4_trans(stage + tb_lane + mi * 512, l[0], l[1], l[2], l[3]);
-    ldsm_x4_trans(stage + tb_lane + mi * 512 + 128, m[0], m[1], m[2], m[3]);
-    ldsm_x4_trans(stage + tb_lane + 1024 + (mi & 1) * 512 + 256 + (mi >> 1) * 128, n[0], n[1], n[2], n[3]);
-  } else {
+  for (int c = 0; c < nchunks; ++c, ++item) {
+    if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) return false;
+    const uint32_t stage = sbase + s * kStageBytes;
+
+    // R^T = v^T - S^T k+^T; T diag(beta) and the first of kr meanwhile
+    float R[2][4][4];
+    {
+      uint32_t x[4][4];              // v^T: channel blocks of 8 rows; register = token block
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ldsm_x4_trans(stage + v_lane + ((((row0 >> 3) + i) & 7) ^ r) * 16, x[i][0], x[i][1], x[i][2], x[i][3]);
+      const int64_t left = tokens - static_cast<int64_t>(c) * kChunk;
+      if (left < kChunk) {           // rows past the sequence end belong to somebody else
+        const int len = static_cast<int>(left);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const uint32_t keep = (8 * nt + 2 * t < len ? 0xffffu : 0u) | (8 * nt + 2 * t + 1 < len ? 0xffff0000u : 0u);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i][nt] &= keep;
+        }
+      }
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          R[vt][nt][0] = bf_lo(x[2 * vt][nt]);
+          R[vt][nt][1] = bf_hi(x[2 * vt][nt]);
+          R[vt][nt][2] = bf_lo(x[2 * vt + 1][nt]);
+          R[vt][nt][3] = bf_hi(x[2 * vt + 1][nt]);
+        }
+    }
+    uint32_t l[4], m[4], n[4];       // T diag(beta): token tiles 0 and 1 (tokens 0-15 only: lower triangle), 2, 3
     ldsm_x4(stage + tb_lane + (mi >> 1) * 512 + (mi & 1) * 128, l[0], l[1], l[2], l[3]);
     ldsm_x4(stage + tb_lane + 1024 + mi * 128, m[0], m[1], m[2], m[3]);
     ldsm_x4(stage + tb_lane + 1536 + mi * 128, n[0], n[1], n[2], n[3]);
-  }
-  uint32_t kr[2][4];
-  ldsm_x4_trans(stage + kr_lane, kr[0][0], kr[0][1], kr[0][2], kr[0][3]);
-  uint32_t u[2][2][4];             // A fragments, k-step = 16 tokens: first of R^T, then of U^T
-  auto as_operand = [&](uint32_t(&d)[2][4], const float(&x)[4][4]) {
+    uint32_t kr[2][4];
+    ldsm_x4_trans(stage + kr_lane, kr[0][0], kr[0][1], kr[0][2], kr[0][3]);
+    // and the state's decay: its copy has been taken
+    const float2* e2 = reinterpret_cast<const float2*>(smem + s * kStageBytes + 8192 + kCrE) + t;
+    bool there = false;
 #pragma unroll
-    for (int ks = 0; ks < 2; ++ks)
+    for (int jt = 0; jt < 16; ++jt) {
+      if (jt == 12) there = mbar_test(bar(B_R), item & 1u);
+      const float2 e = e2[4 * jt];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)  // e & 1: rows + 8, e >> 1: tokens + 8
-        d[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
-  };
+      for (int vt = 0; vt < 2; ++vt) {
+        uint32_t y[4];
 #pragma unroll
-  for (int vt = 0; vt < 2; ++vt) as_operand(u[vt], R[vt]);
-  {
-    float U[2][4][4];
+        for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[vt][jt][k]);
+        mul2(y[0], y[1], e);
+        mul2(y[2], y[3], e);
 #pragma unroll
-    for (int vt = 0; vt < 2; ++vt) {
+        for (int k = 0; k < 4; ++k) S[vt][jt][k] = __uint_as_float(y[k]);
+      }
+    }
+    if (!__all_sync(0xffffffffu, there) && !warp_wait(bar(B_R), item & 1u, abort_flag)) return false;
+    tc_fence_after();
+    uint32_t u[2][2][4];             // A fragments, k-step = 16 tokens: first of R^T, then of U^T
+    auto as_operand = [&](uint32_t(&d)[2][4], const float(&x)[4][4]) {
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) U[vt][nt][0] = U[vt][nt][1] = U[vt][nt][2] = U[vt][nt][3] = 0.f;
-      if (kBack) {
-        mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
-        mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
-        mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[0], n[1]);
-        mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
-        mma_bf16_16816(U[vt][0], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], l[2], l[3]);
-        mma_bf16_16816(U[vt][1], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
-      } else {
+      for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)  // e & 1: rows + 8, e >> 1: tokens + 8
+          d[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
+    };
+    {
+      const uint32_t d = tq + kColD + 64 * (item & 1u);
+      uint32_t y[2][16];
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) tmem_ld_16x256b_x4(d + (static_cast<uint32_t>(16 * vt) << 16), y[vt]);
+      tmem_wait_ld();
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) R[vt][nt][e] += __uint_as_float(y[vt][4 * nt + e]);
+        as_operand(u[vt], R[vt]);
+      }
+    }
+    // U^T = R^T (T diag(beta))^T
+    {
+      float U[2][4][4];
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt) {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) U[vt][nt][0] = U[vt][nt][1] = U[vt][nt][2] = U[vt][nt][3] = 0.f;
         mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
         mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[2], l[3]);
         mma_bf16_16816(U[vt][2], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
@@ -194,64 +199,43 @@ __device__ __forceinline__ void step(float (&S)[2][16][4], uint8_t* smem, uint32
         mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
         mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
       }
-    }
 #pragma unroll
-    for (int vt = 0; vt < 2; ++vt) {
-      as_operand(u[vt], U[vt]);
-      if (kOut) {
-        const uint32_t ut = tq + (static_cast<uint32_t>(16 * vt) << 16) + kColUt + 16 * s;
-        tmem_st_16x128b_x4(ut, u[vt][0], u[vt][1]);
+      for (int vt = 0; vt < 2; ++vt) {
+        as_operand(u[vt], U[vt]);
+        tmem_st_16x128b_x4(tq + (static_cast<uint32_t>(16 * vt) << 16) + kColUt, u[vt][0], u[vt][1]);
       }
     }
-  }
-  // S^T = S^T diag(e) + U^T kr; the next stage's barrier is looked at meanwhile
-  const float2* e2 = reinterpret_cast<const float2*>(smem + s * kStageBytes + 8192 + kCrE) + t;
-  ready = mbar_test(next_full, next_par);
-#pragma unroll
-  for (int jt = 0; jt < 16; ++jt) {
-    const uint32_t(&B)[4] = kr[jt & 1];
-    if (jt < 15) {
-      uint32_t(&N)[4] = kr[(jt + 1) & 1];
-      ldsm_x4_trans(stage + kr_lane + (jt + 1) * 128, N[0], N[1], N[2], N[3]);
-    }
-    const float2 e = e2[4 * jt];
-#pragma unroll
-    for (int vt = 0; vt < 2; ++vt) {
-      uint32_t y[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[vt][jt][k]);
-      mul2(y[0], y[1], e);
-      mul2(y[2], y[3], e);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) S[vt][jt][k] = __uint_as_float(y[k]);
-    }
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-      for (int vt = 0; vt < 2; ++vt)
-        mma_bf16_16816(S[vt][jt], u[vt][ks][0], u[vt][ks][1], u[vt][ks][2], u[vt][ks][3], B[2 * ks], B[2 * ks + 1]);
-  }
-  if (kOut) {
-    tmem_wait_st();
-    tc_fence_before();
-  }
-}
-
-// The chunks of one walk on the recurrence warps, from stage s (phase par) on; ready: that stage is known to be full.
-__device__ __forceinline__ bool walk(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, uint32_t tq, int nchunks, int64_t tokens, int row0, int lane,
-                                     volatile int* abort_flag, int& s, uint32_t& par, bool& ready) {
-  auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
-  for (int c = 0; c < nchunks; ++c) {
-    if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) return false;
-    const int64_t left = tokens - static_cast<int64_t>(c) * kChunk;
+    // S^T = S^T diag(e) + U^T kr, and the copy of it for the next chunk as its halves are done; the next stage's barrier is looked at meanwhile
     const int s1 = s + 1 == kStages ? 0 : s + 1;
     const uint32_t par1 = s1 == 0 ? par ^ 1u : par;
-    step<true, false>(S, smem, sbase, tq, s, left < kChunk ? static_cast<int>(left) : kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
-    __syncwarp();
-    if (lane == 0) {
-      mbar_arrive(bar(B_U + s));
-      mbar_arrive(bar(B_EMPTY + s));
+    const bool more = c + 1 < nchunks;
+    ready = mbar_test(bar(B_FULL + s1), par1);
+#pragma unroll
+    for (int jt = 0; jt < 16; ++jt) {
+      const uint32_t(&B)[4] = kr[jt & 1];
+      if (jt < 15) {
+        uint32_t(&N)[4] = kr[(jt + 1) & 1];
+        ldsm_x4_trans(stage + kr_lane + (jt + 1) * 128, N[0], N[1], N[2], N[3]);
+      }
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+          mma_bf16_16816(S[vt][jt], u[vt][ks][0], u[vt][ks][1], u[vt][ks][2], u[vt][ks][3], B[2 * ks], B[2 * ks + 1]);
+      if (jt == 4) arrive_after_st(B_U);
+      if (more) {
+        if (jt == 8) put_copy(S, tq, 0, 0);
+        if (jt == 9) put_copy(S, tq, 0, 1);
+        if (jt == 13) arrive_after_st(B_S);
+      }
     }
+    if (more) {
+      put_copy(S, tq, 1, 0);
+      put_copy(S, tq, 1, 1);
+      arrive_after_st(B_S + 1);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(B_EMPTY + s));
     s = s1;
     par = par1;
   }
@@ -318,7 +302,7 @@ template <bool kSeg, bool kStream, bool kSlice>
 __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constant__ CUtensorMap tm_v, const ScanParams p, const int walks) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kSmMisc + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kSmMisc);
   Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
@@ -328,13 +312,16 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar(B_FULL + s), 1);
-      mbar_init(bar(B_EMPTY + s), 4 + 1);              // recurrence warps + commit of the output products
-      mbar_init(bar(B_U + s), 4);
+      mbar_init(bar(B_EMPTY + s), 4 + 1);              // recurrence warps + commit of the products on U
     }
-    for (int i = 0; i < kOBufs; ++i) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(B_S + i), 4);
       mbar_init(bar(B_O + i), 1);
       mbar_init(bar(B_O_FREE + i), 4);
     }
+    mbar_init(bar(B_R), 1);
+    mbar_init(bar(B_LAST), 1);
+    mbar_init(bar(B_U), 4);
     fence_mbar_init();
   }
   if (warp == 4) {
@@ -344,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = *tmem_slot, utmem = __shfl_sync(0xffffffffu, tmem, 0);
   bool ok = *abort_flag <= 0;
   grid_dependency_wait();
   if (p.release_next) grid_release_next();
@@ -364,23 +351,19 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
         const volatile Info* f = infos + (i & (kInfos - 1));
         walk_index = f->walk;
         ready = true;
-        if (f->flags & kEnd) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(B_U + s));
-          break;
-        }
+        if (f->flags & kEnd) break;
       }
       const ChainView cv = chain_view<kSeg, kSlice>(p, walk_index);
       load_state(S, cv, row0, lane);
       // (an empty run hands its state through)
-      if (cv.nchunks > 0) ok = walk(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, row0, lane, abort_flag, s, par, ready);
+      if (cv.nchunks > 0) ok = walk(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, row0, lane, abort_flag, s, par, ready, static_cast<uint32_t>(i));
       if (ok && cv.fin_base != nullptr) store_state(S, cv, row0, lane);
       if (!kStream) break;
       i += cv.nchunks;
     }
   } else {
     const int w = warp - 4, mi = lane >> 3, r = lane & 7;
-    const uint32_t tq = tmem + (static_cast<uint32_t>(32 * w) << 16) + kColO;
+    const uint32_t tq = tmem + (static_cast<uint32_t>(32 * w) << 16) + kColD + 32;
     const uint32_t stg = sbase + kSmStg + w * 32 * kStgStride;
     const uint8_t* src = smem + kSmStg + w * 32 * kStgStride + (lane >> 2) * kStgStride + (lane & 3) * 16;
     __nv_bfloat16* const out0 = p.out + static_cast<size_t>(lane >> 2) * p.H * kD + 32 * w + (lane & 3) * 8;
@@ -443,64 +426,76 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       ++copied;
       if (++cs == kStages) cs = 0;
     };
-    // ===== one lane of the first warp: O^T = S^T q+^T + U^T mqk^T of item i ==========================================
-    int issued = 0;                    // items whose commits are under way
-    int ps = 0, po = 0;                // stage and output buffer of the next item, with their phases
-    uint32_t ps_par = 0, po_par = 1;
-    auto products = [&](int i) -> bool {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, 32, 0, 0);
-      const int s = ps, o = po;
-      if (!mbar_wait_parked(bar(B_U + s), ps_par, abort_flag)) return false;
-      if (i >= kOBufs && !mbar_wait_parked(bar(B_O_FREE + o), po_par, abort_flag)) return false;
-      if (++ps == kStages) { ps = 0; ps_par ^= 1u; }
-      if (++po == kOBufs) { po = 0; po_par ^= 1u; }
-      if (kStream && (static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags & kEnd)) {
-        mbar_arrive(bar(B_O + o));
-        return true;
-      }
-      tc_fence_after();
-      const uint32_t base = sbase + s * kStageBytes + 8192;
-      const uint32_t d = tmem + kColO + 32 * o;
-      const uint64_t bq = umma_desc(base + kCrQP, 128, 2048), bm = umma_desc(base + kCrMQK, 128, 512);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) umma_ts(d, tmem + kColSb + 64 * s + 8 * ks, bq + ks * 16, idesc, ks > 0);
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) umma_ts(d, tmem + kColUt + 16 * s + 8 * ks, bm + ks * 16, idesc, 1);
-      umma_commit(bar(B_O + o));
-      umma_commit(bar(B_EMPTY + s));
-      issued = i + 1;
-      return true;
-    };
-
     int n_one = 0;                     // (one walk per CTA) its items
     if (!kStream) n_one = chain_view<kSeg, kSlice>(p, static_cast<int>(blockIdx.x)).nchunks;
     const bool work = kStream || n_one > 0;
     if (w == 1 && lane == 0 && ok && work)
       for (int k = 0; k < kStages && !cur.ended; ++k) copy();
-    if (w == 0 && lane == 0 && ok && work) ok = products(0);
-    bool end_ahead = false;            // (first warp) the end of the stream has been passed on
-    int i = 0, o = 0, es = 0;          // item; its output buffer and its stage with their phases
-    uint32_t o_par = 0, es_par = 0;
-    for (; kStream || i < n_one; ++i) {
-      if (w == 0) {
-        // the products of the next item before the output of this one
-        if (lane == 0 && ok && !end_ahead) {
-          end_ahead = kStream ? (static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags & kEnd) != 0 : i + 1 == n_one;
-          if (!end_ahead) ok = products(i + 1);
+
+    // ===== the first warp: S^T [k+; q+]^T of an item as soon as the copy of S is there, half of k by half; later O^T = S^T q+^T +
+    // U^T mqk^T on top of it.  The output of the item before lies between the two.  (All lanes go through this, with operands
+    // that the compiler can see to be the same in all of them: issued from one lane's branch a product costs 75 cycles.) =====
+    int ps = 0, items = 0;             // stage of the item, with its phase; items begun
+    uint32_t ps_par = 0;
+    bool ended = false;
+    const uint64_t desc_s = umma_desc(sbase + 8192 + kCrKN, 128, 2048), desc_u = umma_desc(sbase + 8192 + kCrMQK, 128, 512);
+    auto products_s = [&](int i) -> bool {
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 64, 0, 0);
+      if (!warp_wait(bar(B_FULL + ps), ps_par, abort_flag)) return false;
+      if (kStream && (static_cast<const volatile Info*>(infos)[i & (kInfos - 1)].flags & kEnd)) {
+        if (lane == 0) mbar_arrive(bar(B_O + (i & 1)));
+        ended = true;
+        return true;
+      }
+      if (i >= 2 && !warp_wait(bar(B_O_FREE + (i & 1)), ((i >> 1) - 1) & 1, abort_flag)) return false;
+      const uint32_t d = utmem + kColD + 64 * (i & 1);
+      const uint64_t b = desc_s + static_cast<uint32_t>(ps * (kStageBytes >> 4));
+      items = i + 1;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (!warp_wait(bar(B_S + half), i & 1, abort_flag)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_ts(d, utmem + kColSb + 32 * half + 8 * k, b + (4 * half + k) * 16, idesc, half + k > 0);
+          if (half == 1) umma_commit(bar(B_R));
         }
         __syncwarp();
       }
+      return true;
+    };
+    auto products_u = [&](int i) -> bool {
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 32, 0, 0);
+      if (!warp_wait(bar(B_U), i & 1, abort_flag)) return false;
+      tc_fence_after();
+      const uint64_t b = desc_u + static_cast<uint32_t>(ps * (kStageBytes >> 4));
+      if (elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) umma_ts(utmem + kColD + 64 * (i & 1) + 32, utmem + kColUt + 8 * ks, b + ks * 16, idesc, 1);
+        umma_commit(bar(B_O + (i & 1)));
+        umma_commit(bar(B_EMPTY + ps));
+      }
+      __syncwarp();
+      if (++ps == kStages) { ps = 0; ps_par ^= 1u; }
+      return true;
+    };
+
+    int o = 0, es = 0;                 // output buffer and stage of the item whose output is written, with their phases
+    uint32_t o_par = 0, es_par = 0;
+    for (int i = 0; kStream || i <= n_one; ++i) {
+      const bool begin = kStream ? !ended : i < n_one;
+      if (w == 0 && ok && begin) ok = products_s(i);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-      if (!__all_sync(0xffffffffu, mbar_wait_parked(bar(B_O + o), o_par, abort_flag))) { ok = false; break; }
-      const volatile Info* f = infos + (i & (kInfos - 1));
-      if (kStream && (f->flags & kEnd)) break;
-      {
+      if (i > 0) {
+        if (!__all_sync(0xffffffffu, mbar_wait_parked(bar(B_O + o), o_par, abort_flag))) { ok = false; break; }
+        const volatile Info* f = infos + ((i - 1) & (kInfos - 1));
+        if (kStream && (f->flags & kEnd)) break;
         const long long off = f->out_off;
         const int len = f->len;
         tc_fence_after();
         uint32_t y[2][16];
-        tmem_ld_16x256b_x4(tq + 32 * o, y[0]);
-        tmem_ld_16x256b_x4(tq + (16u << 16) + 32 * o, y[1]);
+        tmem_ld_16x256b_x4(tq + 64 * o, y[0]);
+        tmem_ld_16x256b_x4(tq + (16u << 16) + 64 * o, y[1]);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
@@ -521,25 +516,21 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           dst += step;
         }
         __syncwarp();
+        if (w == 1 && lane == 0 && !cur.ended) {
+          if (!mbar_wait_parked(bar(B_EMPTY + es), es_par, abort_flag)) ok = false;
+          else copy();
+        }
+        if (++o == 2) { o = 0; o_par ^= 1u; }
+        if (++es == kStages) { es = 0; es_par ^= 1u; }
       }
-      if (w == 1 && lane == 0 && !cur.ended) {
-        if (!mbar_wait_parked(bar(B_EMPTY + es), es_par, abort_flag)) ok = false;
-        else copy();
-      }
-      if (++o == kOBufs) { o = 0; o_par ^= 1u; }
-      if (++es == kStages) { es = 0; es_par ^= 1u; }
+      if (w == 0 && ok && begin && !ended) ok = products_u(i);
     }
-    if (w == 0 && lane == 0 && issued > 0) {
-      // the commits issued last must land before the CTA may exit (a stage that was refilled since has had its commit)
-      const int k = issued - 1;
+    if (w == 0 && items > 0 && elect_one()) {
+      // what was issued must land before the CTA may exit: a commit behind all of it
+      umma_commit(bar(B_LAST));
       const uint64_t t0 = globaltimer_ns();
-      if (!ok) {
-        while (!mbar_try_wait(bar(B_O + k % kOBufs), (k / kOBufs) & 1))
-          if (globaltimer_ns() - t0 > 20000000ull) break;
-      } else if (i - k < kStages) {
-        while (ok && !mbar_try_wait(bar(B_EMPTY + k % kStages), (k / kStages) & 1))
-          if (globaltimer_ns() - t0 > kWaitLimitNs) ok = false;
-      }
+      while (!mbar_try_wait(bar(B_LAST), 0))
+        if (globaltimer_ns() - t0 > (ok ? kWaitLimitNs : 20000000ull)) { ok = false; break; }
     }
     if (w == 1 && lane == 0 && (!ok || *abort_flag > 0)) {
       // (giving up) copies in flight must land before the CTA's shared memory goes away
@@ -570,6 +561,154 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
 // 8 heads of 131072 tokens (lower_bound -2), recurrence with all its passes: 820 -> 340 us, 795 with gates that never decay; 16
 // heads of 32768 tokens, the whole call: 619 -> 365 us (610).  Few chains lose a tenth where nothing decays (1 head of 131072 tokens 338
 // -> 379 us, against 132 otherwise), as M and N had a CTA each.
+// One chunk of a walk without outputs, from stage s, every product on mma.sync.  `ready`: whether the next stage is full already.
+// kBack: the transposed step, S^T Phi^T with Phi = diag(e) + kn^T TB^T kr the chunk's transition and no v: the same products with k+ and
+// kr exchanged and TB transposed.
+template <bool kBack>
+__device__ __forceinline__ void step(float (&S)[2][16][4], uint8_t* smem, uint32_t sbase, int s, int len, int row0, int lane, uint32_t next_full,
+                                     uint32_t next_par, bool& ready) {
+  const int mi = lane >> 3, r = lane & 7, t = lane & 3;
+  const uint32_t kn_lane = 8192 + (kBack ? kCrKR : kCrKN) + (mi >> 1) * 2048 + (mi & 1) * 128 + r * 16;
+  const uint32_t kr_lane = 8192 + (kBack ? kCrKN : kCrKR) + mi * 2048 + r * 16;
+  const uint32_t v_lane = (row0 >> 6) * 4096 + lane * 128;
+  const uint32_t tb_lane = 8192 + kCrTB + r * 16;
+  const uint32_t stage = sbase + s * kStageBytes;
+
+  // R^T = v^T - S^T k+^T: the accumulators start from v^T; operands of a k-step are loaded during the one before
+  float R[2][4][4];
+  if (kBack) {
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) R[vt][nt][0] = R[vt][nt][1] = R[vt][nt][2] = R[vt][nt][3] = 0.f;
+  } else {
+    uint32_t x[4][4];              // v^T: channel blocks of 8 rows; register = token block
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ldsm_x4_trans(stage + v_lane + ((((row0 >> 3) + i) & 7) ^ r) * 16, x[i][0], x[i][1], x[i][2], x[i][3]);
+    if (len < kChunk) {            // rows past the sequence end belong to somebody else
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const uint32_t keep = (8 * nt + 2 * t < len ? 0xffffu : 0u) | (8 * nt + 2 * t + 1 < len ? 0xffff0000u : 0u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i][nt] &= keep;
+      }
+    }
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        R[vt][nt][0] = bf_lo(x[2 * vt][nt]);
+        R[vt][nt][1] = bf_hi(x[2 * vt][nt]);
+        R[vt][nt][2] = bf_lo(x[2 * vt + 1][nt]);
+        R[vt][nt][3] = bf_hi(x[2 * vt + 1][nt]);
+      }
+  }
+  uint32_t bb[2][8];
+  ldsm_x4(stage + kn_lane, bb[0][0], bb[0][1], bb[0][2], bb[0][3]);
+  ldsm_x4(stage + kn_lane + 4096, bb[0][4], bb[0][5], bb[0][6], bb[0][7]);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t a[2][16];               // bf16 copy of the state: A fragments of four k-steps
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        a[vt][2 * j] = pack_bf16(S[vt][8 * half + j][0], S[vt][8 * half + j][1]);
+        a[vt][2 * j + 1] = pack_bf16(S[vt][8 * half + j][2], S[vt][8 * half + j][3]);
+      }
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+      const int ks = 4 * half + k4;
+      const uint32_t(&B)[8] = bb[ks & 1];
+      if (ks < 7) {
+        uint32_t(&N)[8] = bb[(ks + 1) & 1];
+        ldsm_x4(stage + kn_lane + (ks + 1) * 256, N[0], N[1], N[2], N[3]);
+        ldsm_x4(stage + kn_lane + 4096 + (ks + 1) * 256, N[4], N[5], N[6], N[7]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int vt = 0; vt < 2; ++vt)
+          mma_bf16_16816(R[vt][nt], a[vt][4 * k4], a[vt][4 * k4 + 1], a[vt][4 * k4 + 2], a[vt][4 * k4 + 3], B[2 * nt], B[2 * nt + 1]);
+    }
+  }
+  // U^T = R^T (T diag(beta))^T
+  uint32_t l[4], m[4], n[4];       // T diag(beta): token tiles 0 and 1 (tokens 0-15 only: lower triangle), 2, 3; transposed: 0, 1, 2 and 3 (16-31 only)
+  if (kBack) {
+    ldsm_x4_trans(stage + tb_lane + mi * 512, l[0], l[1], l[2], l[3]);
+    ldsm_x4_trans(stage + tb_lane + mi * 512 + 128, m[0], m[1], m[2], m[3]);
+    ldsm_x4_trans(stage + tb_lane + 1024 + (mi & 1) * 512 + 256 + (mi >> 1) * 128, n[0], n[1], n[2], n[3]);
+  } else {
+    ldsm_x4(stage + tb_lane + (mi >> 1) * 512 + (mi & 1) * 128, l[0], l[1], l[2], l[3]);
+    ldsm_x4(stage + tb_lane + 1024 + mi * 128, m[0], m[1], m[2], m[3]);
+    ldsm_x4(stage + tb_lane + 1536 + mi * 128, n[0], n[1], n[2], n[3]);
+  }
+  uint32_t kr[2][4];
+  ldsm_x4_trans(stage + kr_lane, kr[0][0], kr[0][1], kr[0][2], kr[0][3]);
+  uint32_t u[2][2][4];             // A fragments, k-step = 16 tokens: first of R^T, then of U^T
+  auto as_operand = [&](uint32_t(&d)[2][4], const float(&x)[4][4]) {
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)  // e & 1: rows + 8, e >> 1: tokens + 8
+        d[ks][e] = pack_bf16(x[2 * ks + (e >> 1)][2 * (e & 1)], x[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
+  };
+#pragma unroll
+  for (int vt = 0; vt < 2; ++vt) as_operand(u[vt], R[vt]);
+  {
+    float U[2][4][4];
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt) {
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) U[vt][nt][0] = U[vt][nt][1] = U[vt][nt][2] = U[vt][nt][3] = 0.f;
+      if (kBack) {
+        mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
+        mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
+        mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[0], n[1]);
+        mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
+        mma_bf16_16816(U[vt][0], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], l[2], l[3]);
+        mma_bf16_16816(U[vt][1], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
+      } else {
+        mma_bf16_16816(U[vt][0], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[0], l[1]);
+        mma_bf16_16816(U[vt][1], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], l[2], l[3]);
+        mma_bf16_16816(U[vt][2], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], m[0], m[1]);
+        mma_bf16_16816(U[vt][3], u[vt][0][0], u[vt][0][1], u[vt][0][2], u[vt][0][3], n[0], n[1]);
+        mma_bf16_16816(U[vt][2], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], m[2], m[3]);
+        mma_bf16_16816(U[vt][3], u[vt][1][0], u[vt][1][1], u[vt][1][2], u[vt][1][3], n[2], n[3]);
+      }
+    }
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt) as_operand(u[vt], U[vt]);
+  }
+  // S^T = S^T diag(e) + U^T kr; the next stage's barrier is looked at meanwhile
+  const float2* e2 = reinterpret_cast<const float2*>(smem + s * kStageBytes + 8192 + kCrE) + t;
+  ready = mbar_test(next_full, next_par);
+#pragma unroll
+  for (int jt = 0; jt < 16; ++jt) {
+    const uint32_t(&B)[4] = kr[jt & 1];
+    if (jt < 15) {
+      uint32_t(&N)[4] = kr[(jt + 1) & 1];
+      ldsm_x4_trans(stage + kr_lane + (jt + 1) * 128, N[0], N[1], N[2], N[3]);
+    }
+    const float2 e = e2[4 * jt];
+#pragma unroll
+    for (int vt = 0; vt < 2; ++vt) {
+      uint32_t y[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[k] = __float_as_uint(S[vt][jt][k]);
+      mul2(y[0], y[1], e);
+      mul2(y[2], y[3], e);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) S[vt][jt][k] = __uint_as_float(y[k]);
+    }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int vt = 0; vt < 2; ++vt)
+        mma_bf16_16816(S[vt][jt], u[vt][ks][0], u[vt][ks][1], u[vt][ks][2], u[vt][ks][3], B[2 * ks], B[2 * ks + 1]);
+  }
+}
+
 __device__ __forceinline__ bool is_zero(const float (&S)[2][16][4]) {
   uint32_t any = 0;
 #pragma unroll
@@ -641,7 +780,7 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
       ready = false;
       const bool end = static_cast<const volatile Info*>(infos)[c & (kInfos - 1)].flags & kEnd;
       if (!end && !zero) {
-        step<false, true>(S, smem, sbase, 0, s, kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
+        step<true>(S, smem, sbase, s, kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
         if ((c < 16 || (c & 7) == 7) && is_zero(S)) {
           zero = true;
           if (lane == 0) {
@@ -678,7 +817,7 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
         uint32_t par1;
         next(s1, par1);
         const int64_t left = cv.eos - cv.bos - static_cast<int64_t>(c) * kChunk;
-        step<false, false>(S, smem, sbase, 0, s, left < kChunk ? static_cast<int>(left) : kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
+        step<false>(S, smem, sbase, s, left < kChunk ? static_cast<int>(left) : kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
         release(s1, par1);
       }
       if (ok) {
