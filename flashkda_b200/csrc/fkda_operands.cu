@@ -7,8 +7,8 @@
 //   warp  9      loads of the item after next, stores of the record, tril(M)
 //   warp  11     first products [A; M] = [k+; q+] k-^T on tcgen05
 //
-// 770 bytes read and 912 written per token-head: 0.27 ms of HBM time on a million token-heads.  Alone it takes 0.336 ms in a
-// burst of calls (5.2 TB/s, four fifths of the measured copy rate) and 0.380 kept up under the power cap.
+// 770 bytes read and 912 written per token-head: 0.27 ms of HBM time on a million token-heads.  Alone it takes 0.322 ms in a
+// burst of calls (5.5 TB/s, 84 % of the measured copy rate) and 0.366 kept up under the power cap.
 // What it took to get there from 0.379 / 0.413 ms (4 x 8192 tokens x 32 heads, cycles per item and CTA by clock64):
 //   * The row norms went through a warp that also issued the products: an element warp waited 1000 of its 5700 cycles for them.
 //     Every element warp now sums the eight partial sums itself (two rows per lane, handed round by shuffles).  That alone made
@@ -23,6 +23,8 @@
 //     0.358; explicit sleeps of 20 to 100 ns: 0.350.)
 //   * One 4-d copy per tensor instead of two 3-d ones, issued before the next item is decoded (a request costs its issuer 120
 //     cycles), and no prefetch to the L2 any more, which the earlier loads do not need: 0.339 / 0.387 -> 0.336 / 0.380 ms.
+//   * The first products issued by a whole warp (elect.sync) with operands that the compiler can see to be uniform, 300 cycles instead
+//     of 940 between the operands and the element warps' next store: 0.338 / 0.379 -> 0.322 / 0.366 ms.
 //
 // Decay ranges: with G the running log2 decay inside the chunk and P its value after the first 16 tokens, the first products
 // use k+ = khat 2^(G - P) and k- = khat 2^(P - G): both stay inside 2^(+-115.4) for lower_bound >= -5 (16 tokens x 5 x
@@ -430,6 +432,8 @@ __device__ __forceinline__ bool product_role(const PrepParams& p, uint8_t* smem,
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
   bool ok = true;
   int i = 0;
+  tmem = __shfl_sync(0xffffffffu, tmem, 0);
+  n_it = __shfl_sync(0xffffffffu, n_it, 0);
   for (; i < n_it; ++i) {
     const int b = i & 1;
     const uint32_t ph = (i >> 1) & 1;
@@ -442,8 +446,8 @@ __device__ __forceinline__ bool product_role(const PrepParams& p, uint8_t* smem,
     // (the inverse of item i - 4, which used this slot, ended before item i - 2 gave its result back)
     reinterpret_cast<float*>(smem + kSmBeta + (i & 3) * 128)[lane] = lane < f->len ? sigmoid_fast(beta) : 0.f;
     __syncwarp();
-    if (lane == 0) {
-      mbar_arrive(bar(B_D1 + b));
+    if (lane == 0) mbar_arrive(bar(B_D1 + b));
+    if (elect_one()) {       // (operands that are plainly the same in all lanes: from one lane's branch a product costs 100 cycles to issue)
       // rows of the A operand: even items k+ | q+ from row 0 (A in lanes 0-31, M in 32-63); odd items, whose k+ lies behind
       // q+, from row 32 on (M in lanes 32-63, A in 64-95).  What the other rows hold does not matter: nobody reads their lanes.
       constexpr uint32_t idesc = umma_idesc_bf16(128, 32, 0, 0);
@@ -471,7 +475,7 @@ operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const PrepParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kSmMisc + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kSmMisc);
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
