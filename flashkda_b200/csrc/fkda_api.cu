@@ -367,12 +367,13 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
 
 // Where fewer chains than SMs have a CTA each, the SMs beyond them can work out operands meanwhile.  The call is then cut in two
 // time slices, and the second one's operands are computed beside the first one's recurrence, by kSliceWaves waves of two
-// CTAs on each free SM that end with it.  A chunk of the recurrence takes 1.32 us; a CTA of the token-parallel stage 3.7 us per item
-// and 5 us to fill and drain its pipeline.  Returns the chunks of the first slice, or 0 where what the stage is shortened by is
-// not worth it: the second pair of launches costs about 20 us and the stage's share of the recurrence's bandwidth about 4 % of the
-// call.  Gains measured against one piece, chains x chunks: 75 x 512 13 %, 96 x 256 10 %, 110 x 256 7 %, 120 x 512 3 %, 124 x 1024
-// 1.5 %, 128 x 512 and 128 x 1024 nothing to 1 %, 130 x 1024 -0.4 %, 134 x 1024 -3 %, 140 x 2048 -5 %: the line at 5 % of the
-// call lies at 129 chains.  Equal lengths only: a packed batch's lengths, which the slices would have to follow, are on the
+// CTAs on each free SM that end with it.  The costs are those of the kernels at the time of the fit - 1.32 us for a chunk of the
+// recurrence, 3.7 us per item and CTA of the token-parallel stage and 5 us to fill and drain its pipeline; both have become a fifth
+// faster since, and the cut lies where it did: the best of seven was the planned one, or next to it, for 96, 110 and 120 chains of 256
+// chunks, 75 x 512, 80 x 128 and 124 x 1024.  Returns the chunks of the first slice, or 0 where what the stage is shortened by is
+// not worth it: the second pair of launches costs about 20 us, and the stage takes its share of the recurrence's bandwidth.
+// Gains measured against one piece, chains x chunks: 75 x 512 15 %, 80 x 128 11 %, 96 x 256 12 %, 110 x 256 10 %, 120 x 256 10 %, 124 x
+// 1024 14 %, 128 x 512 6 %.  Equal lengths only: a packed batch's lengths, which the slices would have to follow, are on the
 // device.  Chains split over CTAs leave too few SMs free beside them (20 at 32 chains, none at 37 or 74).
 constexpr int kSliceWaves = 2;
 int plan_slice(int64_t chains, int64_t chunks, int sms) {
