@@ -213,6 +213,14 @@ bool fused_short(const fkda_fwd_params* p) {
   return p->cu_seqlens == nullptr && p->T > 0 && (any_t || (p->T <= fkda::kFusedMaxT && (p->flags & 0xff57u) == 0));
 }
 
+// whether the call is one of the per-token kernel, and with it needs no scratch memory: that kernel has no wait whose end a
+// status word could tell
+bool takes_step_kernel(const fkda_fwd_params* p) { return fused_short(p) && p->T <= fkda::kStepMaxT && !(p->flags & FKDA_FLAG_FUSED_ANY_T); }
+int64_t scratch_bytes(const fkda_fwd_params* p, const Layout& L) {
+  if (!(p->flags & FKDA_FLAG_STATUS_UNREAD) || !fused_short(p)) return L.total_bytes;
+  return takes_step_kernel(p) ? 0 : static_cast<int64_t>(fkda::kWsHeaderBytes);
+}
+
 // `whole_call`: the operator (fkda_fwd) rather than one of its stages; `fit`: its plan keeps to the given workspace
 int validate(const fkda_fwd_params* p, Layout* L, bool whole_call = false, bool fit = false) {
   if (!p) return fail(FKDA_ERR_INVALID_ARGUMENT, "params is NULL");
@@ -238,10 +246,11 @@ int validate(const fkda_fwd_params* p, Layout* L, bool whole_call = false, bool 
   if (p->N * p->H > 0x7fffffffLL) return fail(FKDA_ERR_INVALID_ARGUMENT, "N*H exceeds 2^31-1 chains");
   if (!make_layout(T_total, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, L, fit ? p->workspace_bytes : kAnyRoom)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
   if (L->chunks_per_head * p->H > 0x7fffffffLL) return fail(FKDA_ERR_INVALID_ARGUMENT, "too many (chunk, head) pairs for one call");
+  // (a caller who can read the status word sized the workspace by fkda_get_workspace_size, which is held to)
+  const int64_t needed = whole_call ? scratch_bytes(p, *L) : L->total_bytes;
+  if (needed == 0) return FKDA_OK;
   if (!p->workspace) return fail(FKDA_ERR_INVALID_ARGUMENT, "workspace is NULL");
   if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return fail(FKDA_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
-  // (a caller who can read the status word sized the workspace by fkda_get_workspace_size, which is held to)
-  const int64_t needed = whole_call && (p->flags & FKDA_FLAG_STATUS_UNREAD) && fused_short(p) ? fkda::kWsHeaderBytes : L->total_bytes;
   if (p->workspace_bytes < needed)
     return fail(FKDA_ERR_WORKSPACE_TOO_SMALL, "workspace has %lld bytes, %lld needed", (long long)p->workspace_bytes, (long long)needed);
   return FKDA_OK;
@@ -484,7 +493,7 @@ int do_fwd(const fkda_fwd_params* p, void* cuda_stream, bool fit) {
     // short fixed-length sequences (a continuation step): one fused kernel, no operand records
     cudaError_t e = clear_status(p, stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(status)");
-    if (p->T <= fkda::kStepMaxT && !(p->flags & FKDA_FLAG_FUSED_ANY_T)) {
+    if (takes_step_kernel(p)) {
       e = fkda::launch_step(prep_params(p, L), scan_params(p, L), stream);
       if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
       return FKDA_OK;
@@ -558,7 +567,7 @@ int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes) {
   Layout L;
   if (!p || !bytes) return fail(FKDA_ERR_INVALID_ARGUMENT, "NULL pointer");
   if (!make_layout(p->B * p->T, p->H, p->N, p->cu_seqlens ? 1 : 0, p->T, p->flags, &L)) return fail(FKDA_ERR_INVALID_ARGUMENT, "bad sizes");
-  *bytes = (p->flags & FKDA_FLAG_STATUS_UNREAD) && fused_short(p) ? fkda::kWsHeaderBytes : L.total_bytes;
+  *bytes = scratch_bytes(p, L);
   return FKDA_OK;
 }
 

@@ -94,7 +94,9 @@ PyObject* fwd_fast(PyObject*, PyObject* const* a, Py_ssize_t n) {
     int64_t bytes = 0;
     if (fkda_fwd_scratch_bytes(&p, &bytes) != FKDA_OK) Py_RETURN_FALSE;
     // freed when the call returns: the caching allocator hands a block only to later work of the same stream
-    c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(bytes));
+    // (none for a decode step, where asking for it would be a tenth of the call)
+    c10::DataPtr ws;
+    if (bytes > 0) ws = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(bytes));
     p.workspace = ws.get();
     p.workspace_bytes = bytes;
     void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();

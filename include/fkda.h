@@ -82,7 +82,8 @@ typedef struct fkda_fwd_params {
   const void* initial_state; /* [N][H][128 v][128 k] of state_dtype, or NULL (start from zero) */
   void* final_state;         /* same shape and dtype, or NULL                                   */
   const int64_t* cu_seqlens; /* device int64 [N+1], or NULL for B equal-length sequences        */
-  void* workspace;           /* >= fkda_get_workspace_size bytes, 256-byte aligned              */
+  void* workspace;           /* >= fkda_get_workspace_size bytes, 256-byte aligned (may be NULL where
+                                fkda_fwd_scratch_bytes says 0)                                  */
   int64_t workspace_bytes;
   int64_t B;                 /* batch; must be 1 when cu_seqlens is given                       */
   int64_t T;                 /* tokens per batch row (total tokens when cu_seqlens is given)    */
@@ -109,7 +110,8 @@ int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen
                                int64_t* bytes);
 
 /* The same for one call: the bytes of workspace that fkda_fwd will need for exactly these sizes and flags (`workspace`,
- * `workspace_bytes` and the data pointers other than cu_seqlens are not looked at). */
+ * `workspace_bytes` and the data pointers other than cu_seqlens are not looked at).  None (0) with
+ * FKDA_FLAG_STATUS_UNREAD for a fixed-length call of at most four tokens per sequence. */
 int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes);
 
 /* The plan of the recurrence over long sequences: into how many runs (1 = none), walked in parallel, fkda_fwd cuts the

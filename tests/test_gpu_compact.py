@@ -339,3 +339,16 @@ def test_runs_whose_maps_last_or_vanish(lasting, packed, state):
                                      initial_state=x["initial_state"], cu_seqlens=x["cu_seqlens"])
     assert max_abs(out.cpu(), o64) <= OUT_MAX_ABS and rel_fro(out.cpu(), o64) <= 1e-2
     assert rel_fro(fin.cpu(), s64) <= STATE_REL
+
+
+@pytest.mark.parametrize("T,asks", [(1, 0), (4, 0), (5, 1), (40, 1)])
+def test_a_decode_step_asks_for_no_scratch_memory(T, asks):
+    w = Workload("d", H=4, B=3, T=T, state_in="fp32", state_out="fp32", seed=T)
+    x = make_inputs(w, device="cuda")
+    call = lambda: F.fwd(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                         initial_state=x["initial_state"], final_state=x["final_state"])
+    call()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    call()
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] - before == asks
