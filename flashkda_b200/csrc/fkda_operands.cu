@@ -75,14 +75,12 @@ struct Info {
 };
 static_assert(sizeof(Info) == 32, "info");
 
+// Where an item lies (all but ha, which takes a load from memory).
 template <bool kSlice>
 __device__ __forceinline__ Info decode(const PrepParams& p, unsigned item) {
   Info r;
   r.h = static_cast<int>(item % static_cast<unsigned>(p.H));        // consecutive items: consecutive heads of a chunk, adjacent in memory
   r.gc = static_cast<int>(item / static_cast<unsigned>(p.H));
-  const float ha = 0.5f * ex2f(__ldg(p.A_log + r.h) * kLog2e);
-  // (off zero and infinity: a gate input of minus infinity stands for a token that is not there)
-  r.ha = ha < 1e-30f ? 1e-30f : ha > 1e30f ? 1e30f : ha;
   r.pad[0] = r.pad[1] = 0;
   if (p.cu_seqlens != nullptr) {
     int lo = 0, hi = p.N - 1;
@@ -105,6 +103,11 @@ __device__ __forceinline__ Info decode(const PrepParams& p, unsigned item) {
     r.len = rem < kChunk ? static_cast<int>(rem) : kChunk;
   }
   return r;
+}
+__device__ __forceinline__ float gate_factor(const PrepParams& p, int h) {
+  const float ha = 0.5f * ex2f(__ldg(p.A_log + h) * kLog2e);
+  // (off zero and infinity: a gate input of minus infinity stands for a token that is not there)
+  return ha < 1e-30f ? 1e-30f : ha > 1e30f ? 1e30f : ha;
 }
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait_parked(bar, parity, abort_flag));
@@ -343,29 +346,36 @@ __device__ __forceinline__ bool copy_role(const PrepParams& p, const CUtensorMap
                                           uint32_t sbase, uint32_t tmem, int n_it, int lane, volatile int* abort_flag) {
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
   Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
-  auto load = [&](int i) {
-    const Info* f = infos + (i & (kInfos - 1));
+  auto load = [&](int i, const Info& f) {
     const uint32_t full = bar(B_IN + (i & 1)), dst = sbase + kSmSlot + (i & 1) * kSlotBytes;
-    const int tc = static_cast<int>(f->t0), h = f->h;
+    const int tc = static_cast<int>(f.t0), h = f.h;
     mbar_arrive_expect_tx(full, kSlotBytes + 512);
     tma_load_4d(dst, tq, 0, tc, 0, h, full);
     tma_load_4d(dst + 8192, tk, 0, tc, 0, h, full);
     tma_load_4d(dst + 16384, tg, 0, tc, 0, h, full);
     bulk_g2s(sbase + kSmBias + (i & 1) * 512, p.dt_bias + static_cast<size_t>(h) * kD, 512, full);
   };
-  auto look_ahead = [&](int i) {
-    infos[i & (kInfos - 1)] = decode<kSlice>(p, blockIdx.x + static_cast<unsigned>(i) * gridDim.x);
+  auto look_ahead = [&](int i, Info f) {
+    f.ha = gate_factor(p, f.h);
+    infos[i & (kInfos - 1)] = f;
   };
+  auto item = [&](int i) { return decode<kSlice>(p, blockIdx.x + static_cast<unsigned>(i) * gridDim.x); };
   int loaded = 0;
   bool ok = true;
   if (lane == 0) {
+    // the first items' loads before their gate factor, which has to come from memory; the barrier also waits for what is said about them
     for (int i = 0; i < 2 && i < n_it; ++i) {
-      look_ahead(i);
-      if (i == 1 && p.first_load_only) break;        // test aid: a wait that nothing completes
-      load(i);
-      ++loaded;
+      const Info f = item(i);
+      const bool first_only = i == 1 && p.first_load_only;       // test aid: a wait that nothing completes
+      if (!first_only) {
+        load(i, f);
+        ++loaded;
+      }
+      look_ahead(i, f);
+      if (first_only) break;
+      mbar_arrive(bar(B_IN + i));
     }
-    if (n_it > 2) look_ahead(2);
+    if (n_it > 2) look_ahead(2, item(2));
   }
   __syncwarp();
   for (int i = 0; i < n_it; ++i) {
@@ -380,10 +390,11 @@ __device__ __forceinline__ bool copy_role(const PrepParams& p, const CUtensorMap
       bulk_commit();
       bulk_wait_read0();             // (also the tril(M) of the item before)
       if (i + 2 < n_it && !p.first_load_only) {
-        load(i + 2);
+        load(i + 2, infos[(i + 2) & (kInfos - 1)]);
+        mbar_arrive(bar(B_IN + b));
         ++loaded;
       }
-      if (i + 3 < n_it) look_ahead(i + 3);
+      if (i + 3 < n_it) look_ahead(i + 3, item(i + 3));
     }
     __syncwarp();
     if (!warp_wait(bar(B_D1 + b), ph, abort_flag)) { ok = false; break; }
@@ -483,7 +494,7 @@ operands_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // the swizzled tiles need this alignment: report instead of computing garbage (below zero: a wait limit, test aid)
     *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(B_IN + i), 1);
+      mbar_init(bar(B_IN + i), 2);                     // the copies, and what is said about the item
       mbar_init(bar(B_NORMP + i), 8);
       mbar_init(bar(B_OPS + i), 8);
       mbar_init(bar(B_D1 + i), 2);                     // the commit, and the warp that leaves sigmoid(beta) beside it
