@@ -544,7 +544,10 @@ struct ChainView {
   int fin_stride;              // elements per row there (128; a transition map's slot: kSegMapStride)
   bool write_out, zero_up;
 };
+// What follows from a chain's sequence, head, tokens and first record.
 template <bool kSeg, bool kSlice = false>   // kSlice: minds the time slice of ScanParams
+__device__ __forceinline__ void chain_finish(const ScanParams& p, ChainView& cv, int seg, int variant);
+template <bool kSeg, bool kSlice = false>
 __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) {
   ChainView cv;
   int chain = block, seg = 0, variant = 0;
@@ -572,6 +575,11 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
     cv.eos = cv.bos + p.T;
     cv.chunk_base = cv.n * static_cast<int>((p.T + kChunk - 1) / kChunk);
   }
+  chain_finish<kSeg, kSlice>(p, cv, seg, variant);
+  return cv;
+}
+template <bool kSeg, bool kSlice>
+__device__ __forceinline__ void chain_finish(const ScanParams& p, ChainView& cv, int seg, int variant) {
   const bool skipped = p.skip_short && cv.eos - cv.bos <= kStepMaxT;
   cv.nchunks = skipped ? 0 : static_cast<int>((cv.eos - cv.bos + kChunk - 1) / kChunk);
   {  // never read past the records of this head, whatever cu_seqlens claims
@@ -643,7 +651,6 @@ __device__ __forceinline__ ChainView chain_view(const ScanParams& p, int block) 
   }
   cv.write_out = !kSeg || variant == 0;
   cv.zero_up = kSeg && variant == 2;
-  return cv;
 }
 
 }  // namespace fkda

@@ -42,7 +42,9 @@ constexpr int kInfos = 16;
 constexpr int kSmInfo = kSmStg + 4 * 32 * kStgStride;
 constexpr int kSmBars = kSmInfo + kInfos * 32;
 constexpr int kSmMisc = kSmBars + 256;
-constexpr int kSmem = kSmMisc + 16;
+constexpr int kWalkInfos = 8;                      // (persistent form) more than stages, and a walk has an item at least
+constexpr int kSmWalks = kSmMisc + 16;
+constexpr int kSmem = kSmWalks + kWalkInfos * 48;
 static_assert(kSmem <= 227 * 1024, "shared memory plan");
 // tensor memory columns.  One copy of S and of U each: when the products of a chunk on S are complete, those of the chunk
 // before on U are too (one thread issues both), and the state's copy may be written over.
@@ -68,9 +70,17 @@ struct Info {
   long long out_off;   // element offset of the first token's row in `out`
   int len;             // valid tokens
   int flags;
-  int walk;            // index of the walk (chain, or run of a chain) for chain_view
+  int walk;            // (persistent form) which WalkInfo
   int pad[3];
 };
+// What it says about a walk, so that the recurrence warps need not look the chain up again (three dependent loads).
+struct WalkInfo {
+  const void* init_base;
+  void* fin_base;
+  long long tokens;
+  int nchunks, init_mode, fin_fp32, pad[3];
+};
+static_assert(sizeof(WalkInfo) == 48, "walk info");
 static_assert(sizeof(Info) == 32, "info");
 enum { kEnd = 1 };
 
@@ -345,15 +355,24 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     uint32_t par = 0;
     bool ready = false;
     for (int i = 0; ok;) {
-      int walk_index = static_cast<int>(blockIdx.x);
+      ChainView cv{};
       if (kStream) {
         if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
         const volatile Info* f = infos + (i & (kInfos - 1));
-        walk_index = f->walk;
         ready = true;
         if (f->flags & kEnd) break;
+        const WalkInfo* wi = reinterpret_cast<const WalkInfo*>(smem + kSmWalks) + f->walk;
+        cv.init_base = wi->init_base;
+        cv.init_mode = wi->init_mode;
+        cv.fin_base = wi->fin_base;
+        cv.fin_fp32 = wi->fin_fp32;
+        cv.fin_stride = kD;
+        cv.bos = 0;
+        cv.eos = wi->tokens;
+        cv.nchunks = wi->nchunks;
+      } else {
+        cv = chain_view<kSeg, kSlice>(p, static_cast<int>(blockIdx.x));
       }
-      const ChainView cv = chain_view<kSeg, kSlice>(p, walk_index);
       load_state(S, cv, row0, lane);
       // (an empty run hands its state through)
       if (cv.nchunks > 0) ok = walk(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, row0, lane, abort_flag, s, par, ready, static_cast<uint32_t>(i));
@@ -371,6 +390,33 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
 
     // ===== one lane of the second warp: the stream of chunks into the ring ==========================================
     struct { long long bos, eos; const uint8_t* rec; int walk, h, c, n, turn; bool ended; } cur{};
+    // The next walk, looked up a step per item (a packed batch: the counter, the order by length, then the sequence's ends and first record
+    // are loads that depend on one another; in a row they would keep this warp's output waiting for more than a chunk's time).
+    struct { ChainView cv; int walk, step; } next{};
+    auto look = [&]() {
+      if (!kStream || next.step >= 3) return;
+      if (next.step == 0) {
+        const int base = cur.turn * static_cast<int>(gridDim.x);
+        next.walk = p.next_walk != nullptr ? atomicAdd(p.next_walk, 1)
+                    : base + ((cur.turn & 1) ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x));
+        ++cur.turn;
+      } else if (next.walk >= walks || next.walk < 0) {
+        next.step = 2;
+      } else if (next.step == 1) {
+        const int slot = next.walk / p.H;
+        next.cv.h = next.walk - slot * p.H;
+        next.cv.n = p.seq_order != nullptr ? p.seq_order[slot] : slot;
+      } else if (p.cu_seqlens != nullptr) {
+        next.cv.bos = p.cu_seqlens[next.cv.n];
+        next.cv.eos = p.cu_seqlens[next.cv.n + 1];
+        next.cv.chunk_base = p.chunk_prefix[next.cv.n];
+      } else {
+        next.cv.bos = static_cast<int64_t>(next.cv.n) * p.T;
+        next.cv.eos = next.cv.bos + p.T;
+        next.cv.chunk_base = next.cv.n * static_cast<int>((p.T + kChunk - 1) / kChunk);
+      }
+      ++next.step;
+    };
     int copied = 0;
     int cs = 0;                        // stage of the next item
     auto copy = [&]() {
@@ -383,13 +429,22 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           return;
         }
         for (;;) {
-          const int base = cur.turn * static_cast<int>(gridDim.x);
-          const int walk = !kStream ? static_cast<int>(blockIdx.x) : p.next_walk != nullptr ? atomicAdd(p.next_walk, 1)
-                           : base + ((cur.turn & 1) ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x));
-          ++cur.turn;
-          const bool past = walk >= walks || walk < 0;
           ChainView cv{};
-          if (!past) cv = chain_view<kSeg, kSlice>(p, walk);
+          bool past = false;
+          if (kStream) {
+            while (next.step < 3) look();
+            next.step = 0;
+            past = next.walk >= walks || next.walk < 0;
+            if (!past) {
+              cv = next.cv;
+              cv.bos = cv.bos < 0 ? 0 : (cv.bos > p.T_total ? p.T_total : cv.bos);
+              cv.eos = cv.eos < cv.bos ? cv.bos : (cv.eos > p.T_total ? p.T_total : cv.eos);
+              chain_finish<false>(p, cv, 0, 0);
+            }
+          } else {
+            ++cur.turn;
+            cv = chain_view<kSeg, kSlice>(p, static_cast<int>(blockIdx.x));
+          }
           if (past || (kStream && cv.nchunks == 0 && p.N <= kOrderMax)) {
             // (The last round may be shorter than the grid: a CTA without a walk in it is done, there is no round after it.
             // Skipped sequences come last in the order by length.)
@@ -401,16 +456,27 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
             return;
           }
           if (kStream && cv.nchunks == 0) continue;
-          cur.walk = walk;
+          cur.walk = (cur.walk + 1) & (kWalkInfos - 1);
           cur.h = cv.h;
           cur.bos = cv.bos;
           cur.eos = cv.eos;
           cur.c = 0;
           cur.n = cv.nchunks;
           cur.rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
+          if (kStream) {
+            WalkInfo* wi = reinterpret_cast<WalkInfo*>(smem + kSmWalks) + cur.walk;
+            wi->init_base = cv.init_base;
+            wi->init_mode = cv.init_mode;
+            wi->fin_base = cv.fin_base;
+            wi->fin_fp32 = cv.fin_fp32;
+            wi->tokens = cv.eos - cv.bos;
+            wi->nchunks = cv.nchunks;
+          }
           if (copied > 0 && (cv.init_mode == 1 || cv.init_mode == 2)) bulk_prefetch_l2(cv.init_base, kD * kD * (cv.init_mode == 1 ? 4 : 2));
           break;
         }
+      } else {
+        look();
       }
       const long long t0 = cur.bos + static_cast<long long>(cur.c) * kChunk;
       f->out_off = (t0 * p.H + cur.h) * kD;
