@@ -79,7 +79,7 @@ struct Layout {
 // chunks.  The first pass has a CTA for every run but the last, which works out the run's map M and offset N; the second one a CTA
 // per run.  Where the gates' decay makes M vanish, which the first pass finds out (fkda_recur.cu), its two walks are a few chunks
 // long; where it does not, they are as long as the run and the maps are chained.  The plan is made for the former, among those that cost in the
-// latter at most a tenth more than whole sequences and a twelfth more than the best plan for it; of plans within 6 % and 3 us,
+// latter at most a tenth more than whole sequences and a twelfth more than the best plan for it; of plans within 5 % and 3 us,
 // which is what the costs are off by, the one with the fewest runs.  The one planner: the workspace size, the launch and fkda_plan_segments ask here.
 // Its costs are those of the default path's kernels, in hundredths of a microsecond, fitted to 150 timed calls of 1 to 48
 // heads and 64 to 4096 chunks, half of them without decay: a chunk step of a chain split over four or two CTAs (fkda_recur_split.cu) or
@@ -87,7 +87,7 @@ struct Layout {
 // beside their steps, and every round of CTAs after the first; the chaining of the maps per run and round of its CTAs.  (The
 // two-stage form walks its runs by the same plan.)
 int plan_runs(int64_t chains, int64_t chunks, int64_t most, int sms, int* len) {
-  constexpr int64_t kQuad = 59, kHalf = 87, kOne = 135, kQuiet = 95, kVanish = 9, kPasses = 1300, kRound = 640, kChaining = 160, kMostRuns = 160, kLeast = 10;
+  constexpr int64_t kQuad = 59, kHalf = 87, kOne = 108, kQuiet = 95, kVanish = 9, kPasses = 1300, kRound = 640, kChaining = 160, kMostRuns = 160, kLeast = 10;
   *len = 0;
   if (chains <= 0 || chains * 3 > sms || chunks < 48) return 1;
   const int64_t whole = (chains * 4 <= sms ? kQuad : kHalf) * chunks;
@@ -112,7 +112,7 @@ int plan_runs(int64_t chains, int64_t chunks, int64_t most, int sms, int* len) {
       if (c.lasting * 12 > least_lasting * 13 || c.lasting * 100 > whole * 110 || c.vanishing * 100 > whole * 97) continue;
       if (pass == 1) {
         if (c.vanishing < best) best = c.vanishing;
-      } else if (c.vanishing * 1000 <= best * 1058 && c.vanishing <= best + 300) {
+      } else if (c.vanishing * 100 <= best * 105 && c.vanishing <= best + 300) {
         best_n = static_cast<int>(n);
         break;
       }

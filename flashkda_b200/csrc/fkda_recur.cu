@@ -625,8 +625,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
 // whose gates hold some channel to the end costs what it always did, a walk each for M and N, plus the test for zero (a hundred
 // cycles in the first sixteen chunks and then in every eighth).
 // 8 heads of 131072 tokens (lower_bound -2), recurrence with all its passes: 820 -> 340 us, 795 with gates that never decay; 16
-// heads of 32768 tokens, the whole call: 619 -> 365 us (610).  Few chains lose a tenth where nothing decays (1 head of 131072 tokens 338
-// -> 379 us, against 132 otherwise), as M and N had a CTA each.
+// heads of 32768 tokens, the whole call: 619 -> 365 us (610); the walks themselves have become faster since (281 and 733 us).  Few
+// chains lose a tenth where nothing decays (1 head of 131072 tokens 338 -> 379 us, against 132 otherwise), as M and N had a CTA each.
 // One chunk of a walk without outputs, from stage s, every product on mma.sync.  `ready`: whether the next stage is full already.
 // kBack: the transposed step, S^T Phi^T with Phi = diag(e) + kn^T TB^T kr the chunk's transition and no v: the same products with k+ and
 // kr exchanged and TB transposed.
