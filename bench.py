@@ -446,7 +446,7 @@ def main():
     # stages of the default path, each alone over the workspace of a whole call, or of the two-stage form where a flag selects it.
     varlen = x["cu_seqlens"] is not None
     fused = not varlen and 0 < T <= 32 and (args.flags & 0xFF57) == 0
-    one_kernel = "refmode" if args.flags & F.FLAG_REFERENCE_ROUNDING else ("step" if T <= 4 else "short16") if fused else None
+    one_kernel = "refmode" if args.flags & F.FLAG_REFERENCE_ROUNDING else ("step" if T <= 4 else "short8" if T <= 8 else "short16") if fused else None
     two_stage = args.flags & ~(F.FLAG_SCAN_NO_SEGMENTS | F.FLAG_NO_FUSED_SHORT | F.FLAG_OPERANDS_PER_ITEM) or \
         (varlen and args.flags & F.FLAG_SCAN_NO_SEGMENTS)
     stages = []
@@ -622,7 +622,7 @@ def main():
 SHORT16_TRAFFIC_BYTES_PER_CHAIN = 140_100   # profiles/short16_kernel_B128xT16xH32.md (T = 16, fp32 state in and out)
 # operands, recurrence: profiles/operands_kernel_recur_kernel_B8xT1024xH16.md; prepare, scan (two-stage form):
 # profiles/prepare_pipe_kernel_prepare_tc4_kernel_B8xT1024xH16.md, profiles/prepare_kernel_scan2_kernel_B8xT1024xH16.md
-TRAFFIC_BYTES_PER_TOKEN_HEAD = {"operands": 1287, "recurrence": 1352, "prepare": 1774, "scan": 1313}
+TRAFFIC_BYTES_PER_TOKEN_HEAD = {"operands": 1274, "recurrence": 1364, "prepare": 1774, "scan": 1313}
 
 if __name__ == "__main__":
     main()
