@@ -448,7 +448,7 @@ struct ScanParams {
   int seg_chunks;              // 0: one CTA per whole sequence
   int n_segs;
   int seg_pass;                // 1 or 2; over compact records kSegMaps or kSegWalks
-  float* seg_buf;              // fp32 [(n*H + h)][n_segs][3] slots: 0 = M, 1 = N, 2 = state at the start of the run
+  float* seg_buf;              // fp32 [(n*H + h)][n_segs][3] slots: 0 = M, 1 = N, 2 = state at the start of the run (of run 0: over compact records)
   const int* select;           // device word, or nullptr: the kernel runs only if *select == select_want
   int select_want;
   const int* seg_chunks_dev;   // varlen batches: run length decided on the device from the longest sequence (else nullptr)
@@ -620,7 +620,9 @@ __device__ __forceinline__ void chain_finish(const ScanParams& p, ChainView& cv,
       }
       cv.fin_fp32 = 1;
     } else {
-      if (seg > 0) {
+      // (run 0 over compact records: the caller's state, which maps_kernel has put there, so that this pass may write the final
+      // state over it)
+      if (seg > 0 || (p.seg_pass == kSegWalks && cv.init_mode != 0)) {
         cv.init_mode = 1;
         cv.init_base = slots + (seg * 3 + 2) * kSegSlotFloats;
       }

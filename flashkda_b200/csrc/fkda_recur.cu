@@ -898,6 +898,22 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
               *reinterpret_cast<float2*>(N + (row0 + 16 * vt + g + 8 * i) * kD + 8 * jt + 2 * t) = make_float2(S[vt][jt][2 * i], S[vt][jt][2 * i + 1]);
       }
     }
+  } else if (warp != 5 && run == 0 && ok) {
+    // (the warps without a part in the walks) The caller's state goes where the second pass starts run 0 from: by then the CTA of the
+    // last run may have written the final state over it, which may be the same tensor.
+    float4* dst = reinterpret_cast<float4*>(p.seg_buf + ((static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 + 2) * kSegSlotFloats);
+    const int first = (warp == 4 ? 0 : warp - 5) * 32 + lane;
+#pragma unroll 4
+    for (int i = first; i < kD * kD / 4; i += 3 * 32) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (cv.init_mode == 1) {
+        x = __ldg(static_cast<const float4*>(cv.init_base) + i);
+      } else if (cv.init_mode == 2) {
+        const uint2 y = __ldg(static_cast<const uint2*>(cv.init_base) + i);
+        x = make_float4(bf_lo(y.x), bf_hi(y.x), bf_lo(y.y), bf_hi(y.y));
+      }
+      dst[i] = x;
+    }
   } else if (warp == 5 && lane == 0 && ok) {
     const uint8_t* rec = p.records + (static_cast<size_t>(cv.h) * p.total_chunks + cv.chunk_base) * kCrBytes;
     int item = 0;

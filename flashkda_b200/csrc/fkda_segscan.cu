@@ -46,7 +46,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
   lo = __float_as_uint(x - __uint_as_float(hi)) & 0xffffe000u;
 }
 
-// Z_start[run + 1] = Z_start[run] M[run] + N[run] for run = first .. n_segs-2, Z_start[0] the caller's state; rows of Z are independent, so each CTA
+// Z_start[run + 1] = Z_start[run] M[run] + N[run] for run = first .. n_segs-2, Z_start[first] in its slot; rows of Z are independent, so each CTA
 // carries eight of them through all runs, as Z^T[run + 1] = M^T Z^T + N^T.  The maps arrive by bulk copies (one per map: its
 // slot holds it with padded rows) three runs ahead.  The products run on the tensor cores in tf32 with both operands split into a leading and a
 // trailing part (three mma per tile: the error of the split, about 2^-21 relative, is that of an fp32 product), fp32
@@ -59,7 +59,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
 // which the instruction caches no longer hold (1.7 us).
 // Runs whose map is zero (`flagged`: their words are looked at) are left out: the state behind such a run is in its slot already.
 __global__ void __launch_bounds__(kCmbThreads, 1)
-seg_combine_kernel(float* seg_buf, int n_segs, int first, int flagged, const void* initial_state, int state_fp32, int* status, int wait_limit_us, int stop_maps_after) {
+seg_combine_kernel(float* seg_buf, int n_segs, int first, int flagged, int* status, int wait_limit_us, int stop_maps_after) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   const uint32_t sbase = smem_u32(smem);
@@ -123,25 +123,7 @@ seg_combine_kernel(float* seg_buf, int n_segs, int first, int flagged, const voi
     }
   };
   float x[4], next_n[4];                 // N of a run is fetched one run ahead
-  if (list[0] > 0) {
-    load_rows(slots + (list[0] * 3 + 2) * kSegSlotFloats, x);      // the state at the start of that run
-  } else {
-    const size_t at = (static_cast<size_t>(blockIdx.x) * kD + r_base + 2 * t) * kD + n0 + 2 * g;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (initial_state == nullptr) {
-        x[i] = x[2 + i] = 0.f;
-      } else if (state_fp32) {
-        const float2 y = *reinterpret_cast<const float2*>(static_cast<const float*>(initial_state) + at + i * kD);
-        x[i] = y.x;
-        x[2 + i] = y.y;
-      } else {
-        const uint32_t y = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(initial_state) + at + i * kD);
-        x[i] = bf_lo(y);
-        x[2 + i] = bf_hi(y);
-      }
-    }
-  }
+  load_rows(slots + (list[0] * 3 + 2) * kSegSlotFloats, x);      // the state at the start of that run
   if (half == 0) put_z(n0, x);
   load_rows(slots + (list[0] * 3 + 1) * kSegSlotFloats, next_n);
   // this warp's columns of a map, split: [k-step][leading, trailing part][A fragment]
@@ -250,7 +232,7 @@ cudaError_t launch_scan_segmented(const ScanParams& base, int n_segs, int seg_ch
     if (e != cudaSuccess) return e;
     const dim3 grid(static_cast<unsigned>(chains), kD / kCmbRows);
     e = launch_after(seg_combine_kernel, grid, kCmbThreads, kCmbSmemBytes, stream, seg_buf, n_segs, v != nullptr ? 0 : 1,
-                     v != nullptr && p.stop_maps_after == 0 ? 1 : 0, p.initial_state, p.state_fp32, p.status, p.map_wait_limit_us, p.stop_maps_after);
+                     v != nullptr && p.stop_maps_after == 0 ? 1 : 0, p.status, p.map_wait_limit_us, p.stop_maps_after);
     if (e != cudaSuccess) return e;
   }
   p.seg_pass = v != nullptr ? kSegWalks : 2;

@@ -80,7 +80,7 @@ typedef struct fkda_fwd_params {
   const float* A_log;        /* fp32 [H]                                                        */
   const float* dt_bias;      /* fp32 [H][128]                                                   */
   const void* initial_state; /* [N][H][128 v][128 k] of state_dtype, or NULL (start from zero) */
-  void* final_state;         /* same shape and dtype, or NULL                                   */
+  void* final_state;         /* same shape and dtype, or NULL; may be initial_state itself       */
   const int64_t* cu_seqlens; /* device int64 [N+1], or NULL for B equal-length sequences        */
   void* workspace;           /* >= fkda_get_workspace_size bytes, 256-byte aligned (may be NULL where
                                 fkda_fwd_scratch_bytes says 0)                                  */

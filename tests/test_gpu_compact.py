@@ -206,6 +206,40 @@ def test_the_call_walks_the_runs_that_the_planner_reports(H, T, packed):
         assert bool((states != 0x5A).any(-1).all()), "fewer runs than reported"
 
 
+@pytest.mark.parametrize("state", ["bf16", "fp32"])
+@pytest.mark.parametrize("H,T,lens", [(2, 32 * 700, None), (8, 8192, None), (2, 0, [32 * 200 + 9, 0, 32 * 180, 32 * 3 + 1]), (3, 0, [9000, 40])],
+                         ids=["two_heads", "eight_heads", "packed", "packed_empty_last_runs"])
+def test_states_may_be_updated_in_place_by_calls_that_are_cut_into_runs(H, T, lens, state):
+    """`initial_state is final_state`, as a server keeps them: the bits of a call with separate tensors.  The last run, which in the packed
+    batches is empty for the shorter sequence and stores at once, works beside run 0; so run 0 starts from the copy that the first
+    pass has left in its slot."""
+    w = Workload("in place", H=H, T=T, seq_lens=lens, state_in=state, state_out=state, state_std=0.5, seed=H)
+    x = make_inputs(w, device="cuda")
+    args = (x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"])
+    tokens, chains = x["q"].shape[1], w.N * H
+    runs = F.plan_segments(chains, (tokens // w.N + 31) // 32)[0]
+    if lens:
+        runs = min(runs, F.plan_segments(chains, (tokens * 4 // (w.N * 3) + 31) // 32)[0])
+    assert runs > 1
+    off, rec, per_head = F.workspace_layout(tokens, H, w.N, lens is not None, T)
+    slots, floats = off + rec * per_head * H, 128 * 136
+    ws = torch.full((max(F.get_workspace_size(tokens, H, w.N), slots + chains * runs * 3 * floats * 4),), 0xFF, dtype=torch.uint8, device="cuda")
+    before = x["initial_state"].clone()
+    F.fwd(*args, initial_state=x["initial_state"], final_state=x["final_state"], cu_seqlens=x["cu_seqlens"], workspace=ws)
+    assert F.read_status(ws) == 0
+    assert torch.equal(x["initial_state"], before)
+    taken = ws[slots:slots + chains * runs * 3 * floats * 4].view(torch.float32).view(w.N, H, runs, 3, floats)[:, :, 0, 2, :128 * 128]
+    taken = taken.reshape(before.shape)
+    for n in range(w.N):
+        if lens is None or lens[n] > 4:          # (the others are the per-token kernel's)
+            assert torch.equal(taken[n], before[n].float()), n
+    out, fin = x["out"].clone(), x["final_state"].clone()
+    for _ in range(20):
+        both = before.clone()
+        F.fwd(*args, initial_state=both, final_state=both, cu_seqlens=x["cu_seqlens"], workspace=ws)
+        assert torch.equal(x["out"].view(torch.int16), out.view(torch.int16)) and torch.equal(both, fin)
+
+
 @pytest.mark.parametrize("state", [None, "bf16", "fp32"])
 @pytest.mark.parametrize("B,T", [(1, 1), (3, 4), (2, 5), (5, 15), (5, 16), (3, 17), (2, 31), (2, 32), (400, 3)])
 def test_short_sequences_match_the_recurrence(B, T, state):
