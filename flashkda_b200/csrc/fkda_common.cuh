@@ -474,8 +474,12 @@ constexpr int64_t kSegSlotFloats = 128 * kSegMapStride;   // every slot has room
 // Passes over runs on the compact records (ScanParams::seg_pass; 1 and 2 are the two-stage form's): maps of all runs but the last,
 // walks of all runs.
 constexpr int kSegMaps = 3, kSegWalks = 4;
-// Whether the map of a run is zero to the last bit: behind its offset's rows.
+// Words behind the rows of a run's offset: whether its map is zero to the last bit; how many runs of the chain are done, with
+// kSegBad for each of them that left something other than finite numbers (run 0's counts); a bit per row v of S^T that did ([4]).
 __device__ __forceinline__ int* seg_zero_word(float* slots, int run) { return reinterpret_cast<int*>(slots + (run * 3 + 1) * kSegSlotFloats + kD * kD); }
+__device__ __forceinline__ int* seg_done_word(float* slots) { return seg_zero_word(slots, 0) + 1; }
+__device__ __forceinline__ uint32_t* seg_bad_rows(float* slots, int run) { return reinterpret_cast<uint32_t*>(seg_zero_word(slots, run)) + 4; }
+constexpr int kSegBad = 0x10000;
 constexpr int kDefaultSms = 148;       // SMs of a B200: assumed where no device can be asked
 
 // SM count of the current device, asked once per device and cached; the kernel-selection rules, the planner of the

@@ -302,6 +302,55 @@ __device__ __forceinline__ void store_state(const float (&S)[2][16][4], const Ch
   }
 }
 
+// (runs) The rows of a warp that hold an infinity or not-a-number, a bit each.
+__device__ __forceinline__ uint32_t bad_rows(const float (&S)[2][16][4]) {
+  uint32_t rows = 0;
+#pragma unroll
+  for (int vt = 0; vt < 2; ++vt)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t most = 0;
+#pragma unroll
+      for (int jt = 0; jt < 16; ++jt)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) most = max(most, __float_as_uint(S[vt][jt][2 * i + k]) & 0x7fffffffu);
+      const uint32_t lanes = __ballot_sync(0xffffffffu, most >= 0x7f800000u);
+#pragma unroll
+      for (int g = 0; g < 8; ++g) rows |= (lanes >> (4 * g) & 15u) != 0u ? 1u << (16 * vt + 8 * i + g) : 0u;
+    }
+  return rows;
+}
+
+// (runs, at the end of a CTA) A row of S^T that holds an infinity or not-a-number once holds one to the end of its sequence, and every
+// output of that channel is one: R = v - S k+, U and S e + U kr take in the whole row.  A map that was found to be zero says
+// otherwise: the runs behind it start from its offset, whatever is in front.  So the last CTA of a chain to come here, where some run
+// has left such rows, writes not-a-number over what the runs behind that one have made of them.  Other calls pay
+// for an atomic at the end of each CTA: 0.8 to 1.4 us of 48 to 600.
+__device__ __forceinline__ void spoil_runs(const ScanParams& p, float* slots, volatile int* last, bool bad) {
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    int done;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(done) : "l"(seg_done_word(slots)), "r"(bad ? 1 + kSegBad : 1) : "memory");
+    *last = (done & (kSegBad - 1)) == p.n_segs - 1 && (bad || done >= kSegBad);
+  }
+  __syncthreads();
+  if (!*last) return;
+  const ChainView cv = chain_view<false>(p, static_cast<int>(blockIdx.x) / p.n_segs);
+  const int v = tid & (kD - 1), part = tid / kD, run_len = p.seg_chunks_dev != nullptr ? *p.seg_chunks_dev : p.seg_chunks;
+  int run = 0;
+  while (run < p.n_segs - 1 && !(__ldcg(seg_bad_rows(slots, run) + (v >> 5)) >> (v & 31) & 1u)) ++run;
+  if (run == p.n_segs - 1) return;
+  const int64_t chunk = static_cast<int64_t>(run + 1) * run_len, covered = cv.bos + static_cast<int64_t>(cv.nchunks) * kChunk;
+  const int64_t end = covered < cv.eos ? covered : cv.eos;
+  for (int64_t t = cv.bos + chunk * kChunk + part; t < end; t += kThreads / kD)
+    p.out[(t * p.H + cv.h) * kD + v] = __ushort_as_bfloat16(0x7fff);
+  if (cv.fin_base != nullptr && part == 0)
+    for (int k = 0; k < kD; ++k) {
+      if (cv.fin_fp32) static_cast<uint32_t*>(cv.fin_base)[v * kD + k] = 0x7fffffffu;
+      else static_cast<uint16_t*>(cv.fin_base)[v * kD + k] = 0x7fffu;
+    }
+}
+
 // kStream: the CTA is persistent and goes through its walks (whole chains; with kSeg runs of a chain, see fkda_segscan.cu) as
 // one stream of chunks, so that records, v and state of the next walk are on their way while the last chunks of this one
 // are computed.  Equal lengths: walks in turn, every other round backwards; packed batches take the next longest
@@ -317,9 +366,14 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kSmMisc);
   Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
   auto bar = [&](int i) { return sbase + kSmBars + 8 * i; };
+  // (runs) whether some rows are not finite at the end, the chain's slots (unless the recurrence could not begin)
+  volatile int* bad = reinterpret_cast<volatile int*>(smem + kSmMisc + 8);
+  float** chain_slots = reinterpret_cast<float**>(smem + kSmWalks);
   if (tid == 0) {
     // the swizzled tiles need this alignment: report instead of computing garbage (below zero: a wait limit, test aid)
     *abort_flag = (sbase & 1023u) != 0u ? 1 : -p.wait_limit_us;
+    *bad = 0;
+    if (kSeg) *chain_slots = nullptr;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar(B_FULL + s), 1);
       mbar_init(bar(B_EMPTY + s), 4 + 1);              // recurrence warps + commit of the products on U
@@ -377,6 +431,15 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
       // (an empty run hands its state through)
       if (cv.nchunks > 0) ok = walk(S, smem, sbase, tq, cv.nchunks, cv.eos - cv.bos, row0, lane, abort_flag, s, par, ready, static_cast<uint32_t>(i));
       if (ok && cv.fin_base != nullptr) store_state(S, cv, row0, lane);
+      if (kSeg) {
+        const uint32_t rows = ok ? bad_rows(S) : 0u;
+        if (lane == 0) {
+          float* slots = p.seg_buf + (static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 * kSegSlotFloats;
+          seg_bad_rows(slots, static_cast<int>(blockIdx.x) % p.n_segs)[warp] = rows;
+          if (rows != 0u) *bad = 1;
+          if (warp == 0) *chain_slots = slots;
+        }
+      }
       if (!kStream) break;
       i += cv.nchunks;
     }
@@ -614,13 +677,14 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     tc_fence_after();
     tmem_dealloc(tmem, kTmemCols);
   }
+  if (kSeg && *chain_slots != nullptr) spoil_runs(p, *chain_slots, reinterpret_cast<volatile int*>(smem + kSmMisc + 12), *bad != 0);
 }
 
 // ---- maps of runs (fkda_segscan.cu) ---------------------------------------------------------------------------------------
 // A CTA per (chain, run but the last): first the run's transition map M, from its last chunk to its first, then its offset N,
 // the walk from a zero state.  Walked backwards, Q <- Q Phi^T from the identity, the rows of M^T = Q never meet each other either, and
 // after c chunks Q is the map of the run's last c chunks: once it is zero to the last bit (103 nats of decay; a few hundred
-// tokens of ordinary gates), so is M, and nothing in front of those chunks can be seen behind the run.  Both walks then end there:
+// tokens of ordinary gates), so is M, and nothing finite in front of those chunks can be seen behind the run (spoil_runs sees to the rest).  Both walks then end there:
 // what they cost is a handful of chunks instead of two runs, and chaining such runs costs nothing at all.  A run
 // whose gates hold some channel to the end costs what it always did, a walk each for M and N, plus the test for zero (a hundred
 // cycles in the first sixteen chunks and then in every eighth).
@@ -901,8 +965,10 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
   } else if (warp != 5 && run == 0 && ok) {
     // (the warps without a part in the walks) The caller's state goes where the second pass starts run 0 from: by then the CTA of the
     // last run may have written the final state over it, which may be the same tensor.
-    float4* dst = reinterpret_cast<float4*>(p.seg_buf + ((static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 + 2) * kSegSlotFloats);
+    float* slots = p.seg_buf + (static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 * kSegSlotFloats;
+    float4* dst = reinterpret_cast<float4*>(slots + 2 * kSegSlotFloats);
     const int first = (warp == 4 ? 0 : warp - 5) * 32 + lane;
+    if (first == 0) *seg_done_word(slots) = 0;
 #pragma unroll 4
     for (int i = first; i < kD * kD / 4; i += 3 * 32) {
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);

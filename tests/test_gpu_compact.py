@@ -375,6 +375,40 @@ def test_runs_whose_maps_last_or_vanish(lasting, packed, state):
     assert rel_fro(fin.cpu(), s64) <= STATE_REL
 
 
+@pytest.mark.parametrize("where", ["state", "v", "k", "g", "beta", "q"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")], ids=["nan", "inf"])
+@pytest.mark.parametrize("lens,state", [((16384,), "fp32"), ((9000, 3000, 3), "fp32"), ((6400, 6400), "bf16")], ids=["equal", "packed", "packed_bf16"])
+def test_not_a_number_reaches_to_the_end_of_a_sequence_cut_into_runs(lens, state, value, where):
+    """With gates that forget everything within a run: what is not finite reaches as far as in the walk of a whole sequence, which
+    runs that start from a vanished map would cut short.  Everything else is as close as the two forms are."""
+    H = 2
+    w = Workload("nan", H=H, seq_lens=list(lens), state_in=state, state_out=state, seed=91)
+    x = make_inputs(w, device="cuda")
+    assert F.plan_segments(len(lens) * H, (sum(lens) // len(lens) + 31) // 32)[0] > 1
+    if where == "state":
+        x["initial_state"][0, 0, 5, 7] = value
+        x["initial_state"][len(lens) - 1, 1, 100, 3] = value
+    elif where == "beta":
+        x["beta"][0, 2100, 1] = value if value != value else -value       # (sigmoid(inf) is a number)
+    else:
+        x[where][0, 700, 0, 33] = value
+        x[where][0, 5000, 1, 4] = value
+    inputs = {n: x[n] for n in ("q", "k", "v", "g", "beta")}
+    common = (x["A_log"], x["dt_bias"], x["lower_bound"])
+    packed = x["cu_seqlens"] if len(lens) > 1 else None
+    F.fwd(*inputs.values(), x["scale"], x["out"], *common, initial_state=x["initial_state"], final_state=x["final_state"], cu_seqlens=packed)
+    a = 0
+    for n, length in enumerate(lens):
+        part = {name: t[:, a:a + length].contiguous() for name, t in inputs.items()}
+        out, fin = torch.empty_like(part["v"]), torch.empty_like(x["final_state"][n:n + 1])
+        F.fwd(*part.values(), x["scale"], out, *common, initial_state=x["initial_state"][n:n + 1], final_state=fin, flags=F.FLAG_SCAN_NO_SEGMENTS)
+        for got, want in ((x["out"][:, a:a + length], out), (x["final_state"][n:n + 1], fin)):
+            finite = torch.isfinite(want)
+            assert torch.equal(torch.isfinite(got), finite), (n, int((torch.isfinite(got) != finite).sum()))
+            assert not finite.any() or max_abs(got[finite], want[finite]) <= OUT_MAX_ABS
+        a += length
+
+
 @pytest.mark.parametrize("T,asks", [(1, 0), (4, 0), (5, 1), (40, 1)])
 def test_a_decode_step_asks_for_no_scratch_memory(T, asks):
     w = Workload("d", H=4, B=3, T=T, state_in="fp32", state_out="fp32", seed=T)
