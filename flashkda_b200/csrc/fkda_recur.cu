@@ -43,6 +43,7 @@ constexpr int kSmInfo = kSmStg + 4 * 32 * kStgStride;
 constexpr int kSmBars = kSmInfo + kInfos * 32;
 constexpr int kSmMisc = kSmBars + 256;
 constexpr int kWalkInfos = 8;                      // (persistent form) more than stages, and a walk has an item at least
+constexpr int kClaimAhead = 6;                     // (persistent form) items left of a walk to copy when the next one is claimed
 constexpr int kSmWalks = kSmMisc + 16;
 constexpr int kSmem = kSmWalks + kWalkInfos * 48;
 static_assert(kSmem <= 227 * 1024, "shared memory plan");
@@ -454,7 +455,11 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
     // ===== one lane of the second warp: the stream of chunks into the ring ==========================================
     struct { long long bos, eos; const uint8_t* rec; int walk, h, c, n, turn; bool ended; } cur{};
     // The next walk, looked up a step per item (a packed batch: the counter, the order by length, then the sequence's ends and first record
-    // are loads that depend on one another; in a row they would keep this warp's output waiting for more than a chunk's time).
+    // are loads that depend on one another; in a row they would keep this warp's output waiting for more than a chunk's time).  Not
+    // before the walk's last items: what a CTA holds nobody else can take, and walks are handed out longest first.  With the look-up begun at
+    // a walk's second item one SM had a sequence of 6400 tokens behind the one of 16384: 16384 + 4 x 6400 + 60 x 64 tokens on 32
+    // heads 1283 us, now 1056; 96 decode tokens among four prompts 236.2 -> 237.3.  Three items ahead, one for each step, 200
+    // short sequences need 417 us, as the last step's loads are waited for; six ahead 414.5.
     struct { ChainView cv; int walk, step; } next{};
     auto look = [&]() {
       if (!kStream || next.step >= 3) return;
@@ -538,7 +543,7 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
           if (copied > 0 && (cv.init_mode == 1 || cv.init_mode == 2)) bulk_prefetch_l2(cv.init_base, kD * kD * (cv.init_mode == 1 ? 4 : 2));
           break;
         }
-      } else {
+      } else if (cur.n - cur.c <= kClaimAhead) {
         look();
       }
       const long long t0 = cur.bos + static_cast<long long>(cur.c) * kChunk;

@@ -409,6 +409,31 @@ def test_not_a_number_reaches_to_the_end_of_a_sequence_cut_into_runs(lens, state
         a += length
 
 
+def test_the_longest_sequence_of_a_skewed_batch_sets_the_time():
+    """Persistent recurrence: the walks are handed out longest first, and a CTA takes its next one near the end of its walk.  Taken with
+    the first items, one of four sequences of 200 chunks waits behind the one of 512 on the same SM: 712 chunks instead of 512
+    (measured 843 us against 621 for the longest alone; now 626).  The bound lies halfway between the two: 1 + 200 / 512 / 2."""
+    def stage_time(lens):
+        w = Workload("skew", H=32, seq_lens=lens, state_out="fp32", seed=8)
+        x = make_inputs(w, device="cuda")
+        args = (x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["out"], x["A_log"], x["dt_bias"], x["lower_bound"])
+        ws = torch.empty(F.get_workspace_size(sum(lens), w.H, w.N), dtype=torch.uint8, device="cuda")
+        F.operands(*args, cu_seqlens=x["cu_seqlens"], workspace=ws)
+        times = []
+        for _ in range(9):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            F.recurrence(*args, final_state=x["final_state"], cu_seqlens=x["cu_seqlens"], workspace=ws)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        return sorted(times)[len(times) // 2]
+
+    alone, skewed = stage_time([16384] + [64] * 124), stage_time([16384] + [6400] * 4 + [64] * 60)
+    print(f"longest alone {alone:.3f} ms, skewed {skewed:.3f} ms")
+    assert skewed <= alone * 1.195
+
+
 @pytest.mark.parametrize("T,asks", [(1, 0), (4, 0), (5, 1), (40, 1)])
 def test_a_decode_step_asks_for_no_scratch_memory(T, asks):
     w = Workload("d", H=4, B=3, T=T, state_in="fp32", state_out="fp32", seed=T)
