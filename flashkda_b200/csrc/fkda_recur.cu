@@ -967,20 +967,24 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
               *reinterpret_cast<float2*>(N + (row0 + 16 * vt + g + 8 * i) * kD + 8 * jt + 2 * t) = make_float2(S[vt][jt][2 * i], S[vt][jt][2 * i + 1]);
       }
     }
-  } else if (warp != 5 && run == 0 && ok) {
+  } else if (warp != 5 && ok) {
     // (the warps without a part in the walks) The caller's state goes where the second pass starts run 0 from: by then the CTA of the
-    // last run may have written the final state over it, which may be the same tensor.
-    float* slots = p.seg_buf + (static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 * kSegSlotFloats;
+    // last run may have written the final state over it, which may be the same tensor.  A share for every CTA of the chain: all
+    // of it takes one CTA longer than walks that vanish (8 heads of 131072 tokens 592 -> 599 us).
+    const size_t chain = static_cast<size_t>(cv.n) * p.H + cv.h;
+    float* slots = p.seg_buf + chain * p.n_segs * 3 * kSegSlotFloats;
     float4* dst = reinterpret_cast<float4*>(slots + 2 * kSegSlotFloats);
-    const int first = (warp == 4 ? 0 : warp - 5) * 32 + lane;
+    const float4* wide = static_cast<const float4*>(p.initial_state) + chain * (kD * kD / 4);
+    const uint2* narrow = static_cast<const uint2*>(p.initial_state) + chain * (kD * kD / 4);
+    const int first = (run * 3 + (warp == 4 ? 0 : warp - 5)) * 32 + lane;
     if (first == 0) *seg_done_word(slots) = 0;
-#pragma unroll 4
-    for (int i = first; i < kD * kD / 4; i += 3 * 32) {
+#pragma unroll 8
+    for (int i = first; i < kD * kD / 4; i += (p.n_segs - 1) * 3 * 32) {
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (cv.init_mode == 1) {
-        x = __ldg(static_cast<const float4*>(cv.init_base) + i);
-      } else if (cv.init_mode == 2) {
-        const uint2 y = __ldg(static_cast<const uint2*>(cv.init_base) + i);
+      if (p.initial_state != nullptr && p.state_fp32) {
+        x = __ldg(wide + i);
+      } else if (p.initial_state != nullptr) {
+        const uint2 y = __ldg(narrow + i);
         x = make_float4(bf_lo(y.x), bf_hi(y.x), bf_lo(y.y), bf_hi(y.y));
       }
       dst[i] = x;
