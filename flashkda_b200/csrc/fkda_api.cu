@@ -214,8 +214,10 @@ bool fused_short(const fkda_fwd_params* p) {
 }
 
 // whether the call is one of the per-token kernel, and with it needs no scratch memory: that kernel has no wait whose end a
-// status word could tell
-bool takes_step_kernel(const fkda_fwd_params* p) { return fused_short(p) && p->T <= fkda::kStepMaxT && !(p->flags & FKDA_FLAG_FUSED_ANY_T); }
+// status word could tell (FKDA_FLAG_REFERENCE_ROUNDING, not among the flags that fused_short looks at, comes first and clears the header)
+bool takes_step_kernel(const fkda_fwd_params* p) {
+  return fused_short(p) && p->T <= fkda::kStepMaxT && !(p->flags & (FKDA_FLAG_FUSED_ANY_T | FKDA_FLAG_REFERENCE_ROUNDING));
+}
 int64_t scratch_bytes(const fkda_fwd_params* p, const Layout& L) {
   if (!(p->flags & FKDA_FLAG_STATUS_UNREAD) || !fused_short(p)) return L.total_bytes;
   return takes_step_kernel(p) ? 0 : static_cast<int64_t>(fkda::kWsHeaderBytes);

@@ -111,7 +111,8 @@ int fkda_workspace_bytes_exact(int64_t T_total, int64_t H, int64_t N, int varlen
 
 /* The same for one call: the bytes of workspace that fkda_fwd will need for exactly these sizes and flags (`workspace`,
  * `workspace_bytes` and the data pointers other than cu_seqlens are not looked at).  None (0) with
- * FKDA_FLAG_STATUS_UNREAD for a fixed-length call of at most four tokens per sequence. */
+ * FKDA_FLAG_STATUS_UNREAD for a fixed-length call of at most four tokens per sequence (a header's bytes where
+ * FKDA_FLAG_REFERENCE_ROUNDING is given too). */
 int fkda_fwd_scratch_bytes(const fkda_fwd_params* p, int64_t* bytes);
 
 /* The plan of the recurrence over long sequences: into how many runs (1 = none), walked in parallel, fkda_fwd cuts the

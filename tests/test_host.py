@@ -121,6 +121,23 @@ def test_c_abi_rejects_bad_params_without_a_gpu():
     assert L.fkda_fwd(ctypes.byref(p), None) == -1 and "aligned" in F.last_error()
 
 
+@pytest.mark.parametrize("T", [1, 4])
+def test_reference_rounding_needs_the_header_also_where_a_decode_step_needs_no_workspace(T):
+    """That form clears the header whatever else is asked for."""
+    from flashkda_b200._binding import FwdParams
+    L, unread, header = F.lib(), 0x40000, 256
+    asked = ctypes.c_int64(-1)
+
+    def params(flags, workspace=None, size=0):
+        return FwdParams(*([0x1000] * 8), None, None, None, workspace, size, 2, T, 2, 2, 0.1, -5.0, 0, flags)
+    assert L.fkda_fwd_scratch_bytes(ctypes.byref(params(unread)), ctypes.byref(asked)) == 0 and asked.value == 0
+    p = params(unread | F.FLAG_REFERENCE_ROUNDING)
+    assert L.fkda_fwd_scratch_bytes(ctypes.byref(p), ctypes.byref(asked)) == 0 and asked.value == header
+    assert L.fkda_fwd(ctypes.byref(p), None) == -1 and "workspace is NULL" in F.last_error()
+    p = params(unread | F.FLAG_REFERENCE_ROUNDING, 0x3000, header - 1)
+    assert L.fkda_fwd(ctypes.byref(p), None) == -2 and "workspace has" in F.last_error()
+
+
 def test_segment_planner_is_consistent_with_the_workspace_size():
     """Few long chains are cut into runs; many chains or short sequences are not.  The last run is never empty and
     the workspace grows by three fp32 slots of 128 x 136 floats per (chain, run)."""
