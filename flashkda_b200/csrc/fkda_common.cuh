@@ -519,18 +519,25 @@ struct SmemOptIn {
 
 // Launch that lets the kernel's set-up overlap with the end of the stream's previous kernel (grid_dependency_wait).
 template <class... Params, class... Args>
-inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch_clusters_after(void (*kernel)(Params...), dim3 grid, unsigned cluster, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_clusters_after(kernel, grid, 1, threads, smem, stream, args...);
 }
 
 // What one CTA of a recurrence kernel walks: a whole (sequence, head) chain, or, in the segment-parallel form (kSeg), one

@@ -694,8 +694,8 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
 // whose gates hold some channel to the end costs what it always did, a walk each for M and N, plus the test for zero (a hundred
 // cycles in the first sixteen chunks and then in every eighth).
 // 8 heads of 131072 tokens (lower_bound -2), recurrence with all its passes: 820 -> 340 us, 795 with gates that never decay; 16
-// heads of 32768 tokens, the whole call: 619 -> 365 us (610); the walks themselves have become faster since (281 and 733 us).  Few
-// chains lose a tenth where nothing decays (1 head of 131072 tokens 338 -> 379 us, against 132 otherwise), as M and N had a CTA each.
+// heads of 32768 tokens, the whole call: 619 -> 365 us (610); the walks themselves have become faster since (281 and 733 us).  (Few
+// chains where nothing decays: kPair below.)
 // One chunk of a walk without outputs, from stage s, every product on mma.sync.  `ready`: whether the next stage is full already.
 // kBack: the transposed step, S^T Phi^T with Phi = diag(e) + kn^T TB^T kr the chunk's transition and no v: the same products with k+ and
 // kr exchanged and TB transposed.
@@ -855,12 +855,29 @@ __device__ __forceinline__ bool is_zero(const float (&S)[2][16][4]) {
   return !__any_sync(0xffffffffu, (any << 1) != 0u);
 }
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Into another CTA's shared memory, at the place that `smem` is here.
+__device__ __forceinline__ void cluster_store(uint32_t smem, uint32_t cta, int x) {
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.relaxed.cluster.shared::cluster.b32 [a], %2;\n\t}" ::"r"(smem), "r"(cta), "r"(x) : "memory");
+}
+
+// kPair: a cluster of two CTAs per run.  The first one does as above but for the offset of a run whose map lasts, which the second
+// one walks beside it from the run's first chunk; it leaves off when the first one tells it that the map has vanished.  Taken where all
+// clusters are resident at once: there M and N in turn are the longest path of a call whose gates hold.  Whole calls without
+// decay, M and N in turn and beside one another, heads x tokens: 1 x 4096 80.0 -> 69.8 us, 1 x 16384 in 32 runs 132.6 -> 117.1, 2 x 22400 in 37
+// 161.6 -> 144.5, 4 x 4128 85.1 -> 74.6, 1 x 131072 in 75 359.1 -> 307.4; where maps vanish the cluster costs 0.6 to 2.8 us.  (Runs of
+// more CTAs than that gain nothing: the second round is as long as the second walk.)
+template <bool kPair>
 __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant__ CUtensorMap tm_v, const ScanParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool offset_only = kPair && (blockIdx.x & 1u) != 0u;     // (the cluster's second CTA)
+  const int block = static_cast<int>(kPair ? blockIdx.x >> 1 : blockIdx.x);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kSmMisc + 4);
-  int* zeros = reinterpret_cast<int*>(smem + kSmMisc + 8);       // warps whose rows of the map are zero ...
+  int* zeros = reinterpret_cast<int*>(smem + kSmMisc + 8);       // warps whose rows of the map are zero (second CTA: 4 once the first has said so) ...
   int* longest = reinterpret_cast<int*>(smem + kSmMisc + 12);    // ... after so many chunks
   Info* infos = reinterpret_cast<Info*>(smem + kSmInfo);
   constexpr int B_TURN = B_U;                                    // M is done, N may be fetched
@@ -876,11 +893,12 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
     mbar_init(bar(B_TURN), 4);
     fence_mbar_init();
   }
-  __syncthreads();
+  if (kPair) cluster_sync();
+  else __syncthreads();
   bool ok = *abort_flag <= 0;
   grid_dependency_wait();
-  const ChainView cv = chain_view<true>(p, static_cast<int>(blockIdx.x));
-  const int n = ok ? cv.nchunks : 0, run = static_cast<int>(blockIdx.x) % (p.n_segs - 1);
+  const ChainView cv = chain_view<true>(p, block);
+  const int n = ok ? cv.nchunks : 0, run = block % (p.n_segs - 1);
   if (warp < 4) {
     float* slots = p.seg_buf + (static_cast<size_t>(cv.n) * p.H + cv.h) * p.n_segs * 3 * kSegSlotFloats;
     const int row0 = 32 * warp, g = lane >> 2, t = lane & 3;
@@ -907,7 +925,7 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
       par = par1;
     };
     fill(1.f);
-    for (int c = 0; ok; ++c) {
+    for (int c = 0; ok && !offset_only; ++c) {
       if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
       int s1;
       uint32_t par1;
@@ -929,10 +947,12 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
       if (end) break;
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    const bool all_zero = *static_cast<volatile int*>(zeros) == 4;
+    const bool all_zero = !offset_only && *static_cast<volatile int*>(zeros) == 4;
     const int first = all_zero ? n - *static_cast<volatile int*>(longest) : 0;
+    if (kPair && ok && all_zero && tid == 0) cluster_store(smem_u32(zeros), 1, 4);
+    bool left_off = false;
     if (ok) {
-      if (!all_zero) {           // M, transposed back
+      if (!all_zero && !offset_only) {           // M, transposed back
         float* M = slots + (run * 3 + 0) * kSegSlotFloats;
 #pragma unroll
         for (int vt = 0; vt < 2; ++vt)
@@ -941,13 +961,15 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
 #pragma unroll
             for (int i = 0; i < 4; ++i) M[(8 * jt + 2 * t + (i & 1)) * kSegMapStride + row0 + 16 * vt + g + 8 * (i >> 1)] = S[vt][jt][i];
       }
-      if (tid == 0) *seg_zero_word(slots, run) = all_zero;
+      if (tid == 0 && !offset_only) *seg_zero_word(slots, run) = all_zero;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(B_TURN));
       fill(0.f);
       ready = false;
-      for (int c = first; c < n; ++c) {
+      const bool mine = !kPair || offset_only || all_zero;
+      for (int c = first; mine && c < n; ++c) {
         if (!__all_sync(0xffffffffu, ready) && !warp_wait(bar(B_FULL + s), par, abort_flag)) { ok = false; break; }
+        if (offset_only && (static_cast<const volatile Info*>(infos)[c & (kInfos - 1)].flags & kEnd)) { left_off = true; break; }
         int s1;
         uint32_t par1;
         next(s1, par1);
@@ -955,7 +977,7 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
         step<false>(S, smem, sbase, s, left < kChunk ? static_cast<int>(left) : kChunk, row0, lane, bar(B_FULL + s1), par1, ready);
         release(s1, par1);
       }
-      if (ok) {
+      if (ok && mine && !left_off) {
         // behind a map of zero the offset is the state at the start of the next run
         float* N = all_zero ? slots + ((run + 1) * 3 + 2) * kSegSlotFloats : slots + (run * 3 + 1) * kSegSlotFloats;
 #pragma unroll
@@ -967,7 +989,7 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
               *reinterpret_cast<float2*>(N + (row0 + 16 * vt + g + 8 * i) * kD + 8 * jt + 2 * t) = make_float2(S[vt][jt][2 * i], S[vt][jt][2 * i + 1]);
       }
     }
-  } else if (warp != 5 && ok) {
+  } else if (warp != 5 && ok && !offset_only) {
     // (the warps without a part in the walks) The caller's state goes where the second pass starts run 0 from: by then the CTA of the
     // last run may have written the final state over it, which may be the same tensor.  A share for every CTA of the chain: all
     // of it takes one CTA longer than walks that vanish (8 heads of 131072 tokens 592 -> 599 us).
@@ -1014,11 +1036,18 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
       return true;
     };
     bool more = true;
-    for (int c = n - 1; more && c >= 0 && *static_cast<volatile int*>(zeros) < 4; --c) more = put(c, false);
-    more = more && put(-1, false);
-    if (more && !mbar_wait_parked(bar(B_TURN), 0, abort_flag)) more = ok = false;
-    if (more)
-      for (int c = *static_cast<volatile int*>(zeros) == 4 ? n - *static_cast<volatile int*>(longest) : 0; more && c < n; ++c) more = put(c, true);
+    if (offset_only) {
+      int c = 0;
+      for (; more && c < n && *static_cast<volatile int*>(zeros) < 4; ++c) more = put(c, true);
+      if (more && c < n) more = put(-1, false);
+    } else {
+      for (int c = n - 1; more && c >= 0 && *static_cast<volatile int*>(zeros) < 4; --c) more = put(c, false);
+      more = more && put(-1, false);
+      if (more && !mbar_wait_parked(bar(B_TURN), 0, abort_flag)) more = ok = false;
+      const bool all_zero = *static_cast<volatile int*>(zeros) == 4;
+      if (more && (!kPair || all_zero))
+        for (int c = all_zero ? n - *static_cast<volatile int*>(longest) : 0; more && c < n; ++c) more = put(c, true);
+    }
     if (!ok || *abort_flag > 0 || !more) {
       // (giving up) copies in flight must land before the CTA's shared memory goes away
       for (int c = item > kStages ? item - kStages : 0; c < item; ++c) {
@@ -1029,7 +1058,8 @@ __global__ void __launch_bounds__(kThreads, 1) maps_kernel(const __grid_constant
     }
   }
   if (!ok || *abort_flag > 0) atomicCAS(p.status, kStatusOk, kStatusWaitTimeout);
-  __syncthreads();
+  if (kPair) cluster_sync();                                     // (what the first CTA stores into goes away with the second)
+  else __syncthreads();
 }
 
 }  // namespace recur
@@ -1042,10 +1072,12 @@ cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream
   CUtensorMap tv;
   if (!make_map(&tv, v, p.T_total, p.H)) return cudaErrorInvalidValue;
   if (p.seg_chunks > 0 && p.seg_pass == kSegMaps) {
-    static SmemOptIn opt_in;
-    cudaError_t e = opt_in.ensure(recur::maps_kernel, recur::kSmem);
+    const bool pair = walks * 2 <= device_sm_count();
+    const auto maps = pair ? recur::maps_kernel<true> : recur::maps_kernel<false>;
+    static SmemOptIn opt_in[2];
+    cudaError_t e = opt_in[pair].ensure(maps, recur::kSmem);
     if (e != cudaSuccess) return e;
-    return launch_after(recur::maps_kernel, static_cast<unsigned>(walks), recur::kThreads, recur::kSmem, stream, tv, p);
+    return launch_clusters_after(maps, static_cast<unsigned>(pair ? 2 * walks : walks), pair ? 2 : 1, recur::kThreads, recur::kSmem, stream, tv, p);
   }
   // More walks than SMs and short ones on average: one persistent CTA per SM.  (At 24 chunks the 3 us a walk costs more
   // in a CTA of its own are what the tighter chunk loop saves.)

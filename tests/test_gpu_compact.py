@@ -375,6 +375,29 @@ def test_runs_whose_maps_last_or_vanish(lasting, packed, state):
     assert rel_fro(fin.cpu(), s64) <= STATE_REL
 
 
+@pytest.mark.parametrize("lasting", ["all", "none", "odd"])
+@pytest.mark.parametrize("H,T,beside", [(1, 32 * 100 + 1, True), (4, 32 * 128, True), (12, 32 * 160, False)])
+def test_maps_and_offsets_beside_one_another_and_in_turn(H, T, beside, lasting):
+    """The first pass over runs, with M and N of a run in two CTAs of a cluster where all of them are resident at once, else in turn in one."""
+    w = Workload("b", H=H, T=T, state_in="fp32", state_out="fp32", state_std=0.5, seed=T + H, lower_bound=-2.0)
+    runs, length = F.plan_segments(H, (T + 31) // 32)
+    assert runs > 2 and (H * (runs - 1) * 2 <= torch.cuda.get_device_properties(0).multi_processor_count) == beside
+    x = make_inputs(w)
+    for r in range(runs):
+        if lasting == "all" or (lasting == "odd" and r % 2 == 1):
+            x["g"][:, r * length * 32:(r + 1) * length * 32] = -12.0
+    x["A_log"].fill_(0.5)
+    xc = to_cuda(x)
+    ws = torch.full((F.get_workspace_size(T, H, 1),), 0xFF, dtype=torch.uint8, device="cuda")
+    F.fwd(xc["q"], xc["k"], xc["v"], xc["g"], xc["beta"], x["scale"], xc["out"], xc["A_log"], xc["dt_bias"], x["lower_bound"],
+          initial_state=xc["initial_state"], final_state=xc["final_state"], workspace=ws)
+    assert F.read_status(ws) == 0
+    o64, s64 = oracle.recurrence_f64(x["q"], x["k"], x["v"], x["g"], x["beta"], x["scale"], x["A_log"], x["dt_bias"], x["lower_bound"],
+                                     initial_state=x["initial_state"])
+    assert max_abs(xc["out"].cpu(), o64) <= OUT_MAX_ABS and rel_fro(xc["out"].cpu(), o64) <= 1e-2
+    assert rel_fro(xc["final_state"].cpu(), s64) <= STATE_REL
+
+
 @pytest.mark.parametrize("where", ["state", "v", "k", "g", "beta", "q"])
 @pytest.mark.parametrize("value", [float("nan"), float("inf")], ids=["nan", "inf"])
 @pytest.mark.parametrize("lens,state", [((16384,), "fp32"), ((9000, 3000, 3), "fp32"), ((6400, 6400), "bf16")], ids=["equal", "packed", "packed_bf16"])
