@@ -78,9 +78,13 @@ struct Layout {
 // How many runs to cut each sequence of a batch into (1 = walk whole sequences), at most `most` of them, and their length in
 // chunks.  The first pass has a CTA for every run but the last, which works out the run's map M and offset N; the second one a CTA
 // per run.  Where the gates' decay makes M vanish, which the first pass finds out (fkda_recur.cu), its two walks are a few chunks
-// long; where it does not, they are as long as the run and the maps are chained.  The plan is made for the former, among those that cost in the
-// latter at most a tenth more than whole sequences and a twelfth more than the best plan for it; of plans within 5 % and 3 us,
-// which is what the costs are off by, the one with the fewest runs.  The one planner: the workspace size, the launch and fkda_plan_segments ask here.
+// long; where it does not, they are as long as the run, beside one another if a CTA for each is resident, and the maps are chained.  The plan
+// is made for the former, among those that cost in the latter at most a tenth more than whole sequences and no more than `before`: the
+// best plan of the form that walked M and N forwards in a CTA each whatever the gates (its own fitted costs), which a call that never forgets
+// must not fall behind.  Microseconds without decay / with, chains x chunks, that form, a twelfth above the best plan instead, now:
+// 1 x 4096 346, 372 / 122, 305 / 145; 2 x 700 154, 166 / 74, 143 / 81; 3 x 700 169, 172 / 84, 152 / 96; 1 x 1500 207, 225 / 82, 203 / 86.
+// Where that form was not worth it, a twelfth above the best plan: 24 x 256 265 / 162 against 239 in whole sequences.
+// Of plans within 5 % and 3 us, which is what the costs are off by, the one with the fewest runs.  The one planner: the workspace size, the launch and fkda_plan_segments ask here.
 // Its costs are those of the default path's kernels, in hundredths of a microsecond, fitted to 150 timed calls of 1 to 48
 // heads and 64 to 4096 chunks, half of them without decay: a chunk step of a chain split over four or two CTAs (fkda_recur_split.cu) or
 // in one CTA (fkda_recur.cu), the latter with and without outputs; the chunks that a map takes to vanish; what the passes cost
@@ -92,12 +96,16 @@ int plan_runs(int64_t chains, int64_t chunks, int64_t most, int sms, int* len) {
   if (chains <= 0 || chains * 3 > sms || chunks < 48) return 1;
   const int64_t whole = (chains * 4 <= sms ? kQuad : kHalf) * chunks;
   auto rounds = [&](int64_t ctas) { return (ctas + sms - 1) / sms; };
-  struct Cost { int64_t vanishing, lasting; };
+  struct Cost { int64_t vanishing, lasting, before; };
   auto cost = [&](int64_t n, int64_t l) {
     const int64_t r1 = rounds(chains * (n - 1)), r2 = rounds(chains * n), common = r2 * kOne * l + kPasses + (r1 + r2 - 2) * kRound;
-    return Cost{common + r1 * 2 * kQuiet * (l < kVanish ? l : kVanish), common + r1 * 2 * kQuiet * l + kChaining * (n - 1) * rounds(chains * 16)};
+    const int64_t walks = chains * (n - 1) * 2 <= sms ? 1 : r1 * 2;
+    const int64_t b1 = rounds(chains * (2 * n - 3)), b2 = rounds(chains * (n - 1));
+    const bool slow_end = (chains - 1) * (2 * n - 3) >= (b1 - 1) * sms;      // run 0, with outputs, was in its first pass
+    return Cost{common + r1 * 2 * kQuiet * (l < kVanish ? l : kVanish), common + walks * kQuiet * l + kChaining * (n - 1) * rounds(chains * 16),
+                (slow_end ? (b1 - 1) * 88 + 132 : b1 * 88) * l + b2 * 132 * l + 1100 + (b1 + b2 - 2) * kRound + 165 * (n - 2) * rounds(chains * 16)};
   };
-  int64_t least_lasting = INT64_MAX, best = INT64_MAX;
+  int64_t least_lasting = INT64_MAX, before = whole, best = INT64_MAX;
   int best_n = 1;
   for (int pass = 0; pass < 3; ++pass) {
     for (int64_t n = 3; n <= (most < kMostRuns ? most : kMostRuns); ++n) {
@@ -107,9 +115,10 @@ int plan_runs(int64_t chains, int64_t chunks, int64_t most, int sms, int* len) {
       const Cost c = cost(n, l);
       if (pass == 0) {
         if (c.lasting < least_lasting) least_lasting = c.lasting;
+        if (c.before < before) before = c.before;
         continue;
       }
-      if (c.lasting * 12 > least_lasting * 13 || c.lasting * 100 > whole * 110 || c.vanishing * 100 > whole * 97) continue;
+      if (c.lasting > (before == whole ? least_lasting * 13 / 12 : before > least_lasting ? before : least_lasting) || c.lasting * 100 > whole * 110 || c.vanishing * 100 > whole * 97) continue;
       if (pass == 1) {
         if (c.vanishing < best) best = c.vanishing;
       } else if (c.vanishing * 100 <= best * 105 && c.vanishing <= best + 300) {

@@ -376,7 +376,7 @@ def test_runs_whose_maps_last_or_vanish(lasting, packed, state):
 
 
 @pytest.mark.parametrize("lasting", ["all", "none", "odd"])
-@pytest.mark.parametrize("H,T,beside", [(1, 32 * 100 + 1, True), (4, 32 * 128, True), (12, 32 * 160, False)])
+@pytest.mark.parametrize("H,T,beside", [(1, 32 * 100 + 1, True), (4, 32 * 128, True), (16, 32 * 256, False)])
 def test_maps_and_offsets_beside_one_another_and_in_turn(H, T, beside, lasting):
     """The first pass over runs, with M and N of a run in two CTAs of a cluster where all of them are resident at once, else in turn in one."""
     w = Workload("b", H=H, T=T, state_in="fp32", state_out="fp32", state_std=0.5, seed=T + H, lower_bound=-2.0)
