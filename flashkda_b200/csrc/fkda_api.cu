@@ -392,8 +392,9 @@ int do_scan(const fkda_fwd_params* p, const Layout& L, cudaStream_t stream) {
 // faster since, and the cut lies where it did: the best of seven was the planned one, or next to it, for 96, 110 and 120 chains of 256
 // chunks, 75 x 512, 80 x 128 and 124 x 1024.  Returns the chunks of the first slice, or 0 where what the stage is shortened by is
 // not worth it: the second pair of launches costs about 20 us, and the stage takes its share of the recurrence's bandwidth.
-// Gains measured against one piece, chains x chunks: 75 x 512 15 %, 80 x 128 11 %, 96 x 256 12 %, 110 x 256 10 %, 120 x 256 10 %, 124 x
-// 1024 14 %, 128 x 512 6 %.  Equal lengths only: a packed batch's lengths, which the slices would have to follow, are on the
+// Gains measured against one piece, chains x chunks: 75 x 512 14 %, 80 x 128 10 %, 96 x 256 10 %, 110 x 256 7 %, 120 x 256 5 to 9 %, 126 x
+// 256 5 %, 124 x 1024 2 to 6 %, 128 x 512 -2 to 3 %; beyond the line 130 x 2048, 134 x 2048 and 140 x 2048 1 %, 144 x 1024 and 147 x 2048
+// -1 to -5 %.  Equal lengths only: a packed batch's lengths, which the slices would have to follow, are on the
 // device.  Chains split over CTAs leave too few SMs free beside them (20 at 32 chains, none at 37 or 74).
 constexpr int kSliceWaves = 2;
 int plan_slice(int64_t chains, int64_t chunks, int sms) {

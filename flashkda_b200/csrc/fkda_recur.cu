@@ -352,11 +352,11 @@ __device__ __forceinline__ void spoil_runs(const ScanParams& p, float* slots, vo
     }
 }
 
-// kStream: the CTA is persistent and goes through its walks (whole chains; with kSeg runs of a chain, see fkda_segscan.cu) as
+// kStream: the CTA is persistent and goes through its walks (whole chains) as
 // one stream of chunks, so that records, v and state of the next walk are on their way while the last chunks of this one
 // are computed.  Equal lengths: walks in turn, every other round backwards; packed batches take the next longest
-// sequence from a device counter.  Otherwise one walk per CTA: a chunk costs 8 % less (2470 against 2680 cycles: the loop
-// has no registers to spare and every value kept for the stream is felt), a walk 3 us more.
+// sequence from a device counter.  Otherwise one walk per CTA: a chunk costs 5 to 8 % less (768 chains of 64 chunks 467 against 500
+// us), a walk up to 3 us more.
 // kSlice: one walk per CTA, a time slice of it (ScanParams::slice_*).
 template <bool kSeg, bool kStream, bool kSlice>
 __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constant__ CUtensorMap tm_v, const ScanParams p, const int walks) {
@@ -1079,8 +1079,10 @@ cudaError_t launch_recur(const ScanParams& p, const __nv_bfloat16* v, cudaStream
     if (e != cudaSuccess) return e;
     return launch_clusters_after(maps, static_cast<unsigned>(pair ? 2 * walks : walks), pair ? 2 : 1, recur::kThreads, recur::kSmem, stream, tv, p);
   }
-  // More walks than SMs and short ones on average: one persistent CTA per SM.  (At 24 chunks the 3 us a walk costs more
-  // in a CTA of its own are what the tighter chunk loop saves.)
+  // More walks than SMs and short ones on average: one persistent CTA per SM.  Stage alone, a CTA per walk against this form: 2048 equal
+  // chains of 8 chunks 222 / 206 us, of 10 256 / 243; 768 of 8 99.3 / 98.9, of 12 123 / 126, of 24 196 / 206; 24 ragged sequences x 32
+  // heads of 12 chunks on average 132 / 124, of 20 160 / 156, of 28 214 / 215, of 40 303 / 312.  The line lies where ragged
+  // batches, which gain by the order by length, break even; a few rounds of equal chains of 12 to 24 chunks lose up to a twentieth by it.
   const int64_t sms = device_sm_count();
   const bool stream_form = p.seg_chunks == 0 && walks > sms && (p.T_total + static_cast<int64_t>(p.N) * (kChunk / 2)) / kChunk <= 24 * static_cast<int64_t>(p.N);
   // (a time slice is for fewer walks than SMs; its own form, as what it looks up costs the others 0.8 %)
