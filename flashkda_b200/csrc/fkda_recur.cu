@@ -276,7 +276,7 @@ __device__ __forceinline__ void load_state(float (&S)[2][16][4], const ChainView
 #pragma unroll
       for (int jt = 0; jt < 16; ++jt)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) S[vt][jt][i] = (cv.init_mode == 3 && 8 * jt + 2 * t + (i & 1) == v + 8 * (i >> 1)) ? 1.f : 0.f;
+        for (int i = 0; i < 4; ++i) S[vt][jt][i] = 0.f;
     }
   }
 }
@@ -286,11 +286,11 @@ __device__ __forceinline__ void store_state(const float (&S)[2][16][4], const Ch
   for (int vt = 0; vt < 2; ++vt) {
     const int v = row0 + 16 * vt + g;
     if (cv.fin_fp32) {
-      float* dst = static_cast<float*>(cv.fin_base) + static_cast<size_t>(v) * cv.fin_stride + 2 * t;
+      float* dst = static_cast<float*>(cv.fin_base) + v * kD + 2 * t;
 #pragma unroll
       for (int jt = 0; jt < 16; ++jt) {
         *reinterpret_cast<float2*>(dst + 8 * jt) = make_float2(S[vt][jt][0], S[vt][jt][1]);
-        *reinterpret_cast<float2*>(dst + 8 * cv.fin_stride + 8 * jt) = make_float2(S[vt][jt][2], S[vt][jt][3]);
+        *reinterpret_cast<float2*>(dst + 8 * kD + 8 * jt) = make_float2(S[vt][jt][2], S[vt][jt][3]);
       }
     } else {
       __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(cv.fin_base) + v * kD + 2 * t;
@@ -421,7 +421,6 @@ __global__ void __launch_bounds__(kThreads, 1) recur_kernel(const __grid_constan
         cv.init_mode = wi->init_mode;
         cv.fin_base = wi->fin_base;
         cv.fin_fp32 = wi->fin_fp32;
-        cv.fin_stride = kD;
         cv.bos = 0;
         cv.eos = wi->tokens;
         cv.nchunks = wi->nchunks;
